@@ -249,9 +249,9 @@ def tolerance(case):
     # Measured against restatements in 64 bits: linears, groups and MoE 2e-7 to 3e-7 in fp32, the cache 1e-7; one rounding to
     # bf16 on the way out 1.7e-3; a bf16 block of three linears 3.4e-3 to 4.6e-3.
     if case["kind"] == "stack":
-        # fp32, but cache codes and routed experts are whole numbers: a last-bit difference (1e-6 in the embeddings moves the
-        # logits by 2e-6 to 1.4e-5) tips one of the hundreds of thousands of codes now and then
-        return {"rel": 2e-4}
+        # fp32, but cache codes are whole numbers: last-bit differences (3e-7 in the embeddings) move the logits by 7e-7, and
+        # by 1e-4 to 4e-4 where they tip one of the hundreds of thousands of codes, as one in six such differences does
+        return {"rel": 2e-3}
     if case.get("dtype", "f32") == "bf16":
         return {"rel": 1e-2 if case["kind"] == "mlp" else 7e-3}
     return {"rel": 1.5e-6}
