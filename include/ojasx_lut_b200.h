@@ -306,6 +306,11 @@ OJASX_API int ojasx_b200_kvq_append(OjasxKvqHandle handle, const void* d_k, cons
  * every cached token; scale <= 0 means 1/sqrt(head_dim) (ojasx_lut_kv_cache.cpp:74-76). */
 OJASX_API int ojasx_b200_kvq_decode(OjasxKvqHandle handle, const void* d_q, void* d_out, float scale, int io_dtype,
                                     void* stream);
+/* A chunk of n_positions prompt tokens per sequence: d_k, d_v [n_positions, B, kv_heads, head_dim] are appended and
+ * d_q [n_positions, B, q_heads, head_dim] attends, every position to the tokens up to itself, into d_out (same shape as
+ * d_q).  As n_positions appends and decodes in turn, up to fp32 rounding of the attention.  -2: the cache is too small. */
+OJASX_API int ojasx_b200_kvq_prefill(OjasxKvqHandle handle, const void* d_k, const void* d_v, const void* d_q, void* d_out,
+                                     int n_positions, float scale, int io_dtype, void* stream);
 OJASX_API void ojasx_b200_kvq_destroy(OjasxKvqHandle handle);
 
 /* ---- Per-token operators of a decoder step (no counterpart in the reference, which leaves them to the

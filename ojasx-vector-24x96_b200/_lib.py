@@ -91,6 +91,7 @@ SIGNATURES = {
     "ojasx_b200_kvq_append": (_i, [_vp, _vp, _vp, _i, _vp]),
     "ojasx_b200_kvq_decode": (_i, [_vp, _vp, _vp, _f, _i, _vp]),
     "ojasx_b200_kvq_decode_gather": (_i, [_vp, _vp, _vp, _f, _i, _i, _i, _vp, _vp]),
+    "ojasx_b200_kvq_prefill": (_i, [_vp, _vp, _vp, _vp, _vp, _i, _f, _i, _vp]),
     "ojasx_b200_kvq_destroy": (None, [_vp]),
     "ojasx_b200_kvq_set_static_plan": (_i, [_vp, _i]),
     "ojasx_b200_kvq_sync_len": (_i, [_vp]),

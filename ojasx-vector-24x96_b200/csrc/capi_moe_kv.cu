@@ -65,7 +65,7 @@ MoeProblem MoeHandle::problem(const void* x, void* y, const int* idx, const floa
 KvqHandle::~KvqHandle() {
     DeviceGuard g(dev);
     cudaFree(k_codes); cudaFree(v_codes); cudaFree(k_cb); cudaFree(v_cb); cudaFree(seq_lens); cudaFree(error_flag); cudaFree(counters);
-    cudaFree(partials);
+    cudaFree(partials); cudaFree(pos_partials);
 }
 
 LegacyKvHandle::~LegacyKvHandle() {
@@ -332,6 +332,10 @@ void ojasx_destroy_moe(OjasxMoEHandle handle) {
 }
 
 /* ------------------------------------------------------------------------- codebook-VQ KV */
+// Positions one batched decode launch takes (a chunk of prompt positions too short for the prefill kernel, or of a
+// shape that kernel does not cover).
+static constexpr int kKvqDecodePositions = 16;
+
 OjasxKvqHandle ojasx_b200_kvq_create(int batch, int kv_heads, int q_heads, int head_dim, int block_dim, int max_seq_len,
                                      const float* k_codebook, const float* v_codebook) {
     if (batch <= 0 || kv_heads <= 0 || q_heads <= 0 || q_heads % kv_heads || head_dim <= 0 || block_dim <= 0 ||
@@ -350,7 +354,8 @@ OjasxKvqHandle ojasx_b200_kvq_create(int batch, int kv_heads, int q_heads, int h
     if (rc == OJX_OK) rc = upload((void**)&h->v_cb, v_codebook, cbb);
     if (rc == OJX_OK) rc = upload((void**)&h->seq_lens, nullptr, sizeof(int) * (size_t)batch);
     if (rc == OJX_OK) rc = upload((void**)&h->error_flag, nullptr, sizeof(int));
-    if (rc == OJX_OK) rc = upload((void**)&h->counters, nullptr, sizeof(int) * ((size_t)batch + (size_t)batch * kv_heads));
+    // append: [B]; decode: [B * Hkv], and as many again for every position of a batched decode (kvq_prefill)
+    if (rc == OJX_OK) rc = upload((void**)&h->counters, nullptr, sizeof(int) * ((size_t)batch + (size_t)(1 + kKvqDecodePositions) * batch * kv_heads));
     if (rc != OJX_OK) { delete h; return nullptr; }
     return h;
 }
@@ -455,6 +460,52 @@ static int kvq_decode_impl(OjasxKvqHandle handle, const void* d_q, void* d_out, 
     P.out_heads = out_heads;
     P.out_head0 = out_head0;
     return launch_kvq_decode(P, static_cast<cudaStream_t>(stream), link);
+}
+
+int ojasx_b200_kvq_prefill(OjasxKvqHandle handle, const void* d_k, const void* d_v, const void* d_q, void* d_out, int n_positions,
+                           float scale, int io_dtype, void* stream) {
+    if (!handle || !d_k || !d_v || !d_q || !d_out || n_positions <= 0 || (io_dtype != OJX_F32 && io_dtype != OJX_BF16)) return OJX_ERR_ARG;
+    auto* h = static_cast<KvqHandle*>(handle);
+    if (!h->static_plan && h->host_len + n_positions > h->max_seq) return OJX_ERR_RANGE;
+    cudaStream_t s = static_cast<cudaStream_t>(stream);
+    const size_t esz = io_dtype == OJX_BF16 ? 2 : 4;
+    const size_t kv_pos = esz * h->B * h->Hkv * h->head_dim, q_pos = esz * h->B * h->Hq * h->head_dim;
+    DeviceGuard g(h->dev);
+    KvqProblem P = kvq_problem(h, io_dtype);
+    P.scale = scale > 0.0f ? scale : 1.0f / std::sqrt((float)h->head_dim);
+    P.new_k = d_k; P.new_v = d_v; P.q = d_q; P.out = d_out; P.n_pos = n_positions;
+    // The prefill kernel walks a CTA's whole context for 64 query rows; it pays once its CTAs fill half the GPU or the
+    // context is short.  Few positions on a long context split the context instead: the decode kernel with a position axis.
+    const int R = h->Hq / h->Hkv, cached = h->static_plan ? h->max_seq : h->host_len;
+    const long long ctas = (long long)((n_positions * R + 63) / 64) * h->Hkv * h->B;
+    if (n_positions >= kKvqDecodePositions && kvq_prefill_supported(P) && (2 * ctas >= num_sms() || cached <= 1024)) {
+        int rc = launch_kvq_append_many(P, s);
+        if (rc != OJX_OK) return rc;
+        rc = launch_kvq_prefill_attention(P, s);
+        if (rc == OJX_OK) rc = launch_kvq_advance(P, s);
+        if (rc == OJX_OK && !h->static_plan) h->host_len += n_positions;
+        return rc;
+    }
+    for (int p0 = 0; p0 < n_positions; p0 += kKvqDecodePositions) {
+        P.n_pos = std::min(kKvqDecodePositions, n_positions - p0);
+        P.new_k = static_cast<const char*>(d_k) + p0 * kv_pos;
+        P.new_v = static_cast<const char*>(d_v) + p0 * kv_pos;
+        P.q = static_cast<const char*>(d_q) + p0 * q_pos;
+        P.out = static_cast<char*>(d_out) + p0 * q_pos;
+        const int T = h->static_plan ? h->max_seq : h->host_len + P.n_pos;
+        plan_kvq_decode(P, T, num_sms());
+        // scratch of its own: a captured decode step keeps a pointer to the other one
+        const size_t need = sizeof(float) * (size_t)kKvqDecodePositions * h->B * h->Hkv * kvq_max_splits(h->max_seq) * R * (h->head_dim + 2);
+        int rc = ensure_capacity(&h->pos_partials, &h->pos_partials_cap, need);
+        if (rc != OJX_OK) return rc;
+        P.partials = static_cast<float*>(h->pos_partials);
+        P.split_done = h->counters + h->B + (size_t)h->B * h->Hkv;
+        if ((rc = launch_kvq_append_many(P, s)) != OJX_OK) return rc;
+        if ((rc = launch_kvq_decode(P, s)) != OJX_OK) return rc;
+        if ((rc = launch_kvq_advance(P, s)) != OJX_OK) return rc;
+        if (!h->static_plan) h->host_len += P.n_pos;
+    }
+    return OJX_OK;
 }
 
 int ojasx_b200_kvq_set_static_plan(OjasxKvqHandle handle, int enabled) {

@@ -116,6 +116,8 @@ struct KvqProblem {
     float scale;
     int out_heads;          // query heads of a row of `out` (0: Hq); > Hq when this cache holds a KV-head shard and
     int out_head0;          // writes its heads at [out_head0, out_head0 + Hq) of the gathered output
+    int n_pos;              // > 0: a chunk of prompt positions; q, out [n_pos, B, Hq, head_dim], new_k, new_v [n_pos, B, Hkv, head_dim],
+                            // seq_lens holds the lengths before the chunk and position s sees seq_lens[b] + s + 1 tokens
 };
 
 inline int round_up(int a, int b) { return (a + b - 1) / b * b; }

@@ -96,7 +96,8 @@ __global__ void __launch_bounds__(kKvThreads) kvq_append_kernel(const __grid_con
 }
 
 // ------------------------------------------------------------------------------ kvq decode
-// grid = (splits, Hkv, B); a CTA owns tokens [split*chunk, (split+1)*chunk) of one (sequence, KV head)
+// grid = (splits, Hkv, B), or (splits, Hkv, positions * B) for a chunk of prompt positions whose tokens are
+// cached already; a CTA owns tokens [split*chunk, (split+1)*chunk) of one (position, sequence, KV head)
 // and walks them in passes of kSub tokens with a running maximum (online softmax), so the query table
 // [G,256,R] is built once per CTA however long its range is.
 //
@@ -167,7 +168,7 @@ __device__ __forceinline__ void st_heads(float* p, const float (&o)[R]) {
 // The CTA that arrives last merges the partials of the R query heads: M = max m_c, weights
 // exp(m_c - M), splits in index order -- so a decode is one launch.  The counter returns to zero.
 template <int R>
-__device__ __forceinline__ void kvq_merge_if_last(const KvqProblem& P, int b, int h, const PeerLink& link) {
+__device__ __forceinline__ void kvq_merge_if_last(const KvqProblem& P, int b /* blockIdx.z */, int h, const PeerLink& link) {
     __shared__ int s_last;
     __threadfence();   // this thread's partial is visible device-wide before the CTA is counted
     __syncthreads();
@@ -232,14 +233,14 @@ __global__ void __launch_bounds__(kvq_decode_threads(R, D), 1) kvq_decode_kernel
     uint32_t* vct = reinterpret_cast<uint32_t*>(mfin + R);         // [2][ceil(G/4)][kSub + pad] words of four codes
     const int vrow = kSub + kKvVctPad, Gq = (G + 3) >> 2;
 
-    const int b = blockIdx.z, h = blockIdx.y, split = blockIdx.x;
-    const int T = P.seq_lens[b];
+    const int z = blockIdx.z, b = P.n_pos > 0 ? z % P.B : z, h = blockIdx.y, split = blockIdx.x;
+    const int T = P.n_pos > 0 ? min(P.seq_lens[b] + z / P.B + 1, P.max_seq) : P.seq_lens[b];
     const int t_begin = split * P.chunk;
     const int t_end = min(T, t_begin + P.chunk);
-    float* part = P.partials + ((((size_t)b * P.Hkv + h) * P.n_chunks + split) * R) * (hd + 2);
+    float* part = P.partials + ((((size_t)z * P.Hkv + h) * P.n_chunks + split) * R) * (hd + 2);
     if (t_begin >= t_end) {  // range beyond this sequence: neutral partial
         for (int i = tid; i < R * (hd + 2); i += kThreads) part[i] = (i % (hd + 2)) == 0 ? -INFINITY : 0.0f;
-        kvq_merge_if_last<R>(P, b, h, link);
+        kvq_merge_if_last<R>(P, z, h, link);
         peer_signal_when_last(link, gridDim.x * gridDim.y * gridDim.z);
         return;
     }
@@ -247,7 +248,7 @@ __global__ void __launch_bounds__(kvq_decode_threads(R, D), 1) kvq_decode_kernel
     const uint8_t* kc = P.k_codes + (((size_t)b * P.Hkv + h) * P.max_seq) * G;
     const uint8_t* vc = P.v_codes + (((size_t)b * P.Hkv + h) * P.max_seq) * G;
 
-    for (int i = tid; i < R * hd; i += kThreads) qs[i] = load_io(P.q, ((size_t)b * P.Hq + (size_t)h * R) * hd + i, P.io_dtype);
+    for (int i = tid; i < R * hd; i += kThreads) qs[i] = load_io(P.q, ((size_t)z * P.Hq + (size_t)h * R) * hd + i, P.io_dtype);
     for (int i0 = tid; i0 < 256 * kPieces * vrep; i0 += 4 * kThreads) {   // consecutive threads, consecutive 16-byte slots
         float4 val[4];
 #pragma unroll
@@ -596,7 +597,7 @@ __global__ void __launch_bounds__(kvq_decode_threads(R, D), 1) kvq_decode_kernel
             part[(size_t)r * (hd + 2) + 1] = l;
         }
     }
-    kvq_merge_if_last<R>(P, b, h, link);
+    kvq_merge_if_last<R>(P, z, h, link);
     peer_signal_when_last(link, gridDim.x * gridDim.y * gridDim.z);
 }
 
@@ -616,7 +617,7 @@ size_t kvq_decode_smem(const KvqProblem& P, int R) { return kvq_decode_smem_copi
 // the least (waves of CTAs, one per SM) x (range + the table set-up and the fill and drain of the
 // score/value pipeline, together worth about 1000 tokens) wins.
 void plan_kvq_decode(KvqProblem& P, int T, int sms) {
-    const int heads = P.B * P.Hkv, slots = sms;
+    const int heads = (P.n_pos > 0 ? P.n_pos : 1) * P.B * P.Hkv, slots = sms;
     const int max_s = std::min(kKvMaxSplits, (T + 255) / 256);
     long best = -1;
     P.chunk = round_up(std::max(T, 1), 64);
@@ -667,7 +668,7 @@ static int launch_decode_t(const KvqProblem& P, cudaStream_t s, const PeerLink& 
         OJX_CUDA_TRY(cudaFuncSetAttribute(kvq_decode_kernel<R, D>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
         if (cur_dev >= 0 && cur_dev < 64) configured[cur_dev] = smem;
     }
-    kvq_decode_kernel<R, D><<<dim3(P.n_chunks, P.Hkv, P.B), kvq_decode_threads(R, D), smem, s>>>(Q, link);
+    kvq_decode_kernel<R, D><<<dim3(P.n_chunks, P.Hkv, P.n_pos > 0 ? P.n_pos * P.B : P.B), kvq_decode_threads(R, D), smem, s>>>(Q, link);
     OJX_CUDA_TRY(cudaGetLastError());
     count_launch(1);
     return OJX_OK;

@@ -1,0 +1,439 @@
+// Codebook-VQ KV cache, a chunk of prompt positions at once: every position's key and value are
+// encoded by one launch and every position attends to the tokens up to itself by another.  The
+// reference handles a prompt in one model call (ojasx_24x96/engine.py:153-175); its attention over
+// a cache is the online softmax of ojasx_24x96/long_context.py:92-176.
+//
+// Appending and decoding position by position cost two launches per position and layer: a chunk
+// of 512 positions took 512 x (14.7 + 5.6) us plus the gaps between launches, 13 ms per layer.
+#include <cuda_fp16.h>
+
+#include <algorithm>
+
+#include "common.cuh"
+#include "handles.h"
+#include "launch.h"
+
+namespace ojx {
+
+__device__ __forceinline__ float pf_load(const void* p, size_t i, int dtype) {
+    return dtype == OJX_BF16 ? __bfloat162float(reinterpret_cast<const __nv_bfloat16*>(p)[i])
+                             : reinterpret_cast<const float*>(p)[i];
+}
+
+// ------------------------------------------------------------------------------------ append
+// grid = (2 * Hkv * G, ceil(positions * B / 128)).  A block encodes one (k|v, head, group) of 128
+// rows: thread = row, the 256 centroids and their squared norms broadcast from shared memory.  Same
+// distance and the same first-minimum rule as kvq_append_kernel (every dot product a sequential fp32
+// sum of rounded products), so the codes are equal.  Bound: fp32 issue, 256 x 19 instructions per
+// row and task; a warp per row and task (the one-token kernel) spends as much again on its reduction
+// and reads the centroids once per row.
+constexpr int kPfAppendThreads = 128;
+
+template <int D>
+__global__ void __launch_bounds__(kPfAppendThreads) kvq_append_many_kernel(const __grid_constant__ KvqProblem P) {
+    __shared__ __align__(16) float cb_s[256 * D];
+    __shared__ float cc_s[256];
+    const int G = P.G, task = blockIdx.x;
+    const int which = task / (P.Hkv * G), rem = task - which * P.Hkv * G;
+    const int h = rem / G, g = rem - h * G;
+    const float* cb = (which ? P.v_cb : P.k_cb) + (size_t)h * P.Kcb * D;
+    for (int i = threadIdx.x; i < P.Kcb * D; i += kPfAppendThreads) cb_s[i] = cb[i];
+    __syncthreads();
+    for (int c = threadIdx.x; c < P.Kcb; c += kPfAppendThreads) {
+        float cc = 0.0f;
+#pragma unroll
+        for (int d = 0; d < D; ++d) cc = __fadd_rn(cc, __fmul_rn(cb_s[c * D + d], cb_s[c * D + d]));
+        cc_s[c] = cc;
+    }
+    __syncthreads();
+    const int row = blockIdx.y * kPfAppendThreads + threadIdx.x;
+    if (row >= P.n_pos * P.B) return;
+    const int s = row / P.B, b = row - s * P.B;
+    const int T = P.seq_lens[b] + s;
+    if (T >= P.max_seq) {   // cache full: the token is dropped, the error flag reports it
+        if (task == 0) atomicExch(P.error_flag, 1);
+        return;
+    }
+    const void* src = which ? P.new_v : P.new_k;
+    const size_t base = ((size_t)row * P.Hkv + h) * P.head_dim + (size_t)g * D;
+    float v[D];
+    float vv = 0.0f;
+#pragma unroll
+    for (int d = 0; d < D; ++d) {
+        v[d] = pf_load(src, base + d, P.io_dtype);
+        vv = __fadd_rn(vv, __fmul_rn(v[d], v[d]));
+    }
+    float bd = INFINITY;
+    int bi = 0;
+#pragma unroll 4
+    for (int c = 0; c < P.Kcb; ++c) {
+        const float4* cv = reinterpret_cast<const float4*>(cb_s + c * D);
+        float vc = 0.0f;
+#pragma unroll
+        for (int q = 0; q < D / 4; ++q) {
+            const float4 f = cv[q];
+            vc = __fadd_rn(vc, __fmul_rn(v[4 * q], f.x));
+            vc = __fadd_rn(vc, __fmul_rn(v[4 * q + 1], f.y));
+            vc = __fadd_rn(vc, __fmul_rn(v[4 * q + 2], f.z));
+            vc = __fadd_rn(vc, __fmul_rn(v[4 * q + 3], f.w));
+        }
+        const float dist = __fadd_rn(__fsub_rn(vv, __fmul_rn(2.0f, vc)), cc_s[c]);
+        if (dist < bd) { bd = dist; bi = c; }
+    }
+    uint8_t* codes = which ? P.v_codes : P.k_codes;
+    codes[(((size_t)b * P.Hkv + h) * P.max_seq + T) * G + g] = (uint8_t)bi;
+}
+
+// The sequences' lengths after the chunk (the kernels above and below read the lengths before it).
+__global__ void kvq_advance_kernel(int* seq_lens, int B, int n, int max_seq) {
+    const int b = blockIdx.x * blockDim.x + threadIdx.x;
+    if (b < B) seq_lens[b] = min(seq_lens[b] + n, max_seq);
+}
+
+// --------------------------------------------------------------------------------- attention
+// grid = (tiles of 64 query rows, Hkv, B); a query row is one (position, query head of the KV head).
+// Per tile of 64 tokens the codes are expanded into shared memory once and serve all 64 rows; scores
+// and values are mma.sync products with an online softmax between them, causal per row.
+//
+// fp32 accuracy from fp16 products: every operand is scaled by a power of two (per query row, per
+// codebook, 2^14 for probabilities) so that its largest element is in [2^13, 2^15), and split
+// into x = hi + lo with two fp16 numbers: 22 bits of mantissa down to 2^-24 of the largest element.
+// hi*hi + hi*lo + lo*hi are accumulated in fp32 (the dropped lo*lo is below 2^-22 of hi*hi).
+//
+// Why mma.sync: three products of at most a few GFLOP per chunk and layer are a few microseconds
+// at any tensor rate; what the kernel needs is probabilities that go from the accumulators of the
+// first product to the operand registers of the second.  Two CTAs per SM (88 KB each) hide one
+// another's expansion of the codes.
+constexpr int kPfThreads = 128, kPfRows = 64, kPfTok = 64;
+
+__device__ __forceinline__ void pf_ldsm4(uint32_t addr, uint32_t (&r)[4]) {
+    asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0, %1, %2, %3}, [%4];"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
+                 : "r"(addr));
+}
+__device__ __forceinline__ void pf_ldsm4t(uint32_t addr, uint32_t (&r)[4]) {
+    asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0, %1, %2, %3}, [%4];"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
+                 : "r"(addr));
+}
+__device__ __forceinline__ void pf_mma(float (&c)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
+    asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
+                 : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
+                 : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
+}
+// (a, b) as packed fp16 high parts and the packed fp16 remainders
+__device__ __forceinline__ void pf_split2(float a, float b, uint32_t& hi, uint32_t& lo) {
+    const __half ha = __float2half_rn(a), hb = __float2half_rn(b);
+    const __half la = __float2half_rn(a - __half2float(ha)), lb = __float2half_rn(b - __half2float(hb));
+    const __half2 H = __halves2half2(ha, hb), L = __halves2half2(la, lb);
+    hi = *reinterpret_cast<const uint32_t*>(&H);
+    lo = *reinterpret_cast<const uint32_t*>(&L);
+}
+// power of two that brings a largest magnitude `m` into [2^14, 2^15) (1 for zeros; tiny values stop at 2^100)
+__device__ __forceinline__ float pf_scale(float m) {
+    if (!(m > 0.0f) || m > 3e38f) return 1.0f;
+    int e;
+    frexpf(m, &e);   // m in [2^(e-1), 2^e)
+    return ldexpf(1.0f, min(15 - e, 100));
+}
+
+template <int HD, int D>
+__global__ void __launch_bounds__(kPfThreads) kvq_prefill_kernel(const __grid_constant__ KvqProblem P) {
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    constexpr int LD = HD + 8;                                   // halfs per row: 16 bytes of padding, conflict-free ldmatrix
+    constexpr int G = HD / D, KT = HD / 16;
+    __half* Kh = reinterpret_cast<__half*>(smem_raw);            // [64][LD]
+    __half* Kl = Kh + kPfTok * LD;
+    __half* Vh = Kl + kPfTok * LD;
+    __half* Vl = Vh + kPfTok * LD;
+    __half* cbs = Vl + kPfTok * LD;                              // k hi, k lo, v hi, v lo: [256 * D] each
+    __shared__ float red[2][kPfThreads / 32];
+    __shared__ float row_scale[kPfRows];
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, tq = lane & 3;
+    const int b = blockIdx.z, h = blockIdx.y, R = P.Hq / P.Hkv;
+    const int tile = gridDim.x - 1 - blockIdx.x;                 // the longest contexts start first
+    const int T0 = P.seq_lens[b];
+    const int pos_per = kPfRows / R, s0 = tile * pos_per;
+    const int t_all = min(T0 + min(P.n_pos, s0 + pos_per), P.max_seq);   // tokens the tile's last row sees
+
+    // codebooks of the head, scaled and split
+    float inv_kv[2];
+    {
+        float m[2] = {0.0f, 0.0f};
+        const float* src[2] = {P.k_cb + (size_t)h * P.Kcb * D, P.v_cb + (size_t)h * P.Kcb * D};
+#pragma unroll
+        for (int w = 0; w < 2; ++w)
+            for (int i = tid; i < P.Kcb * D; i += kPfThreads) m[w] = fmaxf(m[w], fabsf(src[w][i]));
+#pragma unroll
+        for (int w = 0; w < 2; ++w) {
+#pragma unroll
+            for (int off = 16; off >= 1; off >>= 1) m[w] = fmaxf(m[w], __shfl_xor_sync(0xffffffffu, m[w], off));
+            if (lane == 0) red[w][warp] = m[w];
+        }
+        __syncthreads();
+#pragma unroll
+        for (int w = 0; w < 2; ++w) {
+            const float sc = pf_scale(fmaxf(fmaxf(red[w][0], red[w][1]), fmaxf(red[w][2], red[w][3])));
+            inv_kv[w] = 1.0f / sc;
+            for (int i = tid; i < 256 * D; i += kPfThreads) {
+                const float x = i < P.Kcb * D ? src[w][i] * sc : 0.0f;
+                const __half hi = __float2half_rn(x);
+                cbs[(2 * w) * 256 * D + i] = hi;
+                cbs[(2 * w + 1) * 256 * D + i] = __float2half_rn(x - __half2float(hi));
+            }
+        }
+    }
+    // query rows: fp32 into the (still unused) K and V tiles, then into registers
+    {
+        float* qs = reinterpret_cast<float*>(smem_raw);          // [64][HD + 4]
+        for (int i = tid; i < kPfRows * HD; i += kPfThreads) {
+            const int row = i / HD, c = i - row * HD, s = s0 + row / R;
+            float v = 0.0f;
+            if (s < P.n_pos) v = pf_load(P.q, (((size_t)s * P.B + b) * P.Hq + (size_t)h * R + row % R) * HD + c, P.io_dtype);
+            qs[row * (HD + 4) + c] = v;
+        }
+        __syncthreads();
+        if (tid < kPfRows) {
+            float m = 0.0f;
+            for (int c = 0; c < HD; ++c) m = fmaxf(m, fabsf(qs[tid * (HD + 4) + c]));
+            row_scale[tid] = pf_scale(m);
+        }
+        __syncthreads();
+    }
+    uint32_t qh[KT][4], ql[KT][4];
+    float descale[2];
+    int limit[2];                                                // last token a row may see
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+        const int row = warp * 16 + g + 8 * i;
+        const float* q = reinterpret_cast<const float*>(smem_raw) + row * (HD + 4);
+        const float sc = row_scale[row];
+        descale[i] = P.scale * (1.0f / sc) * inv_kv[0] * 1.4426950408889634f;   // scores in units of log 2
+        limit[i] = min(T0 + min(s0 + row / R, P.n_pos - 1), P.max_seq - 1);
+#pragma unroll
+        for (int kk = 0; kk < KT; ++kk)
+#pragma unroll
+            for (int j = 0; j < 2; ++j) {
+                const float2 v = *reinterpret_cast<const float2*>(q + kk * 16 + j * 8 + 2 * tq);
+                pf_split2(v.x * sc, v.y * sc, qh[kk][2 * j + i], ql[kk][2 * j + i]);
+            }
+    }
+    __syncthreads();
+
+    float o[HD / 8][4], m_run[2] = {-INFINITY, -INFINITY}, l_run[2] = {0.0f, 0.0f};
+#pragma unroll
+    for (int n = 0; n < HD / 8; ++n)
+#pragma unroll
+        for (int i = 0; i < 4; ++i) o[n][i] = 0.0f;
+
+    const uint8_t* kc = P.k_codes + (((size_t)b * P.Hkv + h) * P.max_seq) * G;
+    const uint8_t* vc = P.v_codes + (((size_t)b * P.Hkv + h) * P.max_seq) * G;
+    // words of four codes (G is a multiple of 4): the next tile's are fetched while this one is computed
+    constexpr int W = kPfTok * G / 4, WPT = (W + kPfThreads - 1) / kPfThreads;
+    uint32_t kw[WPT], vw[WPT];
+    auto fetch = [&](int t0) {
+#pragma unroll
+        for (int u = 0; u < WPT; ++u) {
+            const int i = tid + u * kPfThreads, t = t0 + i / (G / 4);
+            kw[u] = vw[u] = 0u;
+            if (i < W && t < t_all) {
+                kw[u] = *reinterpret_cast<const uint32_t*>(kc + (size_t)t * G + (i % (G / 4)) * 4);
+                vw[u] = *reinterpret_cast<const uint32_t*>(vc + (size_t)t * G + (i % (G / 4)) * 4);
+            }
+        }
+    };
+    auto expand = [&](uint32_t word, const __half* cb, __half* dst) {   // four centroids, D halfs each
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+            const __half* c = cb + ((word >> (8 * q)) & 255u) * D;
+            if constexpr (D == 4) *reinterpret_cast<uint2*>(dst + q * D) = *reinterpret_cast<const uint2*>(c);
+            else {
+#pragma unroll
+                for (int e = 0; e < D / 8; ++e) reinterpret_cast<uint4*>(dst + q * D)[e] = reinterpret_cast<const uint4*>(c)[e];
+            }
+        }
+    };
+    const uint32_t kh_a = static_cast<uint32_t>(__cvta_generic_to_shared(Kh)) + (((lane >> 4) * 8 + (lane & 7)) * LD + ((lane >> 3) & 1) * 8) * 2;
+    const uint32_t vh_a = static_cast<uint32_t>(__cvta_generic_to_shared(Vh)) + ((((lane >> 3) & 1) * 8 + (lane & 7)) * LD + (lane >> 4) * 8) * 2;
+    constexpr uint32_t kPart = kPfTok * LD * 2;                  // bytes from a tile's hi part to its lo part
+
+    fetch(0);
+    for (int t0 = 0; t0 < t_all; t0 += kPfTok) {
+#pragma unroll
+        for (int u = 0; u < WPT; ++u) {
+            const int i = tid + u * kPfThreads;
+            if (i < W) {
+                const int off = (i / (G / 4)) * LD + (i % (G / 4)) * 4 * D;
+                expand(kw[u], cbs, Kh + off);
+                expand(kw[u], cbs + 256 * D, Kl + off);
+                expand(vw[u], cbs + 2 * 256 * D, Vh + off);
+                expand(vw[u], cbs + 3 * 256 * D, Vl + off);
+            }
+        }
+        __syncthreads();
+        if (t0 + kPfTok < t_all) fetch(t0 + kPfTok);
+
+        float s[kPfTok / 8][4];
+#pragma unroll
+        for (int n = 0; n < kPfTok / 8; ++n)
+#pragma unroll
+            for (int i = 0; i < 4; ++i) s[n][i] = 0.0f;
+#pragma unroll
+        for (int kk = 0; kk < KT; ++kk)
+#pragma unroll
+            for (int n2 = 0; n2 < kPfTok / 16; ++n2) {
+                uint32_t bh[4], bl[4];
+                const uint32_t a = kh_a + (n2 * 16 * LD + kk * 16) * 2;
+                pf_ldsm4(a, bh);
+                pf_ldsm4(a + kPart, bl);
+#pragma unroll
+                for (int j = 0; j < 2; ++j) {
+                    pf_mma(s[2 * n2 + j], qh[kk], bl[2 * j], bl[2 * j + 1]);
+                    pf_mma(s[2 * n2 + j], ql[kk], bh[2 * j], bh[2 * j + 1]);
+                    pf_mma(s[2 * n2 + j], qh[kk], bh[2 * j], bh[2 * j + 1]);
+                }
+            }
+        // scale, mask, online softmax (rows g and g + 8 of the warp's sixteen; a row lives in four lanes)
+        float mt[2] = {-INFINITY, -INFINITY};
+#pragma unroll
+        for (int n = 0; n < kPfTok / 8; ++n)
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                const int t = t0 + n * 8 + 2 * tq + (i & 1);
+                s[n][i] = t <= limit[i >> 1] ? s[n][i] * descale[i >> 1] : -INFINITY;
+                mt[i >> 1] = fmaxf(mt[i >> 1], s[n][i]);
+            }
+        float base[2];
+#pragma unroll
+        for (int i = 0; i < 2; ++i) {
+            mt[i] = fmaxf(mt[i], __shfl_xor_sync(0xffffffffu, mt[i], 1));
+            mt[i] = fmaxf(mt[i], __shfl_xor_sync(0xffffffffu, mt[i], 2));
+            const float m = fmaxf(m_run[i], mt[i]);              // finite from the first tile on: every row sees token 0
+            const float alpha = exp2f(m_run[i] - m);
+            m_run[i] = m;
+            base[i] = m;
+            l_run[i] *= alpha;
+#pragma unroll
+            for (int n = 0; n < HD / 8; ++n) {
+                o[n][2 * i] *= alpha;
+                o[n][2 * i + 1] *= alpha;
+            }
+        }
+#pragma unroll
+        for (int n = 0; n < kPfTok / 8; ++n)
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                s[n][i] = exp2f(s[n][i] - base[i >> 1]);
+                l_run[i >> 1] += s[n][i];
+            }
+#pragma unroll
+        for (int j = 0; j < kPfTok / 16; ++j) {
+            uint32_t ph[4], pl[4];
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                const float* c = s[2 * j + (i >> 1)] + (i & 1) * 2;
+                pf_split2(c[0] * 16384.0f, c[1] * 16384.0f, ph[i], pl[i]);
+            }
+#pragma unroll
+            for (int n2 = 0; n2 < HD / 16; ++n2) {
+                uint32_t bh[4], bl[4];
+                const uint32_t a = vh_a + (j * 16 * LD + n2 * 16) * 2;
+                pf_ldsm4t(a, bh);
+                pf_ldsm4t(a + kPart, bl);
+#pragma unroll
+                for (int q = 0; q < 2; ++q) {
+                    pf_mma(o[2 * n2 + q], ph, bl[2 * q], bl[2 * q + 1]);
+                    pf_mma(o[2 * n2 + q], pl, bh[2 * q], bh[2 * q + 1]);
+                    pf_mma(o[2 * n2 + q], ph, bh[2 * q], bh[2 * q + 1]);
+                }
+            }
+        }
+        __syncthreads();   // the tile has been read
+    }
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+        l_run[i] += __shfl_xor_sync(0xffffffffu, l_run[i], 1);
+        l_run[i] += __shfl_xor_sync(0xffffffffu, l_run[i], 2);
+        const int row = warp * 16 + g + 8 * i, s = s0 + row / R;
+        if (s >= P.n_pos) continue;
+        const float inv = inv_kv[1] * (1.0f / 16384.0f) / l_run[i];
+        const size_t base = (((size_t)s * P.B + b) * P.Hq + (size_t)h * R + row % R) * HD;
+#pragma unroll
+        for (int n = 0; n < HD / 8; ++n)
+#pragma unroll
+            for (int e = 0; e < 2; ++e) {
+                const float v = o[n][2 * i + e] * inv;
+                const size_t at = base + n * 8 + 2 * tq + e;
+                if (P.io_dtype == OJX_BF16) reinterpret_cast<__nv_bfloat16*>(P.out)[at] = __float2bfloat16_rn(v);
+                else reinterpret_cast<float*>(P.out)[at] = v;
+            }
+    }
+}
+
+// ------------------------------------------------------------------------------------- host side
+template <int HD, int D>
+static int launch_prefill_t(const KvqProblem& P, cudaStream_t s) {
+    constexpr size_t smem = sizeof(__half) * (4 * (size_t)kPfTok * (HD + 8) + 4 * 256 * (size_t)D);
+    static_assert(sizeof(float) * kPfRows * (HD + 4) <= smem, "query rows are staged in the tiles");
+    OJX_CUDA_TRY(cudaFuncSetAttribute(kvq_prefill_kernel<HD, D>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    const int R = P.Hq / P.Hkv, pos_per = kPfRows / R;
+    kvq_prefill_kernel<HD, D><<<dim3((P.n_pos + pos_per - 1) / pos_per, P.Hkv, P.B), kPfThreads, smem, s>>>(P);
+    OJX_CUDA_TRY(cudaGetLastError());
+    count_launch(1);
+    return OJX_OK;
+}
+
+template <int HD>
+static int launch_prefill_d(const KvqProblem& P, cudaStream_t s) {
+    switch (P.D) {
+        case 4: return launch_prefill_t<HD, 4>(P, s);
+        case 8: return launch_prefill_t<HD, 8>(P, s);
+        case 16: return launch_prefill_t<HD, 16>(P, s);
+        default: return OJX_ERR_UNSUPPORTED;
+    }
+}
+
+bool kvq_prefill_supported(const KvqProblem& P) {
+    const int R = P.Hq / P.Hkv;
+    return R <= kPfRows && kPfRows % R == 0 && P.G % 4 == 0 && P.B <= 65535 && P.Hkv <= 65535 &&
+           (P.head_dim == 64 || P.head_dim == 128) && (P.D == 4 || P.D == 8 || P.D == 16);
+}
+
+int launch_kvq_prefill_attention(const KvqProblem& P, cudaStream_t s) {
+    if (!kvq_prefill_supported(P)) return OJX_ERR_UNSUPPORTED;
+    switch (P.head_dim) {
+        case 64: return launch_prefill_d<64>(P, s);
+        case 128: return launch_prefill_d<128>(P, s);
+        default: return OJX_ERR_UNSUPPORTED;
+    }
+}
+
+template <int D>
+static int launch_append_many_t(const KvqProblem& P, cudaStream_t s) {
+    const long long rows = (long long)P.n_pos * P.B;
+    const long long blocks = (rows + kPfAppendThreads - 1) / kPfAppendThreads;
+    if (blocks > 65535) return OJX_ERR_TOO_LARGE;
+    kvq_append_many_kernel<D><<<dim3(2 * P.Hkv * P.G, (unsigned)blocks), kPfAppendThreads, 0, s>>>(P);
+    OJX_CUDA_TRY(cudaGetLastError());
+    count_launch(1);
+    return OJX_OK;
+}
+
+int launch_kvq_append_many(const KvqProblem& P, cudaStream_t s) {
+    if (!P.new_k || !P.new_v || P.n_pos <= 0) return OJX_ERR_ARG;
+    switch (P.D) {
+        case 4: return launch_append_many_t<4>(P, s);
+        case 8: return launch_append_many_t<8>(P, s);
+        case 16: return launch_append_many_t<16>(P, s);
+        default: return OJX_ERR_UNSUPPORTED;
+    }
+}
+
+int launch_kvq_advance(const KvqProblem& P, cudaStream_t s) {
+    kvq_advance_kernel<<<(P.B + 127) / 128, 128, 0, s>>>(P.seq_lens, P.B, P.n_pos, P.max_seq);
+    OJX_CUDA_TRY(cudaGetLastError());
+    count_launch(1);
+    return OJX_OK;
+}
+
+}  // namespace ojx

@@ -77,6 +77,11 @@ size_t kvq_decode_smem(const KvqProblem& P, int R);
 void plan_kvq_decode(KvqProblem& P, int T, int sms);
 int launch_kvq_append(const KvqProblem& P, cudaStream_t stream);
 int launch_kvq_decode(const KvqProblem& P, cudaStream_t stream, const PeerLink* link = nullptr);
+// --- kv_prefill.cu: a chunk of P.n_pos prompt positions (lengths are advanced last)
+int launch_kvq_append_many(const KvqProblem& P, cudaStream_t stream);
+bool kvq_prefill_supported(const KvqProblem& P);
+int launch_kvq_prefill_attention(const KvqProblem& P, cudaStream_t stream);
+int launch_kvq_advance(const KvqProblem& P, cudaStream_t stream);
 int launch_legacy_append(const float* k, const float* v, int head_dim, int block_dim, uint8_t* k_row, uint8_t* v_row,
                          float* k_scale, float* v_scale, cudaStream_t stream);
 int launch_legacy_attention(const float* q, int head_dim, int block_dim, int T, const uint8_t* k_codes,

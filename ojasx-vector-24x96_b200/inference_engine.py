@@ -169,6 +169,7 @@ class VQDecoderStack:
         self.pos = torch.zeros(batch, dtype=torch.int32, device=self.device)
         self.position = 0
         self._graph = None
+        self._moe_rows = batch       # tokens the MoE scratch of the layers is reserved for
         self._ids = torch.zeros(batch, dtype=torch.int64, device=self.device)
         self._logits = None
         if use_graph:
@@ -305,12 +306,13 @@ class VQDecoderStack:
         """The prompt ``[batch, S]`` into the caches; returns the logits after its last token (one model call over the
         prompt, ``ojasx_24x96/engine.py:153-175``).
 
-        ``batched`` (default on one device): all positions of a chunk of the prompt go through the linears and the MoE
-        as ONE batch -- the regime of the batched kernels: persistent table kernel in fp32, tensor-core dequant GEMM
-        for bf16 -- while attention, whose quantised cache grows a token at a time, appends and decodes position by
-        position.  Results are those of the token-by-token form (every kernel keeps its summation order whatever the
-        batch).  ``max_rows`` bounds batch * positions per chunk (scratch of the MoE grows with it).  Otherwise, and on
-        a stack split over several ranks, the prompt is fed through ``decode_step`` token by token."""
+        ``batched`` (default on one device): all positions of a chunk of the prompt go through the linears, the MoE and
+        the attention as ONE batch -- the regime of the batched kernels: persistent table kernel in fp32, tensor-core
+        dequant GEMM for bf16, causal attention over the chunk (``VQKVCache.prefill``).  Results are those of the
+        token-by-token form: bit for bit through linears and MoE, whose kernels keep their summation order whatever the
+        batch, and in fp32 rounding through the attention of chunks of 16 positions or more.  ``max_rows`` bounds
+        batch * positions per chunk (scratch of the MoE grows with it).  Otherwise, and on a stack split over several
+        ranks, the prompt is fed through ``decode_step`` token by token."""
         if batched is None:
             batched = self.segment is None
         if not batched or self.segment is not None:
@@ -334,6 +336,8 @@ class VQDecoderStack:
         cfg, B = self.cfg, self.batch
         Sc = ids.shape[1]
         rows = B * Sc
+        if rows > self._moe_rows:    # the MoE scratch grows: a captured step would keep pointers to the old one
+            self._moe_rows, self._graph = rows, None
         h = self.embed[ids.t().reshape(-1)].to(self.dtype)
         pos_rows = (self.pos.view(1, B) + torch.arange(Sc, device=self.device, dtype=torch.int32).view(Sc, 1)).reshape(-1).contiguous()
         pending = None
@@ -345,10 +349,7 @@ class VQDecoderStack:
             v = l.v(a).view(rows, cfg.kv_heads, cfg.head_dim)
             rope_qk_(q, k, pos_rows, cfg.rope_theta)
             q4, k4, v4 = (t.view(Sc, B, t.shape[1], cfg.head_dim) for t in (q, k, v))
-            att = torch.empty_like(q4)
-            for s in range(Sc):
-                l.cache.append(k4[s], v4[s])
-                l.cache.decode(q4[s], out=att[s])
+            att = l.cache.prefill(k4, v4, q4)
             o = l.o(att.view(rows, cfg.q_heads * cfg.head_dim))
             m = rmsnorm(h, l.norm2, cfg.rms_eps, add=o)
             pending = l.moe.forward_routed(m, cfg.top_k)

@@ -385,6 +385,20 @@ class VQKVCache:
                                           _stream_ptr(q.device)), "ojasx_b200_kvq_decode")
         return o
 
+    def prefill(self, k: torch.Tensor, v: torch.Tensor, q: torch.Tensor, scale: float = -1.0,
+                out: Optional[torch.Tensor] = None) -> torch.Tensor:
+        """A chunk of prompt positions: ``k``, ``v`` [S, batch, kv_heads, head_dim] are appended and every position of
+        ``q`` [S, batch, q_heads, head_dim] attends to the tokens up to itself."""
+        _require_cuda(q, "q")
+        k2, v2, q2 = k.contiguous(), v.contiguous(), q.contiguous()
+        S = q2.shape[0]
+        assert k2.shape == (S, self.batch, self.kv_heads, self.head_dim) and v2.shape == k2.shape
+        assert q2.shape == (S, self.batch, self.q_heads, self.head_dim) and q2.dtype == k2.dtype == v2.dtype
+        o = torch.empty_like(q2) if out is None else out
+        check(lib().ojasx_b200_kvq_prefill(self._h, k2.data_ptr(), v2.data_ptr(), q2.data_ptr(), o.data_ptr(), S, scale,
+                                           _dtype_code(q2), _stream_ptr(q.device)), "ojasx_b200_kvq_prefill")
+        return o
+
     def close(self):
         if getattr(self, "_h", None):
             lib().ojasx_b200_kvq_destroy(self._h)

@@ -1,0 +1,69 @@
+"""A chunk of prompt positions through the quantised cache against the CPU oracle and against the token-by-token form."""
+import numpy as np
+import pytest
+import torch
+
+from ojasx_b200 import OjasxB200Error, ops
+
+pytestmark = pytest.mark.gpu
+
+
+def _make(seed, B, Hkv, Hq, hd, D, T0, S):
+    rng = np.random.default_rng(seed)
+    sig = 1.0 / np.sqrt(hd)
+    books = [(rng.standard_normal((Hkv, 256, D)) * sig).astype(np.float32) for _ in range(2)]
+    old = [rng.integers(0, 256, (B, Hkv, T0, hd // D), dtype=np.uint8) for _ in range(2)]
+    k, v = ((rng.standard_normal((S, B, Hkv, hd)) * sig).astype(np.float32) for _ in range(2))
+    q = (3.0 * rng.standard_normal((S, B, Hq, hd))).astype(np.float32)
+    return books, old, k, v, q
+
+
+@pytest.mark.parametrize("B,Hkv,Hq,hd,D,T0,S", [
+    (1, 8, 32, 128, 8, 0, 77),       # ragged last tile of rows and of tokens, empty cache
+    (2, 8, 32, 128, 8, 130, 33),     # a cached context, two sequences
+    (1, 2, 2, 64, 4, 63, 65),        # one query head per KV head: 64 positions per tile; tile edges of the context
+    (3, 2, 16, 128, 16, 5, 20),      # eight query heads per KV head
+    (1, 8, 32, 128, 8, 3000, 9),     # few positions on a longer context: decode kernel with a position axis
+    (1, 2, 8, 96, 8, 11, 21),        # head_dim 96: not covered by the prefill kernel, two batched decodes
+])
+def test_prefill_chunk(cuda, oracle, B, Hkv, Hq, hd, D, T0, S):
+    books, old, k, v, q = _make(T0 + S, B, Hkv, Hq, hd, D, T0, S)
+    many, one = (ops.VQKVCache(B, Hkv, Hq, hd, D, T0 + S + 3, *books) for _ in range(2))
+    for c in (many, one):
+        if T0:
+            c.load(*old)
+    kt, vt, qt = (torch.from_numpy(a).to(cuda) for a in (k, v, q))
+    got = many.prefill(kt, vt, qt).cpu().numpy()
+    want = np.stack([(one.append(kt[s], vt[s]), one.decode(qt[s]))[1].cpu().numpy() for s in range(S)])
+    assert many.seq_len == one.seq_len == many.sync_len() == T0 + S
+    a, b = many.read(0, T0 + S), one.read(0, T0 + S)
+    assert np.array_equal(a[0], b[0]) and np.array_equal(a[1], b[1])     # codes: index-exact
+    # fp32 sums in another order, over scores of magnitude ~10: the bounds of the decode tests
+    assert np.allclose(got, want, rtol=1e-4, atol=2e-6), np.abs(got - want).max()
+    R = Hq // Hkv
+    for s, bb, h in [(0, 0, 0), (S // 2, B - 1, Hkv - 1), (S - 1, 0, Hkv - 1)]:
+        ref = oracle.kvq_decode(q[s, bb, h * R:(h + 1) * R], a[0][bb, h, :T0 + s + 1], a[1][bb, h, :T0 + s + 1],
+                                books[0][h], books[1][h], block_dim=D)
+        assert np.allclose(got[s, bb, h * R:(h + 1) * R], ref, rtol=1e-4, atol=2e-6), (s, bb, h)
+    many.crop(T0)
+    bf = many.prefill(kt.bfloat16(), vt.bfloat16(), qt.bfloat16())
+    assert bf.dtype == torch.bfloat16 and torch.isfinite(bf).all()
+    with pytest.raises(OjasxB200Error):
+        many.prefill(kt, vt, qt)                                          # does not fit: -2, nothing is appended
+    assert many.seq_len == T0 + S
+
+
+def test_prefill_operand_range(cuda, oracle):
+    """Queries and codebooks far from 1: the operands of the prefill kernel are scaled per row and per codebook, so the
+    accuracy does not depend on their magnitude."""
+    books, old, k, v, q = _make(3, 1, 2, 8, 128, 8, 64, 16)
+    books = [books[0] * np.float32(2e5), books[1] * np.float32(3e-6)]
+    q = q * np.float32(1e-5)
+    q[3] = 0
+    cache = ops.VQKVCache(1, 2, 8, 128, 8, 100, *books)
+    cache.load(*old)
+    got = cache.prefill(*(torch.from_numpy(a).to(cuda) for a in (k, v, q))).cpu().numpy()
+    kc, vc = cache.read(0, 80)
+    for s in (0, 3, 15):
+        ref = oracle.kvq_decode(q[s, 0, :4], kc[0, 0, :65 + s], vc[0, 0, :65 + s], books[0][0], books[1][0], block_dim=8)
+        assert np.allclose(got[s, 0, :4], ref, rtol=1e-4, atol=2e-6 * 3e-6), s
