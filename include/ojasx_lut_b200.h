@@ -233,6 +233,21 @@ OJASX_API int ojasx_b200_moe_forward_noalloc(OjasxMoEHandle handle, const void* 
                                              const float* d_topk_w, void* d_y, int n_tokens, int k_active,
                                              int io_dtype, void* stream);
 
+/* ojasx_b200_linear_forward with scratch of the caller: bf16 batches up to 31 may then run on the tensor cores, with
+ * the table kernels' result.  ojasx_b200_linear_workspace says how many bytes such a call takes, 16-byte aligned (0: the
+ * call would not use any); calls that overlap in time need scratch of their own. */
+OJASX_API size_t ojasx_b200_linear_workspace(OjasxLinearHandle handle, int batch_size, int io_dtype);
+OJASX_API int ojasx_b200_linear_forward_ws(OjasxLinearHandle handle, const void* d_x, void* d_y, int batch_size,
+                                           int io_dtype, int row_start, int row_stop, void* workspace,
+                                           size_t workspace_bytes, void* stream);
+/* down(silu(gate(x)) * up(x)) for a bf16 batch of 1 to 31, every stage rounded to bf16 as the separate calls round it.
+ * ojasx_b200_mlp_workspace is 0 where the block has to be called layer by layer (then -4). */
+OJASX_API size_t ojasx_b200_mlp_workspace(OjasxLinearHandle gate, OjasxLinearHandle up, OjasxLinearHandle down,
+                                          const void* d_x, int batch_size, int io_dtype);
+OJASX_API int ojasx_b200_mlp_forward(OjasxLinearHandle gate, OjasxLinearHandle up, OjasxLinearHandle down,
+                                     const void* d_x, void* d_y, int batch_size, int io_dtype, void* workspace,
+                                     size_t workspace_bytes, void* stream);
+
 /* ---- Exchange between the GPUs of one box over peer memory, fused into the producing kernel (no counterpart
  * in the reference, which has no multi-device code; the row contract it serves is row_start / row_stop of
  * rvq_fused_gemm, ojasx_24x96/native/ojasx_backend_abi.h:97-111).  Every rank allocates one segment of the same

@@ -54,6 +54,10 @@ SIGNATURES = {
     "ojasx_b200_last_error": (C.c_char_p, []),
     "ojasx_b200_launch_count": (C.c_ulonglong, []),
     "ojasx_b200_linear_forward": (_i, [_vp, _vp, _vp, _i, _i, _i, _i, _vp]),
+    "ojasx_b200_linear_workspace": (_sz, [_vp, _i, _i]),
+    "ojasx_b200_linear_forward_ws": (_i, [_vp, _vp, _vp, _i, _i, _i, _i, _vp, _sz, _vp]),
+    "ojasx_b200_mlp_workspace": (_sz, [_vp, _vp, _vp, _vp, _i, _i]),
+    "ojasx_b200_mlp_forward": (_i, [_vp, _vp, _vp, _vp, _vp, _i, _i, _vp, _sz, _vp]),
     "ojasx_b200_linear_forward_tensor": (_i, [_vp, _vp, _vp, _i, _i, _i, _vp]),
     "ojasx_b200_take_device_error": (_i, []),
     "ojasx_b200_linear_forward_raw": (_i, [_vp, _vp, _vp, _vp, _i, _vp, _vp, _vp, _vp, _vp,

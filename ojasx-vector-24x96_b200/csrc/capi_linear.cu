@@ -1,6 +1,7 @@
 // C ABI, linear-layer part: the reference's ojasx_*linear* handle API on host pointers
 // (split_manifold_lut_experiment/native/src/ojasx_lut_c_api.cpp:31-129) and the ojasx_b200_*
 // device-pointer entry points.  Handles own device copies of every array.
+#include <algorithm>
 #include "../../include/ojasx_lut_b200.h"
 #include "handles.h"
 #include "launch.h"
@@ -186,6 +187,73 @@ int ojasx_b200_linear_forward(OjasxLinearHandle handle, const void* d_x, void* d
         if (min_batch > 0 && batch_size >= min_batch) return launch_dequant_gemm(P, static_cast<cudaStream_t>(stream), &h->dq_lists, h->generation);
     }
     return launch_linear(P, static_cast<cudaStream_t>(stream));
+}
+
+// (code, vector) pairs from which a single linear takes the gather kernel; OJASX_B200_GATHER_MIN_WORK overrides (0: every
+// call that fits, negative: never).  Its second launch costs the host 5 us, which smaller calls do not win back (2560 to
+// 2560 columns, us per call in a loop, table kernels against this: batch 1 15.5 / 22.7, batch 4 22.9 / 22.6, batch 8
+// 24.9 / 22.2; 2560 to 6912, batch 2: 24.9 / 22.8).
+static long long gather_min_work() {
+    const char* e = getenv("OJASX_B200_GATHER_MIN_WORK");
+    return e ? atoll(e) : 3000000;
+}
+
+// Whether the gather kernel (gather_mma.cu) may take a call; the switches of the other paths come first.
+static bool gather_mma_open(const LinearProblem& P, bool csr_sorted) {
+    if (!gather_mma_supported(P) || linear_cluster_disabled() || gather_min_work() < 0) return false;
+    const char* e = getenv("OJASX_B200_TENSOR_MIN_BATCH");
+    const int min_batch = e ? atoi(e) : kTensorMinBatch;
+    return !(min_batch > 0 && P.batch >= min_batch && dequant_gemm_supported(P, csr_sorted));
+}
+
+static bool wants_gather_mma(const LinearProblem& P, bool csr_sorted) {
+    return gather_mma_open(P, csr_sorted) && (long long)(P.row_stop - P.row_start) * P.G * P.batch >= gather_min_work();
+}
+
+size_t ojasx_b200_linear_workspace(OjasxLinearHandle handle, int batch_size, int io_dtype) {
+    if (!handle || batch_size <= 0) return 0;
+    auto* h = static_cast<LinearHandle*>(handle);
+    const LinearProblem P = h->problem(nullptr, nullptr, batch_size, io_dtype, 0, h->out);
+    return gather_mma_supported(P) ? gather_mma_workspace(h->in, batch_size) : 0;
+}
+
+int ojasx_b200_linear_forward_ws(OjasxLinearHandle handle, const void* d_x, void* d_y, int batch_size, int io_dtype,
+                                 int row_start, int row_stop, void* workspace, size_t workspace_bytes, void* stream) {
+    if (!handle || !d_x || !d_y) return OJX_ERR_ARG;
+    auto* h = static_cast<LinearHandle*>(handle);
+    if (batch_size <= 0 || row_start < 0 || row_stop > h->out || row_start >= row_stop) return OJX_ERR_ARG;
+    const LinearProblem P = h->problem(d_x, d_y, batch_size, io_dtype, row_start, row_stop);
+    if (workspace && wants_gather_mma(P, h->csr_sorted) && workspace_bytes >= gather_mma_workspace(h->in, batch_size))
+        return launch_gather_mma(&P, 1, d_x, nullptr, nullptr, workspace, static_cast<cudaStream_t>(stream));
+    return ojasx_b200_linear_forward(handle, d_x, d_y, batch_size, io_dtype, row_start, row_stop, stream);
+}
+
+size_t ojasx_b200_mlp_workspace(OjasxLinearHandle gate, OjasxLinearHandle up, OjasxLinearHandle down, const void* d_x,
+                                int batch_size, int io_dtype) {
+    if (!gate || !up || !down || !d_x || batch_size <= 0) return 0;
+    const LinearHandle* l[3] = {static_cast<LinearHandle*>(gate), static_cast<LinearHandle*>(up), static_cast<LinearHandle*>(down)};
+    if (l[0]->in != l[1]->in || l[0]->out != l[1]->out || l[2]->in != l[0]->out) return 0;
+    for (const LinearHandle* h : l)
+        if (!gather_mma_open(h->problem(d_x, nullptr, batch_size, io_dtype, 0, h->out), h->csr_sorted)) return 0;
+    return std::max(gather_mma_workspace(l[0]->in, batch_size), gather_mma_workspace(l[2]->in, batch_size)) +
+           3 * (size_t)batch_size * l[0]->out * 2;   // and gate, up and the gated vectors
+}
+
+int ojasx_b200_mlp_forward(OjasxLinearHandle gate, OjasxLinearHandle up, OjasxLinearHandle down, const void* d_x, void* d_y,
+                           int batch_size, int io_dtype, void* workspace, size_t workspace_bytes, void* stream) {
+    if (!gate || !up || !down || !d_x || !d_y || !workspace) return OJX_ERR_ARG;
+    const size_t need = ojasx_b200_mlp_workspace(gate, up, down, d_x, batch_size, io_dtype);
+    if (need == 0 || workspace_bytes < need) return OJX_ERR_UNSUPPORTED;
+    auto *g = static_cast<LinearHandle*>(gate), *u = static_cast<LinearHandle*>(up), *d = static_cast<LinearHandle*>(down);
+    cudaStream_t s = static_cast<cudaStream_t>(stream);
+    const size_t one = (size_t)batch_size * g->out * 2;   // a multiple of 16: widths are multiples of 64
+    char* buf = static_cast<char*>(workspace);
+    void *yg = buf, *yu = buf + one, *yh = buf + 2 * one;
+    const LinearProblem P[2] = {g->problem(d_x, yg, batch_size, io_dtype, 0, g->out), u->problem(d_x, yu, batch_size, io_dtype, 0, u->out)};
+    int rc = launch_gather_mma(P, 2, d_x, nullptr, nullptr, buf + 3 * one, s);
+    if (rc != OJX_OK) return rc;
+    const LinearProblem Q = d->problem(yh, d_y, batch_size, io_dtype, 0, d->out);
+    return launch_gather_mma(&Q, 1, yg, yu, yh, buf + 3 * one, s);
 }
 
 int ojasx_b200_linear_forward_gather(OjasxLinearHandle handle, const void* d_x, void* d_y_full, int batch_size, int io_dtype,

@@ -45,6 +45,11 @@ struct DqLists {
 int launch_dequant_gemm(const LinearProblem& P, cudaStream_t stream, DqLists* lists = nullptr, unsigned generation = 0);
 int take_dequant_gemm_error(int* out);
 
+// --- gather_mma.cu: bf16 batches below the tensor-core path, weights gathered into mma.sync operands at fp32 accuracy
+bool gather_mma_supported(const LinearProblem& P);
+size_t gather_mma_workspace(int K, int batch);   // bytes for the prepared activations of one call
+int launch_gather_mma(const LinearProblem* P, int count, const void* x, const void* up, void* h, void* workspace, cudaStream_t s);
+
 // --- moe.cu
 // link: expert-parallel ranks gather every pair's expert output over peer memory before the combine (null: one rank)
 int launch_moe_experts(MoeProblem P, cudaStream_t stream, const PeerLink* link = nullptr);

@@ -17,18 +17,12 @@
 #include "launch.h"
 #include "handles.h"
 #include "peer.cuh"
+#include "silu.cuh"
 #include "../../include/ojasx_lut_b200.h"
 
 #include <mutex>
 
 namespace ojx {
-
-// silu(v) = v / (1 + exp(-v))  (ojasx_lut_cpu.cpp:209-211).  exp is evaluated in double and
-// rounded once, which reproduces a correctly rounded expf in all but ~1e-9 of arguments.
-__device__ __forceinline__ float silu_ref(float v) {
-    const float e = (float)exp((double)(-v));
-    return __fdiv_rn(v, __fadd_rn(1.0f, e));
-}
 
 struct MoePair {
     int token, expert;  // expert is the LOCAL expert index, or -1 when the pair is skipped

@@ -11,6 +11,7 @@ from ._lib import OjasxB200Error, check, lib
 
 _vp = C.c_void_p
 F32, BF16 = 0, 1
+GATHER_BATCHES = range(1, 32)    # bf16 batches that may take the gather kernel (the library decides by shape)
 
 
 def _p(a):
@@ -58,6 +59,7 @@ class VQLinear:
                                             _p(cb), _p(codes), _p(sc), _p(bi))
         if not self._h:
             check(-3, "ojasx_create_linear")
+        self._workspace = {}    # batch -> scratch bytes of a bf16 call
         self.nnz = 0
         if csr is not None:
             rp = np.ascontiguousarray(csr[0], dtype=np.int32)
@@ -87,6 +89,16 @@ class VQLinear:
         rows = row_stop - row_start
         if out is None:
             out = torch.empty((x2.shape[0], rows), device=x.device, dtype=x.dtype)
+        if x2.dtype is torch.bfloat16 and 1 < x2.shape[0] < GATHER_BATCHES.stop:
+            size = self._workspace.get(x2.shape[0])
+            if size is None:
+                size = self._workspace[x2.shape[0]] = lib().ojasx_b200_linear_workspace(self._h, x2.shape[0], BF16)
+            if size:    # scratch of this call, so that calls on several streams do not share it
+                ws = torch.empty(size, device=x.device, dtype=torch.uint8)
+                check(lib().ojasx_b200_linear_forward_ws(self._h, x2.data_ptr(), out.data_ptr(), x2.shape[0], BF16, row_start,
+                                                         row_stop, ws.data_ptr(), size, _stream_ptr(x.device)),
+                      "ojasx_b200_linear_forward_ws")
+                return out.reshape(*x.shape[:-1], rows)
         check(lib().ojasx_b200_linear_forward(self._h, x2.data_ptr(), out.data_ptr(), x2.shape[0], _dtype_code(x2),
                                               row_start, row_stop, _stream_ptr(x.device)),
               "ojasx_b200_linear_forward")
@@ -206,6 +218,17 @@ class VQMLP:
         self._pair = VQLinearGroup([gate, up])   # one launch for gate and up when there is a single token
 
     def forward(self, x: torch.Tensor) -> torch.Tensor:
+        if x.dtype is torch.bfloat16 and x.is_cuda and x.shape[-1] == self.gate.in_features and \
+                x.numel() // self.gate.in_features in GATHER_BATCHES:
+            x2 = x.reshape(-1, self.gate.in_features).contiguous()
+            handles = (self.gate.handle, self.up.handle, self.down.handle)
+            size = lib().ojasx_b200_mlp_workspace(*handles, x2.data_ptr(), x2.shape[0], BF16)
+            if size:
+                ws = torch.empty(size, device=x.device, dtype=torch.uint8)
+                y = torch.empty((x2.shape[0], self.down.out_features), device=x.device, dtype=x.dtype)
+                check(lib().ojasx_b200_mlp_forward(*handles, x2.data_ptr(), y.data_ptr(), x2.shape[0], BF16, ws.data_ptr(), size,
+                                                   _stream_ptr(x.device)), "ojasx_b200_mlp_forward")
+                return y.reshape(*x.shape[:-1], -1)
         if x.numel() == self.gate.in_features:   # one token: gate and up share x and run as one grouped launch
             gu = torch.empty((2, self.gate.out_features), dtype=x.dtype, device=x.device)
             self._pair.forward(x.reshape(-1), gu, shared_x=True)

@@ -1,0 +1,84 @@
+"""bf16 batches below 32: weights gathered into mma.sync operands, against the fp32 oracle."""
+import numpy as np
+import pytest
+import torch
+
+import ojasx_b200
+from ojasx_b200 import ops, synth
+
+pytestmark = pytest.mark.gpu
+
+
+def _oracle(oracle, w, x):
+    return oracle.linear_forward(w.codebook, w.codes, w.scales, w.bias, w.csr, x, block_dim=8)
+
+
+def _close_once_rounded(got, want):
+    """One rounding to bf16 (eight bits of significand: half an ulp is at most 2^-8 of the value) of a sum that differs
+    from the oracle's by fp32 rounding: a few 1e-7 of the row's largest terms, 1e-5 where those are of order one."""
+    return np.all(np.abs(got - want) <= 2.0 ** -8 * np.abs(want) + 1e-5)
+
+
+@pytest.mark.parametrize("K,M,batch", [
+    (512, 300, 2),
+    (64, 16, 8),         # one partial chunk, one tile
+    (256, 33, 9),        # one whole chunk, ragged rows
+    (1088, 200, 16),     # G = 136: eight-byte code loads, an eight-group tail
+    (2560, 2560, 17),
+    (2560, 6912, 31),
+    (6912, 2560, 16),    # K split over a cluster
+    (4736, 130, 25),
+])
+@pytest.mark.parametrize("frac", [0.0, 0.0038])
+def test_gather_mma_against_oracle(cuda, oracle, monkeypatch, K, M, batch, frac):
+    w = synth.make_vq_linear(K + batch, K, M, block_dim=8, outlier_frac=frac, with_scales=True, with_bias=True)
+    x = np.random.default_rng(batch).standard_normal((batch, K)).astype(np.float32)
+    x *= np.float32(2.0) ** np.random.default_rng(K).integers(-20, 20, size=(batch, 1))   # every vector has its own scale
+    xb = synth.to_bf16_f32(x)
+    want = _oracle(oracle, w, xb)
+    layer = ops.VQLinear.from_weights(w)
+    xt = torch.from_numpy(xb).to(cuda).bfloat16()
+    monkeypatch.setenv("OJASX_B200_GATHER_MIN_WORK", "0")
+    n0 = ojasx_b200.launch_count()
+    got = layer(xt).float().cpu().numpy()
+    assert ojasx_b200.launch_count() - n0 == 2          # activations, rows
+    size = np.abs(want).max(axis=1, keepdims=True)      # vectors of 2^-20 .. 2^20: compare at one scale
+    assert _close_once_rounded(got / size, want / size)
+    a, b = M // 3, M - 1                                # a row slice is the same rows
+    part = layer(xt, a, b).float().cpu().numpy()
+    assert _close_once_rounded(part / size, want[:, a:b] / size)
+    monkeypatch.setenv("OJASX_B200_GATHER_MIN_WORK", "-1")
+    table = layer(xt).float().cpu().numpy()             # the table kernels: the oracle's sums, rounded
+    assert np.mean(got != table) <= 1e-5, np.mean(got != table)
+
+
+def test_gather_mma_infinities_and_nan(cuda, oracle, monkeypatch):
+    """A vector with an infinity or NaN is evaluated in the reference's order; its neighbours are untouched."""
+    monkeypatch.setenv("OJASX_B200_GATHER_MIN_WORK", "0")
+    w = synth.make_vq_linear(5, 512, 100, block_dim=8, with_scales=True)
+    x = synth.to_bf16_f32(np.random.default_rng(0).standard_normal((12, 512)).astype(np.float32))
+    clean = ops.VQLinear.from_weights(w)(torch.from_numpy(x).to(cuda).bfloat16()).float().cpu().numpy()
+    x[1, 300], x[4, 0], x[7, 511], x[7, 3] = np.inf, np.nan, -np.inf, np.inf
+    x[9] = 0.0
+    got = ops.VQLinear.from_weights(w)(torch.from_numpy(x).to(cuda).bfloat16()).float().cpu().numpy()
+    with np.errstate(all="ignore"):
+        want = synth.to_bf16_f32(_oracle(oracle, w, x))
+    for t in range(12):
+        if t in (1, 4, 7):
+            assert np.array_equal(got[t], want[t], equal_nan=True)
+        elif t != 9:
+            assert np.array_equal(got[t], clean[t])
+    assert np.all(got[9] == 0)
+
+
+@pytest.mark.parametrize("K,M,batch", [(2560, 6912, 16), (1088, 2112, 8), (1536, 2048, 31)])
+def test_mlp_block_equals_its_layers(cuda, K, M, batch):
+    ws = [synth.make_vq_linear(90 + i, *s, block_dim=8) for i, s in enumerate([(K, M), (K, M), (M, K)])]
+    gate, up, down = (ops.VQLinear.from_weights(w) for w in ws)
+    x = torch.randn(batch, K, device=cuda, generator=torch.Generator(cuda).manual_seed(batch)).bfloat16()
+    n0 = ojasx_b200.launch_count()
+    got = ops.VQMLP(gate, up, down)(x)
+    assert ojasx_b200.launch_count() - n0 == 4
+    want = down(ops.silu_mul(gate(x), up(x)))
+    # a gate or up value whose rounding tips moves one of M terms of an output by 2^-8 of itself
+    assert torch.allclose(got.float(), want.float(), rtol=2 ** -7, atol=2 ** -8 * want.float().abs().max().item() / 8)
