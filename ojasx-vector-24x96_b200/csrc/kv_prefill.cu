@@ -220,7 +220,7 @@ __global__ void __launch_bounds__(kPfThreads) kvq_prefill_kernel(const __grid_co
     }
     __syncthreads();
 
-    float o[HD / 8][4], m_run[2] = {-INFINITY, -INFINITY}, l_run[2] = {0.0f, 0.0f};
+    float o[HD / 8][4], m_run[2] = {-INFINITY, -INFINITY}, l_run[2] = {0.0f, 0.0f}, l_err[2] = {0.0f, 0.0f};
 #pragma unroll
     for (int n = 0; n < HD / 8; ++n)
 #pragma unroll
@@ -254,7 +254,7 @@ __global__ void __launch_bounds__(kPfThreads) kvq_prefill_kernel(const __grid_co
         }
     };
     const uint32_t kh_a = static_cast<uint32_t>(__cvta_generic_to_shared(Kh)) + (((lane >> 4) * 8 + (lane & 7)) * LD + ((lane >> 3) & 1) * 8) * 2;
-    const uint32_t vh_a = static_cast<uint32_t>(__cvta_generic_to_shared(Vh)) + ((((lane >> 3) & 1) * 8 + (lane & 7)) * LD + (lane >> 4) * 8) * 2;
+    const uint32_t vt_a = static_cast<uint32_t>(__cvta_generic_to_shared(Vh)) + lane * LD * 2;   // row = token of a 32-token step
     constexpr uint32_t kPart = kPfTok * LD * 2;                  // bytes from a tile's hi part to its lo part
 
     fetch(0);
@@ -273,25 +273,33 @@ __global__ void __launch_bounds__(kPfThreads) kvq_prefill_kernel(const __grid_co
         __syncthreads();
         if (t0 + kPfTok < t_all) fetch(t0 + kPfTok);
 
+        // Chains in the tensor cores stay short (the products of two 16-wide steps here, of one below): they truncate,
+        // so that the error of a long chain grows with its length.
         float s[kPfTok / 8][4];
 #pragma unroll
-        for (int n = 0; n < kPfTok / 8; ++n)
+        for (int n2 = 0; n2 < kPfTok / 16; ++n2)
 #pragma unroll
-            for (int i = 0; i < 4; ++i) s[n][i] = 0.0f;
+            for (int k2 = 0; k2 < KT; k2 += 2) {
+                float t[2][4];
 #pragma unroll
-        for (int kk = 0; kk < KT; ++kk)
+                for (int i = 0; i < 8; ++i) t[i >> 2][i & 3] = 0.0f;
 #pragma unroll
-            for (int n2 = 0; n2 < kPfTok / 16; ++n2) {
-                uint32_t bh[4], bl[4];
-                const uint32_t a = kh_a + (n2 * 16 * LD + kk * 16) * 2;
-                pf_ldsm4(a, bh);
-                pf_ldsm4(a + kPart, bl);
+                for (int kk = k2; kk < k2 + 2; ++kk) {
+                    uint32_t bh[4], bl[4];
+                    const uint32_t a = kh_a + (n2 * 16 * LD + kk * 16) * 2;
+                    pf_ldsm4(a, bh);
+                    pf_ldsm4(a + kPart, bl);
 #pragma unroll
-                for (int j = 0; j < 2; ++j) {
-                    pf_mma(s[2 * n2 + j], qh[kk], bl[2 * j], bl[2 * j + 1]);
-                    pf_mma(s[2 * n2 + j], ql[kk], bh[2 * j], bh[2 * j + 1]);
-                    pf_mma(s[2 * n2 + j], qh[kk], bh[2 * j], bh[2 * j + 1]);
+                    for (int j = 0; j < 2; ++j) {
+                        pf_mma(t[j], qh[kk], bl[2 * j], bl[2 * j + 1]);
+                        pf_mma(t[j], ql[kk], bh[2 * j], bh[2 * j + 1]);
+                        pf_mma(t[j], qh[kk], bh[2 * j], bh[2 * j + 1]);
+                    }
                 }
+#pragma unroll
+                for (int j = 0; j < 2; ++j)
+#pragma unroll
+                    for (int i = 0; i < 4; ++i) s[2 * n2 + j][i] = k2 == 0 ? t[j][i] : s[2 * n2 + j][i] + t[j][i];
             }
         // scale, mask, online softmax (rows g and g + 8 of the warp's sixteen; a row lives in four lanes)
         float mt[2] = {-INFINITY, -INFINITY};
@@ -303,7 +311,7 @@ __global__ void __launch_bounds__(kPfThreads) kvq_prefill_kernel(const __grid_co
                 s[n][i] = t <= limit[i >> 1] ? s[n][i] * descale[i >> 1] : -INFINITY;
                 mt[i >> 1] = fmaxf(mt[i >> 1], s[n][i]);
             }
-        float base[2];
+        float base[2], l_tile[2] = {0.0f, 0.0f};
 #pragma unroll
         for (int i = 0; i < 2; ++i) {
             mt[i] = fmaxf(mt[i], __shfl_xor_sync(0xffffffffu, mt[i], 1));
@@ -313,6 +321,7 @@ __global__ void __launch_bounds__(kPfThreads) kvq_prefill_kernel(const __grid_co
             m_run[i] = m;
             base[i] = m;
             l_run[i] *= alpha;
+            l_err[i] *= alpha;
 #pragma unroll
             for (int n = 0; n < HD / 8; ++n) {
                 o[n][2 * i] *= alpha;
@@ -324,29 +333,43 @@ __global__ void __launch_bounds__(kPfThreads) kvq_prefill_kernel(const __grid_co
 #pragma unroll
             for (int i = 0; i < 4; ++i) {
                 s[n][i] = exp2f(s[n][i] - base[i >> 1]);
-                l_run[i >> 1] += s[n][i];
+                l_tile[i >> 1] += s[n][i];
             }
 #pragma unroll
-        for (int j = 0; j < kPfTok / 16; ++j) {
-            uint32_t ph[4], pl[4];
+        for (int i = 0; i < 2; ++i) {   // compensated: thousands of additions follow on a long context
+            const float y = l_tile[i] - l_err[i], t = __fadd_rn(l_run[i], y);
+            l_err[i] = __fsub_rn(__fsub_rn(t, l_run[i]), y);
+            l_run[i] = t;
+        }
+        uint32_t ph[kPfTok / 16][4], pl[kPfTok / 16][4];
+#pragma unroll
+        for (int j = 0; j < kPfTok / 16; ++j)
 #pragma unroll
             for (int i = 0; i < 4; ++i) {
                 const float* c = s[2 * j + (i >> 1)] + (i & 1) * 2;
-                pf_split2(c[0] * 16384.0f, c[1] * 16384.0f, ph[i], pl[i]);
+                pf_split2(c[0] * 16384.0f, c[1] * 16384.0f, ph[j][i], pl[j][i]);
             }
 #pragma unroll
-            for (int n2 = 0; n2 < HD / 16; ++n2) {
-                uint32_t bh[4], bl[4];
-                const uint32_t a = vh_a + (j * 16 * LD + n2 * 16) * 2;
+        for (int n1 = 0; n1 < HD / 8; ++n1) {   // a tile's products are added to one another, then to the output
+            float sum[4];
+#pragma unroll
+            for (int j2 = 0; j2 < kPfTok / 16; j2 += 2) {
+                uint32_t bh[4], bl[4];          // eight dimensions of 32 tokens
+                const uint32_t a = vt_a + (j2 * 16 * LD + n1 * 8) * 2;
                 pf_ldsm4t(a, bh);
                 pf_ldsm4t(a + kPart, bl);
 #pragma unroll
-                for (int q = 0; q < 2; ++q) {
-                    pf_mma(o[2 * n2 + q], ph, bl[2 * q], bl[2 * q + 1]);
-                    pf_mma(o[2 * n2 + q], pl, bh[2 * q], bh[2 * q + 1]);
-                    pf_mma(o[2 * n2 + q], ph, bh[2 * q], bh[2 * q + 1]);
+                for (int j = 0; j < 2; ++j) {
+                    float t[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+                    pf_mma(t, ph[j2 + j], bl[2 * j], bl[2 * j + 1]);
+                    pf_mma(t, pl[j2 + j], bh[2 * j], bh[2 * j + 1]);
+                    pf_mma(t, ph[j2 + j], bh[2 * j], bh[2 * j + 1]);
+#pragma unroll
+                    for (int i = 0; i < 4; ++i) sum[i] = j2 + j == 0 ? t[i] : sum[i] + t[i];
                 }
             }
+#pragma unroll
+            for (int i = 0; i < 4; ++i) o[n1][i] += sum[i];
         }
         __syncthreads();   // the tile has been read
     }
