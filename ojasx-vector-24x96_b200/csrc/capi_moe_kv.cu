@@ -348,6 +348,7 @@ OjasxKvqHandle ojasx_b200_kvq_create(int batch, int kv_heads, int q_heads, int h
     int rc = cudaGetDevice(&h->dev) == cudaSuccess ? OJX_OK : OJX_ERR_CUDA;
     const size_t codes = (size_t)batch * kv_heads * max_seq_len * h->G;
     const size_t cbb = sizeof(float) * (size_t)kv_heads * 256 * block_dim;
+    for (size_t i = 0; i < cbb / sizeof(float) && h->finite_books; ++i) h->finite_books = std::isfinite(k_codebook[i]) && std::isfinite(v_codebook[i]);
     if (rc == OJX_OK) rc = upload((void**)&h->k_codes, nullptr, codes);
     if (rc == OJX_OK) rc = upload((void**)&h->v_codes, nullptr, codes);
     if (rc == OJX_OK) rc = upload((void**)&h->k_cb, k_codebook, cbb);
@@ -408,11 +409,9 @@ static KvqProblem kvq_problem(const KvqHandle* h, int io) {
     P.seq_lens = h->seq_lens; P.error_flag = h->error_flag; P.partials = static_cast<float*>(h->partials);
     P.append_done = h->counters; P.split_done = h->counters + h->B;
     P.B = h->B; P.Hkv = h->Hkv; P.Hq = h->Hq; P.head_dim = h->head_dim; P.D = h->D; P.G = h->G; P.Kcb = 256;
-    P.max_seq = h->max_seq; P.io_dtype = io;
+    P.max_seq = h->max_seq; P.io_dtype = io; P.finite_books = h->finite_books;
     return P;
 }
-
-static int kvq_max_splits(int max_seq) { return std::min(kKvMaxSplits, (max_seq + 255) / 256); }
 
 int ojasx_b200_kvq_append(OjasxKvqHandle handle, const void* d_k, const void* d_v, int io_dtype, void* stream) {
     if (!handle || !d_k || !d_v || (io_dtype != OJX_F32 && io_dtype != OJX_BF16)) return OJX_ERR_ARG;

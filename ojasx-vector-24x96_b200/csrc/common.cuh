@@ -111,6 +111,7 @@ struct KvqProblem {
     int* split_done;        // [B, Hkv] decode CTAs of a (sequence, head) that have written their partial (returns to 0)
     int B, Hkv, Hq, head_dim, D, G, Kcb, max_seq;
     int chunk, n_chunks;
+    int finite_books;       // both codebooks hold finite numbers only (checked when the cache is created)
     int v_copies;           // copies of the value codebook in the decode kernel's shared memory (1 or 8)
     int io_dtype;
     float scale;

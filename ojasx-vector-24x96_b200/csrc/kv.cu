@@ -12,6 +12,7 @@
 //     per-token abs-max scale (ojasx_lut_kv_cache.cpp:16-132, softmax of
 //     ojasx_lut_c_api.cpp:178-191).
 #include <algorithm>
+#include <cstdlib>
 
 #include "common.cuh"
 #include "launch.h"
@@ -37,6 +38,7 @@ __device__ __forceinline__ float load_io(const void* p, size_t i, int dtype) {
 // the length before they count), so an append is one launch.
 template <int D>
 __global__ void __launch_bounds__(kKvThreads) kvq_append_kernel(const __grid_constant__ KvqProblem P) {
+    cudaTriggerProgrammaticLaunchCompletion();   // a decode behind this launch may prepare its tables
     const int b = blockIdx.y;
     const int T = P.seq_lens[b];
     if (T >= P.max_seq) {   // cache full: nothing is written, the error flag reports it
@@ -616,8 +618,22 @@ size_t kvq_decode_smem(const KvqProblem& P, int R) { return kvq_decode_smem_copi
 // Splits of the context: a CTA's range is a multiple of 64 tokens; among the split counts the one with
 // the least (waves of CTAs, one per SM) x (range + the table set-up and the fill and drain of the
 // score/value pipeline, together worth about 1000 tokens) wins.
+static bool kvq_decode_by_mma(const KvqProblem& P) {
+    const char* e = getenv("OJASX_B200_KV_DECODE");   // "table" keeps the query-table kernel
+    return kvq_decode_mma_supported(P) && !(e && e[0] == 't');
+}
+
 void plan_kvq_decode(KvqProblem& P, int T, int sms) {
     const int heads = (P.n_pos > 0 ? P.n_pos : 1) * P.B * P.Hkv, slots = sms;
+    if (kvq_decode_by_mma(P)) {
+        // chunks are shared out evenly over the SMs: an SM's share, 32 to 256 tokens (a tile for each of 16 warps), and
+        // no more chunks per sequence than the scratch holds
+        const long long share = ((long long)heads * std::max(T, 1) + sms - 1) / sms;
+        P.chunk = round_up((int)std::min<long long>(share, 256), 32);
+        P.chunk = std::max(P.chunk, round_up((std::max(T, 1) + kvq_max_splits(T) - 1) / kvq_max_splits(T), 32));
+        P.n_chunks = (std::max(T, 1) + P.chunk - 1) / P.chunk;
+        return;
+    }
     const int max_s = std::min(kKvMaxSplits, (T + 255) / 256);
     long best = -1;
     P.chunk = round_up(std::max(T, 1), 64);
@@ -690,6 +706,7 @@ int launch_kvq_decode(const KvqProblem& P, cudaStream_t s, const PeerLink* lk) {
     if (!P.q || !P.out || !P.partials || !P.seq_lens) return OJX_ERR_ARG;
     if (P.G > kKvMaxGroups || P.Hq % P.Hkv != 0) return OJX_ERR_UNSUPPORTED;
     if (P.head_dim > 2 * kKvThreads || P.head_dim % 4 != 0) return OJX_ERR_UNSUPPORTED;
+    if (kvq_decode_by_mma(P)) return launch_kvq_decode_mma(P, s, link);
     switch (P.Hq / P.Hkv) {
         case 1: return launch_decode_r<1>(P, s, link);
         case 2: return launch_decode_r<2>(P, s, link);

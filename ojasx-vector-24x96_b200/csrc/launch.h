@@ -80,8 +80,13 @@ constexpr int kKvMaxSplits = 256;   // context splits of one (sequence, KV head)
 size_t kvq_decode_smem(const KvqProblem& P, int R);
 // Fills P.chunk (tokens per CTA) and P.n_chunks (<= kKvMaxSplits) for a context of T tokens.
 void plan_kvq_decode(KvqProblem& P, int T, int sms);
+// Most splits a plan for up to T tokens makes.
+inline int kvq_max_splits(int T) { return T <= 0 ? 1 : T > 64 * kKvMaxSplits ? kKvMaxSplits : (T + 63) / 64; }
 int launch_kvq_append(const KvqProblem& P, cudaStream_t stream);
 int launch_kvq_decode(const KvqProblem& P, cudaStream_t stream, const PeerLink* link = nullptr);
+// --- kv_decode_mma.cu: decode for block_dim 8 and head_dim 64 or 128 (launch_kvq_decode takes it where it fits)
+bool kvq_decode_mma_supported(const KvqProblem& P);
+int launch_kvq_decode_mma(const KvqProblem& P, cudaStream_t stream, const PeerLink& link);
 // --- kv_prefill.cu: a chunk of P.n_pos prompt positions (lengths are advanced last)
 int launch_kvq_append_many(const KvqProblem& P, cudaStream_t stream);
 bool kvq_prefill_supported(const KvqProblem& P);

@@ -1,0 +1,107 @@
+"""Decode on mma.sync operands gathered from the codebooks against the query-table kernel and 64-bit attention."""
+import numpy as np
+import pytest
+import torch
+
+import ojasx_b200
+from ojasx_b200 import ops
+
+pytestmark = pytest.mark.gpu
+
+
+def _cache(B, Hk, R, hd, T, cap, seed):
+    rng = np.random.default_rng(seed)
+    books = [(rng.standard_normal((Hk, 256, 8)) / np.sqrt(hd)).astype(np.float32) for _ in range(2)]
+    codes = [rng.integers(0, 256, (B, Hk, T, hd // 8), dtype=np.uint8) for _ in range(2)]
+    cache = ops.VQKVCache(B, Hk, Hk * R, hd, 8, cap, *books)
+    cache.load(*codes)
+    return cache, books, codes, rng
+
+
+def _exact(books, codes, q, scale):
+    B, Hk = codes[0].shape[:2]
+    R = q.shape[1] // Hk
+    out = np.zeros(q.shape, np.float64)
+    for b in range(B):
+        for h in range(Hk):
+            k, v = (books[i][h].astype(np.float64)[codes[i][b, h]].reshape(codes[i].shape[2], -1) for i in range(2))
+            s = q[b, h * R:(h + 1) * R].astype(np.float64) @ k.T * scale
+            p = np.exp(s - s.max(-1, keepdims=True))
+            out[b, h * R:(h + 1) * R] = p @ v / p.sum(-1, keepdims=True)
+    return out
+
+
+@pytest.mark.parametrize("R,hd", [(4, 64), (4, 128), (8, 64), (8, 128)])
+@pytest.mark.parametrize("T", [1, 16, 17, 257, 1001, 5000])
+def test_decode_against_table_kernel_and_64_bits(cuda, monkeypatch, R, hd, T):
+    B, Hk = 2, 3
+    cache, books, codes, rng = _cache(B, Hk, R, hd, T, T + 3, R * hd + T)
+    q = rng.standard_normal((B, Hk * R, hd)).astype(np.float32) * 4       # scores of a few units: some tokens dominate
+    q[0, 0] *= 1e-6                                                       # heads of other sizes
+    q[1, -1] *= 1e4
+    qt = torch.from_numpy(q).to(cuda)
+    got = cache.decode(qt)
+    half = cache.decode(qt.bfloat16())
+    cache.set_static_plan(True)
+    planned = cache.decode(qt)
+    cache.set_static_plan(False)
+    monkeypatch.setenv("OJASX_B200_KV_DECODE", "table")
+    table = cache.decode(qt).cpu().numpy()
+    want = _exact(books, codes, q, 1.0 / np.sqrt(hd))
+    # a rounding of the scores (2^-24 of their largest terms, up to 1e4 units for the last head) is a relative error of p
+    err = np.abs(got.cpu().numpy() - want).max(-1)
+    ref = np.abs(table - want).max(-1)
+    size = np.abs(want).max(-1)
+    assert np.all(err <= 2 * ref + 1e-6 * size), (err / size, ref / size)
+    assert np.allclose(planned.cpu().numpy(), got.cpu().numpy(), rtol=0, atol=float((2 * ref + 2e-6 * size).max()))
+    bf = _exact(books, codes, qt.bfloat16().float().cpu().numpy(), 1.0 / np.sqrt(hd))
+    assert np.all(np.abs(half.float().cpu().numpy() - bf).max(-1) <= 2.0 ** -8 * np.abs(bf).max(-1) + 4 * ref + 1e-6 * size)
+
+
+def test_append_and_decode_in_one_stream_and_under_capture(cuda):
+    """A decode prepares its tables while the append before it runs, and still sees the appended token."""
+    cache, books, codes, rng = _cache(1, 2, 4, 128, 40, 64, 9)
+    k, v = (torch.from_numpy(rng.standard_normal((20, 1, 2, 128)).astype(np.float32)).to(cuda) for _ in range(2))
+    q = torch.from_numpy(rng.standard_normal((20, 1, 8, 128)).astype(np.float32)).to(cuda)
+    outs = []
+    for t in range(20):
+        cache.append(k[t], v[t])
+        outs.append(cache.decode(q[t]).cpu().numpy())
+    kc, vc = cache.read(0, 60)
+    for t in range(20):
+        want = _exact(books, [kc[:, :, :41 + t], vc[:, :, :41 + t]], q[t].cpu().numpy(), 1.0 / np.sqrt(128))
+        assert np.allclose(outs[t], want, rtol=1e-5, atol=1e-6 * np.abs(want).max())
+    cache.crop(40)
+    cache.set_static_plan(True)
+    cache.append(k[0], v[0])
+    cache.decode(q[0])
+    torch.cuda.synchronize()
+    cache.crop(40)
+    kk, vv, qq, o = k[0].clone(), v[0].clone(), q[0].clone(), torch.empty_like(q[0])
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        cache.append(kk, vv)
+        cache.decode(qq, out=o)
+    for t in range(20):
+        kk.copy_(k[t]); vv.copy_(v[t]); qq.copy_(q[t])
+        graph.replay()
+        assert np.allclose(o.cpu().numpy(), outs[t], rtol=1e-5, atol=1e-6)
+
+
+def test_codebooks_with_infinities_keep_the_table_kernel(cuda, monkeypatch):
+    """High and low parts of an infinity are NaN: caches whose codebooks are not finite stay on the query-table kernel."""
+    rng = np.random.default_rng(0)
+    books = [(rng.standard_normal((1, 256, 8)) * 0.1).astype(np.float32) for _ in range(2)]
+    books[1][0, 7, 3] = np.inf
+    cache = ops.VQKVCache(1, 1, 4, 64, 8, 32, *books)
+    codes = rng.integers(8, 256, (1, 1, 20, 8), dtype=np.uint8)
+    codes2 = codes.copy()
+    codes2[0, 0, 5, 2] = 7
+    q = torch.from_numpy(rng.standard_normal((1, 4, 64)).astype(np.float32)).to(cuda)
+    for c in (codes, codes2):
+        cache.load(codes, c)
+        got = cache.decode(q).cpu().numpy()
+        monkeypatch.setenv("OJASX_B200_KV_DECODE", "table")
+        assert np.array_equal(got, cache.decode(q).cpu().numpy(), equal_nan=True)
+        monkeypatch.delenv("OJASX_B200_KV_DECODE")
+        assert np.isfinite(got).all() == (c is codes)
