@@ -91,7 +91,8 @@ struct MoeProblem {
                               // (ResidualVQFusedExperts._apply_gate, ojasx_24x96/module.py:646-651); <= 0: no clamp
     const int* chain_ctl;     // [1 + pairs] claim counter and per-slot flags of moe_experts_chain_kernel (zeroed by the plan kernel), or null
     int lut_blocks;           // layout of lut_in: 0 = [token][group][256]; 1 = 16-group blocks (moe_prebuild_kernel);
-                              // 2 = per-slice images of the chain walk's table area (moe_chain_prebuild_kernel)
+                              // 2 = per-slice images of the chain walk's table area (moe_chain_prebuild_kernel);
+                              // 3 = no tables: the fragments of moe_gather.cu, made by the expert launches
 };
 
 // Codebook-VQ KV cache of one layer.  Device pointers.

@@ -181,7 +181,7 @@ __global__ void __launch_bounds__(kGmMaxWarps * 32, 2) gm_linear_kernel(const __
 #pragma unroll
                 for (int i = 0; i < 4; ++i) acc[m][n][i] = 0.0f;
         const uint4* frag = A.frag + (size_t)c * 8 * kVecs * 4;
-        gm_chunk<MT, NT>(acc, w, min(16, P.G - c * kGmChunk), table, [&](int j, int n) { return __ldg(frag + (size_t)j * kVecs * 4 + boff[n]); });
+        gm_chunk<MT, NT, 16>(acc, w, min(16, P.G - c * kGmChunk), table, [&](int j, int n) { return __ldg(frag + (size_t)j * kVecs * 4 + boff[n]); });
         const bool first = c == c_begin + warp;
 #pragma unroll
         for (int n = 0; n < NT; ++n) {

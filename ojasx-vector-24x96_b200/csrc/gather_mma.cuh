@@ -116,7 +116,9 @@ __device__ __forceinline__ void gm_load_codes(uint32_t (&w)[4], const uint8_t* r
 // acc += (weights of MT x 16 rows, one chunk) x (NT x 8 vectors).  w: the lane's codes (row lane & 15 of each tile,
 // half lane >> 4).  load(j, n): the lane's 16 bytes of fragments of tile n for steps 2j and 2j + 1.  table: shared address
 // of the lane's copy ((lane & 7) * 16 from the table's start).
-template <int MT, int NT, class Load>
+// kFlush: steps whose products are accumulated in the tensor cores before they are added to acc in fp32 (the tensor
+// cores truncate, so a chain's error grows with its length); 16: all of them.
+template <int MT, int NT, int kFlush, class Load>
 __device__ __forceinline__ void gm_chunk(float (&acc)[MT][NT][4], const uint32_t (&w)[MT][4], int steps, uint32_t table, Load load) {
     uint4 b[NT], bn[NT];
 #pragma unroll
@@ -130,6 +132,7 @@ __device__ __forceinline__ void gm_chunk(float (&acc)[MT][NT][4], const uint32_t
         gm_ldsm4(at + kGmTable / 2, lo);
     };
     uint32_t hi[2][4], lo[2][4];
+    float part[MT][NT][4];
     read(0, 0, hi[0], lo[0]);
 #pragma unroll
     for (int j = 0; j < 8; ++j) {
@@ -146,10 +149,23 @@ __device__ __forceinline__ void gm_chunk(float (&acc)[MT][NT][4], const uint32_t
                 for (int m = 0; m < MT; ++m) {
                     const int at = (2 * j + s) * MT + m, cur = at & 1, next = at + 1;
                     if (next < 16 * MT) read(next / MT, next % MT, hi[cur ^ 1], lo[cur ^ 1]);
+                    if (kFlush < 16 && (2 * j + s) % kFlush == 0) {
 #pragma unroll
-                    for (int n = 0; n < NT; ++n) gm_mma(acc[m][n], lo[cur], s ? b[n].z : b[n].x, s ? b[n].w : b[n].y);
+                        for (int n = 0; n < NT; ++n)
 #pragma unroll
-                    for (int n = 0; n < NT; ++n) gm_mma(acc[m][n], hi[cur], s ? b[n].z : b[n].x, s ? b[n].w : b[n].y);
+                            for (int e = 0; e < 4; ++e) part[m][n][e] = 0.0f;
+                    }
+                    auto& sum = kFlush < 16 ? part : acc;
+#pragma unroll
+                    for (int n = 0; n < NT; ++n) gm_mma(sum[m][n], lo[cur], s ? b[n].z : b[n].x, s ? b[n].w : b[n].y);
+#pragma unroll
+                    for (int n = 0; n < NT; ++n) gm_mma(sum[m][n], hi[cur], s ? b[n].z : b[n].x, s ? b[n].w : b[n].y);
+                    if (kFlush < 16 && (2 * j + s) % kFlush == kFlush - 1) {
+#pragma unroll
+                        for (int n = 0; n < NT; ++n)
+#pragma unroll
+                            for (int e = 0; e < 4; ++e) acc[m][n][e] += part[m][n][e];
+                    }
                 }
         }
     }

@@ -72,6 +72,9 @@ bool moe_fused_wanted(const MoeProblem& P);   // shape fits and enough routed pa
 int launch_moe_fused(MoeProblem P, cudaStream_t stream, const PeerLink* link = nullptr);   // work list, token tables (unless lut_ready), experts
 int launch_moe_prebuild_blocks(const void* x, int io_dtype, int n_tokens, int H, int D, const float* codebook, int Kcb,
                                float* out, cudaStream_t stream);
+// --- moe_gather.cu: experts that several tokens are routed to, on mma.sync operands gathered from the codebooks
+bool moe_gather_wanted(const MoeProblem& P);
+int launch_moe_gather(const MoeProblem& P, cudaStream_t s, const PeerLink& link);   // all but the combine
 int take_moe_fused_error(int* out);
 int take_moe_bulk_copy_error(int* out);   // moe.cu: a bounded wait for a bulk table copy ran out
 

@@ -25,6 +25,7 @@
 #include "launch.h"
 #include "handles.h"
 #include "peer.cuh"
+#include "block_scan.cuh"
 
 #include <cstdlib>
 
@@ -652,31 +653,6 @@ __global__ void __launch_bounds__(kThreads, 1) moe_fused_kernel(const __grid_con
 // into chunks of 4, 2 and 1 pairs of one expert (the largest chunks first in the list, so that the CTAs
 // that start last get the short ones).  plan[0] = chunks, plan[1] = work counter (zeroed), plan[4..] =
 // sorted pair ids, then the chunks.  One CTA; counting sort on the local expert id.
-__device__ __forceinline__ int block_exclusive_scan(int v, int* warp_tot /* [33] shared */, int* total) {
-    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nwarp = blockDim.x >> 5;
-    int inc = v;
-#pragma unroll
-    for (int off = 1; off < 32; off <<= 1) {
-        const int o = __shfl_up_sync(0xffffffffu, inc, off);
-        if (lane >= off) inc += o;
-    }
-    __syncthreads();   // warp_tot may still be read from the previous scan
-    if (lane == 31) warp_tot[wid] = inc;
-    __syncthreads();
-    if (wid == 0) {
-        int t = lane < nwarp ? warp_tot[lane] : 0;
-#pragma unroll
-        for (int off = 1; off < 32; off <<= 1) {
-            const int o = __shfl_up_sync(0xffffffffu, t, off);
-            if (lane >= off) t += o;
-        }
-        warp_tot[lane] = t;
-    }
-    __syncthreads();
-    *total = warp_tot[nwarp - 1];
-    return inc - v + (wid > 0 ? warp_tot[wid - 1] : 0);
-}
-
 __device__ __forceinline__ int plan_local_expert(const MoeProblem& P, int pair) {
     const int e = P.topk_idx[pair] - P.expert_offset;
     const float w = P.topk_w[pair];
