@@ -509,35 +509,64 @@ __global__ void __launch_bounds__(256) moe_router_logits_kernel(const float* __r
     peer_signal_when_last(link, gridDim.x * gridDim.y);
 }
 
-// Batches: a block scores eight experts (a warp each) for eight tokens at a time from a shared-memory tile of x, so a
-// router row is read once per eight tokens instead of once per token.  Every (token, expert) sum is formed exactly as
-// in router_logits_block: lane l adds columns l, l + 32, ... in order, then the same butterfly.
+// Batches: a block scores EPW experts per warp for eight tokens at a time from a shared-memory tile of x, so a router row is
+// read once per eight tokens and an element of x once per EPW experts.  Every (token, expert) sum is formed exactly as in
+// router_logits_block: lane l adds columns l, l + 32, ... in order, then the same butterfly.  Bound: issue slots (a multiply
+// and an addition per product) from four experts per warp on, shared-memory reads below; the next tile of x is fetched
+// while this one is used.  256 tokens, 512 experts, hidden 2560, us, one expert per warp and four: fp32 77 / 49, bf16
+// (element by element before) 179 / 49.
 constexpr int kLogitTokens = 8, kLogitCols = 512;
+template <int EPW>
 __global__ void __launch_bounds__(256) moe_router_logits_tiled_kernel(const float* __restrict__ Wr, const void* __restrict__ x,
                                                                       int io_dtype, int n_tokens, int H, int E,
                                                                       float* __restrict__ logits, int e_begin, int e_end,
                                                                       const __grid_constant__ PeerLink link) {
     __shared__ __align__(16) float xs[kLogitTokens][kLogitCols];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int e = e_begin + blockIdx.x * 8 + warp, t0 = blockIdx.y * kLogitTokens;
-    const bool live = e < e_end;
-    const float* w = Wr + (size_t)(live ? e : e_begin) * H;
-    const size_t esz = io_dtype == OJX_BF16 ? 2 : 4;
-    float acc[kLogitTokens];
+    const int e0 = e_begin + (blockIdx.x * 8 + warp) * EPW, t0 = blockIdx.y * kLogitTokens;
+    const bool live = e0 < e_end;
+    const float* w[EPW];
 #pragma unroll
-    for (int tt = 0; tt < kLogitTokens; ++tt) acc[tt] = 0.0f;
+    for (int k = 0; k < EPW; ++k) w[k] = Wr + (size_t)min(e0 + k, e_end - 1) * H;
+    const bool bf16 = io_dtype == OJX_BF16;
+    const size_t esz = bf16 ? 2 : 4;
+    float acc[EPW][kLogitTokens];
+#pragma unroll
+    for (int k = 0; k < EPW; ++k)
+#pragma unroll
+        for (int tt = 0; tt < kLogitTokens; ++tt) acc[k][tt] = 0.0f;
+    // tiles as 16-byte pieces: four of fp32, two of bf16 per thread
+    const bool pieces = (H & 7) == 0 && (reinterpret_cast<uintptr_t>(x) & 15) == 0;
+    uint4 next[4];
+    auto fetch = [&](int c0) {
+        const int per = bf16 ? kLogitCols / 8 : kLogitCols / 4, width = bf16 ? 8 : 4;
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+            const int i = threadIdx.x + u * 256, tt = i / per, j = (i - tt * per) * width, t = t0 + tt;
+            next[u] = make_uint4(0u, 0u, 0u, 0u);
+            if (tt < kLogitTokens && t < n_tokens && c0 + j < H)
+                next[u] = *reinterpret_cast<const uint4*>(static_cast<const char*>(x) + ((size_t)t * H + c0 + j) * esz);
+        }
+    };
+    auto place = [&]() {
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+            const int i = threadIdx.x + u * 256;
+            const uint32_t v[4] = {next[u].x, next[u].y, next[u].z, next[u].w};
+            if (!bf16) reinterpret_cast<uint4*>(&xs[0][0])[i] = next[u];
+            else if (u < 2) {
+                float4* at = reinterpret_cast<float4*>(&xs[0][0]) + 2 * i;
+                at[0] = make_float4(__uint_as_float(v[0] << 16), __uint_as_float(v[0] & 0xffff0000u), __uint_as_float(v[1] << 16), __uint_as_float(v[1] & 0xffff0000u));
+                at[1] = make_float4(__uint_as_float(v[2] << 16), __uint_as_float(v[2] & 0xffff0000u), __uint_as_float(v[3] << 16), __uint_as_float(v[3] & 0xffff0000u));
+            }
+        }
+    };
+    if (pieces) fetch(0);
     for (int c0 = 0; c0 < H; c0 += kLogitCols) {
         const int nc = min(kLogitCols, H - c0);
         __syncthreads();   // the previous tile has been read
-        if (io_dtype == OJX_F32 && (H & 3) == 0 && (reinterpret_cast<uintptr_t>(x) & 15) == 0) {   // 16-byte pieces
-            const float* xf = static_cast<const float*>(x);
-            for (int i = threadIdx.x; i < kLogitTokens * kLogitCols / 4; i += 256) {
-                const int tt = i / (kLogitCols / 4), j = (i - tt * (kLogitCols / 4)) * 4, t = t0 + tt;
-                float4 v = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-                if (t < n_tokens && j < nc) v = *reinterpret_cast<const float4*>(xf + (size_t)t * H + c0 + j);
-                *reinterpret_cast<float4*>(&xs[tt][j]) = v;
-            }
-        } else {
+        if (pieces) place();
+        else {
             for (int i = threadIdx.x; i < kLogitTokens * kLogitCols; i += 256) {
                 const int tt = i / kLogitCols, j = i - tt * kLogitCols, t = t0 + tt;
                 float v = 0.0f;
@@ -549,31 +578,40 @@ __global__ void __launch_bounds__(256) moe_router_logits_tiled_kernel(const floa
             }
         }
         __syncthreads();
+        if (pieces && c0 + kLogitCols < H) fetch(c0 + kLogitCols);
         if (live) {
             int cc = lane;
-            for (; cc + 3 * 32 < nc; cc += 4 * 32) {   // four router weights in flight, additions still in column order
-                float wv[4];
-#pragma unroll
-                for (int u = 0; u < 4; ++u) wv[u] = __ldg(w + c0 + cc + 32 * u);
+            for (; cc + 3 * 32 < nc; cc += 4 * 32) {   // four weights of every expert in flight, additions still in column order
+                float wv[EPW][4];
 #pragma unroll
                 for (int u = 0; u < 4; ++u)
 #pragma unroll
-                    for (int tt = 0; tt < kLogitTokens; ++tt) acc[tt] = __fadd_rn(acc[tt], __fmul_rn(wv[u], xs[tt][cc + 32 * u]));
-            }
-            for (; cc < nc; cc += 32) {
-                const float wv = __ldg(w + c0 + cc);
+                    for (int k = 0; k < EPW; ++k) wv[k][u] = __ldg(w[k] + c0 + cc + 32 * u);
 #pragma unroll
-                for (int tt = 0; tt < kLogitTokens; ++tt) acc[tt] = __fadd_rn(acc[tt], __fmul_rn(wv, xs[tt][cc]));
+                for (int u = 0; u < 4; ++u)
+#pragma unroll
+                    for (int tt = 0; tt < kLogitTokens; ++tt) {
+                        const float xv = xs[tt][cc + 32 * u];
+#pragma unroll
+                        for (int k = 0; k < EPW; ++k) acc[k][tt] = __fadd_rn(acc[k][tt], __fmul_rn(wv[k][u], xv));
+                    }
             }
+            for (; cc < nc; cc += 32)
+#pragma unroll
+                for (int tt = 0; tt < kLogitTokens; ++tt)
+#pragma unroll
+                    for (int k = 0; k < EPW; ++k) acc[k][tt] = __fadd_rn(acc[k][tt], __fmul_rn(__ldg(w[k] + c0 + cc), xs[tt][cc]));
         }
     }
 #pragma unroll
-    for (int tt = 0; tt < kLogitTokens; ++tt) {
-        float part = acc[tt];
+    for (int k = 0; k < EPW; ++k)
 #pragma unroll
-        for (int off = 16; off >= 1; off >>= 1) part = __fadd_rn(part, __shfl_xor_sync(0xffffffffu, part, off));
-        if (live && lane == 0 && t0 + tt < n_tokens) peer_store(link, logits + (size_t)(t0 + tt) * E + e, part);
-    }
+        for (int tt = 0; tt < kLogitTokens; ++tt) {
+            float part = acc[k][tt];
+#pragma unroll
+            for (int off = 16; off >= 1; off >>= 1) part = __fadd_rn(part, __shfl_xor_sync(0xffffffffu, part, off));
+            if (e0 + k < e_end && lane == 0 && t0 + tt < n_tokens) peer_store(link, logits + (size_t)(t0 + tt) * E + e0 + k, part);
+        }
     peer_signal_when_last(link, gridDim.x * gridDim.y);
 }
 
@@ -1021,8 +1059,12 @@ int launch_moe_router(const float* Wr, const void* x, int io_dtype, int n_tokens
             default: return OJX_ERR_UNSUPPORTED;
         }
     } else if (n_tokens >= kLogitTokens) {
-        moe_router_logits_tiled_kernel<<<dim3(lx, (n_tokens + kLogitTokens - 1) / kLogitTokens), 256, 0, s>>>(Wr, x, io_dtype, n_tokens, H, E, logits,
-                                                                                                          e_begin, e_end, link);
+        // most experts per warp that still leave a block for every SM
+        const int ty = (n_tokens + kLogitTokens - 1) / kLogitTokens, sms = num_sms();
+        const dim3 g4((ne + 31) / 32, ty), g2((ne + 15) / 16, ty), g1(lx, ty);
+        if ((int)(g4.x * g4.y) >= sms) moe_router_logits_tiled_kernel<4><<<g4, 256, 0, s>>>(Wr, x, io_dtype, n_tokens, H, E, logits, e_begin, e_end, link);
+        else if ((int)(g2.x * g2.y) >= sms) moe_router_logits_tiled_kernel<2><<<g2, 256, 0, s>>>(Wr, x, io_dtype, n_tokens, H, E, logits, e_begin, e_end, link);
+        else moe_router_logits_tiled_kernel<1><<<g1, 256, 0, s>>>(Wr, x, io_dtype, n_tokens, H, E, logits, e_begin, e_end, link);
     } else {
         moe_router_logits_kernel<<<dim3(lx, ly), 256, 0, s>>>(Wr, x, io_dtype, n_tokens, H, E, logits, e_begin, e_end, link);
     }
