@@ -21,35 +21,44 @@ __device__ __forceinline__ void st_io(void* p, size_t i, int dt, float v) {
 // (the residual add that precedes the norm), with the sum also written back to x.  A thread keeps its
 // elements in registers between the two passes (up to kNormKeep of them; rows longer than
 // 256 * kNormKeep re-read the rest), and the row sum is a shuffle tree per warp plus one exchange.
+// Latency-bound (one row of a decode step): every load of the row is issued before the first is used, 5.0 -> 3.0 us
+// at one row of 2560, 7.7 -> 4.6 at 32.
 constexpr int kNormKeep = 16;
 
+template <bool kBf16>
 __global__ void __launch_bounds__(256) rmsnorm_kernel(void* __restrict__ x, const void* __restrict__ add,
-                                                      const float* __restrict__ w, void* __restrict__ out, int H, float eps,
-                                                      int io_dtype) {
+                                                      const float* __restrict__ w, void* __restrict__ out, int H, float eps) {
+    constexpr int dt = kBf16 ? OJX_BF16 : OJX_F32;
     __shared__ float red[8];
     const size_t base = (size_t)blockIdx.x * H;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    float keep[kNormKeep];
+    float keep[kNormKeep], more[kNormKeep], wk[kNormKeep];
     float ss = 0.0f;
-    auto element = [&](int i) {   // the (updated) value of x[r, i] as it is stored, i.e. rounded to the io dtype
-        float v = ld_io(x, base + i, io_dtype);
-        if (add) {
-            v += ld_io(add, base + i, io_dtype);
-            if (io_dtype == OJX_BF16) v = __bfloat162float(__float2bfloat16_rn(v));
-            st_io(x, base + i, io_dtype, v);
-        }
-        return v;
-    };
-    float wk[kNormKeep];   // the weights do not depend on the row sum: asked for now, used after it
+    const bool adds = add != nullptr;
 #pragma unroll
     for (int u = 0; u < kNormKeep; ++u) {
         const int i = tid + u * 256;
-        keep[u] = i < H ? element(i) : 0.0f;
+        keep[u] = i < H ? ld_io(x, base + i, dt) : 0.0f;
+        more[u] = adds && i < H ? ld_io(add, base + i, dt) : 0.0f;
         wk[u] = i < H ? w[i] : 0.0f;
+    }
+    // the (updated) value of x[r, i] as it is stored, i.e. rounded to the io dtype
+    auto rounded = [](float v) { return kBf16 ? __bfloat162float(__float2bfloat16_rn(v)) : v; };
+#pragma unroll
+    for (int u = 0; u < kNormKeep; ++u) {
+        const int i = tid + u * 256;
+        if (adds && i < H) {
+            keep[u] = rounded(keep[u] + more[u]);
+            st_io(x, base + i, dt, keep[u]);
+        }
         ss += keep[u] * keep[u];
     }
     for (int i = tid + kNormKeep * 256; i < H; i += 256) {
-        const float v = element(i);
+        float v = ld_io(x, base + i, dt);
+        if (adds) {
+            v = rounded(v + ld_io(add, base + i, dt));
+            st_io(x, base + i, dt, v);
+        }
         ss += v * v;
     }
 #pragma unroll
@@ -63,9 +72,9 @@ __global__ void __launch_bounds__(256) rmsnorm_kernel(void* __restrict__ x, cons
 #pragma unroll
     for (int u = 0; u < kNormKeep; ++u) {
         const int i = tid + u * 256;
-        if (i < H) st_io(out, base + i, io_dtype, keep[u] * inv * wk[u]);
+        if (i < H) st_io(out, base + i, dt, keep[u] * inv * wk[u]);
     }
-    for (int i = tid + kNormKeep * 256; i < H; i += 256) st_io(out, base + i, io_dtype, ld_io(x, base + i, io_dtype) * inv * w[i]);
+    for (int i = tid + kNormKeep * 256; i < H; i += 256) st_io(out, base + i, dt, ld_io(x, base + i, dt) * inv * w[i]);
 }
 
 // Rotate-half rotary embedding in place on q [B, Hq, hd] and k [B, Hkv, hd] at positions pos[b].
@@ -102,7 +111,9 @@ int ojasx_b200_rmsnorm(void* d_x, const void* d_add, const float* d_weight, void
                        int io_dtype, void* stream) {
     if (!d_x || !d_weight || !d_out || rows <= 0 || hidden <= 0) return OJX_ERR_ARG;
     if (io_dtype != OJX_F32 && io_dtype != OJX_BF16) return OJX_ERR_ARG;
-    rmsnorm_kernel<<<rows, 256, 0, static_cast<cudaStream_t>(stream)>>>(d_x, d_add, d_weight, d_out, hidden, eps, io_dtype);
+    const cudaStream_t s = static_cast<cudaStream_t>(stream);
+    if (io_dtype == OJX_BF16) rmsnorm_kernel<true><<<rows, 256, 0, s>>>(d_x, d_add, d_weight, d_out, hidden, eps);
+    else rmsnorm_kernel<false><<<rows, 256, 0, s>>>(d_x, d_add, d_weight, d_out, hidden, eps);
     OJX_CUDA_TRY(cudaGetLastError());
     count_launch(1);
     return OJX_OK;
