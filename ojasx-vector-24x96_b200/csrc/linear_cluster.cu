@@ -305,7 +305,11 @@ static bool plan_cluster_group(const LinearProblem* Ps, int count, ClusterPlan* 
     if (P0.D != 4 && P0.D != 8 && P0.D != 16 && P0.D != 32) return false;
     // Measured on B200 (2560->6912): 12.5 us against 22.7 us for the persistent kernel at batch 1,
     // but 33 us against 24.7 us at batch 4, where the persistent kernel's larger tiles win.
-    if (P0.batch > 2 || rows_total * P0.batch > 32768) return false;
+    // A single problem's time goes with its rows here and hardly at all there (each CTA's table dominates); the lines cross
+    // near 12 k rows x vectors whatever the width.  us, this kernel / the persistent one: 2560 columns 8192 rows 15.6 / 21.5,
+    // 12000 22.7 / 21.8, 32768 39.0 / 23.5; 6912 columns 8192 45.2 / 49.2, 16384 75.7 / 50.5; 1024 columns 12000 10.6 / 11.6,
+    // 32768 22.4 / 12.5; two vectors, 4096 columns: 4096 rows 26.5 / 31.2, 8192 37.6 / 32.0.
+    if (P0.batch > 2 || rows_total * P0.batch > (count == 1 ? 12288 : 32768)) return false;
     const int TC = P0.G / 16, sms = num_sms();
     double best = 1e30;
     bool found = false;
