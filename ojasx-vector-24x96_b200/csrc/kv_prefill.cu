@@ -98,7 +98,10 @@ __global__ void kvq_advance_kernel(int* seq_lens, int B, int n, int max_seq) {
 // fp32 accuracy from fp16 products: every operand is scaled by a power of two (per query row, per
 // codebook, 2^14 for probabilities) so that its largest element is in [2^13, 2^15), and split
 // into x = hi + lo with two fp16 numbers: 22 bits of mantissa down to 2^-24 of the largest element.
-// hi*hi + hi*lo + lo*hi are accumulated in fp32 (the dropped lo*lo is below 2^-22 of hi*hi).
+// hi*hi + hi*lo + lo*hi are accumulated in fp32 (the dropped lo*lo is below 2^-22 of hi*hi), in runs short
+// enough that the tensor cores' truncation does not show (error against 64 bits with 1000 positions behind
+// 4000 tokens: 1.7e-7; 3.7e-7 with whole tiles accumulated there; 1.1e-7 position by position).  78 us per
+// layer of 512 positions with 32 query heads (70 with the long runs).
 //
 // Why mma.sync: three products of at most a few GFLOP per chunk and layer are a few microseconds
 // at any tensor rate; what the kernel needs is probabilities that go from the accumulators of the
@@ -416,9 +419,10 @@ static int launch_prefill_d(const KvqProblem& P, cudaStream_t s) {
     }
 }
 
+// High and low parts of an infinity are NaN, so codebooks with one keep the decode kernel.
 bool kvq_prefill_supported(const KvqProblem& P) {
     const int R = P.Hq / P.Hkv;
-    return R <= kPfRows && kPfRows % R == 0 && P.G % 4 == 0 && P.B <= 65535 && P.Hkv <= 65535 &&
+    return P.finite_books && R <= kPfRows && kPfRows % R == 0 && P.G % 4 == 0 && P.B <= 65535 && P.Hkv <= 65535 &&
            (P.head_dim == 64 || P.head_dim == 128) && (P.D == 4 || P.D == 8 || P.D == 16);
 }
 

@@ -105,3 +105,17 @@ def test_codebooks_with_infinities_keep_the_table_kernel(cuda, monkeypatch):
         assert np.array_equal(got, cache.decode(q).cpu().numpy(), equal_nan=True)
         monkeypatch.delenv("OJASX_B200_KV_DECODE")
         assert np.isfinite(got).all() == (c is codes)
+
+
+def test_prefill_of_a_cache_with_infinite_centroids_equals_position_by_position(cuda):
+    rng = np.random.default_rng(3)
+    books = [(rng.standard_normal((1, 256, 8)) * 0.1).astype(np.float32) for _ in range(2)]
+    books[0][0, 9, 1] = np.inf
+    k, v = (torch.from_numpy(rng.standard_normal((20, 1, 1, 64)).astype(np.float32) * 0.1).to(cuda) for _ in range(2))
+    q = torch.from_numpy(rng.standard_normal((20, 1, 4, 64)).astype(np.float32)).to(cuda)
+    chunk, one = (ops.VQKVCache(1, 1, 4, 64, 8, 32, *books) for _ in range(2))
+    got = chunk.prefill(k, v, q)
+    for s in range(20):
+        one.append(k[s], v[s])
+        want = one.decode(q[s])
+        assert torch.allclose(got[s], want, rtol=1e-5, atol=1e-6, equal_nan=True)
