@@ -27,7 +27,8 @@ def _dtype_code(t: torch.Tensor) -> int:
 
 
 def _stream_ptr(device) -> int:
-    return torch.cuda.current_stream(device).cuda_stream
+    """The current stream of a tensor's device (the raw handle: a Stream object costs as much as the launch it is for)."""
+    return torch._C._cuda_getCurrentRawStream(device.index)
 
 
 def _require_cuda(t: torch.Tensor, name: str) -> None:
