@@ -6,10 +6,10 @@
 //
 // The table kernels spend one shared-memory gather and one addition per code and vector.  Here a code costs 32 bytes of
 // shared-memory reads whatever the batch.  SwiGLU block of widths 2560 and 6912, us, before and now: batch 1 55 -> 37, 16
-// 139 -> 50 (before the rule of gm_plan was fitted: 2 91 -> 43, 8 117 -> 49, 31 195 -> 117).  What is left is latency: launches, building the table, the
-// outliers' gathers and the ordered sums; clocks of a CTA at 2560 to 6912 columns and batch 16: 4.4 k before the
-// activations are there, 8.2 k for the products (a third of the shared-memory rate), 6.2 k for partial sums and outliers,
-// 6.0 k for the sums evaluated again.
+// 139 -> 50 (before the rule of gm_plan was fitted: 2 91 -> 43, 8 117 -> 49, 31 195 -> 117).  What is left is latency:
+// launches, building the table, the outliers' gathers and the ordered sums; clocks of a CTA at 2560 to 6912 columns and
+// batch 16: 4.4 k before the activations are there, 8.2 k for the products (a third of the shared-memory rate), 6.2 k for
+// partial sums and outliers, 6.0 k for the sums evaluated again.
 #include <algorithm>
 #include <atomic>
 
