@@ -206,6 +206,7 @@ __global__ void __launch_bounds__(kGmMaxWarps * 32, 2) gm_linear_kernel(const __
             for (int v = 1; v < live; ++v) s += part[(size_t)v * kRows * kLd + at];
             part[at] = s;
         }
+        __syncwarp();   // the barrier is an aligned one
         asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
     }
     // Sums too close to a rounding boundary of bf16 to decide: listed in the dead table, evaluated in order below.

@@ -118,8 +118,10 @@ __device__ __forceinline__ void gm_load_codes(uint32_t (&w)[4], const uint8_t* r
 // of the lane's copy ((lane & 7) * 16 from the table's start).
 // kFlush: steps whose products are accumulated in the tensor cores before they are added to acc in fp32 (the tensor
 // cores truncate, so a chain's error grows with its length); 16: all of them.
+// The lanes meet first: ldmatrix and mma need all 32 of them converged, and callers come from loops of per-lane length.
 template <int MT, int NT, int kFlush, class Load>
 __device__ __forceinline__ void gm_chunk(float (&acc)[MT][NT][4], const uint32_t (&w)[MT][4], int steps, uint32_t table, Load load) {
+    __syncwarp();
     uint4 b[NT], bn[NT];
 #pragma unroll
     for (int n = 0; n < NT; ++n) bn[n] = load(0, n);

@@ -184,6 +184,7 @@ __global__ void __launch_bounds__(kKdThreads, 1) kvq_decode_mma_kernel(const __g
             for (int e = 0; e < 4; ++e) o[i][e] = 0.0f;
 
         for (; t0 < t_end; t0 += kKdWarps * 16) {
+            __syncwarp();   // ldmatrix, mma and movmatrix need the warp converged
             uint32_t kw[W], vw[W];
 #pragma unroll
             for (int i = 0; i < W; ++i) {

@@ -275,6 +275,7 @@ __global__ void __launch_bounds__(kPfThreads) kvq_prefill_kernel(const __grid_co
         }
         __syncthreads();
         if (t0 + kPfTok < t_all) fetch(t0 + kPfTok);
+        __syncwarp();   // a lane's fetch depends on its tokens; ldmatrix and mma need the warp converged
 
         // Chains in the tensor cores stay short (the products of two 16-wide steps here, of one below): they truncate,
         // so that the error of a long chain grows with its length.

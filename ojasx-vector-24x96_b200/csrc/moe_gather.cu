@@ -350,6 +350,7 @@ __global__ void __launch_bounds__(kMgUpThreads, 1) moe_gather_up_kernel(const __
         for (int u = units * S.part / kMgParts + warp; u < u1; u += warps) {
             if (S.count <= 8) mg_up_unit<1>(A, S, cols, ld, table, inv_cb, u);
             else mg_up_unit<2>(A, S, cols, ld, table, inv_cb, u);
+            __syncwarp();   // lanes without a pair have left the unit early
         }
     }
 }
@@ -411,6 +412,7 @@ __global__ void __launch_bounds__(kMgDownThreads, 2) moe_gather_down_kernel(cons
         for (int u = units * S.part / kMgParts + warp; u < u1; u += warps) {
             if (S.count <= 4) mg_down_unit<1>(A, S, cols, ld, table, inv_cb, u, link);
             else mg_down_unit<2>(A, S, cols, ld, table, inv_cb, u, link);
+            __syncwarp();
         }
     }
     peer_signal_when_last(link, gridDim.x);

@@ -86,3 +86,29 @@ def test_gather_experts_routed_call_and_non_finite_tokens(cuda, monkeypatch):
     bad[[2, 9, 20]] = True
     assert torch.equal(got[~bad], clean[~bad])
     assert torch.equal(torch.isnan(got[bad]), torch.isnan(table[bad])) and torch.equal(torch.isposinf(got[bad]), torch.isposinf(table[bad]))
+
+
+@pytest.mark.parametrize("B", [1, 3, 5, 13])
+def test_gather_experts_with_outliers_in_few_rows(cuda, oracle, B):
+    """Lanes without a pair leave a unit early and lanes with a long outlier row leave it late; the warp meets again before
+    the next unit's products.  Few pairs per expert and hundreds of entries in every sixteenth row, several units per warp."""
+    H, I, E, k = 1024, 640, 4, 2
+    w = synth.make_vq_moe(B, E, H, I, block_dim=8, outlier_frac=0.0, unit_scales=False)
+    rng = np.random.default_rng(B)
+
+    def long_rows(rows, cols):
+        counts = np.where(np.arange(rows) % 16 == 5, 300, 0)
+        ptr = np.concatenate([[0], np.cumsum(counts)]).astype(np.int32)
+        col = np.concatenate([np.sort(rng.choice(cols, 300, replace=False)) for _ in range(np.count_nonzero(counts))])
+        return ptr, col.astype(np.int32), (rng.standard_normal(len(col)) * 0.1).astype(np.float32)
+
+    w.gate_up_csr, w.down_csr = long_rows(E * 2 * I, H), long_rows(E * H, I)
+    x = synth.to_bf16_f32(rng.standard_normal((B, H)).astype(np.float32))
+    idx = np.stack([rng.choice(E, size=k, replace=False) for _ in range(B)]).astype(np.int32)
+    wts = rng.uniform(0.1, 0.3, size=(B, k)).astype(np.float32)
+    moe = ops.VQMoE(w)
+    n0 = ojasx_b200.launch_count()
+    got = moe.forward(*_args(x, idx, wts)).float().cpu().numpy()
+    assert ojasx_b200.launch_count() - n0 == 6
+    want = _oracle_moe(oracle, w, x, idx, wts)
+    assert np.all(np.abs(got - want) <= ATOL + RTOL * np.abs(want)), np.abs(got - want).max()
