@@ -327,9 +327,9 @@ __global__ void __launch_bounds__(kGmMaxWarps * 32, 2) gm_linear_kernel(const __
                 if (at[u] >= 0) fix_buf[at[u]] = gm_entry(xv[u], P.codebook, code[u], P.Kcb);
         }
         __syncthreads();
-        if (tid < n) {
-            const uint2 l = list[i0 + tid];
-            const float4* v = reinterpret_cast<const float4*>(fix_buf + tid * ld);
+        for (int e = tid; e < n; e += blockDim.x) {   // narrow layers: a pass holds more sums than the CTA has threads
+            const uint2 l = list[i0 + e];
+            const float4* v = reinterpret_cast<const float4*>(fix_buf + e * ld);
             float acc = 0.0f;
 #pragma unroll 4
             for (int i = 0; i < P.G / 4; ++i) {   // G is a multiple of 8

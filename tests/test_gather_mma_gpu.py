@@ -82,3 +82,26 @@ def test_mlp_block_equals_its_layers(cuda, K, M, batch):
     want = down(ops.silu_mul(gate(x), up(x)))
     # a gate or up value whose rounding tips moves one of M terms of an output by 2^-8 of itself
     assert torch.allclose(got.float(), want.float(), rtol=2 ** -7, atol=2 ** -8 * want.float().abs().max().item() / 8)
+
+
+def _table(monkeypatch, layer, x):
+    monkeypatch.setenv("OJASX_B200_GATHER_MIN_WORK", "-1")
+    y = layer(x).float().cpu().numpy()
+    monkeypatch.setenv("OJASX_B200_GATHER_MIN_WORK", "0")
+    return y
+
+
+@pytest.mark.parametrize("K,M", [(64, 300), (64, 20000), (256, 300), (256, 9000), (384, 300), (384, 9000)])
+@pytest.mark.parametrize("batch", [16, 31])
+@pytest.mark.parametrize("fill", [0.0, float("nan")])
+def test_every_listed_sum_is_stored(cuda, monkeypatch, K, M, batch, fill):
+    """Narrow layers: more sums of a tile are evaluated again than the CTA has threads (all but one vector zero or NaN)."""
+    monkeypatch.setenv("OJASX_B200_GATHER_MIN_WORK", "0")
+    layer = ops.VQLinear.from_weights(synth.make_vq_linear(K, K, M, block_dim=8, outlier_frac=0.0))
+    x = torch.full((batch, K), fill, device=cuda, dtype=torch.bfloat16)
+    x[3] = torch.randn(K, device=cuda, generator=torch.Generator(cuda).manual_seed(K)).bfloat16()
+    out = torch.full((batch, M), 12345.0, device=cuda, dtype=torch.bfloat16)
+    n0 = ojasx_b200.launch_count()
+    layer(x, out=out)
+    assert ojasx_b200.launch_count() - n0 == 2
+    assert np.array_equal(out.float().cpu().numpy(), _table(monkeypatch, layer, x), equal_nan=True)
