@@ -33,7 +33,7 @@ struct GmArgs {
     LinearProblem P[kGmProblems];
     int tiles0;                     // row tiles of problem 0
     const uint4* frag;
-    const float* inv;               // [chunks][bp] inverse scale, NaN where a vector has an infinity or NaN in the chunk
+    const float* inv;               // [chunks][bp] inverse scale: 0 where a vector's chunk is all zeros, NaN where it has an infinity or NaN
     const __nv_bfloat16* xT;        // [chunks * 256][bp]
     int chunks, per_split;
     float tol;                      // kGmTolerance
@@ -74,7 +74,9 @@ __global__ void __launch_bounds__(256) gm_prep_kernel(const __nv_bfloat16* __res
         m = __reduce_max_sync(0xffffffffu, m);
         float scale, inv;
         gm_scale(m, scale, inv);
-        if (lane == 0) inv_out[c * bp + t] = m >= 0x7f800000u ? __uint_as_float(0x7fc00000u) : inv;
+        // 0 for zeros: the chunk adds nothing to a sum, so nothing to the bound on its error either (with gm_scale's 1 a padded
+        // vector's sums were all evaluated again: 154 us against 35 with 8 zero vectors of 16, 2560 to 6912 columns)
+        if (lane == 0) inv_out[c * bp + t] = m == 0u ? 0.0f : m >= 0x7f800000u ? __uint_as_float(0x7fc00000u) : inv;
         *reinterpret_cast<uint4*>(&tile[t][lane * 8]) = make_uint4(v[0], v[1], v[2], v[3]);
         // lane = group of the chunk: step lane & 15, half lane >> 4
         uint32_t* at = reinterpret_cast<uint32_t*>(frag + ((size_t)(c * 8 + ((lane & 15) >> 1)) * bp + t) * 4) + (lane & 1) * 2 + (lane >> 4);

@@ -105,3 +105,35 @@ def test_every_listed_sum_is_stored(cuda, monkeypatch, K, M, batch, fill):
     layer(x, out=out)
     assert ojasx_b200.launch_count() - n0 == 2
     assert np.array_equal(out.float().cpu().numpy(), _table(monkeypatch, layer, x), equal_nan=True)
+
+
+def _us(f, n=20):
+    for _ in range(3):
+        f()
+    a, b = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+    times = []
+    for _ in range(n):
+        torch.cuda.synchronize()
+        a.record()
+        f()
+        b.record()
+        b.synchronize()
+        times.append(a.elapsed_time(b) * 1e3)
+    return sorted(times)[n // 2]
+
+
+def test_zero_vectors_and_zero_chunks_cost_nothing_extra(cuda, monkeypatch):
+    """An all-zero chunk of 256 dimensions adds nothing to a sum, so it must not widen the window in which sums are evaluated
+    again.  The bits are the table kernels'; the time is that of dense vectors (a tenth of all sums evaluated again doubles it)."""
+    monkeypatch.setenv("OJASX_B200_GATHER_MIN_WORK", "0")
+    K, M, batch = 2560, 6912, 16
+    layer = ops.VQLinear.from_weights(synth.make_vq_linear(1, K, M, block_dim=8))
+    x = torch.randn(batch, K, device=cuda, generator=torch.Generator(cuda).manual_seed(1)).bfloat16()
+    padded, chunk = x.clone(), x.clone()
+    padded[8:] = 0
+    chunk[:, 512:768] = 0
+    dense = _us(lambda: layer(x))
+    for v in (padded, chunk):
+        took = _us(lambda: layer(v))
+        assert np.array_equal(layer(v).float().cpu().numpy(), _table(monkeypatch, layer, v))
+        assert took < 1.3 * dense, (took, dense)
