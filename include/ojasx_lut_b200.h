@@ -233,8 +233,9 @@ OJASX_API int ojasx_b200_moe_forward_noalloc(OjasxMoEHandle handle, const void* 
                                              const float* d_topk_w, void* d_y, int n_tokens, int k_active,
                                              int io_dtype, void* stream);
 
-/* ojasx_b200_linear_forward with scratch of the caller: bf16 batches up to 31 may then run on the tensor cores, with
- * the table kernels' result.  ojasx_b200_linear_workspace says how many bytes such a call takes, 16-byte aligned (0: the
+/* ojasx_b200_linear_forward with scratch of the caller: bf16 batches up to 31 may then run on the tensor cores.  The result is
+ * an fp32 sum rounded once to bf16; sums near a rounding boundary are formed in the table kernels' order, so that the bits are
+ * theirs (no difference seen; not proven for every input).  ojasx_b200_linear_workspace says how many bytes such a call takes, 16-byte aligned (0: the
  * call would not use any); calls that overlap in time need scratch of their own. */
 OJASX_API size_t ojasx_b200_linear_workspace(OjasxLinearHandle handle, int batch_size, int io_dtype);
 OJASX_API int ojasx_b200_linear_forward_ws(OjasxLinearHandle handle, const void* d_x, void* d_y, int batch_size,

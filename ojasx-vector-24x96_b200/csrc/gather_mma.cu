@@ -2,14 +2,14 @@
 // weight tiles gathered from the codebook straight into mma.sync operands (gather_mma.cuh).  The result is the table
 // kernels': the reference's fp32 row sum, rounded once to bf16.  A sum formed in another order differs from the
 // reference's by a few 1e-7 and rounds the same unless it lies next to a rounding boundary; those (one in a hundred) are
-// listed and evaluated again in the reference's order.
+// listed and evaluated again in the reference's order.  What counts as next to it is kGmTolerance's comment.
 //
 // The table kernels spend one shared-memory gather and one addition per code and vector.  Here a code costs 32 bytes of
-// shared-memory reads whatever the batch.  SwiGLU block of widths 2560 and 6912, us, before and now: batch 1 55 -> 37, 16
-// 139 -> 50 (before the rule of gm_plan was fitted: 2 91 -> 43, 8 117 -> 49, 31 195 -> 117).  What is left is latency:
-// launches, building the table, the outliers' gathers and the ordered sums; clocks of a CTA at 2560 to 6912 columns and
-// batch 16: 4.4 k before the activations are there, 8.2 k for the products (a third of the shared-memory rate), 6.2 k for
-// partial sums and outliers, 6.0 k for the sums evaluated again.
+// shared-memory reads whatever the batch.  SwiGLU block of widths 2560 and 6912, us, table kernels and these: batch 1
+// 55 / 39, 16 138 / 58.  What is left is latency: launches, building the table, the outliers' gathers and the ordered sums;
+// clocks of a CTA at 2560 to 6912 columns and batch 16, with a window that 0.5 % of the sums fell into: 4.4 k before the
+// activations are there, 8.2 k for the products (a third of the shared-memory rate), 6.2 k for partial sums and outliers,
+// 6.0 k for the sums evaluated again.
 #include <algorithm>
 #include <atomic>
 
@@ -23,10 +23,19 @@ namespace ojx {
 constexpr int kGmMaxBatch = 32;
 constexpr int kGmMaxWarps = 10;     // 320 threads, two CTAs per SM
 constexpr int kGmProblems = 2;
-// Sums within tol * (codebook maximum) * sqrt(sum over chunks of squared activation maxima) of a bf16 rounding boundary
-// are evaluated again in the reference's order.  Maxima are bounds by powers of two scaled by 2^-14 each; against the table
-// kernels 1536 left no difference in 1.2 million outputs, 1024 three, 512 twenty-nine, none of this 360.
-constexpr float kGmTolerance = 1536.0f;
+// A sum is evaluated again in the reference's order if a bf16 rounding boundary lies within a window around it.  What the two
+// may differ by, with v the sum, A the sum of the magnitudes of its pieces (chunks, or what a warp or a CTA of a cluster adds
+// up), eps = 2^-24 and G ordered additions:
+//   eps G / 2 |v|            sums of one sign (A = |v|): partial sums grow to |v|; fades out as A grows to 2 |v|
+//   eps 0.5 sqrt(G) A        sums that cancel: partial sums up to (A + |v|) / 2, independent roundings, four deviations
+//   eps (16 |v| + 4 A)       truncation in the tensor cores, 32 products of a chunk: a common shrinking, and what chunks differ by
+//   kGmTolerance             operands of 22 bits and roundings inside a chunk: times (codebook maximum) * sqrt(sum over chunks
+//                            of squared activation maxima), maxima being powers of two scaled by 2^-14 each
+// Not a bound for every input (that takes eps G A, and more than twice as many sums); measured: none of 48 million outputs of
+// Gaussian, one-signed, constant, cancelling, tiny, large, spiked and ramped activations at widths 64 to 6912 differs.  With a
+// window for Gaussian data alone (1536 and 2 eps |v|) 1 in 10 000 of one-signed and 1 in 400 of cancelling sums did; it
+// took 50 us where this takes 58 (SwiGLU block of 2560 and 6912, 16 vectors).
+constexpr float kGmTolerance = 1024.0f;
 constexpr int kGmEntries = 768;     // outliers of a tile brought in before the activations are ready
 
 struct GmArgs {
@@ -36,7 +45,6 @@ struct GmArgs {
     const float* inv;               // [chunks][bp] inverse scale: 0 where a vector's chunk is all zeros, NaN where it has an infinity or NaN
     const __nv_bfloat16* xT;        // [chunks * 256][bp]
     int chunks, per_split;
-    float tol;                      // kGmTolerance
 };
 
 // ------------------------------------------------------------------------------------ activations
@@ -108,8 +116,9 @@ __device__ __forceinline__ float gm_entry(const uint4& x, const float* cb, int c
 }
 
 // grid (row tiles of all problems, splits), cluster (1, splits).  A CTA owns MT x 16 rows and its split's chunks of 256
-// dimensions; warp w takes chunks w, w + warps, ... of them for all rows, so fragments go from L2 to registers and
-// every warp reads whole sectors of the code rows.  Partial sums of the warps, then of the cluster's CTAs, are added
+// dimensions; every warp takes a run of them for all rows, so fragments go from L2 to registers and every warp reads whole
+// sectors of the code rows (a run and not every warps-th chunk: the magnitude of a run's sum then tells how far the ordered
+// partial sums go up, also where the first and the second half of a row cancel).  Partial sums of the warps, then of the cluster's CTAs, are added
 // in chunk order in shared memory.  The table is built while the activations are still being prepared.
 template <int MT, int NT>
 __global__ void __launch_bounds__(kGmMaxWarps * 32, 2) gm_linear_kernel(const __grid_constant__ GmArgs A) {
@@ -131,9 +140,10 @@ __global__ void __launch_bounds__(kGmMaxWarps * 32, 2) gm_linear_kernel(const __
 #pragma unroll
     for (int m = 0; m < MT; ++m) rows[m] = P.codes + (size_t)min(row0 + m * 16 + (lane & 15), P.row_stop - 1) * P.G;
     uint32_t w[MT][4], wn[MT][4];
-    if (c_begin + warp < c_end) {
+    const int run = (c_end - c_begin + warps - 1) / warps, c_first = c_begin + warp * run, c_last = min(c_end, c_first + run);
+    if (c_first < c_last) {
 #pragma unroll
-        for (int m = 0; m < MT; ++m) gm_load_codes(wn[m], rows[m], c_begin + warp, lane >> 4, P.G, wide);
+        for (int m = 0; m < MT; ++m) gm_load_codes(wn[m], rows[m], c_first, lane >> 4, P.G, wide);
     }
     constexpr int kItems = kRows * NT * 2;     // four vectors of one row each
     // the rows this CTA finishes: all of its tile, or its share of the cluster's
@@ -157,20 +167,23 @@ __global__ void __launch_bounds__(kGmMaxWarps * 32, 2) gm_linear_kernel(const __
     cudaGridDependencySynchronize();   // the prepared activations
 
     if (tid < kVecs) {
-        float m = 0.0f;
-        for (int c = 0; c < A.chunks; ++c) m = fmaf(A.inv[c * kVecs + tid], A.inv[c * kVecs + tid], m);
-        tol_s[tid] = sqrtf(m) * inv_cb * A.tol;
+        float top = 0.0f, m = 0.0f;   // relative to the largest: squares of tiny or huge scales leave the range of fp32
+        for (int c = 0; c < A.chunks; ++c) top = fmaxf(top, A.inv[c * kVecs + tid]);
+        const float r = top > 0.0f ? 1.0f / top : 0.0f;
+        for (int c = 0; c < A.chunks; ++c) m = fmaf(A.inv[c * kVecs + tid] * r, A.inv[c * kVecs + tid] * r, m);
+        const float tol = top * inv_cb * sqrtf(m) * kGmTolerance + (float)P.K * 1.4e-45f;   // products may be subnormal
+        tol_s[tid] = tol < 1e28f ? tol : __uint_as_float(0x7fc00000u);                        // ordered partial sums may overflow
         if (tid == 0) n_fix = 0;
     }
     float* mine = part + (size_t)warp * kRows * kLd;
-    for (int c = c_begin + warp; c < c_end; c += warps) {
+    for (int c = c_first; c < c_last; ++c) {
 #pragma unroll
         for (int m = 0; m < MT; ++m)
 #pragma unroll
             for (int i = 0; i < 4; ++i) w[m][i] = wn[m][i];
-        if (c + warps < c_end) {
+        if (c + 1 < c_last) {
 #pragma unroll
-            for (int m = 0; m < MT; ++m) gm_load_codes(wn[m], rows[m], c + warps, lane >> 4, P.G, wide);
+            for (int m = 0; m < MT; ++m) gm_load_codes(wn[m], rows[m], c + 1, lane >> 4, P.G, wide);
         }
         float2 iv[NT];
 #pragma unroll
@@ -184,7 +197,7 @@ __global__ void __launch_bounds__(kGmMaxWarps * 32, 2) gm_linear_kernel(const __
                 for (int i = 0; i < 4; ++i) acc[m][n][i] = 0.0f;
         const uint4* frag = A.frag + (size_t)c * 8 * kVecs * 4;
         gm_chunk<MT, NT, 16>(acc, w, min(16, P.G - c * kGmChunk), table, [&](int j, int n) { return __ldg(frag + (size_t)j * kVecs * 4 + boff[n]); });
-        const bool first = c == c_begin + warp;
+        const bool first = c == c_first;
 #pragma unroll
         for (int n = 0; n < NT; ++n) {
 #pragma unroll
@@ -199,14 +212,19 @@ __global__ void __launch_bounds__(kGmMaxWarps * 32, 2) gm_linear_kernel(const __
     }
     __syncthreads();
 
-    const int live = min(warps, c_end - c_begin);
+    const int live = (c_end - c_begin + run - 1) / run;   // warps that had a run
     const unsigned part_addr = static_cast<unsigned>(__cvta_generic_to_shared(part));
     if (splits > 1) {   // the CTA's sum replaces its first warp's part, the cluster's CTAs read one another's
         for (int i = tid; i < kItems * 4; i += blockDim.x) {
             const int at = (i % kRows) * kLd + i / kRows;
-            float s = part[at];
-            for (int v = 1; v < live; ++v) s += part[(size_t)v * kRows * kLd + at];
+            float s = part[at], a = fabsf(s);
+            for (int v = 1; v < live; ++v) {
+                const float f = part[(size_t)v * kRows * kLd + at];
+                s += f;
+                a += fabsf(f);
+            }
             part[at] = s;
+            part[kRows * kLd + at] = a;   // magnitudes, in the second warp's place (there are at least eight)
         }
         __syncwarp();   // the barrier is an aligned one
         asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
@@ -215,11 +233,11 @@ __global__ void __launch_bounds__(kGmMaxWarps * 32, 2) gm_linear_kernel(const __
     uint2* list = reinterpret_cast<uint2*>(smem_raw);                              // [kItems * 4] (row << 8 | vector, outlier sum)
     float* fix_buf = reinterpret_cast<float*>(smem_raw + kItems * 4 * sizeof(uint2));   // [sums][G + 4] table entries
     const int rows_out = P.row_stop - P.row_start;
-    auto finish = [&](float v, float out, int m) {
+    auto affine = [&](float v, int m) {
         if (P.scales) v = __fmul_rn(v, P.scales[m]);
-        if (P.bias) v = __fadd_rn(v, P.bias[m]);
-        return P.csr.nnz > 0 ? __fadd_rn(v, out) : v;
+        return P.bias ? __fadd_rn(v, P.bias[m]) : v;
     };
+    const float one_sign = ((float)P.G + 64.0f) * 0x1p-25f, cancel = (0.5f * sqrtf((float)P.G) + 4.0f) * 0x1p-24f;
     // Outliers: the tile's entries are contiguous, so all threads multiply (entry, four vectors) pieces into the dead
     // table, then a thread per (row, four vectors) adds its row's products in entry order.
     float4* prod = reinterpret_cast<float4*>(smem_raw);                            // [entries of a pass][NT * 2]
@@ -274,7 +292,7 @@ __global__ void __launch_bounds__(kGmMaxWarps * 32, 2) gm_linear_kernel(const __
     for (int i = 0; i < kPer; ++i) {
         const int item = tid + i * blockDim.x, r = item % kRows, t0 = item / kRows * 4, m = row0 + r;
         if (item >= kItems || r < r_begin || r >= r_end) continue;
-        float s[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+        float s[4] = {0.0f, 0.0f, 0.0f, 0.0f}, mag[4] = {0.0f, 0.0f, 0.0f, 0.0f};
         if (splits > 1) {
             for (int v = 0; v < splits; ++v) {
                 unsigned base;
@@ -284,20 +302,26 @@ __global__ void __launch_bounds__(kGmMaxWarps * 32, 2) gm_linear_kernel(const __
                     float f;
                     asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(f) : "r"(base + q * 4) : "memory");
                     s[q] += f;
+                    asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(f) : "r"(base + (kRows * kLd + q) * 4) : "memory");
+                    mag[q] += f;
                 }
             }
         } else {
             for (int v = 0; v < live; ++v)
 #pragma unroll
-                for (int q = 0; q < 4; ++q) s[q] += part[(size_t)v * kRows * kLd + r * kLd + t0 + q];
+                for (int q = 0; q < 4; ++q) {
+                    const float f = part[(size_t)v * kRows * kLd + r * kLd + t0 + q];
+                    s[q] += f;
+                    mag[q] += fabsf(f);
+                }
         }
         const float scale = P.scales ? fabsf(P.scales[m]) : 1.0f;
 #pragma unroll
         for (int q = 0; q < 4; ++q) {
             const int t = t0 + q;
             if (t >= P.batch) break;
-            const float v = finish(s[q], o[i][q], m);
-            const float tol = fmaf(scale, tol_s[t], fabsf(v) * 1.2e-7f);
+            const float sa = fabsf(s[q]), w = affine(s[q], m), v = P.csr.nnz > 0 ? __fadd_rn(w, o[i][q]) : w;
+            const float tol = scale * (tol_s[t] + one_sign * fmaxf(2.0f * sa - mag[q], 0.0f) + 0x1p-20f * sa + cancel * mag[q]) + 1.8e-7f * (fabsf(w) + fabsf(v));
             const __nv_bfloat16 a = __float2bfloat16_rn(v - tol), b = __float2bfloat16_rn(v + tol);
             if (a == b) reinterpret_cast<__nv_bfloat16*>(P.y)[(size_t)t * rows_out + (m - P.row_start)] = a;
             else list[atomicAdd(&n_fix, 1)] = make_uint2(r << 8 | t, __float_as_uint(o[i][q]));   // NaN is unequal to itself
@@ -342,8 +366,9 @@ __global__ void __launch_bounds__(kGmMaxWarps * 32, 2) gm_linear_kernel(const __
                 acc = __fadd_rn(acc, f.w);
             }
             const int m = row0 + (int)(l.x >> 8), t = l.x & 255;
-            reinterpret_cast<__nv_bfloat16*>(P.y)[(size_t)t * rows_out + (m - P.row_start)] =
-                __float2bfloat16_rn(finish(acc, __uint_as_float(l.y), m));
+            acc = affine(acc, m);
+            if (P.csr.nnz > 0) acc = __fadd_rn(acc, __uint_as_float(l.y));
+            reinterpret_cast<__nv_bfloat16*>(P.y)[(size_t)t * rows_out + (m - P.row_start)] = __float2bfloat16_rn(acc);
         }
         __syncthreads();
     }
@@ -452,7 +477,6 @@ int launch_gather_mma(const LinearProblem* P, int count, const void* x, const vo
     count_launch(1);
     int MT = 1, splits = 1, warps = kGmMaxWarps;
     gm_plan(P, count, A.chunks, NT, &MT, &splits, &warps);
-    A.tol = kGmTolerance;
     A.per_split = (A.chunks + splits - 1) / splits;
     A.tiles0 = (P[0].row_stop - P[0].row_start + MT * 16 - 1) / (MT * 16);
     const int tiles = A.tiles0 + (count > 1 ? (P[1].row_stop - P[1].row_start + MT * 16 - 1) / (MT * 16) : 0);

@@ -137,3 +137,41 @@ def test_zero_vectors_and_zero_chunks_cost_nothing_extra(cuda, monkeypatch):
         took = _us(lambda: layer(v))
         assert np.array_equal(layer(v).float().cpu().numpy(), _table(monkeypatch, layer, v))
         assert took < 1.3 * dense, (took, dense)
+
+
+def _kinds(rng, batch, K):
+    x = rng.standard_normal((batch, K)).astype(np.float32)
+    yield "gaussian", x, 0.0
+    yield "one sign", np.abs(x), 1.0
+    yield "constant", np.ones((batch, K), np.float32) * rng.uniform(0.5, 2, (batch, 1)).astype(np.float32), 1.0
+    half = np.abs(x)
+    half[:, K // 2:] *= -1
+    yield "halves that cancel", half, 1.0
+    yield "tiny", x * np.float32(2.0 ** -70), 0.0
+    yield "tiny, one sign", np.abs(x) * np.float32(2.0 ** -90), 1.0
+    yield "large", x * np.float32(2.0 ** 90), 0.0
+    massive = x.copy()
+    massive[:, 7] *= 3000
+    yield "one massive dimension", massive, 0.0
+    ramp = x * np.float32(2.0) ** np.linspace(-12, 12, K, dtype=np.float32)
+    yield "chunks of different size", ramp, 0.0
+
+
+@pytest.mark.parametrize("K,M,batch", [(64, 4096, 16), (2560, 4096, 16), (6912, 2560, 8)])
+def test_bits_of_the_table_kernels_for_biased_data(cuda, monkeypatch, K, M, batch):
+    """Sums of one sign, sums that cancel and activations of other scales: the window in which sums are formed in the table
+    kernels' order has to cover what the two orders differ by."""
+    monkeypatch.setenv("OJASX_B200_GATHER_MIN_WORK", "0")
+    bad = {}
+    for seed in range(4):
+        rng = np.random.default_rng(K + seed)
+        for kind, x, bias in _kinds(rng, batch, K):
+            w = synth.make_vq_linear(seed, K, M, block_dim=8, outlier_frac=0.0)
+            if bias:
+                w.codebook[:] = np.abs(w.codebook)
+            layer = ops.VQLinear.from_weights(w)
+            xt = torch.from_numpy(x).to(cuda).bfloat16()
+            got = layer(xt).float().cpu().numpy()
+            n = int(np.count_nonzero(got != _table(monkeypatch, layer, xt)))
+            bad[kind] = bad.get(kind, 0) + n
+    assert not any(bad.values()), bad
