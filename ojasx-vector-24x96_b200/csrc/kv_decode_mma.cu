@@ -250,9 +250,11 @@ __global__ void __launch_bounds__(kKdThreads, 1) kvq_decode_mma_kernel(const __g
                 }
             }
             uint32_t ph[2], pl[2];   // tokens 0..7 and 8..15 of the tile
+            // no score above -inf yet: weights 0, or NaN where the scores are (a query with an infinity or NaN), never exp(-inf + inf)
+            const float base[2] = {m_run[0] == -INFINITY ? 0.0f : m_run[0], m_run[1] == -INFINITY ? 0.0f : m_run[1]};
 #pragma unroll
             for (int e = 0; e < 2; ++e) {
-                const float p0 = exp2f(s[2 * e] - m_run[0]), p1 = exp2f(s[2 * e + 1] - m_run[1]);
+                const float p0 = exp2f(s[2 * e] - base[0]), p1 = exp2f(s[2 * e + 1] - base[1]);
                 l_run[0] += p0;
                 l_run[1] += p1;
                 kd_split2(p0 * 16384.0f, p1 * 16384.0f, ph[e], pl[e]);
@@ -315,7 +317,7 @@ __global__ void __launch_bounds__(kKdThreads, 1) kvq_decode_mma_kernel(const __g
         }
         for (int i = tid; i < (n_run - 1) * R; i += kKdThreads) {   // the run's other chunks are in the first one's sums
             part[(size_t)(R + i) * (HD + 2)] = -INFINITY;
-            part[(size_t)(R + i) * (HD + 2) + 1] = 0.0f;
+            part[(size_t)(R + i) * (HD + 2) + 1] = -1.0f;   // no sum: a run's own is never negative
         }
 
         // the CTA that arrives last merges the runs in order; the counter returns to zero
@@ -341,15 +343,17 @@ __global__ void __launch_bounds__(kKdThreads, 1) kvq_decode_mma_kernel(const __g
                 for (int c0 = 0; c0 < nz; c0 += 32) {
                     const int c = c0 + lane;
                     const float* p = base + ((size_t)c * R + warp) * (HD + 2);
-                    const float m = c < nz ? __ldcg(p) : -INFINITY, l = c < nz ? __ldcg(p + 1) : 0.0f;
-                    const unsigned run = __ballot_sync(0xffffffffu, !(l == 0.0f));
-                    const float f = m == -INFINITY ? 0.0f : exp2f(m - M);
-                    if (!(l == 0.0f)) {
+                    const float m = c < nz ? __ldcg(p) : -INFINITY, l = c < nz ? __ldcg(p + 1) : -1.0f;
+                    const bool own = l != -1.0f;   // NaN is unequal
+                    const unsigned run = __ballot_sync(0xffffffffu, own);
+                    // a run of NaN weights has a maximum of -inf and keeps its NaN
+                    const float f = m == -INFINITY ? (l == 0.0f ? 0.0f : 1.0f) : exp2f(m - M);
+                    if (own) {
                         const int at = n + __popc(run & ((1u << lane) - 1u));
                         wgt[warp * nz + at] = f;
                         if (warp == 0) slot[at] = c;
+                        L = fmaf(l, f, L);
                     }
-                    L = fmaf(l, f, L);
                     n += __popc(run);
                 }
 #pragma unroll
@@ -370,7 +374,7 @@ __global__ void __launch_bounds__(kKdThreads, 1) kvq_decode_mma_kernel(const __g
                     acc = f != 0.0f ? fmaf(v, f, acc) : acc;
                 }
                 const float L = l_s[0][r];
-                acc *= L > 0.0f ? 1.0f / L : 0.0f;
+                acc *= L == 0.0f ? 0.0f : 1.0f / L;
                 const size_t oi = ((size_t)z * row_heads + P.out_head0 + (size_t)h * R + r) * HD + c;
                 if (P.io_dtype == OJX_BF16) peer_store(link, reinterpret_cast<__nv_bfloat16*>(P.out) + oi, __float2bfloat16_rn(acc));
                 else peer_store(link, reinterpret_cast<float*>(P.out) + oi, acc);

@@ -119,3 +119,60 @@ def test_prefill_of_a_cache_with_infinite_centroids_equals_position_by_position(
         one.append(k[s], v[s])
         want = one.decode(q[s])
         assert torch.allclose(got[s], want, rtol=1e-5, atol=1e-6, equal_nan=True)
+
+
+@pytest.mark.parametrize("R,hd", [(4, 64), (4, 128), (8, 64), (8, 128)])
+@pytest.mark.parametrize("T", [3, 700, 9000])
+def test_non_finite_queries(cuda, R, hd, T):
+    """An infinity or NaN in the query of one head gives NaN for that head, as attention in 64 bits does, and leaves the other
+    heads as they are; the same in chunks of 15 positions (this kernel) and of 16 (the prefill kernel)."""
+    B, Hk = 2, 2
+    cache, _, _, _ = _cache(B, Hk, R, hd, T, T + 40, T)
+    q = torch.randn(B, Hk * R, hd, device=cuda, generator=torch.Generator(cuda).manual_seed(T))
+    clean = cache.decode(q)
+    for value in (float("inf"), -float("inf"), float("nan")):
+        for dtype in (torch.float32, torch.bfloat16):
+            bad = q.to(dtype)
+            ok = cache.decode(bad)
+            bad = bad.clone()
+            bad[0, 1, 5] = value
+            bad[1, R + 2, hd - 1] = value
+            got = cache.decode(bad)
+            mask = torch.zeros(B, Hk * R, dtype=torch.bool, device=cuda)
+            mask[0, 1] = mask[1, R + 2] = True
+            assert torch.isnan(got[mask]).all(), got[mask]
+            assert torch.equal(got[~mask], ok[~mask])
+    for S in (15, 16):
+        k, v = (torch.randn(S, B, Hk, hd, device=cuda) / hd ** 0.5 for _ in range(2))
+        qs = torch.randn(S, B, Hk * R, hd, device=cuda)
+        a = cache.prefill(k, v, qs)
+        cache.crop(T)
+        qs[S - 1, 0, 1, 5] = float("inf")
+        qs[2, 1, R + 2, 0] = float("nan")
+        b = cache.prefill(k, v, qs)
+        cache.crop(T)
+        mask = torch.zeros(S, B, Hk * R, dtype=torch.bool, device=cuda)
+        mask[S - 1, 0, 1] = mask[2, 1, R + 2] = True
+        assert torch.isnan(b[mask]).all()
+        assert torch.equal(a[~mask], b[~mask])
+
+
+def test_scores_that_overflow_in_one_head(cuda, monkeypatch):
+    """A finite query whose scores are -inf over whole runs of tokens: weights 0 there, as in the table kernel, and the runs of
+    the other heads are merged as ever."""
+    B, Hk, R, hd, T = 1, 2, 4, 128, 9000
+    rng = np.random.default_rng(0)
+    books = [rng.uniform(0.5, 1.5, (Hk, 256, 8)).astype(np.float32) for _ in range(2)]
+    books[0][:, :128] *= 1e-3
+    books[0][:, 128:] *= -1
+    codes = [rng.integers(0, 128, (B, Hk, T, hd // 8), dtype=np.uint8) for _ in range(2)]
+    codes[0][:, :, 100:] += 128                              # 100 tokens of small scores, then large negative ones
+    cache = ops.VQKVCache(B, Hk, Hk * R, hd, 8, T, *books)
+    cache.load(*codes)
+    q = torch.rand(B, Hk * R, hd, device=cuda, generator=torch.Generator(cuda).manual_seed(0)) + 0.5
+    q[0, 2] = 0.0
+    q[0, 6] *= 1e38
+    got = cache.decode(q)
+    monkeypatch.setenv("OJASX_B200_KV_DECODE", "table")
+    want = cache.decode(q)
+    assert torch.isfinite(want).all() and torch.allclose(got, want, rtol=1e-4, atol=2e-6)
