@@ -65,7 +65,7 @@ MoeProblem MoeHandle::problem(const void* x, void* y, const int* idx, const floa
 KvqHandle::~KvqHandle() {
     DeviceGuard g(dev);
     cudaFree(k_codes); cudaFree(v_codes); cudaFree(k_cb); cudaFree(v_cb); cudaFree(seq_lens); cudaFree(error_flag); cudaFree(counters);
-    cudaFree(partials); cudaFree(pos_partials);
+    cudaFree(partials);
 }
 
 LegacyKvHandle::~LegacyKvHandle() {
@@ -427,6 +427,15 @@ int ojasx_b200_kvq_append(OjasxKvqHandle handle, const void* d_k, const void* d_
 static int kvq_decode_impl(OjasxKvqHandle handle, const void* d_q, void* d_out, float scale, int io_dtype, void* stream,
                            int out_heads, int out_head0, const PeerLink* link);
 
+static int kvq_splits(const KvqHandle* h) { return kvq_scratch_splits(h->max_seq, h->B * h->Hkv, num_sms()); }
+
+// The partial sums of a decode, or of a batch of positions.  The size depends on the cache alone, so neither a growing context
+// nor a prefill moves the scratch that a captured decode step points at.
+static int kvq_reserve(KvqHandle* h) {
+    return ensure_capacity(&h->partials, &h->partials_cap,
+                           sizeof(float) * (size_t)h->B * h->Hkv * kvq_splits(h) * (h->Hq / h->Hkv) * (h->head_dim + 2));
+}
+
 int ojasx_b200_kvq_decode(OjasxKvqHandle handle, const void* d_q, void* d_out, float scale, int io_dtype, void* stream) {
     return kvq_decode_impl(handle, d_q, d_out, scale, io_dtype, stream, 0, 0, nullptr);
 }
@@ -447,13 +456,9 @@ static int kvq_decode_impl(OjasxKvqHandle handle, const void* d_q, void* d_out, 
     KvqProblem P = kvq_problem(h, io_dtype);
     P.q = d_q; P.out = d_out;
     P.scale = scale > 0.0f ? scale : 1.0f / std::sqrt((float)h->head_dim);
-    const int T = h->static_plan ? h->max_seq : h->host_len, heads = h->B * h->Hkv;
-    plan_kvq_decode(P, T, num_sms());
-    const int R = h->Hq / h->Hkv;
-    // sized once for the largest split count, so a growing context never reallocates
-    const size_t need = sizeof(float) * (size_t)heads * kvq_max_splits(h->max_seq) * R * (h->head_dim + 2);
+    plan_kvq_decode(P, h->static_plan ? h->max_seq : h->host_len, num_sms(), kvq_splits(h));
     DeviceGuard g(h->dev);
-    int rc = ensure_capacity(&h->partials, &h->partials_cap, need);
+    int rc = kvq_reserve(h);
     if (rc != OJX_OK) return rc;
     P.partials = static_cast<float*>(h->partials);
     P.out_heads = out_heads;
@@ -485,19 +490,19 @@ int ojasx_b200_kvq_prefill(OjasxKvqHandle handle, const void* d_k, const void* d
         if (rc == OJX_OK && !h->static_plan) h->host_len += n_positions;
         return rc;
     }
-    for (int p0 = 0; p0 < n_positions; p0 += kKvqDecodePositions) {
-        P.n_pos = std::min(kKvqDecodePositions, n_positions - p0);
+    // as many positions as the scratch of one decode holds partial sums for
+    const int batch = std::min(kKvqDecodePositions, kvq_splits(h));
+    for (int p0 = 0; p0 < n_positions; p0 += batch) {
+        P.n_pos = std::min(batch, n_positions - p0);
         P.new_k = static_cast<const char*>(d_k) + p0 * kv_pos;
         P.new_v = static_cast<const char*>(d_v) + p0 * kv_pos;
         P.q = static_cast<const char*>(d_q) + p0 * q_pos;
         P.out = static_cast<char*>(d_out) + p0 * q_pos;
         const int T = h->static_plan ? h->max_seq : h->host_len + P.n_pos;
-        plan_kvq_decode(P, T, num_sms());
-        // scratch of its own: a captured decode step keeps a pointer to the other one
-        const size_t need = sizeof(float) * (size_t)kKvqDecodePositions * h->B * h->Hkv * kvq_max_splits(h->max_seq) * R * (h->head_dim + 2);
-        int rc = ensure_capacity(&h->pos_partials, &h->pos_partials_cap, need);
+        plan_kvq_decode(P, T, num_sms(), kvq_splits(h) / P.n_pos);
+        int rc = kvq_reserve(h);
         if (rc != OJX_OK) return rc;
-        P.partials = static_cast<float*>(h->pos_partials);
+        P.partials = static_cast<float*>(h->partials);
         P.split_done = h->counters + h->B + (size_t)h->B * h->Hkv;
         if ((rc = launch_kvq_append_many(P, s)) != OJX_OK) return rc;
         if ((rc = launch_kvq_decode(P, s)) != OJX_OK) return rc;
@@ -513,9 +518,7 @@ int ojasx_b200_kvq_set_static_plan(OjasxKvqHandle handle, int enabled) {
     h->static_plan = enabled != 0;
     if (h->static_plan) {   // size the chunk scratch for the full capacity now, so that decode never allocates
         DeviceGuard g(h->dev);
-        const int heads = h->B * h->Hkv, R = h->Hq / h->Hkv;
-        const size_t need = sizeof(float) * (size_t)heads * kvq_max_splits(h->max_seq) * R * (h->head_dim + 2);
-        return ensure_capacity(&h->partials, &h->partials_cap, need);
+        return kvq_reserve(h);
     }
     return OJX_OK;
 }

@@ -123,8 +123,6 @@ struct KvqHandle {
     int* counters = nullptr;                 // [B] append + [B*Hkv] decode completion counters (zero between launches)
     void* partials = nullptr;
     size_t partials_cap = 0;
-    void* pos_partials = nullptr;            // the same for a decode of several positions (kvq_prefill)
-    size_t pos_partials_cap = 0;
     ~KvqHandle();
 };
 

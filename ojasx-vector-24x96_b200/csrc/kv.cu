@@ -623,18 +623,19 @@ static bool kvq_decode_by_mma(const KvqProblem& P) {
     return kvq_decode_mma_supported(P) && !(e && e[0] == 't');
 }
 
-void plan_kvq_decode(KvqProblem& P, int T, int sms) {
+void plan_kvq_decode(KvqProblem& P, int T, int sms, int max_splits) {
     const int heads = (P.n_pos > 0 ? P.n_pos : 1) * P.B * P.Hkv, slots = sms;
     if (kvq_decode_by_mma(P)) {
-        // chunks are shared out evenly over the SMs: an SM's share, 32 to 256 tokens (a tile for each of 16 warps), and
+        // chunks are shared out evenly over the SMs: an SM's share, 64 to 256 tokens (a tile for each of 16 warps), and
         // no more chunks per sequence than the scratch holds
+        const int most = std::min(max_splits, (std::max(T, 1) + 63) / 64);
         const long long share = ((long long)heads * std::max(T, 1) + sms - 1) / sms;
         P.chunk = round_up((int)std::min<long long>(share, 256), 32);
-        P.chunk = std::max(P.chunk, round_up((std::max(T, 1) + kvq_max_splits(T) - 1) / kvq_max_splits(T), 32));
+        P.chunk = std::max(P.chunk, round_up((std::max(T, 1) + most - 1) / most, 32));
         P.n_chunks = (std::max(T, 1) + P.chunk - 1) / P.chunk;
         return;
     }
-    const int max_s = std::min(kKvMaxSplits, (T + 255) / 256);
+    const int max_s = std::min(max_splits, (T + 255) / 256);
     long best = -1;
     P.chunk = round_up(std::max(T, 1), 64);
     P.n_chunks = 1;

@@ -81,10 +81,15 @@ int take_moe_bulk_copy_error(int* out);   // moe.cu: a bounded wait for a bulk t
 // --- kv.cu
 constexpr int kKvMaxSplits = 256;   // context splits of one (sequence, KV head) in kvq decode
 size_t kvq_decode_smem(const KvqProblem& P, int R);
-// Fills P.chunk (tokens per CTA) and P.n_chunks (<= kKvMaxSplits) for a context of T tokens.
-void plan_kvq_decode(KvqProblem& P, int T, int sms);
-// Most splits a plan for up to T tokens makes.
-inline int kvq_max_splits(int T) { return T <= 0 ? 1 : T > 64 * kKvMaxSplits ? kKvMaxSplits : (T + 63) / 64; }
+// Partial sums that the scratch of a cache holds per (sequence, KV head): one per 256 tokens, or two per SM where there are few
+// heads.  A plan never makes more: its chunks are no shorter than 256 tokens or than an SM's share.  At 128 heads of 4 query
+// heads, head_dim 128 and 16384 tokens 17 MB (one per 64 tokens took 68, and as many for each of 16 positions 1.1 GB).
+inline int kvq_scratch_splits(int max_seq, int heads, int sms) {
+    const int tokens = (max_seq + 255) / 256, fill = (2 * sms + heads - 1) / heads, n = tokens > fill ? tokens : fill;
+    return n < kKvMaxSplits ? n : kKvMaxSplits;
+}
+// Fills P.chunk (tokens per CTA) and P.n_chunks (<= max_splits, what the scratch holds per position) for a context of T tokens.
+void plan_kvq_decode(KvqProblem& P, int T, int sms, int max_splits);
 int launch_kvq_append(const KvqProblem& P, cudaStream_t stream);
 int launch_kvq_decode(const KvqProblem& P, cudaStream_t stream, const PeerLink* link = nullptr);
 // --- kv_decode_mma.cu: decode for block_dim 8 and head_dim 64 or 128 (launch_kvq_decode takes it where it fits)

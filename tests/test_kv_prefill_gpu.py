@@ -67,3 +67,45 @@ def test_prefill_operand_range(cuda, oracle):
     for s in (0, 3, 15):
         ref = oracle.kvq_decode(q[s, 0, :4], kc[0, 0, :65 + s], vc[0, 0, :65 + s], books[0][0], books[1][0], block_dim=8)
         assert np.allclose(got[s, 0, :4], ref, rtol=1e-4, atol=2e-6 * 3e-6), s
+
+
+def _used(f):
+    torch.cuda.synchronize()
+    free = torch.cuda.mem_get_info()[0]
+    f()
+    torch.cuda.synchronize()
+    return free - torch.cuda.mem_get_info()[0]
+
+
+@pytest.mark.parametrize("cap", [8192, 16384, 32768])
+@pytest.mark.parametrize("R", [2, 4])
+def test_scratch_of_a_cache(cuda, cap, R):
+    """Partial sums: one per 256 tokens and query head (and what fills the SMs), for positions of a prompt in one launch too."""
+    rng = np.random.default_rng(0)
+    B, Hk, hd = 16, 8, 128
+    cache = ops.VQKVCache(B, Hk, Hk * R, hd, 8, cap, *(rng.standard_normal((Hk, 256, 8)).astype(np.float32) for _ in range(2)))
+    q = torch.randn(1, B, Hk * R, hd, device=cuda)
+    k, v = (torch.randn(1, B, Hk, hd, device=cuda) for _ in range(2))
+    cache.append(k[0], v[0])
+    torch.empty(64 << 20, device=cuda)                       # outputs come from the allocator's cache
+    used = _used(lambda: (cache.decode(q[0]), cache.prefill(k, v, q)))
+    need = 4 * B * Hk * (cap // 256) * R * (hd + 2)
+    assert used <= need + (8 << 20), (used, need)            # the driver hands memory out in pieces of 2 MB
+
+
+@pytest.mark.parametrize("B,Hkv,R,hd,T0,S", [
+    (1, 1, 4, 64, 20000, 15),        # one head: 256 partial sums, 17 per position
+    (16, 8, 4, 128, 300, 9),         # more heads than half the SMs: three positions per launch
+    (20, 8, 2, 64, 40, 5),           # the table kernel, two per launch
+])
+def test_positions_share_the_scratch_of_one_decode(cuda, B, Hkv, R, hd, T0, S):
+    books, old, k, v, q = _make(7, B, Hkv, Hkv * R, hd, 8, T0, S)
+    many, one = (ops.VQKVCache(B, Hkv, Hkv * R, hd, 8, T0 + S, *books) for _ in range(2))
+    for c in (many, one):
+        c.load(*old)
+    kt, vt, qt = (torch.from_numpy(a).to(cuda) for a in (k, v, q))
+    got = many.prefill(kt, vt, qt)
+    for s in range(S):
+        one.append(kt[s], vt[s])
+        assert torch.allclose(got[s], one.decode(qt[s]), rtol=1e-4, atol=2e-6), s
+    assert many.sync_len() == T0 + S
