@@ -64,7 +64,7 @@ __global__ void __launch_bounds__(kPfAppendThreads) kvq_append_many_kernel(const
         vv = __fadd_rn(vv, __fmul_rn(v[d], v[d]));
     }
     float bd = INFINITY;
-    int bi = 0;
+    int bi = 0x7fffffff;   // code 255 where no distance is finite (NaN or infinite keys), as kvq_append_kernel writes it
 #pragma unroll 4
     for (int c = 0; c < P.Kcb; ++c) {
         const float4* cv = reinterpret_cast<const float4*>(cb_s + c * D);

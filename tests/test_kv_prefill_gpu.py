@@ -109,3 +109,17 @@ def test_positions_share_the_scratch_of_one_decode(cuda, B, Hkv, R, hd, T0, S):
         one.append(kt[s], vt[s])
         assert torch.allclose(got[s], one.decode(qt[s]), rtol=1e-4, atol=2e-6), s
     assert many.sync_len() == T0 + S
+
+
+def test_codes_of_non_finite_keys_and_values(cuda):
+    """Positions in a chunk get the codes that single appends give them, also where no distance to a centroid is finite."""
+    books, _, k, v, q = _make(5, 1, 2, 8, 64, 8, 1, 20)
+    books[0][1, 9, 3] = np.inf
+    k[3, 0, 0, 5], k[4, 0, 1, 63], v[5, 0, 0, 0], v[6], v[7] = np.nan, np.inf, -np.inf, np.nan, 3e38
+    many, one = (ops.VQKVCache(1, 2, 8, 64, 8, 64, *books) for _ in range(2))
+    kt, vt, qt = (torch.from_numpy(a).to(cuda) for a in (k, v, q))
+    many.prefill(kt, vt, qt)
+    for s in range(20):
+        one.append(kt[s], vt[s])
+    a, b = many.read(0, 20), one.read(0, 20)
+    assert np.array_equal(a[0], b[0]) and np.array_equal(a[1], b[1])
