@@ -490,8 +490,8 @@ int ojasx_b200_kvq_prefill(OjasxKvqHandle handle, const void* d_k, const void* d
         if (rc == OJX_OK && !h->static_plan) h->host_len += n_positions;
         return rc;
     }
-    // as many positions as the scratch of one decode holds partial sums for
-    const int batch = std::min(kKvqDecodePositions, kvq_splits(h));
+    // as many positions as the scratch of one decode holds partial sums for, and a grid (z = positions x sequences) takes
+    const int batch = std::max(1, std::min({kKvqDecodePositions, kvq_splits(h), 65535 / h->B}));
     for (int p0 = 0; p0 < n_positions; p0 += batch) {
         P.n_pos = std::min(batch, n_positions - p0);
         P.new_k = static_cast<const char*>(d_k) + p0 * kv_pos;

@@ -21,7 +21,7 @@ __device__ __forceinline__ float pf_load(const void* p, size_t i, int dtype) {
 }
 
 // ------------------------------------------------------------------------------------ append
-// grid = (2 * Hkv * G, ceil(positions * B / 128)).  A block encodes one (k|v, head, group) of 128
+// grid = ceil(positions * B / 128) blocks of rows x 2 * Hkv * G tasks, tasks innermost.  A block encodes one (k|v, head, group) of 128
 // rows: thread = row, the 256 centroids and their squared norms broadcast from shared memory.  Same
 // distance and the same first-minimum rule as kvq_append_kernel (every dot product a sequential fp32
 // sum of rounded products), so the codes are equal.  Bound: fp32 issue, 256 x 19 instructions per
@@ -33,7 +33,7 @@ template <int D>
 __global__ void __launch_bounds__(kPfAppendThreads) kvq_append_many_kernel(const __grid_constant__ KvqProblem P) {
     __shared__ __align__(16) float cb_s[256 * D];
     __shared__ float cc_s[256];
-    const int G = P.G, task = blockIdx.x;
+    const int G = P.G, tasks = 2 * P.Hkv * G, task = blockIdx.x % tasks;
     const int which = task / (P.Hkv * G), rem = task - which * P.Hkv * G;
     const int h = rem / G, g = rem - h * G;
     const float* cb = (which ? P.v_cb : P.k_cb) + (size_t)h * P.Kcb * D;
@@ -46,7 +46,7 @@ __global__ void __launch_bounds__(kPfAppendThreads) kvq_append_many_kernel(const
         cc_s[c] = cc;
     }
     __syncthreads();
-    const int row = blockIdx.y * kPfAppendThreads + threadIdx.x;
+    const int row = (int)(blockIdx.x / tasks) * kPfAppendThreads + threadIdx.x;
     if (row >= P.n_pos * P.B) return;
     const int s = row / P.B, b = row - s * P.B;
     const int T = P.seq_lens[b] + s;
@@ -439,9 +439,9 @@ int launch_kvq_prefill_attention(const KvqProblem& P, cudaStream_t s) {
 template <int D>
 static int launch_append_many_t(const KvqProblem& P, cudaStream_t s) {
     const long long rows = (long long)P.n_pos * P.B;
-    const long long blocks = (rows + kPfAppendThreads - 1) / kPfAppendThreads;
-    if (blocks > 65535) return OJX_ERR_TOO_LARGE;
-    kvq_append_many_kernel<D><<<dim3(2 * P.Hkv * P.G, (unsigned)blocks), kPfAppendThreads, 0, s>>>(P);
+    const long long blocks = (rows + kPfAppendThreads - 1) / kPfAppendThreads * 2 * P.Hkv * P.G;
+    if (rows > 0x7fffffff - kPfAppendThreads || blocks > 0x7fffffff) return OJX_ERR_TOO_LARGE;
+    kvq_append_many_kernel<D><<<(unsigned)blocks, kPfAppendThreads, 0, s>>>(P);
     OJX_CUDA_TRY(cudaGetLastError());
     count_launch(1);
     return OJX_OK;

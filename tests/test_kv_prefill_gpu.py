@@ -123,3 +123,16 @@ def test_codes_of_non_finite_keys_and_values(cuda):
         one.append(kt[s], vt[s])
     a, b = many.read(0, 20), one.read(0, 20)
     assert np.array_equal(a[0], b[0]) and np.array_equal(a[1], b[1])
+
+
+def test_positions_of_many_sequences(cuda):
+    """5000 sequences: 15 positions of them are more than the 65535 a grid takes in z."""
+    B, S = 5000, 15
+    rng = np.random.default_rng(0)
+    books = [rng.standard_normal((1, 256, 16)).astype(np.float32) / 8 for _ in range(2)]
+    many, one = (ops.VQKVCache(B, 1, 1, 64, 16, 20, *books) for _ in range(2))
+    k, v, q = (torch.randn(S, B, 1, 64, device=cuda, generator=torch.Generator(cuda).manual_seed(i)) for i in range(3))
+    got = many.prefill(k, v, q)
+    for s in range(S):
+        one.append(k[s], v[s])
+        assert torch.allclose(got[s], one.decode(q[s]), rtol=1e-4, atol=2e-6)
