@@ -8,6 +8,7 @@
 #include "peer.cuh"
 
 #include <atomic>
+#include <cmath>
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
@@ -55,6 +56,24 @@ int ensure_capacity(void** dptr, size_t* cap, size_t bytes) {
     OJX_CUDA_TRY(cudaMalloc(dptr, want));
     *cap = want;
     return OJX_OK;
+}
+
+bool book_fits_halves(const float* cb, int n, int D) {
+    if (!cb) return true;   // zeros
+    std::vector<float> dim(D, 0.0f), cen(n, 0.0f);
+    float top = 0.0f;
+    for (int c = 0; c < n; ++c)
+        for (int d = 0; d < D; ++d) {
+            const float a = std::fabs(cb[(size_t)c * D + d]);
+            if (!std::isfinite(a)) return false;
+            dim[d] = std::max(dim[d], a);
+            cen[c] = std::max(cen[c], a);
+        }
+    for (float a : dim) top = std::max(top, a);
+    if (top == 0.0f) return true;
+    const float least = top * 0x1p-16f;
+    const auto small = [&](float a) { return a != 0.0f && a < least; };
+    return top >= 0x1p-80f && std::none_of(dim.begin(), dim.end(), small) && std::none_of(cen.begin(), cen.end(), small);
 }
 
 int ensure_pinned(void** hptr, size_t* cap, size_t bytes) {
@@ -132,6 +151,7 @@ OjasxLinearHandle ojasx_create_linear(int in_features, int out_features, int blo
     if (!h) return nullptr;
     h->in = in_features; h->out = out_features; h->D = block_dim; h->Kcb = codebook_size;
     h->G = in_features / block_dim;  // ojasx_lut.h:92
+    h->even_book = book_fits_halves(codebook_data, codebook_size, block_dim);
     if (cudaGetDevice(&h->dev) != cudaSuccess) { set_last_error_msg("no CUDA device"); delete h; return nullptr; }
     int rc = OJX_OK;
     // Null data pointers leave the array zero-filled (codes, codebook) or at its default
@@ -198,16 +218,17 @@ static long long gather_min_work() {
     return e ? atoll(e) : 3000000;
 }
 
-// Whether the gather kernel (gather_mma.cu) may take a call; the switches of the other paths come first.
-static bool gather_mma_open(const LinearProblem& P, bool csr_sorted) {
-    if (!gather_mma_supported(P) || linear_cluster_disabled() || gather_min_work() < 0) return false;
+// Whether the gather kernel (gather_mma.cu) may take a call; the switches of the other paths come first.  With a codebook of wide
+// range its window is wide too and most sums are evaluated twice (one entry of 1e30: 274 us, table kernels 114, 35 without it).
+static bool gather_mma_open(const LinearProblem& P, bool csr_sorted, bool even_book) {
+    if (!even_book || !gather_mma_supported(P) || linear_cluster_disabled() || gather_min_work() < 0) return false;
     const char* e = getenv("OJASX_B200_TENSOR_MIN_BATCH");
     const int min_batch = e ? atoi(e) : kTensorMinBatch;
     return !(min_batch > 0 && P.batch >= min_batch && dequant_gemm_supported(P, csr_sorted));
 }
 
-static bool wants_gather_mma(const LinearProblem& P, bool csr_sorted) {
-    return gather_mma_open(P, csr_sorted) && (long long)(P.row_stop - P.row_start) * P.G * P.batch >= gather_min_work();
+static bool wants_gather_mma(const LinearProblem& P, bool csr_sorted, bool even_book) {
+    return gather_mma_open(P, csr_sorted, even_book) && (long long)(P.row_stop - P.row_start) * P.G * P.batch >= gather_min_work();
 }
 
 size_t ojasx_b200_linear_workspace(OjasxLinearHandle handle, int batch_size, int io_dtype) {
@@ -223,7 +244,7 @@ int ojasx_b200_linear_forward_ws(OjasxLinearHandle handle, const void* d_x, void
     auto* h = static_cast<LinearHandle*>(handle);
     if (batch_size <= 0 || row_start < 0 || row_stop > h->out || row_start >= row_stop) return OJX_ERR_ARG;
     const LinearProblem P = h->problem(d_x, d_y, batch_size, io_dtype, row_start, row_stop);
-    if (workspace && wants_gather_mma(P, h->csr_sorted) && workspace_bytes >= gather_mma_workspace(h->in, batch_size))
+    if (workspace && wants_gather_mma(P, h->csr_sorted, h->even_book) && workspace_bytes >= gather_mma_workspace(h->in, batch_size))
         return launch_gather_mma(&P, 1, d_x, nullptr, nullptr, workspace, static_cast<cudaStream_t>(stream));
     return ojasx_b200_linear_forward(handle, d_x, d_y, batch_size, io_dtype, row_start, row_stop, stream);
 }
@@ -234,7 +255,7 @@ size_t ojasx_b200_mlp_workspace(OjasxLinearHandle gate, OjasxLinearHandle up, Oj
     const LinearHandle* l[3] = {static_cast<LinearHandle*>(gate), static_cast<LinearHandle*>(up), static_cast<LinearHandle*>(down)};
     if (l[0]->in != l[1]->in || l[0]->out != l[1]->out || l[2]->in != l[0]->out) return 0;
     for (const LinearHandle* h : l)
-        if (!gather_mma_open(h->problem(d_x, nullptr, batch_size, io_dtype, 0, h->out), h->csr_sorted)) return 0;
+        if (!gather_mma_open(h->problem(d_x, nullptr, batch_size, io_dtype, 0, h->out), h->csr_sorted, h->even_book)) return 0;
     return std::max(gather_mma_workspace(l[0]->in, batch_size), gather_mma_workspace(l[2]->in, batch_size)) +
            3 * (size_t)batch_size * l[0]->out * 2;   // and gate, up and the gated vectors
 }

@@ -59,6 +59,7 @@ MoeProblem MoeHandle::problem(const void* x, void* y, const int* idx, const floa
     P.n_tokens = n_tokens; P.k_active = k; P.E = E; P.expert_offset = expert_offset;
     P.H = H; P.I = I; P.G = H / D; P.Gi = I / D; P.D = D; P.Kcb = 256; P.io_dtype = io;
     P.gate_limit = gate_limit;
+    P.even_books = even_books;
     return P;
 }
 
@@ -123,6 +124,7 @@ OjasxMoEHandle ojasx_create_moe(int num_experts, int hidden_dim, int intermediat
     if (!h) return nullptr;
     h->E = num_experts; h->E_total = num_experts; h->H = hidden_dim; h->I = intermediate_dim; h->top_k = top_k;
     h->D = block_dim;
+    h->even_books = book_fits_halves(codebook_in, 256, block_dim) && book_fits_halves(codebook_down, 256, block_dim);
     const size_t G = hidden_dim / block_dim, Gi = intermediate_dim / block_dim;
     int rc = cudaGetDevice(&h->dev) == cudaSuccess ? OJX_OK : OJX_ERR_CUDA;
     const size_t cbb = sizeof(float) * 256 * (size_t)block_dim;
@@ -348,7 +350,10 @@ OjasxKvqHandle ojasx_b200_kvq_create(int batch, int kv_heads, int q_heads, int h
     int rc = cudaGetDevice(&h->dev) == cudaSuccess ? OJX_OK : OJX_ERR_CUDA;
     const size_t codes = (size_t)batch * kv_heads * max_seq_len * h->G;
     const size_t cbb = sizeof(float) * (size_t)kv_heads * 256 * block_dim;
-    for (size_t i = 0; i < cbb / sizeof(float) && h->finite_books; ++i) h->finite_books = std::isfinite(k_codebook[i]) && std::isfinite(v_codebook[i]);
+    for (int i = 0; i < kv_heads && h->even_books; ++i) {   // the kernels scale per head
+        const size_t at = (size_t)i * 256 * block_dim;
+        h->even_books = book_fits_halves(k_codebook + at, 256, block_dim) && book_fits_halves(v_codebook + at, 256, block_dim);
+    }
     if (rc == OJX_OK) rc = upload((void**)&h->k_codes, nullptr, codes);
     if (rc == OJX_OK) rc = upload((void**)&h->v_codes, nullptr, codes);
     if (rc == OJX_OK) rc = upload((void**)&h->k_cb, k_codebook, cbb);
@@ -409,7 +414,7 @@ static KvqProblem kvq_problem(const KvqHandle* h, int io) {
     P.seq_lens = h->seq_lens; P.error_flag = h->error_flag; P.partials = static_cast<float*>(h->partials);
     P.append_done = h->counters; P.split_done = h->counters + h->B;
     P.B = h->B; P.Hkv = h->Hkv; P.Hq = h->Hq; P.head_dim = h->head_dim; P.D = h->D; P.G = h->G; P.Kcb = 256;
-    P.max_seq = h->max_seq; P.io_dtype = io; P.finite_books = h->finite_books;
+    P.max_seq = h->max_seq; P.io_dtype = io; P.even_books = h->even_books;
     return P;
 }
 

@@ -93,6 +93,7 @@ struct MoeProblem {
     int lut_blocks;           // layout of lut_in: 0 = [token][group][256]; 1 = 16-group blocks (moe_prebuild_kernel);
                               // 2 = per-slice images of the chain walk's table area (moe_chain_prebuild_kernel);
                               // 3 = no tables: the fragments of moe_gather.cu, made by the expert launches
+    int even_books;           // both codebooks fit pairs of fp16 numbers (book_fits_halves, checked when the handle is created)
 };
 
 // Codebook-VQ KV cache of one layer.  Device pointers.
@@ -112,7 +113,7 @@ struct KvqProblem {
     int* split_done;        // [B, Hkv] decode CTAs of a (sequence, head) that have written their partial (returns to 0)
     int B, Hkv, Hq, head_dim, D, G, Kcb, max_seq;
     int chunk, n_chunks;
-    int finite_books;       // both codebooks hold finite numbers only (checked when the cache is created)
+    int even_books;         // the codebooks fit pairs of fp16 numbers (book_fits_halves, checked when the cache is created)
     int v_copies;           // copies of the value codebook in the decode kernel's shared memory (1 or 8)
     int io_dtype;
     float scale;

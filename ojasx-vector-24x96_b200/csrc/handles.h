@@ -11,6 +11,11 @@ void count_launch(int n);
 int upload(void** dptr, const void* host, size_t bytes);          // cudaMalloc + copy (zero-fill when host == null)
 int ensure_capacity(void** dptr, size_t* cap, size_t bytes);      // grow-only device staging buffer
 int wait_stream(cudaStream_t s);                                  // low-latency stream wait
+// Whether the kernels that hold a codebook [n][D] as pairs of fp16 numbers scaled by its largest magnitude keep fp32 accuracy: such
+// a pair has 22 bits down to 2^-18 of the largest and an error of 2^-39 of it below.  So the entries have to be finite, and the
+// largest of every centroid and of every dimension within 2^16 of the largest of all (zeros aside); then a centroid of any size
+// and an activation of any one dimension see 2^-23.  Magnitudes below 2^-80 are out of the scales' reach.
+bool book_fits_halves(const float* cb, int n, int D);
 int ensure_pinned(void** hptr, size_t* cap, size_t bytes);        // grow-only pinned, device-mapped host buffer
 
 // Makes `dev` current for the lifetime of the guard.
@@ -31,6 +36,7 @@ struct LinearHandle {
     float* bias = nullptr;     // null = none
     int nnz = 0;
     bool has_outlier_arrays = false;
+    bool even_book = true;     // book_fits_halves
     bool csr_sorted = true;    // column indices ascending inside every row (needed by the tensor-core path)
     int* row_ptrs = nullptr;
     int* cols = nullptr;
@@ -81,6 +87,7 @@ struct MoeHandle {
     int expert_offset = 0;
     int H = 0, I = 0, top_k = 0, D = 0;
     float gate_limit = 0.0f;   // <= 0: none
+    bool even_books = true;    // book_fits_halves, both
     float* cb_in = nullptr;
     float* cb_down = nullptr;
     uint8_t* gu_codes = nullptr;
@@ -112,7 +119,7 @@ struct KvqHandle {
     int dev = 0;
     int B = 0, Hkv = 0, Hq = 0, head_dim = 0, D = 0, G = 0, max_seq = 0;
     int host_len = 0;                        // host mirror of the (uniform) cached length
-    bool finite_books = true;                // no infinity or NaN in the codebooks
+    bool even_books = true;                  // book_fits_halves, both codebooks of every head
     bool static_plan = false;                // plan launches for max_seq; only the device-side lengths are consulted
     uint8_t* k_codes = nullptr;
     uint8_t* v_codes = nullptr;

@@ -396,7 +396,7 @@ __global__ void __launch_bounds__(kKdThreads, 1) kvq_decode_mma_kernel(const __g
 
 bool kvq_decode_mma_supported(const KvqProblem& P) {
     const int R = P.Hq / P.Hkv;
-    return P.finite_books && P.D == 8 && (P.G == 8 || P.G == 16) && P.head_dim == P.G * 8 && (R == 4 || R == 8);
+    return P.even_books && P.D == 8 && (P.G == 8 || P.G == 16) && P.head_dim == P.G * 8 && (R == 4 || R == 8);
 }
 
 template <int R, int G>

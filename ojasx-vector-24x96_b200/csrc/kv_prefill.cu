@@ -420,10 +420,10 @@ static int launch_prefill_d(const KvqProblem& P, cudaStream_t s) {
     }
 }
 
-// High and low parts of an infinity are NaN, so codebooks with one keep the decode kernel.
+// Codebooks that high and low parts do not hold to fp32 accuracy (infinities, wide ranges) keep the decode kernel.
 bool kvq_prefill_supported(const KvqProblem& P) {
     const int R = P.Hq / P.Hkv;
-    return P.finite_books && R <= kPfRows && kPfRows % R == 0 && P.G % 4 == 0 && P.B <= 65535 && P.Hkv <= 65535 &&
+    return P.even_books && R <= kPfRows && kPfRows % R == 0 && P.G % 4 == 0 && P.B <= 65535 && P.Hkv <= 65535 &&
            (P.head_dim == 64 || P.head_dim == 128) && (P.D == 4 || P.D == 8 || P.D == 16);
 }
 

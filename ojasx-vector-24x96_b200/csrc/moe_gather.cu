@@ -422,7 +422,7 @@ __global__ void __launch_bounds__(kMgDownThreads, 2) moe_gather_down_kernel(cons
 static size_t mg_smem(int chunks) { return kGmTable + 16 * ((size_t)chunks * 512 + 64); }
 
 bool moe_gather_wanted(const MoeProblem& P) {
-    if (P.io_dtype != OJX_BF16 || !P.lut_in || !P.plan || P.D != 8 || P.G % 8 != 0 || P.Gi % 8 != 0 || P.H != P.G * 8 || P.I != P.Gi * 8 || P.E > 4096) return false;
+    if (P.io_dtype != OJX_BF16 || !P.even_books || !P.lut_in || !P.plan || P.D != 8 || P.G % 8 != 0 || P.Gi % 8 != 0 || P.H != P.G * 8 || P.I != P.Gi * 8 || P.E > 4096) return false;
     if (reinterpret_cast<uintptr_t>(P.x) & 3) return false;   // pairs of bf16 are read as words
     const size_t cx = (P.G + kGmChunk - 1) / kGmChunk, ci = (P.Gi + kGmChunk - 1) / kGmChunk, pairs = (size_t)P.n_tokens * P.k_active;
     if (mg_smem((int)cx) > 224 * 1024 || mg_smem((int)ci) > 110 * 1024) return false;

@@ -175,3 +175,21 @@ def test_bits_of_the_table_kernels_for_biased_data(cuda, monkeypatch, K, M, batc
             n = int(np.count_nonzero(got != _table(monkeypatch, layer, xt)))
             bad[kind] = bad.get(kind, 0) + n
     assert not any(bad.values()), bad
+
+
+@pytest.mark.parametrize("entry", [1e30, float("inf")])
+def test_codebooks_of_wide_range_keep_the_table_kernels(cuda, monkeypatch, entry):
+    """One entry far above the others makes every sum's window wide, so that most would be formed twice."""
+    w = synth.make_vq_linear(5, 2560, 6912, block_dim=8)
+    w.codes[w.codes == 255] = 3
+    x = torch.randn(16, 2560, device=cuda, generator=torch.Generator(cuda).manual_seed(1)).bfloat16()
+    want = ops.VQLinear.from_weights(w)(x)
+    w.codebook[255] = entry                              # no code names it
+    layer = ops.VQLinear.from_weights(w)
+    n0 = ojasx_b200.launch_count()
+    got = layer(x)
+    assert ojasx_b200.launch_count() - n0 == 1           # the table kernel
+    assert torch.equal(got, want)
+    mlp = ops.VQMLP(layer, layer, ops.VQLinear.from_weights(synth.make_vq_linear(6, 6912, 2560, block_dim=8)))
+    g = layer(x)
+    assert torch.equal(mlp(x), mlp.down(ops.silu_mul(g, g)))

@@ -176,3 +176,30 @@ def test_scores_that_overflow_in_one_head(cuda, monkeypatch):
     monkeypatch.setenv("OJASX_B200_KV_DECODE", "table")
     want = cache.decode(q)
     assert torch.isfinite(want).all() and torch.allclose(got, want, rtol=1e-4, atol=2e-6)
+
+
+@pytest.mark.parametrize("which,row,col", [(0, 255, slice(None)), (1, 255, slice(None)), (0, 255, 3), (1, slice(None), 5)])
+@pytest.mark.parametrize("factor", [1e30, 2e6])
+def test_codebooks_of_wide_range_keep_fp32_accuracy(cuda, oracle, which, row, col, factor):
+    """Entries far above the others (a centroid that no token has, a dimension): the others keep their 24 bits."""
+    rng = np.random.default_rng(0)
+    B, Hk, R, hd, T, S = 1, 2, 4, 128, 500, 20
+    books = [(rng.standard_normal((Hk, 256, 8)) / np.sqrt(hd)).astype(np.float32) for _ in range(2)]
+    if isinstance(row, slice):
+        books[which] = books[which].astype(np.float32)
+        books[which][1, row, col] = np.float32(factor) * np.abs(books[which][1, row, col])
+    else:
+        books[which][1, row, col] = factor
+    codes = [rng.integers(0, 255, (B, Hk, T, hd // 8), dtype=np.uint8) for _ in range(2)]
+    cache = ops.VQKVCache(B, Hk, Hk * R, hd, 8, T + S, *books)
+    cache.load(*codes)
+    q = rng.standard_normal((S, B, Hk * R, hd)).astype(np.float32)
+    k, v = (torch.from_numpy((rng.standard_normal((S, B, Hk, hd)) / np.sqrt(hd)).astype(np.float32)).to(cuda) for _ in range(2))
+    got = [cache.decode(torch.from_numpy(q[0]).to(cuda)).cpu().numpy()]
+    got += list(cache.prefill(k, v, torch.from_numpy(q).to(cuda)).cpu().numpy())
+    kc, vc = cache.read(0, T + S)
+    for i, (s, n) in enumerate([(0, T)] + [(s, T + s + 1) for s in range(S)]):
+        want = _exact(books, [kc[:, :, :n], vc[:, :, :n]], q[s], 1.0 / np.sqrt(hd))
+        for d in range(hd):     # dimensions of other sizes: each to its own
+            size = np.abs(want[:, :, d]).max()
+            assert np.abs(got[i][:, :, d] - want[:, :, d]).max() <= 1e-5 * size, (i, d)

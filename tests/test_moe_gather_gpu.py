@@ -112,3 +112,16 @@ def test_gather_experts_with_outliers_in_few_rows(cuda, oracle, B):
     assert ojasx_b200.launch_count() - n0 == 6
     want = _oracle_moe(oracle, w, x, idx, wts)
     assert np.all(np.abs(got - want) <= ATOL + RTOL * np.abs(want)), np.abs(got - want).max()
+
+
+@pytest.mark.parametrize("book", ["codebook", "down_codebook"])
+def test_gather_experts_codebooks_of_wide_range(cuda, book):
+    """A centroid that no code names, far above the others, must not cost them bits."""
+    w = synth.make_vq_moe(5, 4, 512, 128, block_dim=8, outlier_frac=0.0)
+    w.gate_up_codes[w.gate_up_codes == 255] = 3
+    w.down_codes[w.down_codes == 255] = 3
+    x = torch.randn(8, 512, device=cuda, generator=torch.Generator(cuda).manual_seed(1)).bfloat16()
+    want = ops.VQMoE(w).forward_routed(x, 2).float()
+    getattr(w, book)[255] = 1e30
+    got = ops.VQMoE(w).forward_routed(x, 2).float()
+    assert torch.all((got - want).abs() <= 2.0 ** -7 * want.abs() + ATOL)
