@@ -26,9 +26,15 @@ def _dtype_code(t: torch.Tensor) -> int:
     raise TypeError(f"activations must be float32 or bfloat16, got {t.dtype}")
 
 
+# The raw handle of the current stream: a Stream object costs as much as the launch it is for.  Not part of torch's public API,
+# so the public one stands in where a build of torch lacks it.
+_raw_stream = getattr(torch._C, "_cuda_getCurrentRawStream", None) or (lambda index: torch.cuda.current_stream(index).cuda_stream)
+
+
 def _stream_ptr(device) -> int:
-    """The current stream of a tensor's device (the raw handle: a Stream object costs as much as the launch it is for)."""
-    return torch._C._cuda_getCurrentRawStream(device.index)
+    """The current stream of a device, or of the current device where it has no index."""
+    index = device.index
+    return _raw_stream(torch.cuda.current_device() if index is None else index)
 
 
 def _require_cuda(t: torch.Tensor, name: str) -> None:
