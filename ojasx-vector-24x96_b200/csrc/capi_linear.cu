@@ -235,7 +235,7 @@ size_t ojasx_b200_linear_workspace(OjasxLinearHandle handle, int batch_size, int
     if (!handle || batch_size <= 0) return 0;
     auto* h = static_cast<LinearHandle*>(handle);
     const LinearProblem P = h->problem(nullptr, nullptr, batch_size, io_dtype, 0, h->out);
-    return gather_mma_supported(P) ? gather_mma_workspace(h->in, batch_size) : 0;
+    return wants_gather_mma(P, h->csr_sorted, h->even_book) ? gather_mma_workspace(h->in, batch_size) : 0;
 }
 
 int ojasx_b200_linear_forward_ws(OjasxLinearHandle handle, const void* d_x, void* d_y, int batch_size, int io_dtype,

@@ -66,7 +66,6 @@ class VQLinear:
                                             _p(cb), _p(codes), _p(sc), _p(bi))
         if not self._h:
             check(-3, "ojasx_create_linear")
-        self._workspace = {}    # batch -> scratch bytes of a bf16 call
         self.nnz = 0
         if csr is not None:
             rp = np.ascontiguousarray(csr[0], dtype=np.int32)
@@ -97,9 +96,7 @@ class VQLinear:
         if out is None:
             out = torch.empty((x2.shape[0], rows), device=x.device, dtype=x.dtype)
         if x2.dtype is torch.bfloat16 and 1 < x2.shape[0] < GATHER_BATCHES.stop:
-            size = self._workspace.get(x2.shape[0])
-            if size is None:
-                size = self._workspace[x2.shape[0]] = lib().ojasx_b200_linear_workspace(self._h, x2.shape[0], BF16)
+            size = lib().ojasx_b200_linear_workspace(self._h, x2.shape[0], BF16)
             if size:    # scratch of this call, so that calls on several streams do not share it
                 ws = torch.empty(size, device=x.device, dtype=torch.uint8)
                 check(lib().ojasx_b200_linear_forward_ws(self._h, x2.data_ptr(), out.data_ptr(), x2.shape[0], BF16, row_start,

@@ -193,3 +193,22 @@ def test_codebooks_of_wide_range_keep_the_table_kernels(cuda, monkeypatch, entry
     mlp = ops.VQMLP(layer, layer, ops.VQLinear.from_weights(synth.make_vq_linear(6, 6912, 2560, block_dim=8)))
     g = layer(x)
     assert torch.equal(mlp(x), mlp.down(ops.silu_mul(g, g)))
+
+
+@pytest.mark.parametrize("K,M,batch,scratch", [(512, 512, 4, False), (2560, 6912, 2, True), (2560, 6912, 1, False)])
+def test_scratch_only_where_the_gather_kernel_is_taken(cuda, monkeypatch, K, M, batch, scratch):
+    """A layer too small for it launches as before, without an allocation per call; a switch set later is seen."""
+    layer = ops.VQLinear.from_weights(synth.make_vq_linear(5, K, M, block_dim=8))
+    x = torch.randn(batch, K, device=cuda).bfloat16()
+    out = torch.empty(batch, M, device=cuda, dtype=torch.bfloat16)
+
+    def allocations():
+        n0 = torch.cuda.memory_stats()["allocation.all.allocated"]
+        layer(x, out=out)
+        return torch.cuda.memory_stats()["allocation.all.allocated"] - n0
+
+    assert allocations() == int(scratch)
+    monkeypatch.setenv("OJASX_B200_GATHER_MIN_WORK", "0")
+    assert allocations() == int(batch > 1)
+    monkeypatch.setenv("OJASX_B200_GATHER_MIN_WORK", "-1")
+    assert allocations() == 0
