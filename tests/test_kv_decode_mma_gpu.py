@@ -121,11 +121,12 @@ def test_prefill_of_a_cache_with_infinite_centroids_equals_position_by_position(
         assert torch.allclose(got[s], want, rtol=1e-5, atol=1e-6, equal_nan=True)
 
 
-@pytest.mark.parametrize("R,hd", [(4, 64), (4, 128), (8, 64), (8, 128)])
-@pytest.mark.parametrize("T", [3, 700, 9000])
+@pytest.mark.parametrize("R,hd", [(4, 64), (4, 128), (8, 64), (8, 128), (1, 64), (2, 128)])
+@pytest.mark.parametrize("T", [17, 700, 9000])
 def test_non_finite_queries(cuda, R, hd, T):
     """An infinity or NaN in the query of one head gives NaN for that head, as attention in 64 bits does, and leaves the other
-    heads as they are; the same in chunks of 15 positions (this kernel) and of 16 (the prefill kernel)."""
+    heads as they are; the same on the query-table kernel (one or two query heads per KV head) and in chunks of 15 and of 16
+    positions (the decode kernels, the prefill kernel)."""
     B, Hk = 2, 2
     cache, _, _, _ = _cache(B, Hk, R, hd, T, T + 40, T)
     q = torch.randn(B, Hk * R, hd, device=cuda, generator=torch.Generator(cuda).manual_seed(T))
@@ -136,10 +137,10 @@ def test_non_finite_queries(cuda, R, hd, T):
             ok = cache.decode(bad)
             bad = bad.clone()
             bad[0, 1, 5] = value
-            bad[1, R + 2, hd - 1] = value
+            bad[1, R, hd - 1] = value
             got = cache.decode(bad)
             mask = torch.zeros(B, Hk * R, dtype=torch.bool, device=cuda)
-            mask[0, 1] = mask[1, R + 2] = True
+            mask[0, 1] = mask[1, R] = True
             assert torch.isnan(got[mask]).all(), got[mask]
             assert torch.equal(got[~mask], ok[~mask])
     for S in (15, 16):
@@ -148,11 +149,11 @@ def test_non_finite_queries(cuda, R, hd, T):
         a = cache.prefill(k, v, qs)
         cache.crop(T)
         qs[S - 1, 0, 1, 5] = float("inf")
-        qs[2, 1, R + 2, 0] = float("nan")
+        qs[2, 1, R, 0] = float("nan")
         b = cache.prefill(k, v, qs)
         cache.crop(T)
         mask = torch.zeros(S, B, Hk * R, dtype=torch.bool, device=cuda)
-        mask[S - 1, 0, 1] = mask[2, 1, R + 2] = True
+        mask[S - 1, 0, 1] = mask[2, 1, R] = True
         assert torch.isnan(b[mask]).all()
         assert torch.equal(a[~mask], b[~mask])
 
