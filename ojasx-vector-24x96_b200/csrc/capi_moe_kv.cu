@@ -334,9 +334,9 @@ void ojasx_destroy_moe(OjasxMoEHandle handle) {
 }
 
 /* ------------------------------------------------------------------------- codebook-VQ KV */
-// Positions one batched decode launch takes (a chunk of prompt positions too short for the prefill kernel, or of a
-// shape that kernel does not cover).
-static constexpr int kKvqDecodePositions = 16;
+// Most positions that one batched decode launch takes, and fewest that the prefill kernel takes (shorter chunks, and shapes and
+// types that it does not cover, go through the decode kernels).
+static constexpr int kKvqDecodePositions = 64, kKvqPrefillPositions = 16;
 
 OjasxKvqHandle ojasx_b200_kvq_create(int batch, int kv_heads, int q_heads, int head_dim, int block_dim, int max_seq_len,
                                      const float* k_codebook, const float* v_codebook) {
@@ -478,7 +478,7 @@ int ojasx_b200_kvq_prefill(OjasxKvqHandle handle, const void* d_k, const void* d
     if (!h->static_plan && h->host_len + n_positions > h->max_seq) return OJX_ERR_RANGE;
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     const size_t esz = io_dtype == OJX_BF16 ? 2 : 4;
-    const size_t kv_pos = esz * h->B * h->Hkv * h->head_dim, q_pos = esz * h->B * h->Hq * h->head_dim;
+    const size_t q_pos = esz * h->B * h->Hq * h->head_dim;
     DeviceGuard g(h->dev);
     KvqProblem P = kvq_problem(h, io_dtype);
     P.scale = scale > 0.0f ? scale : 1.0f / std::sqrt((float)h->head_dim);
@@ -487,7 +487,7 @@ int ojasx_b200_kvq_prefill(OjasxKvqHandle handle, const void* d_k, const void* d
     // context is short.  Few positions on a long context split the context instead: the decode kernel with a position axis.
     const int R = h->Hq / h->Hkv, cached = h->static_plan ? h->max_seq : h->host_len;
     const long long ctas = (long long)((n_positions * R + 63) / 64) * h->Hkv * h->B;
-    if (n_positions >= kKvqDecodePositions && kvq_prefill_supported(P) && (2 * ctas >= num_sms() || cached <= 1024)) {
+    if (n_positions >= kKvqPrefillPositions && kvq_prefill_supported(P) && (2 * ctas >= num_sms() || cached <= 1024)) {
         int rc = launch_kvq_append_many(P, s);
         if (rc != OJX_OK) return rc;
         rc = launch_kvq_prefill_attention(P, s);
@@ -496,25 +496,24 @@ int ojasx_b200_kvq_prefill(OjasxKvqHandle handle, const void* d_k, const void* d
         return rc;
     }
     // as many positions as the scratch of one decode holds partial sums for, and a grid (z = positions x sequences) takes
-    const int batch = std::max(1, std::min({kKvqDecodePositions, kvq_splits(h), 65535 / h->B}));
-    for (int p0 = 0; p0 < n_positions; p0 += batch) {
-        P.n_pos = std::min(batch, n_positions - p0);
-        P.new_k = static_cast<const char*>(d_k) + p0 * kv_pos;
-        P.new_v = static_cast<const char*>(d_v) + p0 * kv_pos;
-        P.q = static_cast<const char*>(d_q) + p0 * q_pos;
-        P.out = static_cast<char*>(d_out) + p0 * q_pos;
-        const int T = h->static_plan ? h->max_seq : h->host_len + P.n_pos;
-        plan_kvq_decode(P, T, num_sms(), kvq_splits(h) / P.n_pos);
-        int rc = kvq_reserve(h);
-        if (rc != OJX_OK) return rc;
-        P.partials = static_cast<float*>(h->partials);
-        P.split_done = h->counters + h->B + (size_t)h->B * h->Hkv;
-        if ((rc = launch_kvq_append_many(P, s)) != OJX_OK) return rc;
-        if ((rc = launch_kvq_decode(P, s)) != OJX_OK) return rc;
-        if ((rc = launch_kvq_advance(P, s)) != OJX_OK) return rc;
-        if (!h->static_plan) h->host_len += P.n_pos;
+    const int most = h->static_plan ? h->max_seq : h->host_len + n_positions;
+    const int batch = std::max(1, std::min({kKvqDecodePositions, kvq_decode_positions(P, most, num_sms(), kvq_splits(h)), 65535 / h->B}));
+    int rc = kvq_reserve(h);
+    if (rc == OJX_OK) rc = launch_kvq_append_many(P, s);
+    for (int p0 = 0; rc == OJX_OK && p0 < n_positions; p0 += batch) {
+        KvqProblem Q = P;
+        Q.n_pos = std::min(batch, n_positions - p0);
+        Q.pos0 = p0;
+        Q.q = static_cast<const char*>(d_q) + p0 * q_pos;
+        Q.out = static_cast<char*>(d_out) + p0 * q_pos;
+        Q.partials = static_cast<float*>(h->partials);
+        Q.split_done = h->counters + h->B + (size_t)h->B * h->Hkv;
+        plan_kvq_decode(Q, h->static_plan ? h->max_seq : h->host_len + p0 + Q.n_pos, num_sms(), kvq_splits(h) / Q.n_pos);
+        rc = launch_kvq_decode(Q, s);
     }
-    return OJX_OK;
+    if (rc == OJX_OK) rc = launch_kvq_advance(P, s);
+    if (rc == OJX_OK && !h->static_plan) h->host_len += n_positions;
+    return rc;
 }
 
 int ojasx_b200_kvq_set_static_plan(OjasxKvqHandle handle, int enabled) {

@@ -120,7 +120,8 @@ struct KvqProblem {
     int out_heads;          // query heads of a row of `out` (0: Hq); > Hq when this cache holds a KV-head shard and
     int out_head0;          // writes its heads at [out_head0, out_head0 + Hq) of the gathered output
     int n_pos;              // > 0: a chunk of prompt positions; q, out [n_pos, B, Hq, head_dim], new_k, new_v [n_pos, B, Hkv, head_dim],
-                            // seq_lens holds the lengths before the chunk and position s sees seq_lens[b] + s + 1 tokens
+                            // seq_lens holds the lengths before the chunk and position s sees seq_lens[b] + pos0 + s + 1 tokens
+    int pos0;               // positions of the chunk before these (a decode takes a chunk in several launches)
 };
 
 inline int round_up(int a, int b) { return (a + b - 1) / b * b; }

@@ -17,6 +17,11 @@
 // kernel and this: 2048 tokens, 8 KV heads of 4 query heads 16.9 / 12.6; 32768 tokens x 16 215 / 178; 8000 x 4 with 8 query
 // heads 55 / 35; 500 x 16 with 8 query heads of 64 18.0 / 11.8; 130000 62 / 60.  One or two query heads per KV head fill a
 // quarter or half of the columns and lose (8000 x 4: 16.4 / 27.4 and 19.7 / 29.3): they keep the query-table kernel.
+//
+// bf16 queries and outputs only.  A pair of fp16 numbers is one bit short of fp32, and that shows: fp32 outputs were off by 1.03e-7
+// to 1.28e-7 against 64 bits where the query-table kernel's are by 0.85e-7 to 1.2e-7 (500 to 32768 tokens, head_dim 128).
+// Adding every product's high parts in fp32 and reducing the exponents exactly changed nothing.  In bf16 the output's
+// own rounding is 1.7e-3 on either kernel.
 #include <algorithm>
 #include <atomic>
 
@@ -79,7 +84,7 @@ __global__ void __launch_bounds__(kKdThreads, 1) kvq_decode_mma_kernel(const __g
     cudaGridDependencySynchronize();   // the append before this launch: lengths, codes; the query
 
     auto length = [&](int z) {
-        const int T = P.n_pos > 0 ? min(P.seq_lens[z % P.B] + z / P.B + 1, P.max_seq) : P.seq_lens[z];
+        const int T = P.n_pos > 0 ? min(P.seq_lens[z % P.B] + P.pos0 + z / P.B + 1, P.max_seq) : P.seq_lens[z];
         return min(T, P.n_chunks * P.chunk);   // what the plan and its scratch were made for
     };
     auto chunks = [&](int z) { return (length(z) + P.chunk - 1) / P.chunk; };
@@ -396,7 +401,7 @@ __global__ void __launch_bounds__(kKdThreads, 1) kvq_decode_mma_kernel(const __g
 
 bool kvq_decode_mma_supported(const KvqProblem& P) {
     const int R = P.Hq / P.Hkv;
-    return P.even_books && P.D == 8 && (P.G == 8 || P.G == 16) && P.head_dim == P.G * 8 && (R == 4 || R == 8);
+    return P.io_dtype == OJX_BF16 && P.even_books && P.D == 8 && (P.G == 8 || P.G == 16) && P.head_dim == P.G * 8 && (R == 4 || R == 8);
 }
 
 template <int R, int G>

@@ -420,10 +420,13 @@ static int launch_prefill_d(const KvqProblem& P, cudaStream_t s) {
     }
 }
 
-// Codebooks that high and low parts do not hold to fp32 accuracy (infinities, wide ranges) keep the decode kernel.
+// bf16 only: a pair of fp16 numbers is one bit short of fp32, so that fp32 outputs would be off by up to 1.5 times as much as
+// position by position (512 positions 8.3e-8 against 7.8e-8, 1000 behind 4000 tokens 1.6e-7 against 1.1e-7).  fp32 chunks go
+// through the query-table kernel, as many positions a launch as the scratch of a decode holds.  Codebooks that high and low parts do not hold (infinities, wide
+// ranges) do so in bf16 too.
 bool kvq_prefill_supported(const KvqProblem& P) {
     const int R = P.Hq / P.Hkv;
-    return P.even_books && R <= kPfRows && kPfRows % R == 0 && P.G % 4 == 0 && P.B <= 65535 && P.Hkv <= 65535 &&
+    return P.io_dtype == OJX_BF16 && P.even_books && R <= kPfRows && kPfRows % R == 0 && P.G % 4 == 0 && P.B <= 65535 && P.Hkv <= 65535 &&
            (P.head_dim == 64 || P.head_dim == 128) && (P.D == 4 || P.D == 8 || P.D == 16);
 }
 

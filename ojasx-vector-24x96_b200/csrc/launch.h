@@ -90,6 +90,8 @@ inline int kvq_scratch_splits(int max_seq, int heads, int sms) {
 }
 // Fills P.chunk (tokens per CTA) and P.n_chunks (<= max_splits, what the scratch holds per position) for a context of T tokens.
 void plan_kvq_decode(KvqProblem& P, int T, int sms, int max_splits);
+// Positions whose partial sums fit a scratch of max_splits per (sequence, KV head).
+int kvq_decode_positions(KvqProblem P, int T, int sms, int max_splits);
 int launch_kvq_append(const KvqProblem& P, cudaStream_t stream);
 int launch_kvq_decode(const KvqProblem& P, cudaStream_t stream, const PeerLink* link = nullptr);
 // --- kv_decode_mma.cu: decode for block_dim 8 and head_dim 64 or 128 (launch_kvq_decode takes it where it fits)

@@ -204,3 +204,44 @@ def test_codebooks_of_wide_range_keep_fp32_accuracy(cuda, oracle, which, row, co
         for d in range(hd):     # dimensions of other sizes: each to its own
             size = np.abs(want[:, :, d]).max()
             assert np.abs(got[i][:, :, d] - want[:, :, d]).max() <= 1e-5 * size, (i, d)
+
+
+def _rms(a, want):
+    return np.sqrt(((a.astype(np.float64) - want) ** 2).sum() / (want ** 2).sum())
+
+
+@pytest.mark.parametrize("R,hd,T", [(4, 128, 2048), (8, 128, 2048), (4, 64, 700), (8, 128, 9000)])
+@pytest.mark.parametrize("positions", [0, 40])
+def test_fp32_keeps_fp32_accuracy(cuda, monkeypatch, R, hd, T, positions):
+    """fp32 outputs are as close to 64 bits as the query-table kernel's, in a decode and in a chunk of positions (the same
+    splits; a twentieth for the order of the sums); in bf16 both round the same numbers."""
+    B, Hk = 2, 4
+    cache, books, codes, rng = _cache(B, Hk, R, hd, T, T + positions + 1, R + T)
+    S = max(1, positions)
+    k, v = (torch.from_numpy((rng.standard_normal((S, B, Hk, hd)) / np.sqrt(hd)).astype(np.float32)).to(cuda) for _ in range(2))
+    q = torch.from_numpy(rng.standard_normal((S, B, Hk * R, hd)).astype(np.float32)).to(cuda)
+
+    def outputs(dtype, table):
+        if table:
+            monkeypatch.setenv("OJASX_B200_KV_DECODE", "table")
+        cache.crop(T)
+        if positions and not table:
+            out = cache.prefill(k.to(dtype), v.to(dtype), q.to(dtype))
+        else:
+            out = torch.empty(q.shape, dtype=dtype, device=cuda)
+            for s in range(S):
+                if positions:
+                    cache.append(k[s].to(dtype), v[s].to(dtype))
+                cache.decode(q[s].to(dtype), out=out[s])
+        monkeypatch.delenv("OJASX_B200_KV_DECODE", raising=False)
+        return out
+
+    for dtype in (torch.float32, torch.bfloat16):
+        got, table = (outputs(dtype, t).float().cpu().numpy() for t in (False, True))
+        kc, vc = cache.read(0, T + positions) if positions else codes
+        want = np.stack([_exact(books, [kc[:, :, :T + (s + 1 if positions else 0)], vc[:, :, :T + (s + 1 if positions else 0)]],
+                                q[s].to(dtype).float().cpu().numpy(), 1.0 / np.sqrt(hd)) for s in range(S)])
+        if dtype is torch.float32:
+            assert _rms(got, want) <= 1.05 * _rms(table, want), (_rms(got, want), _rms(table, want))
+        else:
+            assert _rms(got, want) <= 1.0005 * _rms(table, want)
