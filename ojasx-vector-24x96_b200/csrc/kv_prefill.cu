@@ -8,6 +8,7 @@
 #include <cuda_fp16.h>
 
 #include <algorithm>
+#include <cfloat>
 
 #include "common.cuh"
 #include "handles.h"
@@ -223,7 +224,8 @@ __global__ void __launch_bounds__(kPfThreads) kvq_prefill_kernel(const __grid_co
     }
     __syncthreads();
 
-    float o[HD / 8][4], m_run[2] = {-INFINITY, -INFINITY}, l_run[2] = {0.0f, 0.0f}, l_err[2] = {0.0f, 0.0f};
+    // The running maximum starts at the lowest finite number: scores of -inf (they may overflow) then weigh 0, those of NaN NaN.
+    float o[HD / 8][4], m_run[2] = {-FLT_MAX, -FLT_MAX}, l_run[2] = {0.0f, 0.0f}, l_err[2] = {0.0f, 0.0f};
 #pragma unroll
     for (int n = 0; n < HD / 8; ++n)
 #pragma unroll
@@ -320,7 +322,7 @@ __global__ void __launch_bounds__(kPfThreads) kvq_prefill_kernel(const __grid_co
         for (int i = 0; i < 2; ++i) {
             mt[i] = fmaxf(mt[i], __shfl_xor_sync(0xffffffffu, mt[i], 1));
             mt[i] = fmaxf(mt[i], __shfl_xor_sync(0xffffffffu, mt[i], 2));
-            const float m = fmaxf(m_run[i], mt[i]);              // finite from the first tile on: every row sees token 0
+            const float m = fmaxf(m_run[i], mt[i]);
             const float alpha = exp2f(m_run[i] - m);
             m_run[i] = m;
             base[i] = m;
@@ -383,7 +385,7 @@ __global__ void __launch_bounds__(kPfThreads) kvq_prefill_kernel(const __grid_co
         l_run[i] += __shfl_xor_sync(0xffffffffu, l_run[i], 2);
         const int row = warp * 16 + g + 8 * i, s = s0 + row / R;
         if (s >= P.n_pos) continue;
-        const float inv = inv_kv[1] * (1.0f / 16384.0f) / l_run[i];
+        const float inv = l_run[i] == 0.0f ? 0.0f : inv_kv[1] * (1.0f / 16384.0f) / l_run[i];
         const size_t base = (((size_t)s * P.B + b) * P.Hq + (size_t)h * R + row % R) * HD;
 #pragma unroll
         for (int n = 0; n < HD / 8; ++n)

@@ -143,9 +143,9 @@ def test_non_finite_queries(cuda, R, hd, T):
             mask[0, 1] = mask[1, R] = True
             assert torch.isnan(got[mask]).all(), got[mask]
             assert torch.equal(got[~mask], ok[~mask])
-    for S in (15, 16):
-        k, v = (torch.randn(S, B, Hk, hd, device=cuda) / hd ** 0.5 for _ in range(2))
-        qs = torch.randn(S, B, Hk * R, hd, device=cuda)
+    for S, dtype in ((15, torch.float32), (16, torch.float32), (15, torch.bfloat16), (16, torch.bfloat16)):
+        k, v = ((torch.randn(S, B, Hk, hd, device=cuda) / hd ** 0.5).to(dtype) for _ in range(2))
+        qs = torch.randn(S, B, Hk * R, hd, device=cuda).to(dtype)
         a = cache.prefill(k, v, qs)
         cache.crop(T)
         qs[S - 1, 0, 1, 5] = float("inf")
@@ -245,3 +245,28 @@ def test_fp32_keeps_fp32_accuracy(cuda, monkeypatch, R, hd, T, positions):
             assert _rms(got, want) <= 1.05 * _rms(table, want), (_rms(got, want), _rms(table, want))
         else:
             assert _rms(got, want) <= 1.0005 * _rms(table, want)
+
+
+
+def test_chunk_whose_first_scores_overflow(cuda, monkeypatch):
+    """A tile of 64 tokens whose scores are all -inf for one head, before tokens of finite scores: weights 0, as one by one."""
+    B, Hk, R, hd, T, S = 1, 2, 4, 128, 200, 16
+    rng = np.random.default_rng(0)
+    books = [rng.uniform(0.5, 1.5, (Hk, 256, 8)).astype(np.float32) for _ in range(2)]
+    books[0][:, :128] *= 1e-3
+    books[0][:, 128:] *= -1
+    codes = [rng.integers(0, 128, (B, Hk, T, hd // 8), dtype=np.uint8) for _ in range(2)]
+    codes[0][:, :, :100] += 128
+    cache = ops.VQKVCache(B, Hk, Hk * R, hd, 8, T + S, *books)
+    cache.load(*codes)
+    k = torch.zeros(S, B, Hk, hd, device=cuda, dtype=torch.bfloat16)
+    q = torch.rand(S, B, Hk * R, hd, device=cuda, generator=torch.Generator(cuda).manual_seed(0)) + 0.5
+    q[:, 0, 6] *= 1e38
+    q = q.bfloat16()
+    got = cache.prefill(k, k, q)
+    cache.crop(T)
+    monkeypatch.setenv("OJASX_B200_KV_DECODE", "table")
+    for s in range(S):
+        cache.append(k[s], k[s])
+        want = cache.decode(q[s])
+        assert torch.isfinite(want).all() and torch.allclose(got[s].float(), want.float(), rtol=2 ** -7, atol=1e-5), s
