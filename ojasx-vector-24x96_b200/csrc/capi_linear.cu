@@ -209,26 +209,43 @@ int ojasx_b200_linear_forward(OjasxLinearHandle handle, const void* d_x, void* d
     return launch_linear(P, static_cast<cudaStream_t>(stream));
 }
 
-// (code, vector) pairs from which a single linear takes the gather kernel; OJASX_B200_GATHER_MIN_WORK overrides (0: every
-// call that fits, negative: never).  Its second launch costs the host 5 us, which smaller calls do not win back (2560 to
-// 2560 columns, us per call in a loop, table kernels against this: batch 1 15.5 / 22.7, batch 4 22.9 / 22.6, batch 8
-// 24.9 / 22.2; 2560 to 6912, batch 2: 24.9 / 22.8).
-static long long gather_min_work() {
+// OJASX_B200_GATHER_MIN_WORK: (code, vector) pairs from which a single linear takes the gather kernel, instead of gather_pays
+// (0: every call that fits, negative: never).
+static bool gather_min_work(long long* pairs) {
     const char* e = getenv("OJASX_B200_GATHER_MIN_WORK");
-    return e ? atoll(e) : 3000000;
+    if (e) *pairs = atoll(e);
+    return e != nullptr;
+}
+
+// Whether the gather kernel is the faster one for a single linear.  us on the device, fitted to a sweep of ten widths, six row
+// counts and five batches: the table kernel takes 4.5 + 0.052 per group + 0.4 per million (code, vector) pairs, this path
+// 9 + 2.5 per million codes + 0.16 per million pairs + 0.2 per thousand rows.  Its second launch keeps a call of a Python loop
+// above 18.5 us, where the other's floor is 13.4, so it also takes a table time of 17.  us per call in a loop, tables / this:
+//   1024 columns: 4096 rows x 16 vectors 16.6 / 18.5, x 31 20.6 / 18.6; 16384 x 8 20.1 / 20.9, x 16 25.3 / 24.7
+//   2560 columns: 8192 rows x 2 24.7 / 18.6; 16384 x 2 25.5 / 26.9, x 4 29.3 / 28.9
+// Widths of other than whole 128 dimensions take the tables' slow walk (2112 to 2048, 4 vectors: 36.9 / 18.5), one or two
+// vectors and few rows the cluster kernel (4096 to 4096, 2 vectors: 28.8 / 18.9): there three million pairs decide.
+static bool gather_pays(const LinearProblem& P) {
+    const double rows = P.row_stop - P.row_start, codes = rows * P.G * 1e-6, pairs = codes * P.batch;
+    if (pairs < 3.0) return false;
+    if (P.G % 16 != 0 || (P.batch <= 2 && rows * P.batch <= 12288)) return true;
+    return 4.5 + 0.052 * P.G + 0.4 * pairs >= std::max(17.0, 9.0 + 2.5 * codes + 0.16 * pairs + 0.2e-3 * rows);
 }
 
 // Whether the gather kernel (gather_mma.cu) may take a call; the switches of the other paths come first.  With a codebook of wide
 // range its window is wide too and most sums are evaluated twice (one entry of 1e30: 274 us, table kernels 114, 35 without it).
 static bool gather_mma_open(const LinearProblem& P, bool csr_sorted, bool even_book) {
-    if (!even_book || !gather_mma_supported(P) || linear_cluster_disabled() || gather_min_work() < 0) return false;
+    long long least = 0;
+    if (!even_book || !gather_mma_supported(P) || linear_cluster_disabled() || (gather_min_work(&least) && least < 0)) return false;
     const char* e = getenv("OJASX_B200_TENSOR_MIN_BATCH");
     const int min_batch = e ? atoi(e) : kTensorMinBatch;
     return !(min_batch > 0 && P.batch >= min_batch && dequant_gemm_supported(P, csr_sorted));
 }
 
 static bool wants_gather_mma(const LinearProblem& P, bool csr_sorted, bool even_book) {
-    return gather_mma_open(P, csr_sorted, even_book) && (long long)(P.row_stop - P.row_start) * P.G * P.batch >= gather_min_work();
+    if (!gather_mma_open(P, csr_sorted, even_book)) return false;
+    long long least = 0;
+    return gather_min_work(&least) ? (long long)(P.row_stop - P.row_start) * P.G * P.batch >= least : gather_pays(P);
 }
 
 size_t ojasx_b200_linear_workspace(OjasxLinearHandle handle, int batch_size, int io_dtype) {

@@ -3,6 +3,7 @@ import numpy as np
 import pytest
 import torch
 
+import ojasx_b200
 from ojasx_b200 import ops, synth
 
 pytestmark = pytest.mark.gpu
@@ -54,3 +55,21 @@ def test_rmsnorm_register_limit(cuda, rows, hidden, dtype):
     # sums of up to 4097 squares in fp32 in a tree of 256 threads, one rounding to the output type
     tol = 2.0 ** -8 if dtype == torch.bfloat16 else 2.0 ** -20
     assert torch.all((got.double() - want).abs() <= tol * want.abs() + 1e-6)
+
+
+@pytest.mark.parametrize("K,M,batch,gather", [
+    (1024, 3456, 8, False), (1024, 3456, 16, False), (1024, 8192, 31, True),     # narrow: the tables win up to many vectors
+    (2560, 8192, 2, True), (2560, 16384, 2, False), (2560, 16384, 16, True),     # many rows, few vectors
+    (2560, 2304, 4, False), (2560, 2432, 4, True),                               # three million pairs
+    (1600, 2048, 8, True),                                                       # not whole 128 dimensions
+    (4096, 4096, 2, True),                                                       # against the cluster kernel
+])
+def test_linear_tables_and_gathered_operands_meet(cuda, monkeypatch, K, M, batch, gather):
+    """The rule that gives a bf16 layer to one kernel or the other, and the bits of both."""
+    layer = ops.VQLinear.from_weights(synth.make_vq_linear(K + M, K, M, block_dim=8))
+    x = torch.randn(batch, K, device=cuda, generator=torch.Generator(cuda).manual_seed(M)).bfloat16()
+    n0 = ojasx_b200.launch_count()
+    got = layer(x)
+    assert ojasx_b200.launch_count() - n0 == (2 if gather else 1)
+    monkeypatch.setenv("OJASX_B200_GATHER_MIN_WORK", "-1" if gather else "0")
+    assert torch.equal(layer(x), got)
