@@ -94,9 +94,9 @@ def test_scratch_of_a_cache(cuda, cap, R):
 
 
 @pytest.mark.parametrize("B,Hkv,R,hd,T0,S", [
-    (1, 1, 4, 64, 20000, 15),        # one head: 256 partial sums, 17 per position
+    (1, 1, 4, 64, 20000, 15),        # one head: three positions of 79 splits per launch
     (16, 8, 4, 128, 300, 9),         # more heads than half the SMs: three positions per launch
-    (20, 8, 2, 64, 40, 5),           # the table kernel, two per launch
+    (20, 8, 2, 64, 40, 5),           # two per launch
 ])
 def test_positions_share_the_scratch_of_one_decode(cuda, B, Hkv, R, hd, T0, S):
     books, old, k, v, q = _make(7, B, Hkv, Hkv * R, hd, 8, T0, S)
