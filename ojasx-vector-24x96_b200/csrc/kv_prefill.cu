@@ -5,12 +5,10 @@
 //
 // Appending and decoding position by position cost two launches per position and layer: a chunk
 // of 512 positions took 512 x (14.7 + 5.6) us plus the gaps between launches, 13 ms per layer.
-#include <cuda_fp16.h>
-
 #include <algorithm>
 #include <cfloat>
 
-#include "common.cuh"
+#include "gather_mma.cuh"
 #include "handles.h"
 #include "launch.h"
 
@@ -110,21 +108,6 @@ __global__ void kvq_advance_kernel(int* seq_lens, int B, int n, int max_seq) {
 // another's expansion of the codes.
 constexpr int kPfThreads = 128, kPfRows = 64, kPfTok = 64;
 
-__device__ __forceinline__ void pf_ldsm4(uint32_t addr, uint32_t (&r)[4]) {
-    asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0, %1, %2, %3}, [%4];"
-                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
-                 : "r"(addr));
-}
-__device__ __forceinline__ void pf_ldsm4t(uint32_t addr, uint32_t (&r)[4]) {
-    asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0, %1, %2, %3}, [%4];"
-                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
-                 : "r"(addr));
-}
-__device__ __forceinline__ void pf_mma(float (&c)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
-    asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
-                 : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
-                 : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
-}
 // (a, b) as packed fp16 high parts and the packed fp16 remainders
 __device__ __forceinline__ void pf_split2(float a, float b, uint32_t& hi, uint32_t& lo) {
     const __half ha = __float2half_rn(a), hb = __float2half_rn(b);
@@ -293,13 +276,13 @@ __global__ void __launch_bounds__(kPfThreads) kvq_prefill_kernel(const __grid_co
                 for (int kk = k2; kk < k2 + 2; ++kk) {
                     uint32_t bh[4], bl[4];
                     const uint32_t a = kh_a + (n2 * 16 * LD + kk * 16) * 2;
-                    pf_ldsm4(a, bh);
-                    pf_ldsm4(a + kPart, bl);
+                    gm_ldsm4(a, bh);
+                    gm_ldsm4(a + kPart, bl);
 #pragma unroll
                     for (int j = 0; j < 2; ++j) {
-                        pf_mma(t[j], qh[kk], bl[2 * j], bl[2 * j + 1]);
-                        pf_mma(t[j], ql[kk], bh[2 * j], bh[2 * j + 1]);
-                        pf_mma(t[j], qh[kk], bh[2 * j], bh[2 * j + 1]);
+                        gm_mma(t[j], qh[kk], bl[2 * j], bl[2 * j + 1]);
+                        gm_mma(t[j], ql[kk], bh[2 * j], bh[2 * j + 1]);
+                        gm_mma(t[j], qh[kk], bh[2 * j], bh[2 * j + 1]);
                     }
                 }
 #pragma unroll
@@ -362,14 +345,14 @@ __global__ void __launch_bounds__(kPfThreads) kvq_prefill_kernel(const __grid_co
             for (int j2 = 0; j2 < kPfTok / 16; j2 += 2) {
                 uint32_t bh[4], bl[4];          // eight dimensions of 32 tokens
                 const uint32_t a = vt_a + (j2 * 16 * LD + n1 * 8) * 2;
-                pf_ldsm4t(a, bh);
-                pf_ldsm4t(a + kPart, bl);
+                gm_ldsm4t(a, bh);
+                gm_ldsm4t(a + kPart, bl);
 #pragma unroll
                 for (int j = 0; j < 2; ++j) {
                     float t[4] = {0.0f, 0.0f, 0.0f, 0.0f};
-                    pf_mma(t, ph[j2 + j], bl[2 * j], bl[2 * j + 1]);
-                    pf_mma(t, pl[j2 + j], bh[2 * j], bh[2 * j + 1]);
-                    pf_mma(t, ph[j2 + j], bh[2 * j], bh[2 * j + 1]);
+                    gm_mma(t, ph[j2 + j], bl[2 * j], bl[2 * j + 1]);
+                    gm_mma(t, pl[j2 + j], bh[2 * j], bh[2 * j + 1]);
+                    gm_mma(t, ph[j2 + j], bh[2 * j], bh[2 * j + 1]);
 #pragma unroll
                     for (int i = 0; i < 4; ++i) sum[i] = j2 + j == 0 ? t[i] : sum[i] + t[i];
                 }
