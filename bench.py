@@ -799,7 +799,7 @@ def bench_stack(args, E):
                         "decode_tokens_per_s": round(B * args.stack_new / dt_dec, 1),
                         "ms_per_decode_step": round(dt_dec / args.stack_new * 1e3, 3),
                         "prompt": args.stack_prompt, "new_tokens": args.stack_new, "dtype": args.stack_dtype,
-                        "prefill": "positions batched through linears and MoE, attention position by position" if E.seg is None
+                        "prefill": "positions batched through linears, MoE and attention" if E.seg is None
                                    else "token by token through the sharded decode step",
                         "bytes_per_step_estimate": int(step_bytes),
                         "roofline": hbm_roofline(step_bytes, dt_dec / args.stack_new, E.world,

@@ -1,4 +1,4 @@
-// Products of a VQ-coded weight tile with a few activation vectors on the tensor cores, at fp32 accuracy.
+// Products of a VQ-coded weight tile with a few activation vectors on the tensor cores, at 22 bits and fp32 sums.
 //
 // The 8-dimensional centroids are the rows that ldmatrix reads: an 8x8 matrix of fp16 is eight 16-byte rows at
 // any eight addresses, so the lanes hand it the addresses of the centroids that the code bytes name and the A
@@ -7,7 +7,7 @@
 // 16-byte bank group q and the eight rows of a matrix read eight different copies, four wavefronts for 32 codes
 // whatever the codes are.
 //
-// fp32 accuracy from fp16 operands: the codebook is scaled by a power of two (largest element in [2^14, 2^15)) and
+// 22 bits from fp16 operands: the codebook is scaled by a power of two (largest element in [2^14, 2^15)) and
 // split into x = hi + lo, 22 bits of mantissa; activations are scaled the same way per vector and 256 dimensions.
 // A bf16 activation is then one exact fp16 number (elements 2^29 below the largest of their 256 lose bits), and
 // hi * x + lo * x is accumulated in fp32.

@@ -13,13 +13,14 @@
 // with its own running maximum, so the main loop has no barrier; the warps are merged at the end of a run, the runs by the
 // last CTA of a (sequence, head).
 // Bound: shared-memory wavefronts, 4 per ldmatrix: 64 bytes of K and V centroid parts per code pair, 8 clocks per token at
-// 16 groups and 1 for the softmax's shuffles; measured 12 (L1 pipe 85 % busy, tensor pipe 34 %).  us per decode, query-table
-// kernel and this: 2048 tokens, 8 KV heads of 4 query heads 16.9 / 12.6; 32768 tokens x 16 215 / 178; 8000 x 4 with 8 query
-// heads 55 / 35; 500 x 16 with 8 query heads of 64 18.0 / 11.8; 130000 62 / 60.  One or two query heads per KV head fill a
-// quarter or half of the columns and lose (8000 x 4: 16.4 / 27.4 and 19.7 / 29.3): they keep the query-table kernel.
+// 16 groups and 1 for the softmax's shuffles; measured 12 (L1 pipe 75 % busy, tensor pipe 29 % at 16384 tokens x 8).  us per
+// decode, query-table kernel and this: 2048 tokens, 8 KV heads of 4 query heads 17.2 / 12.3; 32768 tokens x 16 213 / 180; 8000 x
+// 4 with 8 query heads 55.7 / 34.4; 500 x 16 with 8 query heads of 64 17.7 / 11.5; 8000 x 4 with 4 of 64 19.2 / 15.9.  One or two
+// query heads per KV head fill a quarter or half of the columns and lose (8000 x 4: 16.4 / 27.4 and 19.7 / 29.3): they keep the
+// query-table kernel.
 //
 // bf16 queries and outputs only.  A pair of fp16 numbers is one bit short of fp32, and that shows: fp32 outputs were off by 1.03e-7
-// to 1.28e-7 against 64 bits where the query-table kernel's are by 0.85e-7 to 1.2e-7 (500 to 32768 tokens, head_dim 128).
+// to 1.28e-7 against 64 bits where the query-table kernel's are by 0.85e-7 to 1.17e-7 (500 to 8000 tokens, head_dim 128).
 // Adding every product's high parts in fp32 and reducing the exponents exactly changed nothing.  In bf16 the output's
 // own rounding is 1.7e-3 on either kernel.
 #include <algorithm>

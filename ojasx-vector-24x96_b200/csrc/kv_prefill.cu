@@ -94,13 +94,10 @@ __global__ void kvq_advance_kernel(int* seq_lens, int B, int n, int max_seq) {
 // Per tile of 64 tokens the codes are expanded into shared memory once and serve all 64 rows; scores
 // and values are mma.sync products with an online softmax between them, causal per row.
 //
-// fp32 accuracy from fp16 products: every operand is scaled by a power of two (per query row, per
-// codebook, 2^14 for probabilities) so that its largest element is in [2^13, 2^15), and split
-// into x = hi + lo with two fp16 numbers: 22 bits of mantissa down to 2^-24 of the largest element.
-// hi*hi + hi*lo + lo*hi are accumulated in fp32 (the dropped lo*lo is below 2^-22 of hi*hi), in runs short
-// enough that the tensor cores' truncation does not show (error against 64 bits with 1000 positions behind
-// 4000 tokens: 1.7e-7; 3.7e-7 with whole tiles accumulated there; 1.1e-7 position by position).  78 us per
-// layer of 512 positions with 32 query heads (70 with the long runs).
+// bf16 queries, keys and values as fp16 products: every operand is scaled by a power of two (per query row, per codebook, 2^14 for
+// probabilities) so that its largest element is in [2^14, 2^15), and split into x = hi + lo with two fp16 numbers: 22 bits of
+// mantissa.  hi*hi + hi*lo + lo*hi are accumulated in fp32, in runs short enough that the tensor cores' truncation does not show:
+// 8.3e-8 against 64 bits before the output is rounded, 512 positions.  78 us per layer of 512 positions with 32 query heads.
 //
 // Why mma.sync: three products of at most a few GFLOP per chunk and layer are a few microseconds
 // at any tensor rate; what the kernel needs is probabilities that go from the accumulators of the

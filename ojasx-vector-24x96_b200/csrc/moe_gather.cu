@@ -6,7 +6,9 @@
 // The table kernels spend a shared-memory gather per (code, token) and copy a token's 393 KB table for every pair.  Here a
 // code costs 32 bytes of shared-memory reads for up to sixteen tokens (eight in the down pass).  256 tokens of 512 experts
 // (hidden 2560, inter 640, top-10): expert passes 1.08 -> 0.74 ms; of 64 experts, the whole layer: 1.17 -> 0.54 ms.
-// Shared-memory pipe 85 % busy in the gate/up pass; a quarter of both passes are the outliers' reads of single elements.
+// L1 pipe 83 % busy in the gate/up pass, 81 % in the down pass (128 tokens of 64 experts); a quarter of both passes are the
+// outliers' reads of single elements.  Codebooks and intermediate vectors have 22 bits here; of the outputs 2.0e-4 to 2.9e-4 are
+// not the 64-bit result rounded to bf16, of the table kernels' 2.4e-4 to 4.1e-4 (ten layers of five shapes, fewer in each).
 //
 //   moe_gather_plan_kernel   pairs grouped by expert, cut into items of up to sixteen pairs
 //   moe_gather_prep_kernel   vectors as fp16 hi + lo fragments, scaled by a power of two per vector (tokens, then inter)
@@ -31,8 +33,12 @@
 namespace ojx {
 
 constexpr int kMgPairs = 16;                 // pairs of an item; the down pass takes them in two halves
+// As many warps as 96 registers a thread leave room for: 20 per SM, in one CTA (gate/up: the table and sixteen columns of the
+// hidden width fill the SM) or in two (down).  A warp takes units of 16 intermediate indices, or 32 hidden rows, of an item's
+// part; a part of fewer units than warps leaves the rest idle (inter 256: 8 of 20 in gate/up).  Two parts per item let SMs
+// that finish early share the last items.
 constexpr int kMgUpThreads = 640, kMgDownThreads = 320;
-constexpr int kMgParts = 2;                  // parts of an item that are claimed on their own
+constexpr int kMgParts = 2;
 
 struct MgArgs {
     MoeProblem P;

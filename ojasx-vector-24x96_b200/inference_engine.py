@@ -309,8 +309,9 @@ class VQDecoderStack:
         ``batched`` (default on one device): all positions of a chunk of the prompt go through the linears, the MoE and
         the attention as ONE batch -- the regime of the batched kernels: persistent table kernel in fp32, tensor-core
         dequant GEMM for bf16, causal attention over the chunk (``VQKVCache.prefill``).  Results are those of the
-        token-by-token form: bit for bit through linears and MoE, whose kernels keep their summation order whatever the
-        batch, and in fp32 rounding through the attention of chunks of 16 positions or more.  ``max_rows`` bounds
+        token-by-token form up to rounding: in fp32 bit for bit through linears and MoE, whose kernels keep their summation
+        order whatever the batch; in bf16 the kernels for batches add in other orders and the GEMM rounds its weights to
+        bf16.  ``max_rows`` bounds
         batch * positions per chunk (scratch of the MoE grows with it).  Otherwise, and on a stack split over several
         ranks, the prompt is fed through ``decode_step`` token by token."""
         if batched is None:
