@@ -119,7 +119,7 @@ def _us(f, n=20):
         b.record()
         b.synchronize()
         times.append(a.elapsed_time(b) * 1e3)
-    return sorted(times)[n // 2]
+    return min(times)    # the host may stall any call, but not make one faster
 
 
 def test_zero_vectors_and_zero_chunks_cost_nothing_extra(cuda, monkeypatch):

@@ -83,9 +83,14 @@ def test_scratch_of_a_cache(cuda, cap, R):
     """Partial sums: one per 256 tokens and query head (and what fills the SMs), for positions of a prompt in one launch too."""
     rng = np.random.default_rng(0)
     B, Hk, hd = 16, 8, 128
-    cache = ops.VQKVCache(B, Hk, Hk * R, hd, 8, cap, *(rng.standard_normal((Hk, 256, 8)).astype(np.float32) for _ in range(2)))
+    books = [rng.standard_normal((Hk, 256, 8)).astype(np.float32) for _ in range(2)]
     q = torch.randn(1, B, Hk * R, hd, device=cuda)
     k, v = (torch.randn(1, B, Hk, hd, device=cuda) for _ in range(2))
+    first = ops.VQKVCache(B, Hk, Hk * R, hd, 8, 16, *books)  # kernels are loaded on their first launch
+    first.append(k[0], v[0])
+    first.decode(q[0])
+    first.prefill(k, v, q)
+    cache = ops.VQKVCache(B, Hk, Hk * R, hd, 8, cap, *books)
     cache.append(k[0], v[0])
     torch.empty(64 << 20, device=cuda)                       # outputs come from the allocator's cache
     used = _used(lambda: (cache.decode(q[0]), cache.prefill(k, v, q)))
