@@ -12,6 +12,7 @@
 //     per-token abs-max scale (ojasx_lut_kv_cache.cpp:16-132, softmax of
 //     ojasx_lut_c_api.cpp:178-191).
 #include <algorithm>
+#include <cfloat>
 #include <cstdlib>
 
 #include "common.cuh"
@@ -192,14 +193,14 @@ __device__ __forceinline__ void kvq_merge_if_last(const KvqProblem& P, int b /* 
         float L = 0.0f, o = 0.0f;
         for (int c = 0; c < P.n_chunks; ++c) {
             const float* p = base + ((size_t)c * R + r) * (hd + 2);
-            const float m = __ldcg(p), l = __ldcg(p + 1);
-            if (m != -INFINITY || !(l == 0.0f)) {   // NaN weights (of a NaN query) have no maximum and stay NaN
-                const float wgt = m == -INFINITY ? 1.0f : __expf(m - M);
-                L += l * wgt;
+            const float m = __ldcg(p);
+            if (m != -INFINITY) {
+                const float wgt = __expf(m - M);
+                L += __ldcg(p + 1) * wgt;
                 o = fmaf(__ldcg(p + 2 + col), wgt, o);
             }
         }
-        o *= L == 0.0f ? 0.0f : 1.0f / L;
+        o *= L > 0.0f ? 1.0f / L : 0.0f;   // NaN stays NaN
         // a KV-head shard writes its heads into the gathered output of every rank (link.n > 0)
         const int row_heads = P.out_heads > 0 ? P.out_heads : P.Hq;
         const size_t oi = ((size_t)b * row_heads + P.out_head0 + (size_t)h * R + r) * hd + col;
@@ -298,11 +299,13 @@ __global__ void __launch_bounds__(kvq_decode_threads(R, D), 1) kvq_decode_kernel
     const int vu = vt_id / stripes, vst = vt_id - vu * stripes;   // unit, stripe
     const int vg = vu * kGp;                                      // first group of the unit
 
+    // Running maxima start at the lowest finite number: scores of -inf then weigh 0 and those of a NaN query NaN, and a partial
+    // of either counts in the merge (an empty range has -inf).
     if (score_warp) {
         float m_run[R], l_loc[R];
 #pragma unroll
         for (int r = 0; r < R; ++r) {
-            m_run[r] = -INFINITY;
+            m_run[r] = -FLT_MAX;
             l_loc[r] = 0.0f;
         }
         // G == 16 (one 16-byte row per token): the rows of the next pass are fetched a pass ahead, so the
@@ -470,7 +473,7 @@ __global__ void __launch_bounds__(kvq_decode_threads(R, D), 1) kvq_decode_kernel
                 float m = m_run[r];
 #pragma unroll
                 for (int w = 0; w < kWarpsHalf; ++w) m = fmaxf(m, wr[w * R + r]);
-                if (m != -INFINITY) l_loc[r] *= __expf(m_run[r] - m);   // factor 0 on the first pass (m_run = -inf, m finite)
+                l_loc[r] *= __expf(m_run[r] - m);
                 m_run[r] = m;
             }
             if (tid == 0) {
@@ -484,7 +487,7 @@ __global__ void __launch_bounds__(kvq_decode_threads(R, D), 1) kvq_decode_kernel
                     float p[R];
 #pragma unroll
                     for (int r = 0; r < R; ++r) {
-                        p[r] = __expf(s[j][r] - (m_run[r] == -INFINITY ? 0.0f : m_run[r]));   // every score -inf: 0; NaN: NaN
+                        p[r] = __expf(s[j][r] - m_run[r]);
                         l_loc[r] += p[r];
                     }
                     st_heads<R>(scb + (size_t)t * R, p);
@@ -505,7 +508,7 @@ __global__ void __launch_bounds__(kvq_decode_threads(R, D), 1) kvq_decode_kernel
         float m_run[R], o[kGp][R][D];
 #pragma unroll
         for (int r = 0; r < R; ++r) {
-            m_run[r] = -INFINITY;
+            m_run[r] = -FLT_MAX;
 #pragma unroll
             for (int i = 0; i < kGp; ++i)
 #pragma unroll
@@ -522,7 +525,7 @@ __global__ void __launch_bounds__(kvq_decode_threads(R, D), 1) kvq_decode_kernel
 #pragma unroll
             for (int r = 0; r < R; ++r) {
                 const float m = mpub[buf * R + r];
-                const float alpha = m == -INFINITY ? 1.0f : __expf(m_run[r] - m);
+                const float alpha = __expf(m_run[r] - m);
                 m_run[r] = m;
 #pragma unroll
                 for (int i = 0; i < kGp; ++i)
