@@ -66,7 +66,7 @@ MoeProblem MoeHandle::problem(const void* x, void* y, const int* idx, const floa
 KvqHandle::~KvqHandle() {
     DeviceGuard g(dev);
     cudaFree(k_codes); cudaFree(v_codes); cudaFree(k_cb); cudaFree(v_cb); cudaFree(seq_lens); cudaFree(error_flag); cudaFree(counters);
-    cudaFree(partials);
+    cudaFree(partials); cudaFree(pos_partials);
 }
 
 LegacyKvHandle::~LegacyKvHandle() {
@@ -362,6 +362,11 @@ OjasxKvqHandle ojasx_b200_kvq_create(int batch, int kv_heads, int q_heads, int h
     if (rc == OJX_OK) rc = upload((void**)&h->error_flag, nullptr, sizeof(int));
     // append: [B]; decode: [B * Hkv], and as many again for every position of a batched decode (kvq_prefill)
     if (rc == OJX_OK) rc = upload((void**)&h->counters, nullptr, sizeof(int) * ((size_t)batch + (size_t)(1 + kKvqDecodePositions) * batch * kv_heads));
+    // The partial sums of a decode: their size depends on the cache alone and they are allocated with it, so no decode waits for an
+    // allocation (half a millisecond of a first call) and none moves what a captured step points at.
+    h->splits = kvq_scratch_splits(max_seq_len, batch * kv_heads, num_sms());
+    h->pos_splits = kvq_position_splits(h->splits, batch * kv_heads, num_sms());
+    if (rc == OJX_OK) rc = upload((void**)&h->partials, nullptr, sizeof(float) * (size_t)batch * kv_heads * h->splits * (q_heads / kv_heads) * (head_dim + 2));
     if (rc != OJX_OK) { delete h; return nullptr; }
     return h;
 }
@@ -411,7 +416,7 @@ int ojasx_b200_kvq_reset(OjasxKvqHandle handle) {
 static KvqProblem kvq_problem(const KvqHandle* h, int io) {
     KvqProblem P{};
     P.k_codes = h->k_codes; P.v_codes = h->v_codes; P.k_cb = h->k_cb; P.v_cb = h->v_cb;
-    P.seq_lens = h->seq_lens; P.error_flag = h->error_flag; P.partials = static_cast<float*>(h->partials);
+    P.seq_lens = h->seq_lens; P.error_flag = h->error_flag; P.partials = h->partials;
     P.append_done = h->counters; P.split_done = h->counters + h->B;
     P.B = h->B; P.Hkv = h->Hkv; P.Hq = h->Hq; P.head_dim = h->head_dim; P.D = h->D; P.G = h->G; P.Kcb = 256;
     P.max_seq = h->max_seq; P.io_dtype = io; P.even_books = h->even_books;
@@ -431,15 +436,6 @@ int ojasx_b200_kvq_append(OjasxKvqHandle handle, const void* d_k, const void* d_
 
 static int kvq_decode_impl(OjasxKvqHandle handle, const void* d_q, void* d_out, float scale, int io_dtype, void* stream,
                            int out_heads, int out_head0, const PeerLink* link);
-
-static int kvq_splits(const KvqHandle* h) { return kvq_scratch_splits(h->max_seq, h->B * h->Hkv, num_sms()); }
-
-// The partial sums of a decode, or of a batch of positions.  The size depends on the cache alone, so neither a growing context
-// nor a prefill moves the scratch that a captured decode step points at.
-static int kvq_reserve(KvqHandle* h) {
-    return ensure_capacity(&h->partials, &h->partials_cap,
-                           sizeof(float) * (size_t)h->B * h->Hkv * kvq_splits(h) * (h->Hq / h->Hkv) * (h->head_dim + 2));
-}
 
 int ojasx_b200_kvq_decode(OjasxKvqHandle handle, const void* d_q, void* d_out, float scale, int io_dtype, void* stream) {
     return kvq_decode_impl(handle, d_q, d_out, scale, io_dtype, stream, 0, 0, nullptr);
@@ -461,11 +457,8 @@ static int kvq_decode_impl(OjasxKvqHandle handle, const void* d_q, void* d_out, 
     KvqProblem P = kvq_problem(h, io_dtype);
     P.q = d_q; P.out = d_out;
     P.scale = scale > 0.0f ? scale : 1.0f / std::sqrt((float)h->head_dim);
-    plan_kvq_decode(P, h->static_plan ? h->max_seq : h->host_len, num_sms(), kvq_splits(h));
+    plan_kvq_decode(P, h->static_plan ? h->max_seq : h->host_len, num_sms(), h->splits);
     DeviceGuard g(h->dev);
-    int rc = kvq_reserve(h);
-    if (rc != OJX_OK) return rc;
-    P.partials = static_cast<float*>(h->partials);
     P.out_heads = out_heads;
     P.out_head0 = out_head0;
     return launch_kvq_decode(P, static_cast<cudaStream_t>(stream), link);
@@ -495,10 +488,14 @@ int ojasx_b200_kvq_prefill(OjasxKvqHandle handle, const void* d_k, const void* d
         if (rc == OJX_OK && !h->static_plan) h->host_len += n_positions;
         return rc;
     }
-    // as many positions as the scratch of one decode holds partial sums for, and a grid (z = positions x sequences) takes
+    // as many positions as the scratch holds partial sums for, and a grid (z = positions x sequences) takes
     const int most = h->static_plan ? h->max_seq : h->host_len + n_positions;
-    const int batch = std::max(1, std::min({kKvqDecodePositions, kvq_decode_positions(P, most, num_sms(), kvq_splits(h)), 65535 / h->B}));
-    int rc = kvq_reserve(h);
+    const int batch = std::max(1, std::min({kKvqDecodePositions, kvq_decode_positions(P, most, num_sms(), h->pos_splits), 65535 / h->B}));
+    int rc = OJX_OK;
+    if (h->pos_splits > h->splits) {   // few heads: under a megabyte or two, always of one size
+        rc = ensure_capacity(&h->pos_partials, &h->pos_partials_cap, sizeof(float) * (size_t)h->B * h->Hkv * h->pos_splits * R * (h->head_dim + 2));
+        P.partials = static_cast<float*>(h->pos_partials);
+    }
     if (rc == OJX_OK) rc = launch_kvq_append_many(P, s);
     for (int p0 = 0; rc == OJX_OK && p0 < n_positions; p0 += batch) {
         KvqProblem Q = P;
@@ -506,9 +503,8 @@ int ojasx_b200_kvq_prefill(OjasxKvqHandle handle, const void* d_k, const void* d
         Q.pos0 = p0;
         Q.q = static_cast<const char*>(d_q) + p0 * q_pos;
         Q.out = static_cast<char*>(d_out) + p0 * q_pos;
-        Q.partials = static_cast<float*>(h->partials);
         Q.split_done = h->counters + h->B + (size_t)h->B * h->Hkv;
-        plan_kvq_decode(Q, h->static_plan ? h->max_seq : h->host_len + p0 + Q.n_pos, num_sms(), kvq_splits(h) / Q.n_pos);
+        plan_kvq_decode(Q, h->static_plan ? h->max_seq : h->host_len + p0 + Q.n_pos, num_sms(), h->pos_splits / Q.n_pos);
         rc = launch_kvq_decode(Q, s);
     }
     if (rc == OJX_OK) rc = launch_kvq_advance(P, s);
@@ -520,10 +516,6 @@ int ojasx_b200_kvq_set_static_plan(OjasxKvqHandle handle, int enabled) {
     if (!handle) return OJX_ERR_ARG;
     auto* h = static_cast<KvqHandle*>(handle);
     h->static_plan = enabled != 0;
-    if (h->static_plan) {   // size the chunk scratch for the full capacity now, so that decode never allocates
-        DeviceGuard g(h->dev);
-        return kvq_reserve(h);
-    }
     return OJX_OK;
 }
 

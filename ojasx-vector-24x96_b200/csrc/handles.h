@@ -128,8 +128,11 @@ struct KvqHandle {
     int* seq_lens = nullptr;
     int* error_flag = nullptr;
     int* counters = nullptr;                 // [B] append + [B*Hkv] decode completion counters (zero between launches)
-    void* partials = nullptr;
-    size_t partials_cap = 0;
+    float* partials = nullptr;               // [B * Hkv][splits] sums of a decode, allocated with the cache
+    int splits = 0;
+    void* pos_partials = nullptr;            // [B * Hkv][pos_splits] the same for prompt positions, where that is more
+    size_t pos_partials_cap = 0;
+    int pos_splits = 0;
     ~KvqHandle();
 };
 

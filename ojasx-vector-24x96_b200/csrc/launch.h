@@ -81,11 +81,18 @@ int take_moe_bulk_copy_error(int* out);   // moe.cu: a bounded wait for a bulk t
 // --- kv.cu
 constexpr int kKvMaxSplits = 256;   // context splits of one (sequence, KV head) in kvq decode
 size_t kvq_decode_smem(const KvqProblem& P, int R);
-// Partial sums that the scratch of a cache holds per (sequence, KV head): one per 256 tokens, or two per SM where there are few
-// heads.  A plan never makes more: its chunks are no shorter than 256 tokens or than an SM's share.  At 128 heads of 4 query
-// heads, head_dim 128 and 16384 tokens 17 MB (one per 64 tokens took 68, and as many for each of 16 positions 1.1 GB).
+// Partial sums that a decode may need per (sequence, KV head): one per 256 tokens, or where there are few heads what shares the
+// tokens out over the SMs.  A plan never makes more: its chunks are no shorter than 256 tokens or than an SM's share (64 at
+// least).  At 128 heads of 4 query heads, head_dim 128 and 16384 tokens 17 MB (one per 64 tokens took 68, and as many for each of
+// 16 positions 1.1 GB).
 inline int kvq_scratch_splits(int max_seq, int heads, int sms) {
-    const int tokens = (max_seq + 255) / 256, fill = (2 * sms + heads - 1) / heads, n = tokens > fill ? tokens : fill;
+    const int tokens = (max_seq + 255) / 256, least = (max_seq + 63) / 64, share = (sms + heads - 1) / heads;
+    const int few = least < share ? least : share, n = tokens > few ? tokens : few;
+    return n < kKvMaxSplits ? n : kKvMaxSplits;
+}
+// The same for positions of a prompt: enough for two CTAs per SM.
+inline int kvq_position_splits(int splits, int heads, int sms) {
+    const int fill = (2 * sms + heads - 1) / heads, n = splits > fill ? splits : fill;
     return n < kKvMaxSplits ? n : kKvMaxSplits;
 }
 // Fills P.chunk (tokens per CTA) and P.n_chunks (<= max_splits, what the scratch holds per position) for a context of T tokens.

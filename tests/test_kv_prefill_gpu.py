@@ -80,7 +80,8 @@ def _used(f):
 @pytest.mark.parametrize("cap", [8192, 16384, 32768])
 @pytest.mark.parametrize("R", [2, 4])
 def test_scratch_of_a_cache(cuda, cap, R):
-    """Partial sums: one per 256 tokens and query head (and what fills the SMs), for positions of a prompt in one launch too."""
+    """Partial sums: one per 256 tokens and query head (and what fills the SMs), for positions of a prompt in one
+    launch too; allocated with the cache, not in its first call."""
     rng = np.random.default_rng(0)
     B, Hk, hd = 16, 8, 128
     books = [rng.standard_normal((Hk, 256, 8)).astype(np.float32) for _ in range(2)]
@@ -90,12 +91,13 @@ def test_scratch_of_a_cache(cuda, cap, R):
     first.append(k[0], v[0])
     first.decode(q[0])
     first.prefill(k, v, q)
-    cache = ops.VQKVCache(B, Hk, Hk * R, hd, 8, cap, *books)
-    cache.append(k[0], v[0])
     torch.empty(64 << 20, device=cuda)                       # outputs come from the allocator's cache
-    used = _used(lambda: (cache.decode(q[0]), cache.prefill(k, v, q)))
-    need = 4 * B * Hk * (cap // 256) * R * (hd + 2)
+    made = []
+    used = _used(lambda: made.append(ops.VQKVCache(B, Hk, Hk * R, hd, 8, cap, *books)))
+    need = 2 * B * Hk * cap * (hd // 8) + 4 * B * Hk * (cap // 256) * R * (hd + 2)
     assert used <= need + (8 << 20), (used, need)            # the driver hands memory out in pieces of 2 MB
+    cache = made[0]
+    assert _used(lambda: (cache.append(k[0], v[0]), cache.decode(q[0]), cache.prefill(k, v, q))) == 0
 
 
 @pytest.mark.parametrize("B,Hkv,R,hd,T0,S", [
