@@ -93,6 +93,7 @@ struct MoeProblem {
     int lut_blocks;           // layout of lut_in: 0 = [token][group][256]; 1 = 16-group blocks (moe_prebuild_kernel);
                               // 2 = per-slice images of the chain walk's table area (moe_chain_prebuild_kernel);
                               // 3 = no tables: the fragments of moe_gather.cu, made by the expert launches
+                              // 4 = no tables: moe_gate_up_quad_kernel builds them for four tokens at a time
     int even_books;           // both codebooks fit pairs of fp16 numbers (book_fits_halves, checked when the handle is created)
 };
 

@@ -75,6 +75,15 @@ int launch_moe_prebuild_blocks(const void* x, int io_dtype, int n_tokens, int H,
 // --- moe_gather.cu: experts that several tokens are routed to, on mma.sync operands gathered from the codebooks
 bool moe_gather_wanted(const MoeProblem& P);
 int launch_moe_gather(const MoeProblem& P, cudaStream_t s, const PeerLink& link);   // all but the combine
+// Work list of the two: pairs grouped by expert, cut into items of up to `width` pairs.  plan [4 + 5 * pairs]: [0] items, [1], [2]
+// claim counters, [3] pairs, sorted pair ids, then (expert, first, count, -) per item.
+int launch_moe_item_plan(const MoeProblem& P, int* plan, int width, cudaStream_t s);
+// --- lut_quad.cu: four vectors at a time in the reference's order of additions
+bool quad_linear_pays(const LinearProblem& P);
+int launch_quad_linear(LinearProblem P, cudaStream_t s, const PeerLink& link);
+bool moe_quad_wanted(const MoeProblem& P);
+int launch_moe_quad(const MoeProblem& P, cudaStream_t s, const PeerLink& link);   // all but the combine
+int take_quad_error(int* out);
 int take_moe_fused_error(int* out);
 int take_moe_bulk_copy_error(int* out);   // moe.cu: a bounded wait for a bulk table copy ran out
 

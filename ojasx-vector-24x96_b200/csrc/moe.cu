@@ -959,7 +959,7 @@ static int launch_moe_experts_t(const MoeProblem& P, cudaStream_t s, const PeerL
 }
 
 // Layout of the token tables this forward wants (MoeProblem::lut_blocks).
-int moe_table_layout(const MoeProblem& P) { return moe_fused_wanted(P) ? 1 : moe_gather_wanted(P) ? 3 : moe_chain_wanted(P) ? 2 : 0; }
+int moe_table_layout(const MoeProblem& P) { return moe_fused_wanted(P) ? 1 : moe_gather_wanted(P) ? 3 : moe_quad_wanted(P) ? 4 : moe_chain_wanted(P) ? 2 : 0; }
 
 int launch_moe_experts(MoeProblem P, cudaStream_t s, const PeerLink* lk) {
     if (!P.x || !P.y || !P.topk_idx || !P.topk_w || !P.inter || !P.expert_out) return OJX_ERR_ARG;
@@ -970,8 +970,8 @@ int launch_moe_experts(MoeProblem P, cudaStream_t s, const PeerLink* lk) {
     const int layout = moe_table_layout(P);
     if (P.lut_ready && P.lut_blocks != layout) P.lut_ready = 0;   // tables were built in another layout: rebuild
     P.lut_blocks = layout;
-    if (layout == 3) {
-        const int rc = launch_moe_gather(P, s, link);
+    if (layout >= 3) {
+        const int rc = layout == 3 ? launch_moe_gather(P, s, link) : launch_moe_quad(P, s, link);
         if (rc != OJX_OK) return rc;
         const int n = P.n_tokens * P.H;
         moe_combine_kernel<<<(n + 255) / 256, 256, 0, s>>>(P, link);
@@ -1054,7 +1054,7 @@ int launch_moe_router(const float* Wr, const void* x, int io_dtype, int n_tokens
     const PeerLink& link = lk ? *lk : none;
     if (link.n <= 0) { e_begin = 0; e_end = E; }
     if (e_begin < 0 || e_end > E || e_begin > e_end) return OJX_ERR_ARG;
-    if (lut_blocks == 3) lut_out = nullptr;   // no tables
+    if (lut_blocks >= 3) lut_out = nullptr;   // no tables
     if (lut_out && lut_blocks) {   // tables in a layout of one of the whole-expert kernels: a launch of their own
         const int rc = lut_blocks == 2 ? launch_moe_chain_images(x, io_dtype, n_tokens, H, D, codebook, Kcb, lut_out, s)
                                        : launch_moe_prebuild_blocks(x, io_dtype, n_tokens, H, D, codebook, Kcb, lut_out, s);

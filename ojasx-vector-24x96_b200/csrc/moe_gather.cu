@@ -10,7 +10,7 @@
 // outliers' reads of single elements.  Codebooks and intermediate vectors have 22 bits here; of the outputs 2.0e-4 to 2.9e-4 are
 // not the 64-bit result rounded to bf16, of the table kernels' 2.4e-4 to 4.1e-4 (ten layers of five shapes, fewer in each).
 //
-//   moe_gather_plan_kernel   pairs grouped by expert, cut into items of up to sixteen pairs
+//   moe_item_plan_kernel     pairs grouped by expert, cut into items of up to sixteen pairs
 //   moe_gather_prep_kernel   vectors as fp16 hi + lo fragments, scaled by a power of two per vector (tokens, then inter)
 //   moe_gather_up_kernel     item x part of the intermediate indices: silu(gate) * up
 //   moe_gather_down_kernel   item x half of its pairs x part of the hidden rows
@@ -58,7 +58,7 @@ __device__ __forceinline__ int mg_local_expert(const MoeProblem& P, int pair) {
     return (e < 0 || e >= P.E || fabsf(P.topk_w[pair]) < 1e-8f) ? -1 : e;
 }
 
-__global__ void __launch_bounds__(1024) moe_gather_plan_kernel(const __grid_constant__ MoeProblem P, int* __restrict__ plan) {
+__global__ void __launch_bounds__(1024) moe_item_plan_kernel(const __grid_constant__ MoeProblem P, int width, int* __restrict__ plan) {
     extern __shared__ int plan_smem[];
     int *cnt = plan_smem, *start = plan_smem + P.E;
     __shared__ int warp_tot[33];
@@ -77,15 +77,15 @@ __global__ void __launch_bounds__(1024) moe_gather_plan_kernel(const __grid_cons
     int np = 0, ni = 0, tp, ti;
     for (int e = lo; e < hi; ++e) {
         np += cnt[e];
-        ni += (cnt[e] + kMgPairs - 1) / kMgPairs;
+        ni += (cnt[e] + width - 1) / width;
     }
     int bp = block_exclusive_scan(np, warp_tot, &tp), bi = block_exclusive_scan(ni, warp_tot, &ti);
     for (int e = lo; e < hi; ++e) {
         start[e] = bp;
-        for (int c = 0; c < cnt[e]; c += kMgPairs, ++bi) {
+        for (int c = 0; c < cnt[e]; c += width, ++bi) {
             items[4 * bi] = e;
             items[4 * bi + 1] = bp + c;
-            items[4 * bi + 2] = min(kMgPairs, cnt[e] - c);
+            items[4 * bi + 2] = min(width, cnt[e] - c);
         }
         bp += cnt[e];
     }
@@ -443,6 +443,13 @@ bool moe_gather_wanted(const MoeProblem& P) {
     return e ? expect >= atoll(e) : expect >= 400 && 2 * expect >= 7LL * P.E;
 }
 
+int launch_moe_item_plan(const MoeProblem& P, int* plan, int width, cudaStream_t s) {
+    moe_item_plan_kernel<<<1, 1024, sizeof(int) * 2 * (size_t)P.E, s>>>(P, width, plan);
+    OJX_CUDA_TRY(cudaGetLastError());
+    count_launch(1);
+    return OJX_OK;
+}
+
 int launch_moe_gather(const MoeProblem& P, cudaStream_t s, const PeerLink& link) {
     static std::atomic<bool> configured[64];   // the kernels' opt-in, once per device
     int dev = 0;
@@ -464,8 +471,8 @@ int launch_moe_gather(const MoeProblem& P, cudaStream_t s, const PeerLink& link)
     A.i_frag = p + (size_t)P.n_tokens * A.chunks_x * 64;
     A.x_inv = reinterpret_cast<const float*>(A.i_frag + (size_t)pairs * A.chunks_i * 64);
     A.i_inv = A.x_inv + P.n_tokens;
-    moe_gather_plan_kernel<<<1, 1024, sizeof(int) * 2 * (size_t)P.E, s>>>(P, A.plan);
-    OJX_CUDA_TRY(cudaGetLastError());
+    const int rc = launch_moe_item_plan(P, A.plan, kMgPairs, s);
+    if (rc != OJX_OK) return rc;
     moe_gather_prep_kernel<<<P.n_tokens, 128, 0, s>>>(P.x, P.io_dtype, P.H, A.chunks_x, nullptr, nullptr, const_cast<uint4*>(A.x_frag),
                                                       const_cast<float*>(A.x_inv));
     OJX_CUDA_TRY(cudaGetLastError());
@@ -476,7 +483,7 @@ int launch_moe_gather(const MoeProblem& P, cudaStream_t s, const PeerLink& link)
     OJX_CUDA_TRY(cudaGetLastError());
     moe_gather_down_kernel<<<2 * sms, kMgDownThreads, mg_smem(A.chunks_i), s>>>(A, link);
     OJX_CUDA_TRY(cudaGetLastError());
-    count_launch(5);
+    count_launch(4);
     return OJX_OK;
 }
 
