@@ -464,6 +464,28 @@ static int kvq_decode_impl(OjasxKvqHandle handle, const void* d_q, void* d_out, 
     return launch_kvq_decode(P, static_cast<cudaStream_t>(stream), link);
 }
 
+// The prefill kernels walk a CTA's whole context for 64 query rows; few positions on a long context split the context instead: the
+// decode kernel with a position axis.  bf16: the former once its CTAs fill half the GPU or the context is short.  fp32: by estimates of
+// both in us, 9.7 per 64 tokens of context (11.2 with two CTAs on an SM) against 16.5 per wave of decode CTAs and thousand tokens, a
+// CTA's tables counting as a thousand.  us per chunk, decode kernel / prefill kernel, 8 KV heads of 4 query heads, head_dim 128:
+//   16 positions behind 0, 500, 1000 tokens 42 / 43, 74 / 126, 88 / 195; 64: 87 / 46, 206 / 130, 327 / 212; 256: 251 / 86, 742 / 169,
+//   1234 / 250.  Under a static plan the context is not known: up to 1024 tokens of capacity it is taken to be short.
+static bool kvq_prefill_pays(const KvqProblem& P, const KvqHandle* h, int cached) {
+    const int R = h->Hq / h->Hkv, sms = num_sms();
+    const long long ctas = (long long)((P.n_pos * R + 63) / 64) * h->Hkv * h->B;
+    if (P.io_dtype == OJX_BF16) return 2 * ctas >= sms || cached <= 1024;
+    if (!kvq_table_decode_fits(P)) return false;   // a chunk is taken where its tokens can be decoded
+    if (h->static_plan && cached <= 1024) return true;
+    const int T = std::min(cached + P.n_pos, h->max_seq);
+    KvqProblem one = P;
+    one.n_pos = 0;
+    plan_kvq_decode(one, T, sms, h->splits);
+    const long long items = (long long)P.n_pos * h->B * h->Hkv * one.n_chunks;
+    const double decode = (double)((items + sms - 1) / sms) * (one.chunk + 1000) * 0.0165;
+    const double prefill = (ctas <= sms ? 9.7 : 11.2 * ((ctas + 2 * sms - 1) / (2 * sms))) * ((T + 63) / 64);
+    return prefill < decode;
+}
+
 int ojasx_b200_kvq_prefill(OjasxKvqHandle handle, const void* d_k, const void* d_v, const void* d_q, void* d_out, int n_positions,
                            float scale, int io_dtype, void* stream) {
     if (!handle || !d_k || !d_v || !d_q || !d_out || n_positions <= 0 || (io_dtype != OJX_F32 && io_dtype != OJX_BF16)) return OJX_ERR_ARG;
@@ -476,11 +498,8 @@ int ojasx_b200_kvq_prefill(OjasxKvqHandle handle, const void* d_k, const void* d
     KvqProblem P = kvq_problem(h, io_dtype);
     P.scale = scale > 0.0f ? scale : 1.0f / std::sqrt((float)h->head_dim);
     P.new_k = d_k; P.new_v = d_v; P.q = d_q; P.out = d_out; P.n_pos = n_positions;
-    // The prefill kernel walks a CTA's whole context for 64 query rows; it pays once its CTAs fill half the GPU or the
-    // context is short.  Few positions on a long context split the context instead: the decode kernel with a position axis.
     const int R = h->Hq / h->Hkv, cached = h->static_plan ? h->max_seq : h->host_len;
-    const long long ctas = (long long)((n_positions * R + 63) / 64) * h->Hkv * h->B;
-    if (n_positions >= kKvqPrefillPositions && kvq_prefill_supported(P) && (2 * ctas >= num_sms() || cached <= 1024)) {
+    if (n_positions >= kKvqPrefillPositions && kvq_prefill_supported(P) && kvq_prefill_pays(P, h, cached)) {
         int rc = launch_kvq_append_many(P, s);
         if (rc != OJX_OK) return rc;
         rc = launch_kvq_prefill_attention(P, s);

@@ -713,6 +713,12 @@ static int launch_decode_r(const KvqProblem& P, cudaStream_t s, const PeerLink& 
     }
 }
 
+bool kvq_table_decode_fits(const KvqProblem& P) {
+    const int R = P.Hq / P.Hkv;
+    return P.G <= kKvMaxGroups && P.Hq % P.Hkv == 0 && (R == 1 || R == 2 || R == 4 || R == 8) && (P.D == 4 || P.D == 8 || P.D == 16) &&
+           kvq_decode_smem(P, R) + 64 <= 227 * 1024;
+}
+
 int launch_kvq_decode(const KvqProblem& P, cudaStream_t s, const PeerLink* lk) {
     const PeerLink none{};
     const PeerLink& link = lk ? *lk : none;

@@ -94,7 +94,7 @@ __global__ void kvq_advance_kernel(int* seq_lens, int B, int n, int max_seq) {
 // Per tile of 64 tokens the codes are expanded into shared memory once and serve all 64 rows; scores
 // and values are mma.sync products with an online softmax between them, causal per row.
 //
-// bf16 queries, keys and values as fp16 products: every operand is scaled by a power of two (per query row, per codebook, 2^14 for
+// bf16 queries, keys and values as fp16 products (fp32 ones have a kernel of their own below): every operand is scaled by a power of two (per query row, per codebook, 2^14 for
 // probabilities) so that its largest element is in [2^14, 2^15), and split into x = hi + lo with two fp16 numbers: 22 bits of
 // mantissa.  hi*hi + hi*lo + lo*hi are accumulated in fp32, in runs short enough that the tensor cores' truncation does not show:
 // 8.3e-8 against 64 bits before the output is rounded, 512 positions.  78 us per layer of 512 positions with 32 query heads.
@@ -379,9 +379,280 @@ __global__ void __launch_bounds__(kPfThreads) kvq_prefill_kernel(const __grid_co
     }
 }
 
+// fp32 queries, keys and values: the same tiles in fp32.  A pair of fp16 numbers is one bit short of fp32 (fp32 outputs would be off by
+// up to 1.5 times as much as position by position), so the products are packed fp32 FMAs here.  128 threads, thread = 8 rows x 4 tokens
+// of the scores and 8 rows x HD/16 dimensions of the outputs; keys and values of a tile are expanded one after the other into the same
+// place, so that two CTAs (105 KB each) share an SM.  Sums are formed in short runs: a score's even and odd dimensions apart, outputs in
+// runs of 32 tokens, and of 512 tokens, which are added up in `out`.  Relative error against 64 bits (2-norm), position by position
+// through the decode kernel and here: 512 positions 1.02e-7 / 9.9e-8, 1000 behind 4000 tokens 1.08e-7 / 8.6e-8, 32 7.5e-8 / 7.3e-8.
+// Bound: fp32 FMAs (8.2 k clocks per tile of 64 x 64 x 128 with packed pairs) and the latency of shared memory; two CTAs take 21 k for
+// two tiles.  us per chunk of 512 positions with its codes, 8 KV heads of 4 query heads, head_dim 128: 750 / 171; 1000 behind 4000
+// 16740 / 2310.  With the rounding errors of the running outputs kept beside them the score loop had no registers left for its loads
+// (14 k clocks a tile instead of 8); 256 threads of half the rows read shared memory twice as often (no faster).
+constexpr int kPf32Pad = 4, kPf32Run = 32, kPf32Tiles = 8;
+__device__ __forceinline__ uint64_t pf_pack(float a, float b) {
+    uint64_t r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+    return r;
+}
+__device__ __forceinline__ float2 pf_unpack(uint64_t v) {
+    float2 r;
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v));
+    return r;
+}
+__device__ __forceinline__ uint64_t pf_fma2(uint64_t a, uint64_t b, uint64_t c) {
+    uint64_t r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+    return r;
+}
+
+template <int HD, int D>
+__global__ void __launch_bounds__(kPfThreads, D == 16 && HD == 128 ? 1 : 2) kvq_prefill_f32_kernel(const __grid_constant__ KvqProblem P) {
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    constexpr int LD = HD + kPf32Pad, LP = kPfRows + kPf32Pad, G = HD / D, NC = HD / 64;
+    float* Qs = reinterpret_cast<float*>(smem_raw);              // [64][LD]
+    float* Ts = Qs + kPfRows * LD;                               // [64][LD] keys, then values of a tile
+    float* Ps = Ts + kPfTok * LD;                                // [64 tokens][LP rows] probabilities
+    float* cbs = Ps + kPfTok * LP;                               // k, v: [256 * D] each
+    uint8_t* codes = reinterpret_cast<uint8_t*>(cbs + 2 * 256 * D);   // [2 tiles][k, v][64 * G]
+    const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
+    const int b = blockIdx.z, h = blockIdx.y, R = P.Hq / P.Hkv;
+    const int tile = gridDim.x - 1 - blockIdx.x;                 // the longest contexts start first
+    const int T0 = P.seq_lens[b];
+    const int pos_per = kPfRows / R, s0 = tile * pos_per;
+    const int t_all = min(T0 + min(P.n_pos, s0 + pos_per), P.max_seq);   // tokens the tile's last row sees
+
+    const uint8_t* kc = P.k_codes + (((size_t)b * P.Hkv + h) * P.max_seq) * G;
+    const uint8_t* vc = P.v_codes + (((size_t)b * P.Hkv + h) * P.max_seq) * G;
+    constexpr int W = kPfTok * G / 4, WPT = (W + kPfThreads - 1) / kPfThreads;   // words of four codes
+    uint32_t kw[WPT], vw[WPT];
+    auto fetch = [&](int t0) {
+#pragma unroll
+        for (int u = 0; u < WPT; ++u) {
+            const int i = tid + u * kPfThreads, t = t0 + i / (G / 4);
+            kw[u] = vw[u] = 0u;
+            if (i < W && t < t_all) {
+                kw[u] = *reinterpret_cast<const uint32_t*>(kc + (size_t)t * G + (i % (G / 4)) * 4);
+                vw[u] = *reinterpret_cast<const uint32_t*>(vc + (size_t)t * G + (i % (G / 4)) * 4);
+            }
+        }
+    };
+    auto keep = [&](int buf) {
+#pragma unroll
+        for (int u = 0; u < WPT; ++u) {
+            const int i = tid + u * kPfThreads;
+            if (i >= W) break;
+            reinterpret_cast<uint32_t*>(codes + (2 * buf) * kPfTok * G)[i] = kw[u];
+            reinterpret_cast<uint32_t*>(codes + (2 * buf + 1) * kPfTok * G)[i] = vw[u];
+        }
+    };
+    // A tile's keys or values: 16-byte pieces, consecutive threads on consecutive pieces of a token.
+    auto expand = [&](int buf, int which) {
+        const uint8_t* c = codes + (2 * buf + which) * kPfTok * G;
+        const float* cb = cbs + which * 256 * D;
+#pragma unroll 8
+        for (int i = tid; i < kPfTok * HD / 4; i += kPfThreads) {
+            const int t = i / (HD / 4), piece = i % (HD / 4);
+            *reinterpret_cast<float4*>(Ts + t * LD + piece * 4) =
+                *reinterpret_cast<const float4*>(cb + (int)c[t * G + piece / (D / 4)] * D + piece % (D / 4) * 4);
+        }
+    };
+
+    fetch(0);
+    // codebooks and query rows as 16-byte pieces, loads of a batch first
+    const float4 none = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+#pragma unroll 4
+    for (int i = tid; i < 64 * D; i += kPfThreads) {
+        const bool ok = 4 * i < P.Kcb * D;
+        const float4 k = ok ? reinterpret_cast<const float4*>(P.k_cb + (size_t)h * P.Kcb * D)[i] : none;
+        const float4 v = ok ? reinterpret_cast<const float4*>(P.v_cb + (size_t)h * P.Kcb * D)[i] : none;
+        reinterpret_cast<float4*>(cbs)[i] = k;
+        reinterpret_cast<float4*>(cbs + 256 * D)[i] = v;
+    }
+    const bool q16 = (reinterpret_cast<uintptr_t>(P.q) & 15) == 0;
+#pragma unroll 8
+    for (int i = tid; i < kPfRows * HD / 4; i += kPfThreads) {
+        const int row = i / (HD / 4), c = (i - row * (HD / 4)) * 4, s = s0 + row / R;
+        const float* src = static_cast<const float*>(P.q) + (((size_t)s * P.B + b) * P.Hq + (size_t)h * R + row % R) * HD + c;
+        float4 v = none;
+        if (s < P.n_pos) v = q16 ? *reinterpret_cast<const float4*>(src) : make_float4(src[0], src[1], src[2], src[3]);
+        *reinterpret_cast<float4*>(Qs + row * LD + c) = v;
+    }
+    keep(0);
+
+    // The running maximum starts at the lowest finite number: scores of -inf (they may overflow) then weigh 0, those of NaN NaN.
+    float m_run[8], l_run[8], l_err[8];
+    int limit[8];                                                // last token a row may see
+    float m_out[8];                                              // maximum that the sums kept in `out` refer to
+    uint64_t o[8][NC][2];
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+        m_run[i] = m_out[i] = -FLT_MAX;
+        l_run[i] = l_err[i] = 0.0f;
+        limit[i] = min(T0 + min(s0 + (ty * 8 + i) / R, P.n_pos - 1), P.max_seq - 1);
+#pragma unroll
+        for (int c = 0; c < NC; ++c) o[i][c][0] = o[i][c][1] = 0ull;
+    }
+    // The outputs of a run of tiles go to `out`, which keeps the sums of the runs before them until the last one divides by the sum of
+    // the probabilities.
+    int tiles = 0;
+    auto flush = [&](bool last) {
+        const bool first = tiles <= kPf32Tiles && !(last && tiles > kPf32Tiles);
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+            float inv = 1.0f;
+            if (last) {
+                float l = l_run[i];
+#pragma unroll
+                for (int off = 8; off >= 1; off >>= 1) l += __shfl_xor_sync(0xffffffffu, l, off);
+                inv = l == 0.0f ? 0.0f : 1.0f / l;
+            }
+            const int row = ty * 8 + i, s = s0 + row / R;
+            if (s < P.n_pos) {
+                float* out = static_cast<float*>(P.out) + (((size_t)s * P.B + b) * P.Hq + (size_t)h * R + row % R) * HD;
+                const float alpha = first ? 0.0f : expf(m_out[i] - m_run[i]);
+#pragma unroll
+                for (int c = 0; c < NC; ++c)
+#pragma unroll
+                    for (int e = 0; e < 4; ++e) {
+                        const float2 v = pf_unpack(o[i][c][e >> 1]);
+                        const int at = 64 * c + tx * 4 + e;
+                        float sum = e & 1 ? v.y : v.x;
+                        if (!first) sum += out[at] * alpha;
+                        out[at] = last ? sum * inv : sum;
+                    }
+            }
+            m_out[i] = m_run[i];
+#pragma unroll
+            for (int c = 0; c < NC; ++c) o[i][c][0] = o[i][c][1] = 0ull;
+        }
+    };
+    int buf = 0;
+    for (int t0 = 0; t0 < t_all; t0 += kPfTok, buf ^= 1) {
+        __syncthreads();   // codes of the tile are there, the tile before has been used
+        expand(buf, 0);
+        if (t0 + kPfTok < t_all) fetch(t0 + kPfTok);
+        __syncthreads();
+        float s[8][4];
+        {
+            uint64_t a[8][4];                                    // even and odd dimensions apart
+#pragma unroll
+            for (int i = 0; i < 8; ++i)
+#pragma unroll
+                for (int j = 0; j < 4; ++j) a[i][j] = 0ull;
+#pragma unroll 4
+            for (int d = 0; d < HD; d += 4) {
+                ulonglong2 k[4];
+#pragma unroll
+                for (int j = 0; j < 4; ++j) k[j] = *reinterpret_cast<const ulonglong2*>(Ts + (tx + 16 * j) * LD + d);
+#pragma unroll
+                for (int i = 0; i < 8; ++i) {
+                    const ulonglong2 q = *reinterpret_cast<const ulonglong2*>(Qs + (ty * 8 + i) * LD + d);
+#pragma unroll
+                    for (int j = 0; j < 4; ++j) a[i][j] = pf_fma2(q.x, k[j].x, a[i][j]);
+#pragma unroll
+                    for (int j = 0; j < 4; ++j) a[i][j] = pf_fma2(q.y, k[j].y, a[i][j]);
+                }
+            }
+#pragma unroll
+            for (int i = 0; i < 8; ++i)
+#pragma unroll
+                for (int j = 0; j < 4; ++j) {
+                    const float2 f = pf_unpack(a[i][j]);
+                    s[i][j] = f.x + f.y;
+                }
+        }
+        // scale, mask, online softmax (a row lives in sixteen lanes)
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+            float m = m_run[i], l = 0.0f;
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                s[i][j] = t0 + tx + 16 * j <= limit[i] ? s[i][j] * P.scale : -INFINITY;
+                m = fmaxf(m, s[i][j]);
+            }
+#pragma unroll
+            for (int off = 8; off >= 1; off >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, off));
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                s[i][j] = expf(s[i][j] - m);
+                l += s[i][j];
+            }
+            if (m != m_run[i]) {
+                const float alpha = expf(m_run[i] - m);
+                m_run[i] = m;
+                l_run[i] *= alpha;
+                l_err[i] *= alpha;
+#pragma unroll
+                for (int c = 0; c < NC; ++c)
+#pragma unroll
+                    for (int e = 0; e < 2; ++e) {
+                        const float2 v = pf_unpack(o[i][c][e]);
+                        o[i][c][e] = pf_pack(v.x * alpha, v.y * alpha);
+                    }
+            }
+            const float y = l - l_err[i], t = __fadd_rn(l_run[i], y);   // compensated: thousands of additions follow on a long context
+            l_err[i] = __fsub_rn(__fsub_rn(t, l_run[i]), y);
+            l_run[i] = t;
+        }
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            float* p = Ps + (tx + 16 * j) * LP + ty * 8;
+            *reinterpret_cast<float4*>(p) = make_float4(s[0][j], s[1][j], s[2][j], s[3][j]);
+            *reinterpret_cast<float4*>(p + 4) = make_float4(s[4][j], s[5][j], s[6][j], s[7][j]);
+        }
+        __syncthreads();   // the keys have been read
+        expand(buf, 1);
+        if (t0 + kPfTok < t_all) keep(buf ^ 1);
+        __syncthreads();
+#pragma unroll
+        for (int c = 0; c < NC; ++c)
+#pragma unroll 1
+            for (int r0 = 0; r0 < kPfTok && t0 + r0 < t_all; r0 += kPf32Run) {
+                uint64_t a[8][2];
+#pragma unroll
+                for (int i = 0; i < 8; ++i) a[i][0] = a[i][1] = 0ull;
+#pragma unroll 8
+                for (int t = r0; t < r0 + kPf32Run; ++t) {
+                    const float4 p0 = *reinterpret_cast<const float4*>(Ps + t * LP + ty * 8), p1 = *reinterpret_cast<const float4*>(Ps + t * LP + ty * 8 + 4);
+                    const float p[8] = {p0.x, p0.y, p0.z, p0.w, p1.x, p1.y, p1.z, p1.w};
+                    const ulonglong2 v = *reinterpret_cast<const ulonglong2*>(Ts + t * LD + 64 * c + tx * 4);
+                    uint64_t pp[8];
+#pragma unroll
+                    for (int i = 0; i < 8; ++i) pp[i] = pf_pack(p[i], p[i]);
+#pragma unroll
+                    for (int i = 0; i < 8; ++i) a[i][0] = pf_fma2(pp[i], v.x, a[i][0]);
+#pragma unroll
+                    for (int i = 0; i < 8; ++i) a[i][1] = pf_fma2(pp[i], v.y, a[i][1]);
+                }
+#pragma unroll
+                for (int i = 0; i < 8; ++i)
+#pragma unroll
+                    for (int e = 0; e < 2; ++e) {
+                        const float2 sum = pf_unpack(o[i][c][e]), f = pf_unpack(a[i][e]);
+                        o[i][c][e] = pf_pack(sum.x + f.x, sum.y + f.y);
+                    }
+            }
+        if (++tiles % kPf32Tiles == 0 && t0 + kPfTok < t_all) flush(false);
+    }
+    flush(true);
+}
+
 // ------------------------------------------------------------------------------------- host side
 template <int HD, int D>
+static int launch_prefill_f32_t(const KvqProblem& P, cudaStream_t s) {
+    constexpr size_t smem = sizeof(float) * ((size_t)(kPfRows + kPfTok) * (HD + kPf32Pad) + kPfTok * (kPfRows + kPf32Pad) + 2 * 256 * (size_t)D) + 4 * kPfTok * (HD / D);
+    OJX_CUDA_TRY(cudaFuncSetAttribute(kvq_prefill_f32_kernel<HD, D>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    const int pos_per = kPfRows / (P.Hq / P.Hkv);
+    kvq_prefill_f32_kernel<HD, D><<<dim3((P.n_pos + pos_per - 1) / pos_per, P.Hkv, P.B), kPfThreads, smem, s>>>(P);
+    OJX_CUDA_TRY(cudaGetLastError());
+    count_launch(1);
+    return OJX_OK;
+}
+
+template <int HD, int D>
 static int launch_prefill_t(const KvqProblem& P, cudaStream_t s) {
+    if (P.io_dtype == OJX_F32) return launch_prefill_f32_t<HD, D>(P, s);
     constexpr size_t smem = sizeof(__half) * (4 * (size_t)kPfTok * (HD + 8) + 4 * 256 * (size_t)D);
     static_assert(sizeof(float) * kPfRows * (HD + 4) <= smem, "query rows are staged in the tiles");
     OJX_CUDA_TRY(cudaFuncSetAttribute(kvq_prefill_kernel<HD, D>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
@@ -402,13 +673,11 @@ static int launch_prefill_d(const KvqProblem& P, cudaStream_t s) {
     }
 }
 
-// bf16 only: a pair of fp16 numbers is one bit short of fp32, so that fp32 outputs would be off by up to 1.5 times as much as
-// position by position (512 positions 8.3e-8 against 7.8e-8, 1000 behind 4000 tokens 1.6e-7 against 1.1e-7).  fp32 chunks go
-// through the query-table kernel, as many positions a launch as the scratch of a decode holds.  Codebooks that high and low parts do not hold (infinities, wide
-// ranges) do so in bf16 too.
+// Codebooks that high and low parts do not hold (infinities, wide ranges) go position by position: an infinite value of a masked
+// token would be multiplied by its probability of zero.
 bool kvq_prefill_supported(const KvqProblem& P) {
     const int R = P.Hq / P.Hkv;
-    return P.io_dtype == OJX_BF16 && P.even_books && R <= kPfRows && kPfRows % R == 0 && P.G % 4 == 0 && P.B <= 65535 && P.Hkv <= 65535 &&
+    return P.even_books && R <= kPfRows && kPfRows % R == 0 && P.G % 4 == 0 && P.B <= 65535 && P.Hkv <= 65535 &&
            (P.head_dim == 64 || P.head_dim == 128) && (P.D == 4 || P.D == 8 || P.D == 16);
 }
 

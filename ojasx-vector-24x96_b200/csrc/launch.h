@@ -109,6 +109,7 @@ void plan_kvq_decode(KvqProblem& P, int T, int sms, int max_splits);
 // Positions whose partial sums fit a scratch of max_splits per (sequence, KV head).
 int kvq_decode_positions(KvqProblem P, int T, int sms, int max_splits);
 int launch_kvq_append(const KvqProblem& P, cudaStream_t stream);
+bool kvq_table_decode_fits(const KvqProblem& P);   // what the query-table kernel takes: the shapes of fp32 caches
 int launch_kvq_decode(const KvqProblem& P, cudaStream_t stream, const PeerLink* link = nullptr);
 // --- kv_decode_mma.cu: decode for block_dim 8 and head_dim 64 or 128 (launch_kvq_decode takes it where it fits)
 bool kvq_decode_mma_supported(const KvqProblem& P);
