@@ -54,7 +54,8 @@ __global__ void __launch_bounds__(256) gm_prep_kernel(const __nv_bfloat16* __res
                                                       __nv_bfloat16* __restrict__ h, int K, int batch, int bp, uint4* __restrict__ frag,
                                                       float* __restrict__ inv_out, __nv_bfloat16* __restrict__ xT) {
     __shared__ __align__(16) __nv_bfloat16 tile[kGmMaxBatch][256 + 8];
-    cudaTriggerProgrammaticLaunchCompletion();
+    cudaTriggerProgrammaticLaunchCompletion();   // the linear behind this launch builds its tables, which nothing in the stream writes
+    cudaGridDependencySynchronize();
     const int c = blockIdx.x, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int k0 = c * 256 + lane * 8;
     for (int t = warp; t < bp; t += 8) {
@@ -164,6 +165,8 @@ __global__ void __launch_bounds__(kGmMaxWarps * 32, 2) gm_linear_kernel(const __
 #pragma unroll
     for (int n = 0; n < NT; ++n) boff[n] = (n * 8 + (lane >> 2)) * 4 + (lane & 3);
 
+    // (no trigger here: the next preparation's linear would take shared memory and issue slots from this one, SwiGLU block of 16
+    // tokens 53 us without and 62 with)
     cudaGridDependencySynchronize();   // the prepared activations
 
     if (tid < kVecs) {
@@ -470,10 +473,9 @@ int launch_gather_mma(const LinearProblem* P, int count, const void* x, const vo
     for (int p = 0; p < count; ++p) A.P[p] = P[p];
     const int batch = P[0].batch, NT = (batch + 7) / 8;
     gm_carve(A, workspace, P[0].K, batch);
-    gm_prep_kernel<<<A.chunks, 256, 0, s>>>(static_cast<const __nv_bfloat16*>(x), static_cast<const __nv_bfloat16*>(up),
-                                            static_cast<__nv_bfloat16*>(h), P[0].K, batch, NT * 8, const_cast<uint4*>(A.frag),
-                                            const_cast<float*>(A.inv), const_cast<__nv_bfloat16*>(A.xT));
-    OJX_CUDA_TRY(cudaGetLastError());
+    OJX_CUDA_TRY(launch_chained(gm_prep_kernel, A.chunks, 256, 0, s, static_cast<const __nv_bfloat16*>(x), static_cast<const __nv_bfloat16*>(up),
+                                static_cast<__nv_bfloat16*>(h), P[0].K, batch, NT * 8, const_cast<uint4*>(A.frag), const_cast<float*>(A.inv),
+                                const_cast<__nv_bfloat16*>(A.xT)));
     count_launch(1);
     int MT = 1, splits = 1, warps = kGmMaxWarps;
     gm_plan(P, count, A.chunks, NT, &MT, &splits, &warps);

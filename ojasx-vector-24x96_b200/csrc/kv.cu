@@ -39,7 +39,7 @@ __device__ __forceinline__ float load_io(const void* p, size_t i, int dtype) {
 // the length before they count), so an append is one launch.
 template <int D>
 __global__ void __launch_bounds__(kKvThreads) kvq_append_kernel(const __grid_constant__ KvqProblem P) {
-    cudaTriggerProgrammaticLaunchCompletion();   // a decode behind this launch may prepare its tables
+    chain_begin();
     const int b = blockIdx.y;
     const int T = P.seq_lens[b];
     if (T >= P.max_seq) {   // cache full: nothing is written, the error flag reports it
@@ -213,6 +213,7 @@ template <int R, int D>
 __global__ void __launch_bounds__(kvq_decode_threads(R, D), 1) kvq_decode_kernel(const __grid_constant__ KvqProblem P,
                                                                                  const __grid_constant__ PeerLink link) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
+    chain_begin();
     constexpr int kThreads = kvq_decode_threads(R, D), kHalf = kThreads / 2;   // score threads = value threads
     constexpr int kTpt = 2, kSub = kTpt * kHalf;                               // tokens per pass
     constexpr int kWarpsHalf = kHalf / 32, kPieces = D / 4;
@@ -667,8 +668,7 @@ int kvq_decode_positions(KvqProblem P, int T, int sms, int max_splits) {
 template <int D>
 static int launch_append_t(const KvqProblem& P, cudaStream_t s) {
     const int tasks = 2 * P.Hkv * P.G, wpb = kKvThreads / 32;
-    kvq_append_kernel<D><<<dim3((tasks + wpb - 1) / wpb, P.B), kKvThreads, 0, s>>>(P);
-    OJX_CUDA_TRY(cudaGetLastError());
+    OJX_CUDA_TRY(launch_chained(kvq_append_kernel<D>, dim3((tasks + wpb - 1) / wpb, P.B), kKvThreads, 0, s, P));
     count_launch(1);
     return OJX_OK;
 }
@@ -697,8 +697,7 @@ static int launch_decode_t(const KvqProblem& P, cudaStream_t s, const PeerLink& 
         OJX_CUDA_TRY(cudaFuncSetAttribute(kvq_decode_kernel<R, D>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
         if (cur_dev >= 0 && cur_dev < 64) configured[cur_dev] = smem;
     }
-    kvq_decode_kernel<R, D><<<dim3(P.n_chunks, P.Hkv, P.n_pos > 0 ? P.n_pos * P.B : P.B), kvq_decode_threads(R, D), smem, s>>>(Q, link);
-    OJX_CUDA_TRY(cudaGetLastError());
+    OJX_CUDA_TRY(launch_chained(kvq_decode_kernel<R, D>, dim3(P.n_chunks, P.Hkv, P.n_pos > 0 ? P.n_pos * P.B : P.B), kvq_decode_threads(R, D), smem, s, Q, link));
     count_launch(1);
     return OJX_OK;
 }

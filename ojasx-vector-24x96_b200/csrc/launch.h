@@ -4,6 +4,33 @@
 
 namespace ojx {
 
+// Launch of a kernel that begins with chain_begin(): its CTAs may be scheduled while the launch before it in the stream still runs
+// (programmatic dependent launch), so that a chain of short kernels does not pay a launch latency between any two of them.  us, plain
+// launches and these: routed MoE layer at one token (five kernels) 51.2 / 41.4, 32 append + decode pairs of a cache 620 / 568, SwiGLU
+// block of one token (four kernels) 40.2 / 36.1, decode steps of two layers (26 kernels) 238 / 225 each.
+template <class... Params, class... Args>
+inline cudaError_t launch_chained(void (*kernel)(Params...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, Args&&... args) {
+    cudaLaunchAttribute attr{};
+    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = grid;
+    cfg.blockDim = block;
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = s;
+    cfg.attrs = &attr;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, kernel, Params(args)...);
+}
+#ifdef __CUDACC__
+// Waits until everything before this launch in the stream is done and visible, then lets the launch behind it be scheduled.  In this
+// order, so that a kernel that has been scheduled knows that the launch before the last one is complete.
+__device__ __forceinline__ void chain_begin() {
+    cudaGridDependencySynchronize();
+    cudaTriggerProgrammaticLaunchCompletion();
+}
+#endif
+
 struct PeerLink;   // peer.cuh: exchange over peer memory fused into a kernel's epilogue (null / n == 0: none)
 const PeerLink* peer_link_of(void* peer_link_handle);
 

@@ -31,6 +31,7 @@ lut_linear_kernel(const LinearProblem* __restrict__ probs, int nprobs, int total
                   const __grid_constant__ LinearProblem single, int chain_walk, const __grid_constant__ PeerLink link) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     CoreSmem& sm = *reinterpret_cast<CoreSmem*>(smem_raw);
+    chain_begin();
 
     for (int item = blockIdx.x; item < total_items; item += gridDim.x) {
         const LinearProblem P = probs ? find_problem(probs, nprobs, item) : single;
@@ -217,9 +218,8 @@ int launch_linear(LinearProblem P, cudaStream_t stream, const PeerLink* link) {
     if (rc != OJX_OK) return rc;
     const int cap = kCtasPerSm * num_sms();
     const int grid = total < cap ? total : cap;
-    k<<<grid, kThreads, sizeof(CoreSmem), stream>>>(nullptr, 0, total, P, chain_walk_enabled(), L);
+    OJX_CUDA_TRY(launch_chained(k, grid, kThreads, sizeof(CoreSmem), stream, nullptr, 0, total, P, chain_walk_enabled(), L));
     count_launch(1);
-    OJX_CUDA_TRY(cudaGetLastError());
     return OJX_OK;
 }
 
@@ -234,9 +234,8 @@ int launch_linear_group(const LinearProblem* d_probs, int nprobs, int total_item
     const int grid = total_items < cap ? total_items : cap;
     LinearProblem dummy{};
     const PeerLink none{};
-    k<<<grid, kThreads, sizeof(CoreSmem), stream>>>(d_probs, nprobs, total_items, dummy, chain_walk_enabled(), link ? *link : none);
+    OJX_CUDA_TRY(launch_chained(k, grid, kThreads, sizeof(CoreSmem), stream, d_probs, nprobs, total_items, dummy, chain_walk_enabled(), link ? *link : none));
     count_launch(1);
-    OJX_CUDA_TRY(cudaGetLastError());
     return OJX_OK;
 }
 

@@ -65,6 +65,7 @@ __global__ void __launch_bounds__(kClThreads, 1)
 lut_linear_cluster_kernel(const __grid_constant__ ClusterGroup grp, const __grid_constant__ ClusterPlan plan,
                           const __grid_constant__ PeerLink link) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
+    chain_begin();
     const int C = plan.C;
     const int cid_all = blockIdx.x / C;
     int pi = 0;
@@ -237,13 +238,15 @@ static int launch_cluster_t(const ClusterGroup& grp, ClusterPlan plan, cudaStrea
     cfg.blockDim = dim3(kClThreads);
     cfg.dynamicSmemBytes = plan.smem;
     cfg.stream = stream;
-    cudaLaunchAttribute attr[1];
+    cudaLaunchAttribute attr[2];
     attr[0].id = cudaLaunchAttributeClusterDimension;
     attr[0].val.clusterDim.x = plan.C;
     attr[0].val.clusterDim.y = 1;
     attr[0].val.clusterDim.z = 1;
+    attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;   // see launch_chained
+    attr[1].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
-    cfg.numAttrs = 1;
+    cfg.numAttrs = 2;
     cfg.gridDim = dim3(plan.C * plan.n_clusters, grp.P[0].batch);
     if (dry_run) return OJX_OK;
     OJX_CUDA_TRY(cudaLaunchKernelEx(&cfg, kern, grp, plan, link));

@@ -19,6 +19,7 @@ namespace ojx {
 __global__ void __launch_bounds__(kQuThreads, 1) lut_linear_quad_kernel(const __grid_constant__ LinearProblem P, int items, float neg_zero,
                                                                         const __grid_constant__ PeerLink link) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
+    chain_begin();
     if (quad_begin(smem_raw, P.codebook, P.Kcb)) {
         int first = 0;
         const size_t esz = P.io_dtype == OJX_BF16 ? 2 : 4;
@@ -102,6 +103,7 @@ __device__ __forceinline__ void quad_items(const QuadMoe& A, unsigned char* raw,
 __global__ void __launch_bounds__(kQuThreads, 1) moe_gate_up_quad_kernel(const __grid_constant__ QuadMoe A) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     const MoeProblem& P = A.P;
+    chain_begin();
     if (!quad_begin(smem_raw, P.cb_in, P.Kcb)) return;
     int first = 0;
     const size_t esz = P.io_dtype == OJX_BF16 ? 2 : 4;
@@ -140,6 +142,7 @@ __global__ void __launch_bounds__(kQuThreads, 1) moe_gate_up_quad_kernel(const _
 __global__ void __launch_bounds__(kQuThreads, 1) moe_down_quad_kernel(const __grid_constant__ QuadMoe A, const __grid_constant__ PeerLink link) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     const MoeProblem& P = A.P;
+    chain_begin();
     if (quad_begin(smem_raw, P.cb_down, P.Kcb)) {
         int first = 0;
         quad_items(A, smem_raw, 2, [&](const QuadGroup& g, int h0, int n) {
@@ -224,8 +227,7 @@ int launch_quad_linear(LinearProblem P, cudaStream_t s, const PeerLink& link) {
     P.tile_rows = quad_linear_tile(P, &clocks);
     P.tiles = (P.row_stop - P.row_start + P.tile_rows - 1) / P.tile_rows;
     const int items = (P.batch + kQuVecs - 1) / kQuVecs * P.tiles;
-    lut_linear_quad_kernel<<<std::min(items, num_sms()), kQuThreads, kQuSmemBytes, s>>>(P, items, -0.0f, link);
-    OJX_CUDA_TRY(cudaGetLastError());
+    OJX_CUDA_TRY(launch_chained(lut_linear_quad_kernel, std::min(items, num_sms()), kQuThreads, kQuSmemBytes, s, P, items, -0.0f, link));
     count_launch(1);
     return OJX_OK;
 }
@@ -279,10 +281,8 @@ int launch_moe_quad(const MoeProblem& P, cudaStream_t s, const PeerLink& link) {
     QuadMoe pass[2];
     quad_passes(P, pass);
     if ((rc = launch_moe_item_plan(P, pass[0].plan, kQuVecs, s)) != OJX_OK) return rc;
-    moe_gate_up_quad_kernel<<<num_sms(), kQuThreads, kQuSmemBytes, s>>>(pass[0]);
-    OJX_CUDA_TRY(cudaGetLastError());
-    moe_down_quad_kernel<<<num_sms(), kQuThreads, kQuSmemBytes, s>>>(pass[1], link);
-    OJX_CUDA_TRY(cudaGetLastError());
+    OJX_CUDA_TRY(launch_chained(moe_gate_up_quad_kernel, num_sms(), kQuThreads, kQuSmemBytes, s, pass[0]));
+    OJX_CUDA_TRY(launch_chained(moe_down_quad_kernel, num_sms(), kQuThreads, kQuSmemBytes, s, pass[1], link));
     count_launch(2);
     return OJX_OK;
 }

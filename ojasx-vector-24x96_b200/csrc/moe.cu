@@ -41,6 +41,7 @@ __device__ __forceinline__ MoePair decode_pair(const MoeProblem& P, int pair) {
 template <int D>
 __global__ void __launch_bounds__(kThreads, kCtasPerSm) moe_gate_up_kernel(const __grid_constant__ MoeProblem P) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
+    chain_begin();
     CoreSmem& sm = *reinterpret_cast<CoreSmem*>(smem_raw);
     const int total = (P.pair_list ? P.pair_list[0] : P.n_tokens * P.k_active) * P.gu_tiles;
     const size_t esz = P.io_dtype == OJX_BF16 ? 2 : 4;
@@ -95,6 +96,7 @@ template <int D>
 __global__ void __launch_bounds__(kThreads, kCtasPerSm) moe_down_kernel(const __grid_constant__ MoeProblem P,
                                                                         const __grid_constant__ PeerLink link) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
+    chain_begin();
     CoreSmem& sm = *reinterpret_cast<CoreSmem*>(smem_raw);
     const int total = (P.pair_list ? P.pair_list[0] : P.n_tokens * P.k_active) * P.dn_tiles;
     for (int item = blockIdx.x; item < total; item += gridDim.x) {
@@ -209,6 +211,7 @@ __device__ __forceinline__ void moe_gate_up_chain_item(const MoeProblem& P, unsi
 template <int D>
 __global__ void __launch_bounds__(kThreads, kCtasPerSm) moe_gate_up_chain_kernel(const __grid_constant__ MoeProblem P) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
+    chain_begin();
     const int total = P.pair_list ? P.pair_list[0] : P.n_tokens * P.k_active;
     if (!ChainWalker<D>::usable(smem_raw, P.gu_codes, P.cb_in, P.G)) {   // checked on the host as far as it can be; the
         if (threadIdx.x == 0) atomicExch(&g_bulk_copy_timeout, 2);      // shared-memory base only shows here
@@ -290,6 +293,7 @@ template <int D>
 __global__ void __launch_bounds__(kThreads, kCtasPerSm) moe_down_chain_kernel(const __grid_constant__ MoeProblem P,
                                                                               const __grid_constant__ PeerLink link) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
+    chain_begin();
     const int total = P.pair_list ? P.pair_list[0] : P.n_tokens * P.k_active;
     const bool usable = ChainWalker<D>::usable(smem_raw, P.dn_codes, P.cb_down, P.Gi);
     if (!usable && threadIdx.x == 0) atomicExch(&g_bulk_copy_timeout, 2);
@@ -308,6 +312,7 @@ template <int D>
 __global__ void __launch_bounds__(kThreads, kCtasPerSm) moe_experts_chain_kernel(const __grid_constant__ MoeProblem P,
                                                                                  const __grid_constant__ PeerLink link) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
+    chain_begin();
     // (no static shared memory: the walker needs the dynamic area at its fixed address; between two work items all of
     // it is free, so the claimed item is handed round through its first word)
     volatile int* s_item = reinterpret_cast<volatile int*>(smem_raw);
@@ -354,6 +359,7 @@ __global__ void __launch_bounds__(256) moe_chain_prebuild_kernel(const void* __r
                                                                  float* __restrict__ out) {
     constexpr int SG = ChainWalker<D>::SG;
     __shared__ float cb_s[256 * D];
+    chain_begin();
     const int s = blockIdx.x, t = blockIdx.y, nsl = gridDim.x;
     const int g0 = s * SG, ng = min(SG, G - g0);
     const size_t esz = io_dtype == OJX_BF16 ? 2 : 4;
@@ -384,6 +390,7 @@ __global__ void __launch_bounds__(256) moe_chain_prebuild_kernel(const void* __r
 // the local expert id.  list[0] = count, list[1..] = pair ids.
 __global__ void __launch_bounds__(1024) moe_plan_kernel(const __grid_constant__ MoeProblem P, int* __restrict__ list) {
     extern __shared__ int plan_smem[];
+    chain_begin();
     int* cnt = plan_smem;          // [E] pairs per local expert
     int* start = plan_smem + P.E;  // [E] next free slot of the expert
     __shared__ int warp_tot[32];
@@ -442,6 +449,7 @@ __device__ __forceinline__ bool combine_takes(const MoeProblem& P, int pair) {
 }
 
 __global__ void moe_combine_kernel(const __grid_constant__ MoeProblem P, const __grid_constant__ PeerLink link) {
+    chain_begin();
     if (link.n > 0) {   // expert outputs of the other ranks land in expert_out: wait for every rank's flag first
         if (threadIdx.x < 32) peer_wait_warp(link);
         __syncthreads();
@@ -505,6 +513,7 @@ __global__ void __launch_bounds__(256) moe_router_logits_kernel(const float* __r
                                                                 int io_dtype, int n_tokens, int H, int E,
                                                                 float* __restrict__ logits, int e_begin, int e_end,
                                                                 const __grid_constant__ PeerLink link) {
+    chain_begin();
     router_logits_block(Wr, x, io_dtype, n_tokens, H, E, logits, blockIdx.x, blockIdx.y, gridDim.y, e_begin, e_end, link);
     peer_signal_when_last(link, gridDim.x * gridDim.y);
 }
@@ -522,6 +531,7 @@ __global__ void __launch_bounds__(256) moe_router_logits_tiled_kernel(const floa
                                                                       float* __restrict__ logits, int e_begin, int e_end,
                                                                       const __grid_constant__ PeerLink link) {
     __shared__ __align__(16) float xs[kLogitTokens][kLogitCols];
+    chain_begin();
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int e0 = e_begin + (blockIdx.x * 8 + warp) * EPW, t0 = blockIdx.y * kLogitTokens;
     const bool live = e0 < e_end;
@@ -626,6 +636,7 @@ __global__ void __launch_bounds__(256) moe_logits_prebuild_kernel(const float* _
                                                                   float* __restrict__ lut_out, int e_begin, int e_end,
                                                                   const __grid_constant__ PeerLink link) {
     __shared__ float xs[16 * D];
+    chain_begin();
     const int b = blockIdx.x;
     if (b < lx * ly) {
         router_logits_block(Wr, x, io_dtype, n_tokens, H, E, logits, b % lx, b / lx, ly, e_begin, e_end, link);
@@ -648,6 +659,7 @@ __global__ void __launch_bounds__(kTopkWarps * 32) moe_router_topk_kernel(const 
                                                                          float* __restrict__ probs /* [n_tokens, E] scratch */,
                                                                          const __grid_constant__ PeerLink link) {
     extern __shared__ float topk_smem[];  // [kTopkWarps][E]
+    chain_begin();
     if (link.n > 0) {   // the logits of the other ranks' experts arrive over the link
         if (threadIdx.x < 32) peer_wait_warp(link);
         __syncthreads();
@@ -711,6 +723,7 @@ __global__ void __launch_bounds__(kTopkWarps * 32) moe_router_topk_reg_kernel(co
     constexpr int kPer = EPL / kTopkWarps;
     __shared__ __align__(16) float p[32 * EPL];
     __shared__ float red[kTopkWarps], s_sum;
+    chain_begin();
     if (link.n > 0) {   // the logits of the other ranks' experts arrive over the link
         if (threadIdx.x < 32) peer_wait_warp(link);
         __syncthreads();
@@ -879,8 +892,7 @@ size_t moe_table_bytes(int n_tokens, int G, int D) {
 template <int D>
 static int launch_chain_images(const void* x, int io_dtype, int n_tokens, int H, int G, const float* cb, int Kcb, float* out, cudaStream_t s) {
     const int nsl = (G + ChainWalker<D>::SG - 1) / ChainWalker<D>::SG;
-    moe_chain_prebuild_kernel<D><<<dim3(nsl, n_tokens), 256, 0, s>>>(x, io_dtype, H, G, cb, Kcb, out);
-    OJX_CUDA_TRY(cudaGetLastError());
+    OJX_CUDA_TRY(launch_chained(moe_chain_prebuild_kernel<D>, dim3(nsl, n_tokens), 256, 0, s, x, io_dtype, H, G, cb, Kcb, out));
     count_launch(1);
     return OJX_OK;
 }
@@ -894,6 +906,12 @@ int launch_moe_chain_images(const void* x, int io_dtype, int n_tokens, int H, in
     }
 }
 
+static int launch_combine(const MoeProblem& P, const PeerLink& link, cudaStream_t s) {
+    const int n = P.n_tokens * P.H;
+    OJX_CUDA_TRY(launch_chained(moe_combine_kernel, (n + 255) / 256, 256, 0, s, P, link));
+    return OJX_OK;
+}
+
 template <int D>
 static int launch_moe_experts_t(const MoeProblem& P, cudaStream_t s, const PeerLink& link) {
     int rc;
@@ -905,8 +923,7 @@ static int launch_moe_experts_t(const MoeProblem& P, cudaStream_t s, const PeerL
     if (P.pair_list) {
         const size_t hs = sizeof(int) * 2 * (size_t)P.E;
         if (hs > 48 * 1024) OJX_CUDA_TRY(cudaFuncSetAttribute(moe_plan_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)hs));
-        moe_plan_kernel<<<1, 1024, hs, s>>>(P, const_cast<int*>(P.pair_list));
-        OJX_CUDA_TRY(cudaGetLastError());
+        OJX_CUDA_TRY(launch_chained(moe_plan_kernel, 1, 1024, hs, s, P, const_cast<int*>(P.pair_list)));
         ++extra;
     }
     if constexpr (D <= 16) {
@@ -918,17 +935,13 @@ static int launch_moe_experts_t(const MoeProblem& P, cudaStream_t s, const PeerL
             if (P.pair_list && P.chain_ctl && P.dn_tiles == 1 && moe_chain_down_wanted(P) && !(one && one[0] == '0')) {
                 // gate/up and down of every pair from one work queue (no rounded-up wave between the two passes)
                 if ((rc = set_smem(moe_experts_chain_kernel<D>)) != OJX_OK) return rc;
-                moe_experts_chain_kernel<D><<<pairs < sms ? pairs : sms, kThreads, sizeof(CoreSmem), s>>>(P, link);
-                OJX_CUDA_TRY(cudaGetLastError());
-                const int n = P.n_tokens * P.H;
-                moe_combine_kernel<<<(n + 255) / 256, 256, 0, s>>>(P, link);
-                OJX_CUDA_TRY(cudaGetLastError());
+                OJX_CUDA_TRY(launch_chained(moe_experts_chain_kernel<D>, pairs < sms ? pairs : sms, kThreads, sizeof(CoreSmem), s, P, link));
+                if ((rc = launch_combine(P, link, s)) != OJX_OK) return rc;
                 count_launch(2 + extra);
                 return OJX_OK;
             }
             if ((rc = set_smem(moe_gate_up_chain_kernel<D>)) != OJX_OK) return rc;
-            moe_gate_up_chain_kernel<D><<<pairs < sms ? pairs : sms, kThreads, sizeof(CoreSmem), s>>>(P);
-            OJX_CUDA_TRY(cudaGetLastError());
+            OJX_CUDA_TRY(launch_chained(moe_gate_up_chain_kernel<D>, pairs < sms ? pairs : sms, kThreads, sizeof(CoreSmem), s, P));
         }
     }
     if (P.lut_blocks != 2) {
@@ -938,22 +951,18 @@ static int launch_moe_experts_t(const MoeProblem& P, cudaStream_t s, const PeerL
             OJX_CUDA_TRY(cudaGetLastError());
             ++extra;
         }
-        moe_gate_up_kernel<D><<<gu_items < sms ? gu_items : sms, kThreads, sizeof(CoreSmem), s>>>(P);
-        OJX_CUDA_TRY(cudaGetLastError());
+        OJX_CUDA_TRY(launch_chained(moe_gate_up_kernel<D>, gu_items < sms ? gu_items : sms, kThreads, sizeof(CoreSmem), s, P));
     }
     bool chain_down = false;
     if constexpr (D <= 16) {
         if (P.dn_tiles == 1 && moe_chain_down_wanted(P)) {
             if ((rc = set_smem(moe_down_chain_kernel<D>)) != OJX_OK) return rc;
-            moe_down_chain_kernel<D><<<pairs < sms ? pairs : sms, kThreads, sizeof(CoreSmem), s>>>(P, link);
+            OJX_CUDA_TRY(launch_chained(moe_down_chain_kernel<D>, pairs < sms ? pairs : sms, kThreads, sizeof(CoreSmem), s, P, link));
             chain_down = true;
         }
     }
-    if (!chain_down) moe_down_kernel<D><<<dn_items < sms ? dn_items : sms, kThreads, sizeof(CoreSmem), s>>>(P, link);
-    OJX_CUDA_TRY(cudaGetLastError());
-    const int n = P.n_tokens * P.H;
-    moe_combine_kernel<<<(n + 255) / 256, 256, 0, s>>>(P, link);
-    OJX_CUDA_TRY(cudaGetLastError());
+    if (!chain_down) OJX_CUDA_TRY(launch_chained(moe_down_kernel<D>, dn_items < sms ? dn_items : sms, kThreads, sizeof(CoreSmem), s, P, link));
+    if ((rc = launch_combine(P, link, s)) != OJX_OK) return rc;
     count_launch(3 + extra);
     return OJX_OK;
 }
@@ -973,22 +982,18 @@ int launch_moe_experts(MoeProblem P, cudaStream_t s, const PeerLink* lk) {
     if (layout >= 3) {
         const int rc = layout == 3 ? launch_moe_gather(P, s, link) : launch_moe_quad(P, s, link);
         if (rc != OJX_OK) return rc;
-        const int n = P.n_tokens * P.H;
-        moe_combine_kernel<<<(n + 255) / 256, 256, 0, s>>>(P, link);
-        OJX_CUDA_TRY(cudaGetLastError());
-        count_launch(1);
-        return OJX_OK;
+        const int rc2 = launch_combine(P, link, s);
+        if (rc2 == OJX_OK) count_launch(1);
+        return rc2;
     }
     // Whole-expert work items with gate/up and down fused (moe_fused.cu, opt-in); then the ordered combine.
     if (layout == 1) {
         const int rc = launch_moe_fused(P, s, lk);
         if (rc != OJX_ERR_UNSUPPORTED) {
             if (rc != OJX_OK) return rc;
-            const int n = P.n_tokens * P.H;
-            moe_combine_kernel<<<(n + 255) / 256, 256, 0, s>>>(P, link);
-            OJX_CUDA_TRY(cudaGetLastError());
-            count_launch(1);
-            return OJX_OK;
+            const int rc2 = launch_combine(P, link, s);
+            if (rc2 == OJX_OK) count_launch(1);
+            return rc2;
         }
         P.lut_ready = 0;
         P.lut_blocks = moe_chain_wanted(P) ? 2 : 0;
@@ -1068,30 +1073,28 @@ int launch_moe_router(const float* Wr, const void* x, int io_dtype, int n_tokens
         if (!codebook || H % D != 0) return OJX_ERR_ARG;
         const int G = H / D, grid = lx * ly + (G + 15) / 16 * n_tokens;
         switch (D) {
-            case 4: moe_logits_prebuild_kernel<4><<<grid, 256, 0, s>>>(Wr, x, io_dtype, n_tokens, H, E, logits, lx, ly, G, codebook, Kcb, lut_out, e_begin, e_end, link); break;
-            case 8: moe_logits_prebuild_kernel<8><<<grid, 256, 0, s>>>(Wr, x, io_dtype, n_tokens, H, E, logits, lx, ly, G, codebook, Kcb, lut_out, e_begin, e_end, link); break;
-            case 16: moe_logits_prebuild_kernel<16><<<grid, 256, 0, s>>>(Wr, x, io_dtype, n_tokens, H, E, logits, lx, ly, G, codebook, Kcb, lut_out, e_begin, e_end, link); break;
-            case 32: moe_logits_prebuild_kernel<32><<<grid, 256, 0, s>>>(Wr, x, io_dtype, n_tokens, H, E, logits, lx, ly, G, codebook, Kcb, lut_out, e_begin, e_end, link); break;
+            case 4: OJX_CUDA_TRY(launch_chained(moe_logits_prebuild_kernel<4>, grid, 256, 0, s, Wr, x, io_dtype, n_tokens, H, E, logits, lx, ly, G, codebook, Kcb, lut_out, e_begin, e_end, link)); break;
+            case 8: OJX_CUDA_TRY(launch_chained(moe_logits_prebuild_kernel<8>, grid, 256, 0, s, Wr, x, io_dtype, n_tokens, H, E, logits, lx, ly, G, codebook, Kcb, lut_out, e_begin, e_end, link)); break;
+            case 16: OJX_CUDA_TRY(launch_chained(moe_logits_prebuild_kernel<16>, grid, 256, 0, s, Wr, x, io_dtype, n_tokens, H, E, logits, lx, ly, G, codebook, Kcb, lut_out, e_begin, e_end, link)); break;
+            case 32: OJX_CUDA_TRY(launch_chained(moe_logits_prebuild_kernel<32>, grid, 256, 0, s, Wr, x, io_dtype, n_tokens, H, E, logits, lx, ly, G, codebook, Kcb, lut_out, e_begin, e_end, link)); break;
             default: return OJX_ERR_UNSUPPORTED;
         }
     } else if (n_tokens >= kLogitTokens) {
         // most experts per warp that still leave a block for every SM
         const int ty = (n_tokens + kLogitTokens - 1) / kLogitTokens, sms = num_sms();
         const dim3 g4((ne + 31) / 32, ty), g2((ne + 15) / 16, ty), g1(lx, ty);
-        if ((int)(g4.x * g4.y) >= sms) moe_router_logits_tiled_kernel<4><<<g4, 256, 0, s>>>(Wr, x, io_dtype, n_tokens, H, E, logits, e_begin, e_end, link);
-        else if ((int)(g2.x * g2.y) >= sms) moe_router_logits_tiled_kernel<2><<<g2, 256, 0, s>>>(Wr, x, io_dtype, n_tokens, H, E, logits, e_begin, e_end, link);
-        else moe_router_logits_tiled_kernel<1><<<g1, 256, 0, s>>>(Wr, x, io_dtype, n_tokens, H, E, logits, e_begin, e_end, link);
+        const int epw = (int)(g4.x * g4.y) >= sms ? 4 : (int)(g2.x * g2.y) >= sms ? 2 : 1;
+        OJX_CUDA_TRY(launch_chained(epw == 4 ? moe_router_logits_tiled_kernel<4> : epw == 2 ? moe_router_logits_tiled_kernel<2> : moe_router_logits_tiled_kernel<1>,
+                                    epw == 4 ? g4 : epw == 2 ? g2 : g1, 256, 0, s, Wr, x, io_dtype, n_tokens, H, E, logits, e_begin, e_end, link));
     } else {
-        moe_router_logits_kernel<<<dim3(lx, ly), 256, 0, s>>>(Wr, x, io_dtype, n_tokens, H, E, logits, e_begin, e_end, link);
+        OJX_CUDA_TRY(launch_chained(moe_router_logits_kernel, dim3(lx, ly), 256, 0, s, Wr, x, io_dtype, n_tokens, H, E, logits, e_begin, e_end, link));
     }
-    OJX_CUDA_TRY(cudaGetLastError());
     const size_t tsm = sizeof(float) * kTopkWarps * (size_t)E;
     if (tsm > 200 * 1024) return OJX_ERR_TOO_LARGE;
     if (tsm > 48 * 1024) OJX_CUDA_TRY(cudaFuncSetAttribute(moe_router_topk_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tsm));
     const int tgrid = (n_tokens + kTopkWarps - 1) / kTopkWarps;
-    if (E <= 512) moe_router_topk_reg_kernel<16><<<n_tokens, kTopkWarps * 32, 0, s>>>(logits, n_tokens, E, k, idx_out, w_out, probs, link);
-    else moe_router_topk_kernel<<<tgrid, kTopkWarps * 32, tsm, s>>>(logits, n_tokens, E, k, idx_out, w_out, probs, link);
-    OJX_CUDA_TRY(cudaGetLastError());
+    if (E <= 512) OJX_CUDA_TRY(launch_chained(moe_router_topk_reg_kernel<16>, n_tokens, kTopkWarps * 32, 0, s, logits, n_tokens, E, k, idx_out, w_out, probs, link));
+    else OJX_CUDA_TRY(launch_chained(moe_router_topk_kernel, tgrid, kTopkWarps * 32, tsm, s, logits, n_tokens, E, k, idx_out, w_out, probs, link));
     count_launch(2);
     return OJX_OK;
 }

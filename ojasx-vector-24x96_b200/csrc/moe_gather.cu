@@ -60,6 +60,7 @@ __device__ __forceinline__ int mg_local_expert(const MoeProblem& P, int pair) {
 
 __global__ void __launch_bounds__(1024) moe_item_plan_kernel(const __grid_constant__ MoeProblem P, int width, int* __restrict__ plan) {
     extern __shared__ int plan_smem[];
+    chain_begin();
     int *cnt = plan_smem, *start = plan_smem + P.E;
     __shared__ int warp_tot[33];
     const int pairs = P.n_tokens * P.k_active;
@@ -444,8 +445,7 @@ bool moe_gather_wanted(const MoeProblem& P) {
 }
 
 int launch_moe_item_plan(const MoeProblem& P, int* plan, int width, cudaStream_t s) {
-    moe_item_plan_kernel<<<1, 1024, sizeof(int) * 2 * (size_t)P.E, s>>>(P, width, plan);
-    OJX_CUDA_TRY(cudaGetLastError());
+    OJX_CUDA_TRY(launch_chained(moe_item_plan_kernel, 1, 1024, sizeof(int) * 2 * (size_t)P.E, s, P, width, plan));
     count_launch(1);
     return OJX_OK;
 }

@@ -30,6 +30,7 @@ __global__ void __launch_bounds__(256) rmsnorm_kernel(void* __restrict__ x, cons
                                                       const float* __restrict__ w, void* __restrict__ out, int H, float eps) {
     constexpr int dt = kBf16 ? OJX_BF16 : OJX_F32;
     __shared__ float red[8];
+    chain_begin();
     const size_t base = (size_t)blockIdx.x * H;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     float keep[kNormKeep], more[kNormKeep], wk[kNormKeep];
@@ -83,6 +84,7 @@ __global__ void __launch_bounds__(256) rmsnorm_kernel(void* __restrict__ x, cons
 __global__ void rope_qk_kernel(void* __restrict__ q, void* __restrict__ k, const int* __restrict__ pos, int Hq, int Hkv,
                                int hd, float theta, int io_dtype) {
     const int b = blockIdx.y, head = blockIdx.x, half = hd >> 1;
+    chain_begin();
     const float p = (float)pos[b];
     void* buf = head < Hq ? q : k;
     const size_t base = head < Hq ? ((size_t)b * Hq + head) * hd : ((size_t)b * Hkv + (head - Hq)) * hd;
@@ -97,6 +99,7 @@ __global__ void rope_qk_kernel(void* __restrict__ q, void* __restrict__ k, const
 }
 
 __global__ void add_int_kernel(int* p, int n, int delta) {
+    chain_begin();
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i < n) p[i] += delta;
 }
@@ -112,9 +115,7 @@ int ojasx_b200_rmsnorm(void* d_x, const void* d_add, const float* d_weight, void
     if (!d_x || !d_weight || !d_out || rows <= 0 || hidden <= 0) return OJX_ERR_ARG;
     if (io_dtype != OJX_F32 && io_dtype != OJX_BF16) return OJX_ERR_ARG;
     const cudaStream_t s = static_cast<cudaStream_t>(stream);
-    if (io_dtype == OJX_BF16) rmsnorm_kernel<true><<<rows, 256, 0, s>>>(d_x, d_add, d_weight, d_out, hidden, eps);
-    else rmsnorm_kernel<false><<<rows, 256, 0, s>>>(d_x, d_add, d_weight, d_out, hidden, eps);
-    OJX_CUDA_TRY(cudaGetLastError());
+    OJX_CUDA_TRY(launch_chained(io_dtype == OJX_BF16 ? rmsnorm_kernel<true> : rmsnorm_kernel<false>, rows, 256, 0, s, d_x, d_add, d_weight, d_out, hidden, eps));
     count_launch(1);
     return OJX_OK;
 }
@@ -124,16 +125,16 @@ int ojasx_b200_rope_qk(void* d_q, void* d_k, const int* d_positions, int batch, 
     if (!d_q || !d_k || !d_positions || batch <= 0 || q_heads <= 0 || kv_heads <= 0 || head_dim <= 0 || (head_dim & 1)) return OJX_ERR_ARG;
     if (io_dtype != OJX_F32 && io_dtype != OJX_BF16) return OJX_ERR_ARG;
     if (batch > 65535) return OJX_ERR_TOO_LARGE;   // a grid row per sequence
-    rope_qk_kernel<<<dim3(q_heads + kv_heads, batch), (head_dim / 2 + 31) / 32 * 32 < 256 ? (head_dim / 2 + 31) / 32 * 32 : 256, 0, static_cast<cudaStream_t>(stream)>>>(d_q, d_k, d_positions, q_heads, kv_heads, head_dim, theta, io_dtype);
-    OJX_CUDA_TRY(cudaGetLastError());
+    const int threads = (head_dim / 2 + 31) / 32 * 32;
+    OJX_CUDA_TRY(launch_chained(rope_qk_kernel, dim3(q_heads + kv_heads, batch), threads < 256 ? threads : 256, 0, static_cast<cudaStream_t>(stream), d_q, d_k,
+                                d_positions, q_heads, kv_heads, head_dim, theta, io_dtype));
     count_launch(1);
     return OJX_OK;
 }
 
 int ojasx_b200_add_int(int* d_values, int count, int delta, void* stream) {
     if (!d_values || count <= 0) return OJX_ERR_ARG;
-    add_int_kernel<<<(count + 127) / 128, 128, 0, static_cast<cudaStream_t>(stream)>>>(d_values, count, delta);
-    OJX_CUDA_TRY(cudaGetLastError());
+    OJX_CUDA_TRY(launch_chained(add_int_kernel, (count + 127) / 128, 128, 0, static_cast<cudaStream_t>(stream), d_values, count, delta));
     count_launch(1);
     return OJX_OK;
 }
