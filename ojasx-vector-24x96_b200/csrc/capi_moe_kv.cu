@@ -478,7 +478,7 @@ static bool kvq_prefill_pays(const KvqProblem& P, const KvqHandle* h, int cached
     if (h->static_plan && cached <= 1024) return true;
     const int T = std::min(cached + P.n_pos, h->max_seq);
     KvqProblem one = P;
-    one.n_pos = 0;
+    one.n_pos = 1;
     plan_kvq_decode(one, T, sms, h->splits);
     const long long items = (long long)P.n_pos * h->B * h->Hkv * one.n_chunks;
     const double decode = (double)((items + sms - 1) / sms) * (one.chunk + 1000) * 0.013;

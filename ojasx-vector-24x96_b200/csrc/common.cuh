@@ -115,6 +115,7 @@ struct KvqProblem {
     int B, Hkv, Hq, head_dim, D, G, Kcb, max_seq;
     int chunk, n_chunks;
     int even_books;         // the codebooks fit pairs of fp16 numbers (book_fits_halves, checked when the cache is created)
+    int direct;             // decode kernel: ranges of up to so many tokens go without tables (0: none)
     int v_copies;           // copies of the value codebook in the decode kernel's shared memory (1 or 8)
     int io_dtype;
     float scale;

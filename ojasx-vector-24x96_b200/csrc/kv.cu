@@ -190,16 +190,21 @@ __device__ __forceinline__ void kvq_merge_if_last(const KvqProblem& P, int b /* 
         const int r = i / hd, col = i - r * hd;
         float M = -INFINITY;
         for (int c = 0; c < P.n_chunks; ++c) M = fmaxf(M, __ldcg(base + ((size_t)c * R + r) * (hd + 2)));
-        float L = 0.0f, o = 0.0f;
-        for (int c = 0; c < P.n_chunks; ++c) {
-            const float* p = base + ((size_t)c * R + r) * (hd + 2);
-            const float m = __ldcg(p);
-            if (m != -INFINITY) {
-                const float wgt = __expf(m - M);
-                L += __ldcg(p + 1) * wgt;
-                o = fmaf(__ldcg(p + 2 + col), wgt, o);
+        // four sums side by side: shorter chains of roundings, and of loads
+        float Ls[4] = {0.0f, 0.0f, 0.0f, 0.0f}, os[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+        for (int c0 = 0; c0 < P.n_chunks; c0 += 4)
+#pragma unroll
+            for (int u = 0; u < 4; ++u) {
+                const float* p = base + ((size_t)min(c0 + u, P.n_chunks - 1) * R + r) * (hd + 2);
+                const float m = __ldcg(p), l = __ldcg(p + 1), v = __ldcg(p + 2 + col);
+                if (c0 + u < P.n_chunks && m != -INFINITY) {
+                    const float wgt = expf(m - M);
+                    Ls[u] = fmaf(l, wgt, Ls[u]);
+                    os[u] = fmaf(v, wgt, os[u]);
+                }
             }
-        }
+        const float L = (Ls[0] + Ls[1]) + (Ls[2] + Ls[3]);
+        float o = (os[0] + os[1]) + (os[2] + os[3]);
         o *= L > 0.0f ? 1.0f / L : 0.0f;   // NaN stays NaN
         // a KV-head shard writes its heads into the gathered output of every rank (link.n > 0)
         const int row_heads = P.out_heads > 0 ? P.out_heads : P.Hq;
@@ -209,10 +214,157 @@ __device__ __forceinline__ void kvq_merge_if_last(const KvqProblem& P, int b /* 
     }
 }
 
+// Ranges of few tokens, without tables: a token's centroids are multiplied with the queries as they are.  Same products and sums as
+// through the query table (fp32, a group's dimensions in order, then the groups), outputs in runs of kDirectRun tokens.  The tables and
+// the eight copies of the value codebook take a CTA as long as 200 to 300 tokens do here.  us per decode, tables / this, 8 KV heads of
+// 4 query heads of 128: 16 tokens 13.5 / 7.0, 64 13.5 / 7.9, 256 14.4 / 8.7, 1000 15.3 / 11.1; 16 sequences, 64 tokens 14.4 / 8.5, 256
+// 15.0 / 13.8; 8 query heads, 64 17.6 / 11.1, 256 in one range 23.5 / 24.2 (so half as many tokens there).  Error against 64 bits at 64,
+// 256 and 1000 tokens 1.24e-7 / 9.8e-8, 1.24e-7 / 9.6e-8, 1.00e-7 / 8.0e-8.
+// Latency-bound: codes from L2, scores (eight threads per token), softmax (a warp per head), outputs (thread = column and token
+// stripe), each behind a barrier.
+constexpr int kDirectTokens = 256, kDirectRun = 8;
+template <int R, int D>
+constexpr size_t kvq_direct_smem(int G, int hd) {
+    return sizeof(float) * (2 * 256 * D + (size_t)R * hd + kDirectTokens * R + (size_t)kvq_decode_threads(R, D) * R) + 2 * (size_t)kDirectTokens * G;
+}
+template <int R, int D>
+__device__ __forceinline__ void kvq_decode_direct(const KvqProblem& P, unsigned char* smem_raw, int z, int h, const uint8_t* kc, const uint8_t* vc, int n,
+                                                  float* part) {
+    constexpr int kThreads = kvq_decode_threads(R, D);
+    const int G = P.G, hd = P.head_dim, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const float* kcb = reinterpret_cast<const float*>(smem_raw);   // [256][D], put there before the wait
+    const float* vcb = kcb + 256 * D;
+    uint8_t* ks = smem_raw + 2 * 256 * D * sizeof(float);          // [n][G] codes (all of these start on 16-byte boundaries)
+    uint8_t* vs = ks + kDirectTokens * G;
+    float* qs = reinterpret_cast<float*>(vs + kDirectTokens * G);  // [R][hd]
+    float* sc = qs + R * hd;                                       // [n][R]
+    float* sums = sc + kDirectTokens * R;                          // [stripes][R][hd]
+    const int bytes = n * G;
+    if (((reinterpret_cast<uintptr_t>(kc) | reinterpret_cast<uintptr_t>(vc) | (unsigned)bytes) & 15) == 0) {
+        for (int i = tid; i < bytes / 16; i += kThreads) {
+            const uint4 k = reinterpret_cast<const uint4*>(kc)[i], v = reinterpret_cast<const uint4*>(vc)[i];
+            reinterpret_cast<uint4*>(ks)[i] = k;
+            reinterpret_cast<uint4*>(vs)[i] = v;
+        }
+    } else {
+        for (int i = tid; i < bytes; i += kThreads) {
+            ks[i] = kc[i];
+            vs[i] = vc[i];
+        }
+    }
+    for (int i = tid; i < R * hd; i += kThreads) qs[i] = load_io(P.q, ((size_t)z * P.Hq + (size_t)h * R) * hd + i, P.io_dtype);
+    __syncthreads();
+    // scores: groups sub, sub + 8, ... of a token per thread; the queries of two groups stay in registers
+    const int sub = tid & 7;
+    constexpr int kKeep = R * D <= 32 ? 2 : 1;
+    float qk[kKeep][R][D];
+#pragma unroll
+    for (int k = 0; k < kKeep; ++k)
+#pragma unroll
+        for (int r = 0; r < R; ++r)
+            if (sub + 8 * k < G) ld_heads<D>(qs + r * hd + (sub + 8 * k) * D, qk[k][r]);
+    for (int t0 = 0; t0 < n; t0 += kThreads / 8) {
+        const int t = t0 + (tid >> 3);
+        float s[R];
+#pragma unroll
+        for (int r = 0; r < R; ++r) s[r] = 0.0f;
+        if (t < n) {
+            auto add = [&](int g, auto q_of) {
+                float cv[D];
+                ld_heads<D>(kcb + (int)ks[t * G + g] * D, cv);
+#pragma unroll
+                for (int r = 0; r < R; ++r) {
+                    float qv[D], dot = 0.0f;
+                    q_of(r, qv);
+#pragma unroll
+                    for (int d = 0; d < D; ++d) dot = fmaf(qv[d], cv[d], dot);
+                    s[r] += dot;
+                }
+            };
+#pragma unroll
+            for (int k = 0; k < kKeep; ++k)
+                if (sub + 8 * k < G) add(sub + 8 * k, [&](int r, float (&qv)[D]) {
+#pragma unroll
+                    for (int d = 0; d < D; ++d) qv[d] = qk[k][r][d];
+                });
+            for (int g = sub + 8 * kKeep; g < G; g += 8) add(g, [&](int r, float (&qv)[D]) { ld_heads<D>(qs + r * hd + g * D, qv); });
+        }
+#pragma unroll
+        for (int r = 0; r < R; ++r) {
+#pragma unroll
+            for (int off = 4; off >= 1; off >>= 1) s[r] += __shfl_xor_sync(0xffffffffu, s[r], off);
+            if (t < n && sub == r) sc[t * R + r] = s[r] * P.scale;
+        }
+    }
+    __syncthreads();
+    if (warp < R) {
+        float m = -FLT_MAX, l = 0.0f;
+        for (int t = lane; t < n; t += 32) m = fmaxf(m, sc[t * R + warp]);
+#pragma unroll
+        for (int off = 16; off >= 1; off >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, off));
+        for (int t = lane; t < n; t += 32) {
+            const float p = expf(sc[t * R + warp] - m);
+            sc[t * R + warp] = p;
+            l += p;
+        }
+#pragma unroll
+        for (int off = 16; off >= 1; off >>= 1) l += __shfl_xor_sync(0xffffffffu, l, off);
+        if (lane == 0) {
+            part[(size_t)warp * (hd + 2)] = m;
+            part[(size_t)warp * (hd + 2) + 1] = l;
+        }
+    }
+    __syncthreads();
+    const int stripes = kThreads / hd, stripe = tid / hd, col = tid - stripe * hd;   // hd <= kThreads
+    if (stripe < stripes) {
+        float o[R];
+#pragma unroll
+        for (int r = 0; r < R; ++r) o[r] = 0.0f;
+        for (int t0 = stripe; t0 < n; t0 += stripes * kDirectRun) {
+            float a[R];
+#pragma unroll
+            for (int r = 0; r < R; ++r) a[r] = 0.0f;
+#pragma unroll 4
+            for (int u = 0; u < kDirectRun; ++u) {
+                const int t = t0 + u * stripes;
+                if (t < n) {
+                    const float v = vcb[(int)vs[t * G + col / D] * D + col % D];
+                    float p[R];
+                    ld_heads<R>(sc + t * R, p);
+#pragma unroll
+                    for (int r = 0; r < R; ++r) a[r] = fmaf(p[r], v, a[r]);
+                }
+            }
+#pragma unroll
+            for (int r = 0; r < R; ++r) o[r] += a[r];
+        }
+#pragma unroll
+        for (int r = 0; r < R; ++r) sums[((size_t)stripe * R + r) * hd + col] = o[r];
+    }
+    __syncthreads();
+    for (int i = tid; i < R * hd; i += kThreads) {
+        const int r = i / hd, c = i - r * hd;
+        float acc = 0.0f;
+        for (int s2 = 0; s2 < stripes; ++s2) acc += sums[((size_t)s2 * R + r) * hd + c];
+        part[(size_t)r * (hd + 2) + 2 + c] = acc;
+    }
+}
+
 template <int R, int D>
 __global__ void __launch_bounds__(kvq_decode_threads(R, D), 1) kvq_decode_kernel(const __grid_constant__ KvqProblem P,
                                                                                  const __grid_constant__ PeerLink link) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
+    {   // the head's codebooks, which nothing in the stream writes, for a range of few tokens (see kvq_decode_direct)
+        float4* cb = reinterpret_cast<float4*>(smem_raw);
+        const size_t at = (size_t)blockIdx.y * P.Kcb * D / 4;
+        for (int i = threadIdx.x; i < 64 * D; i += kvq_decode_threads(R, D)) {
+            const bool ok = 4 * i < P.Kcb * D;
+            const float4 none = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+            const float4 k = ok ? reinterpret_cast<const float4*>(P.k_cb)[at + i] : none, v = ok ? reinterpret_cast<const float4*>(P.v_cb)[at + i] : none;
+            cb[i] = k;
+            cb[64 * D + i] = v;
+        }
+    }
     chain_begin();
     constexpr int kThreads = kvq_decode_threads(R, D), kHalf = kThreads / 2;   // score threads = value threads
     constexpr int kTpt = 2, kSub = kTpt * kHalf;                               // tokens per pass
@@ -251,6 +403,13 @@ __global__ void __launch_bounds__(kvq_decode_threads(R, D), 1) kvq_decode_kernel
     const int n_passes = (t_end - t_begin + kSub - 1) / kSub;
     const uint8_t* kc = P.k_codes + (((size_t)b * P.Hkv + h) * P.max_seq) * G;
     const uint8_t* vc = P.v_codes + (((size_t)b * P.Hkv + h) * P.max_seq) * G;
+    if (P.direct && t_end - t_begin <= P.direct) {
+        kvq_decode_direct<R, D>(P, smem_raw, z, h, kc + (size_t)t_begin * G, vc + (size_t)t_begin * G, t_end - t_begin, part);
+        kvq_merge_if_last<R>(P, z, h, link);
+        peer_signal_when_last(link, gridDim.x * gridDim.y * gridDim.z);
+        return;
+    }
+    __syncthreads();   // the codebooks' place is the query table's from here on
 
     for (int i = tid; i < R * hd; i += kThreads) qs[i] = load_io(P.q, ((size_t)z * P.Hq + (size_t)h * R) * hd + i, P.io_dtype);
     for (int i0 = tid; i0 < 256 * kPieces * vrep; i0 += 4 * kThreads) {   // consecutive threads, consecutive 16-byte slots
@@ -639,6 +798,13 @@ void plan_kvq_decode(KvqProblem& P, int T, int sms, int max_splits) {
         P.n_chunks = (std::max(T, 1) + P.chunk - 1) / P.chunk;
         return;
     }
+    // few heads: ranges of 64 tokens, which go without tables, if there is an SM for each (more than 16 take longer to merge than they save)
+    const int fine = (std::max(T, 1) + 63) / 64;
+    if (P.n_pos <= 0 && fine <= std::min(max_splits, 16) && heads * fine <= slots) {
+        P.chunk = 64;
+        P.n_chunks = fine;
+        return;
+    }
     // the splits of a single decode, for positions too: a longer split adds more tokens up in a row and is less exact (2048 tokens,
     // fp32, against 64 bits: 1.16e-7 in one split, 0.97e-7 in eight)
     const int max_s = std::min(max_splits, (T + 255) / 256);
@@ -660,7 +826,7 @@ void plan_kvq_decode(KvqProblem& P, int T, int sms, int max_splits) {
 
 int kvq_decode_positions(KvqProblem P, int T, int sms, int max_splits) {
     if (kvq_decode_by_mma(P)) return max_splits;
-    P.n_pos = 0;
+    P.n_pos = 1;
     plan_kvq_decode(P, T, sms, max_splits);
     return max_splits / P.n_chunks;
 }
@@ -690,6 +856,7 @@ static int launch_decode_t(const KvqProblem& P, cudaStream_t s, const PeerLink& 
     if (smem + 64 > 227 * 1024) return OJX_ERR_TOO_LARGE;   // 64: the kernel's few static bytes
     KvqProblem Q = P;
     Q.v_copies = kvq_decode_v_copies(P, R);
+    Q.direct = kvq_direct_smem<R, D>(P.G, P.head_dim) <= smem && P.head_dim <= kvq_decode_threads(R, D) ? (R == 8 ? kDirectTokens / 2 : kDirectTokens) : 0;
     static thread_local size_t configured[64] = {};  // largest opt-in made for this instantiation, per device
     int cur_dev = 0;
     OJX_CUDA_TRY(cudaGetDevice(&cur_dev));

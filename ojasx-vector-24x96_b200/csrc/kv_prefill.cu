@@ -382,14 +382,15 @@ __global__ void __launch_bounds__(kPfThreads) kvq_prefill_kernel(const __grid_co
 // fp32 queries, keys and values: the same tiles in fp32.  A pair of fp16 numbers is one bit short of fp32 (fp32 outputs would be off by
 // up to 1.5 times as much as position by position), so the products are packed fp32 FMAs here.  128 threads, thread = 8 rows x 4 tokens
 // of the scores and 8 rows x HD/16 dimensions of the outputs; keys and values of a tile are expanded one after the other into the same
-// place, so that two CTAs (105 KB each) share an SM.  Sums are formed in short runs: a score's even and odd dimensions apart, outputs in
-// runs of 32 tokens, and of 512 tokens, which are added up in `out`.  Relative error against 64 bits (2-norm), position by position
-// through the decode kernel and here: 512 positions 1.02e-7 / 9.9e-8, 1000 behind 4000 tokens 1.08e-7 / 8.6e-8, 32 7.5e-8 / 7.3e-8.
+// place, so that two CTAs (105 KB each) share an SM.  Sums are formed in short runs: a score in runs of 32 dimensions, even and odd ones apart,
+// outputs in runs of 16 tokens, and of 512 tokens, which are added up in `out`.  Relative error against 64 bits (2-norm), position by
+// position through the query tables and here: 512 positions 1.02e-7 / 9.3e-8, 1000 behind 4000 tokens 1.08e-7 / 8.8e-8, 32 7.5e-8 /
+// 7.1e-8.
 // Bound: fp32 FMAs (8.2 k clocks per tile of 64 x 64 x 128 with packed pairs) and the latency of shared memory; two CTAs take 21 k for
-// two tiles.  us per chunk of 512 positions with its codes, 8 KV heads of 4 query heads, head_dim 128: 750 / 171; 1000 behind 4000
-// 16740 / 2310.  With the rounding errors of the running outputs kept beside them the score loop had no registers left for its loads
+// two tiles.  us per chunk of 512 positions with its codes, 8 KV heads of 4 query heads, head_dim 128: 750 / 173; 1000 behind 4000
+// 16740 / 2340.  With the rounding errors of the running outputs kept beside them the score loop had no registers left for its loads
 // (14 k clocks a tile instead of 8); 256 threads of half the rows read shared memory twice as often (no faster).
-constexpr int kPf32Pad = 4, kPf32Run = 32, kPf32Tiles = 8;
+constexpr int kPf32Pad = 4, kPf32Dims = 32, kPf32Run = 16, kPf32Tiles = 8;
 __device__ __forceinline__ uint64_t pf_pack(float a, float b) {
     uint64_t r;
     asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
@@ -534,14 +535,19 @@ __global__ void __launch_bounds__(kPfThreads, D == 16 && HD == 128 ? 1 : 2) kvq_
         if (t0 + kPfTok < t_all) fetch(t0 + kPfTok);
         __syncthreads();
         float s[8][4];
-        {
+#pragma unroll
+        for (int i = 0; i < 8; ++i)
+#pragma unroll
+            for (int j = 0; j < 4; ++j) s[i][j] = 0.0f;
+#pragma unroll 1
+        for (int d0 = 0; d0 < HD; d0 += kPf32Dims) {
             uint64_t a[8][4];                                    // even and odd dimensions apart
 #pragma unroll
             for (int i = 0; i < 8; ++i)
 #pragma unroll
                 for (int j = 0; j < 4; ++j) a[i][j] = 0ull;
-#pragma unroll 4
-            for (int d = 0; d < HD; d += 4) {
+#pragma unroll
+            for (int d = d0; d < d0 + kPf32Dims; d += 4) {
                 ulonglong2 k[4];
 #pragma unroll
                 for (int j = 0; j < 4; ++j) k[j] = *reinterpret_cast<const ulonglong2*>(Ts + (tx + 16 * j) * LD + d);
@@ -559,7 +565,7 @@ __global__ void __launch_bounds__(kPfThreads, D == 16 && HD == 128 ? 1 : 2) kvq_
 #pragma unroll
                 for (int j = 0; j < 4; ++j) {
                     const float2 f = pf_unpack(a[i][j]);
-                    s[i][j] = f.x + f.y;
+                    s[i][j] += f.x + f.y;
                 }
         }
         // scale, mask, online softmax (a row lives in sixteen lanes)
