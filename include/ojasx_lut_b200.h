@@ -241,7 +241,7 @@ OJASX_API size_t ojasx_b200_linear_workspace(OjasxLinearHandle handle, int batch
 OJASX_API int ojasx_b200_linear_forward_ws(OjasxLinearHandle handle, const void* d_x, void* d_y, int batch_size,
                                            int io_dtype, int row_start, int row_stop, void* workspace,
                                            size_t workspace_bytes, void* stream);
-/* down(silu(gate(x)) * up(x)) for a bf16 batch of 1 to 31, every stage rounded to bf16 as the separate calls round it.
+/* down(silu(gate(x)) * up(x)) for a bf16 batch, every stage rounded to bf16 as the separate calls round it.
  * ojasx_b200_mlp_workspace is 0 where the block has to be called layer by layer (then -4). */
 OJASX_API size_t ojasx_b200_mlp_workspace(OjasxLinearHandle gate, OjasxLinearHandle up, OjasxLinearHandle down,
                                           const void* d_x, int batch_size, int io_dtype);

@@ -192,6 +192,14 @@ int ojasx_set_linear_outliers(OjasxLinearHandle handle, int nnz, const int* row_
     return OJX_OK;
 }
 
+// Whether ojasx_b200_linear_forward takes the tensor cores for a call.
+static bool wants_tensor(const LinearProblem& P, bool csr_sorted) {
+    if (P.io_dtype != OJX_BF16 || !dequant_gemm_supported(P, csr_sorted)) return false;
+    const char* e = getenv("OJASX_B200_TENSOR_MIN_BATCH");   // read per call: a process can time both paths; 0 = never
+    const int min_batch = e ? atoi(e) : kTensorMinBatch;
+    return min_batch > 0 && P.batch >= min_batch;
+}
+
 int ojasx_b200_linear_forward(OjasxLinearHandle handle, const void* d_x, void* d_y, int batch_size, int io_dtype,
                               int row_start, int row_stop, void* stream) {
     if (!handle || !d_x || !d_y) return OJX_ERR_ARG;
@@ -201,11 +209,7 @@ int ojasx_b200_linear_forward(OjasxLinearHandle handle, const void* d_x, void* d
     LinearProblem P = h->problem(d_x, d_y, batch_size, io_dtype, row_start, row_stop);
     // bf16 batches at or above the measured switch-over run on the tensor cores (dequant_gemm.cu);
     // OJASX_B200_TENSOR_MIN_BATCH overrides the threshold (0 = never).
-    if (io_dtype == OJX_BF16 && dequant_gemm_supported(P, h->csr_sorted)) {
-        const char* e = getenv("OJASX_B200_TENSOR_MIN_BATCH");   // read per call: a process can time both paths
-        const int min_batch = e ? atoi(e) : kTensorMinBatch;
-        if (min_batch > 0 && batch_size >= min_batch) return launch_dequant_gemm(P, static_cast<cudaStream_t>(stream), &h->dq_lists, h->generation);
-    }
+    if (wants_tensor(P, h->csr_sorted)) return launch_dequant_gemm(P, static_cast<cudaStream_t>(stream), &h->dq_lists, h->generation);
     return launch_linear(P, static_cast<cudaStream_t>(stream));
 }
 
@@ -271,6 +275,9 @@ size_t ojasx_b200_mlp_workspace(OjasxLinearHandle gate, OjasxLinearHandle up, Oj
     if (!gate || !up || !down || !d_x || batch_size <= 0) return 0;
     const LinearHandle* l[3] = {static_cast<LinearHandle*>(gate), static_cast<LinearHandle*>(up), static_cast<LinearHandle*>(down)};
     if (l[0]->in != l[1]->in || l[0]->out != l[1]->out || l[2]->in != l[0]->out) return 0;
+    bool tensor = true;
+    for (const LinearHandle* h : l) tensor = tensor && wants_tensor(h->problem(d_x, nullptr, batch_size, io_dtype, 0, h->out), h->csr_sorted);
+    if (tensor) return 2 * (size_t)batch_size * l[0]->out * 2;   // gate and up, the gated vectors in gate's place
     for (const LinearHandle* h : l)
         if (!gather_mma_open(h->problem(d_x, nullptr, batch_size, io_dtype, 0, h->out), h->csr_sorted, h->even_book)) return 0;
     return std::max(gather_mma_workspace(l[0]->in, batch_size), gather_mma_workspace(l[2]->in, batch_size)) +
@@ -286,6 +293,18 @@ int ojasx_b200_mlp_forward(OjasxLinearHandle gate, OjasxLinearHandle up, OjasxLi
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     const size_t one = (size_t)batch_size * g->out * 2;   // a multiple of 16: widths are multiples of 64
     char* buf = static_cast<char*>(workspace);
+    if (need == 2 * one) {   // tensor cores
+        const LinearProblem P[2] = {g->problem(d_x, buf, batch_size, io_dtype, 0, g->out), u->problem(d_x, buf + one, batch_size, io_dtype, 0, u->out)};
+        DqLists* const lists[2] = {&g->dq_lists, &u->dq_lists};
+        const unsigned generation[2] = {g->generation, u->generation};
+        int rc = OJX_OK;
+        if (g != u && dequant_gemm_pair_pays(P[0], P[1])) rc = launch_dequant_gemm_pair(P, s, lists, generation);
+        else
+            for (int i = 0; i < 2 && rc == OJX_OK; ++i) rc = launch_dequant_gemm(P[i], s, lists[i], generation[i]);
+        if (rc == OJX_OK) rc = launch_silu_mul(buf, buf + one, buf, (size_t)batch_size * g->out, io_dtype, s);
+        if (rc != OJX_OK) return rc;
+        return launch_dequant_gemm(d->problem(buf, d_y, batch_size, io_dtype, 0, d->out), s, &d->dq_lists, d->generation);
+    }
     void *yg = buf, *yu = buf + one, *yh = buf + 2 * one;
     const LinearProblem P[2] = {g->problem(d_x, yg, batch_size, io_dtype, 0, g->out), u->problem(d_x, yu, batch_size, io_dtype, 0, u->out)};
     int rc = launch_gather_mma(P, 2, d_x, nullptr, nullptr, buf + 3 * one, s);

@@ -13,17 +13,18 @@
 // tcgen05.commit.  After the last K tile the producer warps become the epilogue: tcgen05.ld the
 // accumulator rows, scale, bias, store bf16.
 //
-// A layer has few 128-row tiles (54 for 6912 rows), so the K axis is split over up to four CTAs per
+// A layer has few 128-row tiles (54 for 6912 rows), so the K axis is split over up to eight CTAs per
 // tile until the GPU is full.  The CTAs of a tile form a thread-block cluster: each leaves its raw fp32
 // partial sums in its own shared memory (the stage buffers are idle by then), and after a cluster barrier
 // every CTA adds the partials of its share of the batch columns in split order, reading the other CTAs'
-// copies through distributed shared memory, and applies scale and bias.  (Partial sums through global
+// copies through distributed shared memory, and applies scale and bias (a single CTA does the same on its own).  (Partial sums through global
 // memory with the last CTA to arrive adding them cost 20 of the kernel's 40 microseconds at batch 256.)
 //
 // This path trades the bit-exactness of the table kernels for throughput (weights are rounded to
 // bf16), so it is used only for bf16 I/O, inside the rel 2e-2 tolerance of the bf16 activation path.
 // Every wait on an mbarrier is bounded; on a timeout the kernel raises a flag that the host reads.
 #include <algorithm>
+#include <atomic>
 #include <cstdlib>
 
 #include <cuda.h>   // CUtensorMap and the types of cuTensorMapEncodeTiled (the entry point is looked up at run time)
@@ -86,6 +87,17 @@ __device__ __forceinline__ float dq_ld_cluster(unsigned local_addr, unsigned ran
     return v;
 }
 
+__device__ __forceinline__ unsigned dq_map_cluster(unsigned local_addr, unsigned rank) {
+    unsigned remote;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(remote) : "r"(local_addr), "r"(rank));
+    return remote;
+}
+__device__ __forceinline__ float4 dq_ld_cluster4(unsigned remote) {
+    float4 v;
+    asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(remote) : "memory");
+    return v;
+}
+
 // Shared-memory matrix descriptor of a K-major tile stored with the 128-byte swizzle: rows of 128
 // bytes, groups of 8 rows 1024 bytes apart.
 __device__ __forceinline__ unsigned long long make_desc_sw128(unsigned smem_addr) {
@@ -96,6 +108,24 @@ __device__ __forceinline__ unsigned long long make_desc_sw128(unsigned smem_addr
     d |= (unsigned long long)1 << 46;                            // descriptor version of sm_100
     d |= (unsigned long long)2 << 61;                            // SWIZZLE_128B
     return d;
+}
+
+// The codebook in bf16, `copies` (8 or 4) times: 128 bytes of shared memory hold one centroid for each of eight lanes, or two for each
+// of four pairs, so that the eight lanes that a 16-byte read serves together gather without conflicts (or with those of a pair);
+// with one copy a gather took 2.7 wavefronts for one.
+__device__ __forceinline__ void dq_build_book(uint4* cb16, const float* __restrict__ codebook, int copies, int threads) {
+    const int per = 8 / copies;   // centroids per 128 bytes
+    for (int c = threadIdx.x; c < 256; c += threads) {
+        __nv_bfloat162 h[4];
+        const float4 f0 = reinterpret_cast<const float4*>(codebook)[2 * c], f1 = reinterpret_cast<const float4*>(codebook)[2 * c + 1];
+        h[0] = __floats2bfloat162_rn(f0.x, f0.y);
+        h[1] = __floats2bfloat162_rn(f0.z, f0.w);
+        h[2] = __floats2bfloat162_rn(f1.x, f1.y);
+        h[3] = __floats2bfloat162_rn(f1.z, f1.w);
+        const uint4 v = *reinterpret_cast<uint4*>(h);
+        uint4* row = cb16 + c / per * 8 + c % per;
+        for (int q = 0; q < copies; ++q) row[((q + c) & (copies - 1)) * per] = v;
+    }
 }
 
 struct DequantGemmProblem {
@@ -119,10 +149,68 @@ struct DequantGemmProblem {
     const int* tile_off;
     const int2* tile_ent;       // (row in tile << 8 | column in tile, value / row scale)
     int use_tma;                // X tiles by the copy engine (xmap); 0 = 16-byte cp.async pieces
+    int book_copies;            // copies of the codebook in shared memory (dq_build_book)
 };
 
-__global__ void __launch_bounds__(kDqThreads, 1) vq_dequant_gemm_kernel(const __grid_constant__ DequantGemmProblem P,
+// The CTA's share of a tile's columns, summed over the Z splits in split order, scaled and stored (the eight producer warps).  A
+// thread takes four rows of every eighth column, with up to sixteen 16-byte loads in flight, and stores 8 bytes: with single numbers
+// two splits' sums of 256 columns took 15 k clocks of the kernel's 50 k (2560 to 6912 at batch 256 25.5 us, now 21.3).
+template <int Z>
+__device__ __forceinline__ void dq_reduce(const DequantGemmProblem& P, const unsigned char* tiles, unsigned rank, int N, int nb, int m0, int b0) {
+    constexpr int C = Z == 1 ? 8 : 16 / Z;   // columns at a time
+    const int per = (N + Z - 1) / Z, cfirst = (int)rank * per, clast = min(min(N, nb), cfirst + per), rows_out = P.row_stop - P.row_start;
+    const int warp = threadIdx.x >> 5, r4 = (threadIdx.x & 31) * 4, m = m0 + r4, live = min(4, P.row_stop - m);
+    if (live <= 0) return;
+    float sc[4], bi[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        sc[i] = P.scales && i < live ? P.scales[m + i] : 1.0f;
+        bi[i] = P.bias && i < live ? P.bias[m + i] : 0.0f;
+    }
+    const bool whole = live == 4 && rows_out % 4 == 0 && (reinterpret_cast<uintptr_t>(P.y) & 7) == 0;
+    unsigned part[Z];
+#pragma unroll
+    for (int z = 0; z < Z; ++z) part[z] = dq_map_cluster(smem_u32(tiles) + (unsigned)r4 * 4u, (unsigned)z);
+    for (int bb = cfirst + warp; bb < clast; bb += 8 * C) {
+        float4 pv[C][Z];
+#pragma unroll
+        for (int j = 0; j < C; ++j)
+#pragma unroll
+            for (int z = 0; z < Z; ++z) pv[j][z] = dq_ld_cluster4(part[z] + (unsigned)(min(bb + 8 * j, clast - 1) * kDqBlockM) * 4u);
+#pragma unroll
+        for (int j = 0; j < C; ++j) {
+            const int b = bb + 8 * j;
+            if (b >= clast) break;
+            float r[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+#pragma unroll
+            for (int z = 0; z < Z; ++z) {
+                r[0] += pv[j][z].x; r[1] += pv[j][z].y; r[2] += pv[j][z].z; r[3] += pv[j][z].w;
+            }
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                r[i] = fmaf(r[i], sc[i], bi[i]);
+                if (i < live && sc[i] == 0.0f && P.csr.nnz > 0)  // a zero row scale cannot carry the folded outliers: add them here
+                    for (int q = P.csr.row_ptrs[m + i]; q < P.csr.row_ptrs[m + i + 1]; ++q)
+                        r[i] += P.csr.vals[q] * __bfloat162float(P.x[(size_t)(b0 + b) * P.K + P.csr.cols[q]]);
+            }
+            __nv_bfloat16* y = P.y + (size_t)(b0 + b) * rows_out + (m - P.row_start);
+            if (whole) {
+                const __nv_bfloat162 lo = __floats2bfloat162_rn(r[0], r[1]), hi = __floats2bfloat162_rn(r[2], r[3]);
+                *reinterpret_cast<uint2*>(y) = make_uint2(*reinterpret_cast<const unsigned*>(&lo), *reinterpret_cast<const unsigned*>(&hi));
+            } else {
+#pragma unroll
+                for (int i = 0; i < 4; ++i) if (i < live) y[i] = __float2bfloat16_rn(r[i]);
+            }
+        }
+    }
+}
+
+struct DequantGemmPair { DequantGemmProblem P[2]; };   // row tiles [0, tiles0) of the first, then those of the second
+
+__global__ void __launch_bounds__(kDqThreads, 1) vq_dequant_gemm_kernel(const __grid_constant__ DequantGemmPair pair, int tiles0,
                                                                         const __grid_constant__ CUtensorMap xmap) {
+    const DequantGemmProblem& P = pair.P[(int)blockIdx.x >= tiles0 ? 1 : 0];
+    const int row_tile = (int)blockIdx.x - ((int)blockIdx.x >= tiles0 ? tiles0 : 0);
     extern __shared__ unsigned char dq_smem_raw[];
     // swizzled tiles need 1024-byte alignment; the dynamic segment only promises 16
     unsigned char* dq_smem = dq_smem_raw + ((1024u - (smem_u32(dq_smem_raw) & 1023u)) & 1023u);
@@ -131,8 +219,8 @@ __global__ void __launch_bounds__(kDqThreads, 1) vq_dequant_gemm_kernel(const __
     const int S = P.stages;
     const int a_bytes = kDqBlockM * 128, b_bytes = N * 128, stage_bytes = a_bytes + b_bytes;
     unsigned char* tiles = dq_smem;                                   // [stages][A | B], 1024-byte aligned
-    uint4* cb16 = reinterpret_cast<uint4*>(tiles + S * stage_bytes);   // [256] centroids as 8 bf16
-    unsigned long long* bars = reinterpret_cast<unsigned long long*>(cb16 + 256);
+    uint4* cb16 = reinterpret_cast<uint4*>(tiles + S * stage_bytes);   // [256 * book_copies] centroids as 8 bf16
+    unsigned long long* bars = reinterpret_cast<unsigned long long*>(cb16 + 256 * P.book_copies);
     unsigned* tmem_slot = reinterpret_cast<unsigned*>(bars + 2 * kDqStages + 1);
     int* rp_s = reinterpret_cast<int*>(tmem_slot + 2);                        // [129] row pointers of the CTA's rows
     int* tstart = rp_s + 130;                                                 // [kDqMaxTiles + 1] first entry of each K tile's outlier list
@@ -140,22 +228,19 @@ __global__ void __launch_bounds__(kDqThreads, 1) vq_dequant_gemm_kernel(const __
     int2* csr_s = reinterpret_cast<int2*>(tfill + kDqMaxTiles + 2);           // [csr_cap], 8-byte aligned
     const unsigned full0 = smem_u32(bars), empty0 = full0 + 8 * kDqStages, accum = empty0 + 8 * kDqStages;
 
-    const int m0 = P.row_start + blockIdx.x * kDqBlockM;
+    const int m0 = P.row_start + row_tile * kDqBlockM;
     const int b0 = blockIdx.y * 256;
     const int nb = min(256, P.batch - b0);
     const int rows_out = P.row_stop - P.row_start;
     const int KT_all = P.K / kDqBlockK;
     const int kt0 = blockIdx.z * P.tiles_per_split;                  // this CTA's K tiles: [kt0, kt0 + KT)
     const int KT = min(P.tiles_per_split, KT_all - kt0);
-    const bool split = P.ksplit > 1;
 
-    // codebook -> bf16, one 16-byte entry per centroid
-    for (int c = tid; c < 256; c += kDqThreads) {
-        __nv_bfloat162 h[4];
-#pragma unroll
-        for (int q = 0; q < 4; ++q) h[q] = __floats2bfloat162_rn(P.codebook[c * 8 + 2 * q], P.codebook[c * 8 + 2 * q + 1]);
-        cb16[c] = *reinterpret_cast<uint4*>(h);
-    }
+    dq_build_book(cb16, P.codebook, P.book_copies, kDqThreads);
+    chain_begin();   // (the layer's codebook is written by nothing in the stream; its outlier lists may be)
+    const int bshift = P.book_copies == 8 ? 0 : 1;
+    const uint4* const cb_lane = cb16 + ((lane & 7) >> bshift << bshift);   // this lane's copy
+    auto centroid = [&](unsigned code) { return cb_lane[(code >> bshift) * 8 + (code & bshift)]; };
     // Outliers of this CTA's rows and K range.  Normally they are listed per K tile in shared memory
     // (counting sort: count, prefix, scatter; entry = row << 8 | column in tile, value / row scale), so
     // that the group that builds a tile applies that tile's ~30 entries with one thread each.  If the
@@ -164,7 +249,7 @@ __global__ void __launch_bounds__(kDqThreads, 1) vq_dequant_gemm_kernel(const __
     bool listed = false;
     const bool glists = P.tile_off != nullptr && P.csr.nnz > 0 && KT <= kDqMaxTiles;
     if (glists) {
-        const int* off = P.tile_off + (size_t)blockIdx.x * (KT_all + 1) + kt0;
+        const int* off = P.tile_off + (size_t)row_tile * (KT_all + 1) + kt0;
         for (int i = tid; i <= KT; i += kDqThreads) tstart[i] = off[i];
     } else if (P.csr.nnz > 0 && m0 < P.row_stop) {
         const int n_rows = min(kDqBlockM, P.row_stop - m0);
@@ -317,7 +402,7 @@ __global__ void __launch_bounds__(kDqThreads, 1) vq_dequant_gemm_kernel(const __
 #pragma unroll
                 for (int q = 0; q < 8; ++q) {
                     const unsigned code = (cw[q >> 2] >> ((q & 3) * 8)) & 0xffu;
-                    wv[q] = rok[u] ? cb16[code] : make_uint4(0, 0, 0, 0);
+                    wv[q] = rok[u] ? centroid(code) : make_uint4(0, 0, 0, 0);
                 }
 #pragma unroll
                 for (int q = 0; q < 8; ++q) *reinterpret_cast<uint4*>(arow + ((q ^ r7) << 4)) = wv[q];
@@ -352,19 +437,12 @@ __global__ void __launch_bounds__(kDqThreads, 1) vq_dequant_gemm_kernel(const __
         asm volatile("cp.async.wait_group 0;" ::: "memory");
         // the epilogue and the split reduction address rows as (tid & 127, tid >> 7)
         const int trow = tid & 127, half = tid >> 7;
-        const int m = m0 + trow;
-        const bool row_ok = m < P.row_stop;
-        const float row_scale = (row_ok && P.scales) ? P.scales[m] : 1.0f;
-        int csr_begin = 0, cend_row = 0;
-        if (row_ok && P.csr.nnz > 0) { csr_begin = P.csr.row_ptrs[m]; cend_row = P.csr.row_ptrs[m + 1]; }
         // ---------------- epilogue: accumulator row trow; the two threads of a row split the batch columns
         if (ok) ok = mbar_wait(accum, 0);
         if (ok) {
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-            const float sc = row_scale;
-            const float bi = (row_ok && P.bias) ? P.bias[m] : 0.0f;
             const int cbeg = half * (N >> 1), cstop = cbeg + (N >> 1);
-            float* part = reinterpret_cast<float*>(tiles);   // split: [column][row] fp32, read by the whole cluster
+            float* part = reinterpret_cast<float*>(tiles);   // raw sums [column][row] fp32, read by the whole cluster
             for (int c0 = cbeg; c0 < cstop; c0 += 16) {
                 unsigned v[16];
                 const unsigned taddr = tmem_base + ((unsigned)((warp & 3) * 32) << 16) + (unsigned)c0;
@@ -374,23 +452,9 @@ __global__ void __launch_bounds__(kDqThreads, 1) vq_dequant_gemm_kernel(const __
                       "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15])
                     : "r"(taddr));
                 asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-                if (split) {   // raw partial sums, rows contiguous
 #pragma unroll
-                    for (int j = 0; j < 16; ++j)
-                        if (c0 + j < cstop) part[(c0 + j) * kDqBlockM + trow] = __uint_as_float(v[j]);
-                } else if (row_ok) {
-#pragma unroll
-                    for (int j = 0; j < 16; ++j) {
-                        const int b = c0 + j;
-                        if (b < nb && b < cstop) {
-                            float r = fmaf(__uint_as_float(v[j]), sc, bi);
-                            if (sc == 0.0f)  // a zero row scale cannot carry the folded outliers: add them here
-                                for (int q = csr_begin; q < cend_row; ++q)
-                                    r += P.csr.vals[q] * __bfloat162float(P.x[(size_t)(b0 + b) * P.K + P.csr.cols[q]]);
-                            P.y[(size_t)(b0 + b) * rows_out + (m - P.row_start)] = __float2bfloat16_rn(r);
-                        }
-                    }
-                }
+                for (int j = 0; j < 16; ++j)
+                    if (c0 + j < cstop) part[(c0 + j) * kDqBlockM + trow] = __uint_as_float(v[j]);
             }
         }
     } else if (lane == 0) {
@@ -424,42 +488,23 @@ __global__ void __launch_bounds__(kDqThreads, 1) vq_dequant_gemm_kernel(const __
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"((unsigned)P.tmem_cols) : "memory");
     }
-    if (split) {
-        // Every CTA of the cluster adds the partial sums of its share of the batch columns, in split order (the result
-        // does not depend on timing), and finishes those outputs.  All threads take part in the two cluster barriers;
-        // a CTA whose waits ran out still arrives, so the others are not left waiting.
+    // Every CTA of the cluster (of one without a split) adds the partial sums of its share of the batch columns, in split order
+    // (the result does not depend on timing), and finishes those outputs.  All threads take part in the two cluster barriers;
+    // a CTA whose waits ran out still arrives, so the others are not left waiting.
+    {
         dq_cluster_sync();   // the partial sums of every split are in place
         if (warp < kDqProducers / 32) {
             unsigned rank;
             asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(rank));
-            const int per = (N + P.ksplit - 1) / P.ksplit;
-            const int cfirst = (int)rank * per, clast = min(min(N, nb), cfirst + per);
-            const int trow = tid & 127, half = tid >> 7, m = m0 + trow;
-            if (m < P.row_stop) {
-                const float sc = P.scales ? P.scales[m] : 1.0f, bi = P.bias ? P.bias[m] : 0.0f;
-                const unsigned part0 = smem_u32(tiles);
-                for (int bb = cfirst + half; bb < clast; bb += 8) {   // four columns at a time: all loads first
-                    float pv[4][4];
-#pragma unroll
-                    for (int j = 0; j < 4; ++j)
-#pragma unroll
-                        for (int z = 0; z < 4; ++z)
-                            pv[j][z] = (bb + 2 * j < clast && z < P.ksplit)
-                                           ? dq_ld_cluster(part0 + (unsigned)((bb + 2 * j) * kDqBlockM + trow) * 4u, (unsigned)z) : 0.0f;
-#pragma unroll
-                    for (int j = 0; j < 4; ++j) {
-                        const int b = bb + 2 * j;
-                        if (b >= clast) break;
-                        float acc = 0.0f;
-#pragma unroll
-                        for (int z = 0; z < 4; ++z) if (z < P.ksplit) acc += pv[j][z];
-                        float r = fmaf(acc, sc, bi);
-                        if (sc == 0.0f && P.csr.nnz > 0)  // a zero row scale cannot carry the folded outliers: add them here
-                            for (int q = P.csr.row_ptrs[m]; q < P.csr.row_ptrs[m + 1]; ++q)
-                                r += P.csr.vals[q] * __bfloat162float(P.x[(size_t)(b0 + b) * P.K + P.csr.cols[q]]);
-                        P.y[(size_t)(b0 + b) * rows_out + (m - P.row_start)] = __float2bfloat16_rn(r);
-                    }
-                }
+            switch (P.ksplit) {
+                case 1: dq_reduce<1>(P, tiles, rank, N, nb, m0, b0); break;
+                case 2: dq_reduce<2>(P, tiles, rank, N, nb, m0, b0); break;
+                case 3: dq_reduce<3>(P, tiles, rank, N, nb, m0, b0); break;
+                case 4: dq_reduce<4>(P, tiles, rank, N, nb, m0, b0); break;
+                case 5: dq_reduce<5>(P, tiles, rank, N, nb, m0, b0); break;
+                case 6: dq_reduce<6>(P, tiles, rank, N, nb, m0, b0); break;
+                case 7: dq_reduce<7>(P, tiles, rank, N, nb, m0, b0); break;
+                default: dq_reduce<8>(P, tiles, rank, N, nb, m0, b0); break;
             }
         }
         dq_cluster_sync();   // nobody leaves while its partial sums may still be read
@@ -493,8 +538,8 @@ __global__ void __launch_bounds__(kDq2Threads, 1) vq_dequant_gemm256_kernel(cons
     constexpr int S = kDq2Stages;
     const int a_bytes = 2 * kDqBlockM * 128, b_bytes = N * 128, stage_bytes = a_bytes + b_bytes;
     unsigned char* tiles = dq_smem;                                    // [3][A0 | A1 | B], 1024-byte aligned
-    uint4* cb16 = reinterpret_cast<uint4*>(tiles + S * stage_bytes);    // [256] centroids as 8 bf16
-    unsigned long long* bars = reinterpret_cast<unsigned long long*>(cb16 + 256);
+    uint4* cb16 = reinterpret_cast<uint4*>(tiles + S * stage_bytes);    // [256 * book_copies] centroids as 8 bf16
+    unsigned long long* bars = reinterpret_cast<unsigned long long*>(cb16 + 256 * P.book_copies);
     unsigned* tmem_slot = reinterpret_cast<unsigned*>(bars + 2 * S + 1);
     int* toff = reinterpret_cast<int*>(tmem_slot + 2);                  // [2][kDqMaxTiles + 2] outlier list offsets of both row tiles
     const unsigned full0 = smem_u32(bars), empty0 = full0 + 8 * S, accum = empty0 + 8 * S;
@@ -510,12 +555,11 @@ __global__ void __launch_bounds__(kDq2Threads, 1) vq_dequant_gemm256_kernel(cons
     const bool glists = P.tile_off != nullptr && P.csr.nnz > 0;
     const int row_tiles = (rows_out + kDqBlockM - 1) / kDqBlockM;
 
-    for (int c = tid; c < 256; c += kDq2Threads) {
-        __nv_bfloat162 h[4];
-#pragma unroll
-        for (int q = 0; q < 4; ++q) h[q] = __floats2bfloat162_rn(P.codebook[c * 8 + 2 * q], P.codebook[c * 8 + 2 * q + 1]);
-        cb16[c] = *reinterpret_cast<uint4*>(h);
-    }
+    dq_build_book(cb16, P.codebook, P.book_copies, kDq2Threads);
+    chain_begin();   // (the layer's codebook is written by nothing in the stream; its outlier lists may be)
+    const int bshift = P.book_copies == 8 ? 0 : 1;
+    const uint4* const cb_lane = cb16 + ((lane & 7) >> bshift << bshift);   // this lane's copy
+    auto centroid = [&](unsigned code) { return cb_lane[(code >> bshift) * 8 + (code & bshift)]; };
     for (int i = tid; i < 2 * (kDqMaxTiles + 2); i += kDq2Threads) {
         const int a = i / (kDqMaxTiles + 2), k = i - a * (kDqMaxTiles + 2), rt = 2 * (int)blockIdx.x + a;
         toff[i] = (glists && rt < row_tiles && k <= KT) ? P.tile_off[(size_t)rt * (KT_all + 1) + kt0 + k] : 0;
@@ -612,7 +656,7 @@ __global__ void __launch_bounds__(kDq2Threads, 1) vq_dequant_gemm256_kernel(cons
 #pragma unroll
                 for (int q = 0; q < 8; ++q) {
                     const unsigned code = (cw[q >> 2] >> ((q & 3) * 8)) & 0xffu;
-                    wv[q] = rok[u] ? cb16[code] : make_uint4(0, 0, 0, 0);
+                    wv[q] = rok[u] ? centroid(code) : make_uint4(0, 0, 0, 0);
                 }
 #pragma unroll
                 for (int q = 0; q < 8; ++q) *reinterpret_cast<uint4*>(arow + ((q ^ r7) << 4)) = wv[q];
@@ -732,15 +776,15 @@ __global__ void __launch_bounds__(kDq2Threads, 1) vq_dequant_gemm256_kernel(cons
     }
 }
 
-size_t dequant_gemm256_smem(int n_pad) {
-    return (size_t)kDq2Stages * (2 * kDqBlockM * 128 + (size_t)n_pad * 128) + 256 * 16 + (2 * kDq2Stages + 1) * 8 + 16 +
+size_t dequant_gemm256_smem(int n_pad, int copies) {
+    return (size_t)kDq2Stages * (2 * kDqBlockM * 128 + (size_t)n_pad * 128) + 256 * 16 * (size_t)copies + (2 * kDq2Stages + 1) * 8 + 16 +
            sizeof(int) * 2 * (kDqMaxTiles + 2) + 1024;
 }
 
 constexpr size_t kDqSmemBudget = 226 * 1024;   // dynamic shared memory; the kernel also has a few static bytes
 
-size_t dequant_gemm_smem(int n_pad, int stages, int csr_cap) {
-    return (size_t)stages * (kDqBlockM * 128 + (size_t)n_pad * 128) + 256 * 16 + (2 * kDqStages + 1) * 8 + 16 +
+size_t dequant_gemm_smem(int n_pad, int stages, int csr_cap, int copies) {
+    return (size_t)stages * (kDqBlockM * 128 + (size_t)n_pad * 128) + 256 * 16 * (size_t)copies + (2 * kDqStages + 1) * 8 + 16 +
            sizeof(int) * (130 + 2 * (kDqMaxTiles + 2)) + (size_t)csr_cap * 8 + 1024;
 }
 
@@ -763,12 +807,41 @@ bool dequant_gemm_supported(const LinearProblem& P, bool csr_sorted) {
            (reinterpret_cast<uintptr_t>(P.x) & 15) == 0;
 }
 
+// Clusters of z CTAs of one SM each that are resident at once (a cluster lies inside a GPC); cached per device.
+static int dq_resident_clusters(int z) {
+    static std::atomic<int> cache[64][9];
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return 0;
+    int n = cache[dev][z].load(std::memory_order_relaxed);
+    if (n != 0) return n > 0 ? n : 0;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(64, 1, z);
+    cfg.blockDim = dim3(kDqThreads);
+    cfg.dynamicSmemBytes = kDqSmemBudget;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = 1;
+    attr[0].val.clusterDim.y = 1;
+    attr[0].val.clusterDim.z = z;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    n = 0;
+    if (cudaFuncSetAttribute(vq_dequant_gemm_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kDqSmemBudget) != cudaSuccess ||
+        cudaOccupancyMaxActiveClusters(&n, vq_dequant_gemm_kernel, &cfg) != cudaSuccess) {
+        cudaGetLastError();
+        n = 0;
+    }
+    cache[dev][z].store(n > 0 ? n : -1, std::memory_order_relaxed);
+    return n;
+}
+
 // Splits along K for `ctas` (row tile, batch tile) pairs and KT tiles of 64 columns: fill the SMs, at most
-// four splits (one thread-block cluster), at least eight tiles per split, an even number of tiles per split.
+// zmax splits (one thread-block cluster), at least eight tiles per split, an even number of tiles per split, all clusters resident at
+// once.  us, 6912 to 2560 (20 tiles) at batch 32 and 256 by splits: 4 18.1 / 24.3, 5 15.7 / 21.8, 6 14.1 / 20.4, 7 (two rounds) 25.3 / 36.7.
 static void plan_ksplit(int ctas, int KT, int sms, int zmax, int* ksplit, int* per) {
     int z = sms / (ctas > 0 ? ctas : 1);
     z = z < 1 ? 1 : z > zmax ? zmax : z;
-    while (z > 1 && KT / z < 8) --z;
+    while (z > 1 && (KT / z < 8 || dq_resident_clusters(z) < ctas)) --z;
     int p = (KT + z - 1) / z;
     p += p & 1;
     *per = z > 1 ? p : KT;
@@ -906,8 +979,9 @@ static bool encode_x_map(CUtensorMap* map, const void* x, int K, int batch, int 
                CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
-int launch_dequant_gemm(const LinearProblem& L, cudaStream_t stream, DqLists* lists, unsigned generation) {
-    DequantGemmProblem P{};
+// What the 128-row kernel is given for a layer, but its stages and its split.
+static int dq_problem(DequantGemmProblem* out, const LinearProblem& L, cudaStream_t stream, DqLists* lists, unsigned generation) {
+    DequantGemmProblem& P = *out;
     int* error_flag = nullptr;
     OJX_CUDA_TRY(cudaGetSymbolAddress((void**)&error_flag, g_dq_error));
     P.codes = L.codes; P.codebook = L.codebook; P.scales = L.scales; P.bias = L.bias; P.csr = L.csr;
@@ -922,6 +996,100 @@ int launch_dequant_gemm(const LinearProblem& L, cudaStream_t stream, DqLists* li
     // Outlier lists of the layer (built once) spare every CTA the sort in its prologue and the shared memory for it.
     const bool glists = L.K / kDqBlockK <= kDqMaxTiles && !getenv("OJASX_B200_TENSOR_NO_LISTS") && ensure_dq_lists(lists, L, generation, stream);
     if (glists) { P.tile_off = lists->off; P.tile_ent = lists->ent; }
+    return OJX_OK;
+}
+
+// One launch of the 128-row kernel for a layer, or for two of one width and batch on the same activations.
+static int launch_dq128(DequantGemmProblem* P, const LinearProblem* L, int count, cudaStream_t stream) {
+    bool glists = true;   // outliers of both, where there are any, are listed already
+    for (int i = 0; i < count; ++i) glists = glists && (P[i].tile_off != nullptr || L[i].csr.nnz == 0);
+    // Stage buffers: at least one per producer group.  (A group waits on a stage's "empty" barrier by phase
+    // parity; with fewer stages than groups a group could be two phases ahead of a stage it shares with
+    // another group, and a parity wait cannot tell "two ahead" from "done".)  More stages when the batch
+    // tile is narrow; room for at least 1024 staged outlier entries is kept when every CTA lists its own.
+    const int n_pad = P[0].n_pad;
+    int stages = kDqGroups;
+    const int copies = dequant_gemm_smem(n_pad, stages, glists ? 0 : 1024, 8) <= kDqSmemBudget ? 8 : 4;
+    if (dequant_gemm_smem(n_pad, stages, glists ? 0 : 1024, copies) > kDqSmemBudget) return OJX_ERR_UNSUPPORTED;
+    while (stages < kDqStages && dequant_gemm_smem(n_pad, stages + 1, glists ? 0 : 4096, copies) <= kDqSmemBudget) ++stages;
+    // shared-memory room for the outliers of 128 rows: whatever is left, up to 8192 entries; the
+    // kernel reads entries beyond that from global memory
+    int csr_cap = 0;
+    if (!glists) {
+        const size_t left = kDqSmemBudget - dequant_gemm_smem(n_pad, stages, 0, copies);
+        csr_cap = (int)(left / 8 < 8192 ? left / 8 : 8192);
+    }
+    const size_t smem = dequant_gemm_smem(n_pad, stages, csr_cap, copies);
+    // the opt-in is a per-device attribute of the kernel: remember what each device was given
+    static thread_local size_t configured[64] = {};
+    int cur_dev = 0;
+    OJX_CUDA_TRY(cudaGetDevice(&cur_dev));
+    if (cur_dev < 0 || cur_dev >= 64 || smem > configured[cur_dev]) {
+        OJX_CUDA_TRY(cudaFuncSetAttribute(vq_dequant_gemm_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        if (cur_dev >= 0 && cur_dev < 64) configured[cur_dev] = smem;
+    }
+    int tiles[2] = {0, 0};
+    for (int i = 0; i < count; ++i) tiles[i] = (L[i].row_stop - L[i].row_start + kDqBlockM - 1) / kDqBlockM;
+    dim3 grid(tiles[0] + tiles[1], (L[0].batch + 255) / 256, 1);
+    const int KT = L[0].K / kDqBlockK;
+    int z = 1, per = KT;
+    if (!getenv("OJASX_B200_TENSOR_NO_KSPLIT")) plan_ksplit((int)(grid.x * grid.y), KT, num_sms(), 8, &z, &per);
+    grid.z = z;
+    // X tiles by the copy engine when the tensor map can be made (OJASX_B200_TENSOR_TMA=0 keeps the 16-byte copies)
+    CUtensorMap xmap{};
+    const char* tma_env = getenv("OJASX_B200_TENSOR_TMA");
+    const bool tma = !(tma_env && tma_env[0] == '0') && encode_x_map(&xmap, L[0].x, L[0].K, L[0].batch, n_pad);
+    DequantGemmPair pair{};
+    for (int i = 0; i < count; ++i) {
+        P[i].stages = stages;
+        P[i].book_copies = copies;
+        P[i].csr_cap = csr_cap;
+        P[i].ksplit = z;
+        P[i].tiles_per_split = z > 1 ? per : KT;
+        P[i].use_tma = tma ? 1 : 0;
+        pair.P[i] = P[i];
+    }
+    // the K splits of a tile are one cluster (they exchange partial sums through distributed shared memory)
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = grid;
+    cfg.blockDim = dim3(kDqThreads);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = stream;
+    cudaLaunchAttribute attr[2];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = 1;
+    attr[0].val.clusterDim.y = 1;
+    attr[0].val.clusterDim.z = grid.z;
+    attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;   // see launch_chained
+    attr[1].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 2;
+    OJX_CUDA_TRY(cudaLaunchKernelEx(&cfg, vq_dequant_gemm_kernel, pair, tiles[0], xmap));
+    count_launch(1);
+    return OJX_OK;
+}
+
+// Gate and up of a SwiGLU block in one launch, if their tiles do not need more than a round of the SMs: then nothing, or less, is
+// split along K.  us for both, 2560 to 6912, two launches and one: batch 32 30 / 21, 64 31 / 23, 128 34 / 25, 256 43 / 33.  The block:
+// 62 / 40, 72 / 44, 76 / 50, 94 / 64, with a call into the library for each layer before.
+bool dequant_gemm_pair_pays(const LinearProblem& A, const LinearProblem& B) {
+    const int tiles = (A.row_stop - A.row_start + kDqBlockM - 1) / kDqBlockM + (B.row_stop - B.row_start + kDqBlockM - 1) / kDqBlockM;
+    return A.K == B.K && A.batch == B.batch && A.x == B.x && tiles * ((A.batch + 255) / 256) <= num_sms();
+}
+int launch_dequant_gemm_pair(const LinearProblem* L, cudaStream_t stream, DqLists* const* lists, const unsigned* generation) {
+    DequantGemmProblem P[2]{};
+    for (int i = 0; i < 2; ++i) {
+        const int rc = dq_problem(&P[i], L[i], stream, lists[i], generation[i]);
+        if (rc != OJX_OK) return rc;
+    }
+    return launch_dq128(P, L, 2, stream);
+}
+
+int launch_dequant_gemm(const LinearProblem& L, cudaStream_t stream, DqLists* lists, unsigned generation) {
+    DequantGemmProblem P{};
+    const int rc = dq_problem(&P, L, stream, lists, generation);
+    if (rc != OJX_OK) return rc;
+    const bool glists = P.tile_off != nullptr;
     // Batches of several 256-column tiles: two row tiles per CTA share every X tile (vq_dequant_gemm256_kernel), when
     // the tile pairs fill the GPU without a split along K.  OJASX_B200_TENSOR_ROWS=128 / 256 forces one kernel or the
     // other (256: with a split if the grid is small).
@@ -933,7 +1101,7 @@ int launch_dequant_gemm(const LinearProblem& L, cudaStream_t stream, DqLists* li
         const bool fills = (int)(grid.x * grid.y) * 3 >= num_sms() * 2;
         CUtensorMap xmap{};
         if ((forced == 256 || (forced != 128 && fills)) && !(tma_off && tma_off[0] == '0') && (glists || L.csr.nnz == 0) &&
-            rows > kDqBlockM && P.n_pad >= 64 && dequant_gemm256_smem(P.n_pad) <= kDqSmemBudget &&
+            rows > kDqBlockM && P.n_pad >= 64 && dequant_gemm256_smem(P.n_pad, 4) <= kDqSmemBudget &&
             encode_x_map(&xmap, L.x, L.K, L.batch, P.n_pad)) {
             int z = 1, per = L.K / kDqBlockK;
             if (forced == 256 && !getenv("OJASX_B200_TENSOR_NO_KSPLIT")) plan_ksplit((int)(grid.x * grid.y), L.K / kDqBlockK, num_sms(), 8, &z, &per);
@@ -945,7 +1113,8 @@ int launch_dequant_gemm(const LinearProblem& L, cudaStream_t stream, DqLists* li
                 P.tmem_cols = cols2;
                 P.stages = kDq2Stages;
                 P.use_tma = 1;
-                const size_t smem = dequant_gemm256_smem(P.n_pad);
+                P.book_copies = dequant_gemm256_smem(P.n_pad, 8) <= kDqSmemBudget ? 8 : 4;
+                const size_t smem = dequant_gemm256_smem(P.n_pad, P.book_copies);
                 static thread_local size_t configured2[64] = {};
                 int dev = 0;
                 OJX_CUDA_TRY(cudaGetDevice(&dev));
@@ -959,75 +1128,22 @@ int launch_dequant_gemm(const LinearProblem& L, cudaStream_t stream, DqLists* li
                 cfg.blockDim = dim3(kDq2Threads);
                 cfg.dynamicSmemBytes = smem;
                 cfg.stream = stream;
-                cudaLaunchAttribute attr[1];
+                cudaLaunchAttribute attr[2];
                 attr[0].id = cudaLaunchAttributeClusterDimension;
                 attr[0].val.clusterDim.x = 1;
                 attr[0].val.clusterDim.y = 1;
                 attr[0].val.clusterDim.z = grid.z;
+                attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;   // see launch_chained
+                attr[1].val.programmaticStreamSerializationAllowed = 1;
                 cfg.attrs = attr;
-                cfg.numAttrs = 1;
+                cfg.numAttrs = 2;
                 OJX_CUDA_TRY(cudaLaunchKernelEx(&cfg, vq_dequant_gemm256_kernel, P, xmap));
                 count_launch(1);
                 return OJX_OK;
             }
         }
     }
-    // Stage buffers: at least one per producer group.  (A group waits on a stage's "empty" barrier by phase
-    // parity; with fewer stages than groups a group could be two phases ahead of a stage it shares with
-    // another group, and a parity wait cannot tell "two ahead" from "done".)  More stages when the batch
-    // tile is narrow; room for at least 1024 staged outlier entries is kept when every CTA lists its own.
-    P.stages = kDqGroups;
-    if (dequant_gemm_smem(P.n_pad, P.stages, glists ? 0 : 1024) > kDqSmemBudget) return OJX_ERR_UNSUPPORTED;
-    while (P.stages < kDqStages && dequant_gemm_smem(P.n_pad, P.stages + 1, glists ? 0 : 4096) <= kDqSmemBudget) ++P.stages;
-    // shared-memory room for the outliers of 128 rows: whatever is left, up to 8192 entries; the
-    // kernel reads entries beyond that from global memory
-    P.csr_cap = 0;
-    if (L.csr.nnz > 0 && !glists) {
-        const size_t left = kDqSmemBudget - dequant_gemm_smem(P.n_pad, P.stages, 0);
-        P.csr_cap = (int)(left / 8 < 8192 ? left / 8 : 8192);
-    }
-    const size_t smem = dequant_gemm_smem(P.n_pad, P.stages, P.csr_cap);
-    // the opt-in is a per-device attribute of the kernel: remember what each device was given
-    static thread_local size_t configured[64] = {};
-    int cur_dev = 0;
-    OJX_CUDA_TRY(cudaGetDevice(&cur_dev));
-    if (cur_dev < 0 || cur_dev >= 64 || smem > configured[cur_dev]) {
-        OJX_CUDA_TRY(cudaFuncSetAttribute(vq_dequant_gemm_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-        if (cur_dev >= 0 && cur_dev < 64) configured[cur_dev] = smem;
-    }
-    const int rows = L.row_stop - L.row_start;
-    dim3 grid((rows + kDqBlockM - 1) / kDqBlockM, (L.batch + 255) / 256, 1);
-    P.ksplit = 1;
-    P.tiles_per_split = L.K / kDqBlockK;
-    if (!getenv("OJASX_B200_TENSOR_NO_KSPLIT")) {
-        int z = 1, per = P.tiles_per_split;
-        plan_ksplit((int)(grid.x * grid.y), L.K / kDqBlockK, num_sms(), 4, &z, &per);
-        if (z > 1) {
-            P.ksplit = z;
-            P.tiles_per_split = per;
-            grid.z = z;
-        }
-    }
-    // X tiles by the copy engine when the tensor map can be made (OJASX_B200_TENSOR_TMA=0 keeps the 16-byte copies)
-    CUtensorMap xmap{};
-    const char* tma_env = getenv("OJASX_B200_TENSOR_TMA");
-    P.use_tma = !(tma_env && tma_env[0] == '0') && encode_x_map(&xmap, L.x, L.K, L.batch, P.n_pad) ? 1 : 0;
-    // the K splits of a tile are one cluster (they exchange partial sums through distributed shared memory)
-    cudaLaunchConfig_t cfg{};
-    cfg.gridDim = grid;
-    cfg.blockDim = dim3(kDqThreads);
-    cfg.dynamicSmemBytes = smem;
-    cfg.stream = stream;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeClusterDimension;
-    attr[0].val.clusterDim.x = 1;
-    attr[0].val.clusterDim.y = 1;
-    attr[0].val.clusterDim.z = grid.z;
-    cfg.attrs = attr;
-    cfg.numAttrs = 1;
-    OJX_CUDA_TRY(cudaLaunchKernelEx(&cfg, vq_dequant_gemm_kernel, P, xmap));
-    count_launch(1);
-    return OJX_OK;
+    return launch_dq128(&P, &L, 1, stream);
 }
 
 }  // namespace ojx

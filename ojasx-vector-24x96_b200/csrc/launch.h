@@ -70,6 +70,8 @@ struct DqLists {
     ~DqLists();
 };
 int launch_dequant_gemm(const LinearProblem& P, cudaStream_t stream, DqLists* lists = nullptr, unsigned generation = 0);
+bool dequant_gemm_pair_pays(const LinearProblem& A, const LinearProblem& B);
+int launch_dequant_gemm_pair(const LinearProblem* P, cudaStream_t stream, DqLists* const* lists, const unsigned* generation);
 int take_dequant_gemm_error(int* out);
 
 // --- gather_mma.cu: bf16 batches below the tensor-core path, weights gathered into mma.sync operands at fp32 accuracy

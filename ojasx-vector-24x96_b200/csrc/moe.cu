@@ -822,6 +822,7 @@ __global__ void __launch_bounds__(kTopkWarps * 32) moe_router_topk_reg_kernel(co
 // to the io dtype (the SwiGLU step of a dense VQ MLP block: gate and up are separate VQ linears).
 __global__ void silu_mul_kernel(const void* __restrict__ gate, const void* __restrict__ up, void* __restrict__ out,
                                 size_t n, int io_dtype) {
+    chain_begin();
     const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     if (io_dtype == OJX_BF16) {
@@ -837,8 +838,7 @@ __global__ void silu_mul_kernel(const void* __restrict__ gate, const void* __res
 int launch_silu_mul(const void* gate, const void* up, void* out, size_t n, int io_dtype, cudaStream_t s) {
     if (!gate || !up || !out) return OJX_ERR_ARG;
     if (n == 0) return OJX_OK;
-    silu_mul_kernel<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(gate, up, out, n, io_dtype);
-    OJX_CUDA_TRY(cudaGetLastError());
+    OJX_CUDA_TRY(launch_chained(silu_mul_kernel, (unsigned)((n + 255) / 256), 256, 0, s, gate, up, out, n, io_dtype));
     count_launch(1);
     return OJX_OK;
 }

@@ -222,8 +222,7 @@ class VQMLP:
         self._pair = VQLinearGroup([gate, up])   # one launch for gate and up when there is a single token
 
     def forward(self, x: torch.Tensor) -> torch.Tensor:
-        if x.dtype is torch.bfloat16 and x.is_cuda and x.shape[-1] == self.gate.in_features and \
-                x.numel() // self.gate.in_features in GATHER_BATCHES:
+        if x.dtype is torch.bfloat16 and x.is_cuda and x.shape[-1] == self.gate.in_features and x.numel():
             x2 = x.reshape(-1, self.gate.in_features).contiguous()
             handles = (self.gate.handle, self.up.handle, self.down.handle)
             size = lib().ojasx_b200_mlp_workspace(*handles, x2.data_ptr(), x2.shape[0], BF16)
