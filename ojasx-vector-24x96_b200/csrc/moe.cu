@@ -38,6 +38,12 @@ __device__ __forceinline__ MoePair decode_pair(const MoeProblem& P, int pair) {
     return r;
 }
 
+}  // namespace ojx
+
+#include "moe_few.cuh"
+
+namespace ojx {
+
 template <int D>
 __global__ void __launch_bounds__(kThreads, kCtasPerSm) moe_gate_up_kernel(const __grid_constant__ MoeProblem P) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -912,6 +918,21 @@ static int launch_combine(const MoeProblem& P, const PeerLink& link, cudaStream_
     return OJX_OK;
 }
 
+// Plans of the kernels for a handful of pairs (moe_few.cuh); bytes = 0: the row-per-lane kernels.  OJASX_B200_MOE_FEW=0 keeps those.
+static bool moe_few_wanted(const MoeProblem& P, int G, const void* codes) {
+    if (P.pair_list || P.n_tokens * P.k_active > kMoePlanMinPairs || (G & 7) != 0 || (reinterpret_cast<uintptr_t>(codes) & 7) != 0) return false;
+    const char* e = std::getenv("OJASX_B200_MOE_FEW");
+    return !(e && e[0] == '0');
+}
+static MoeFewPlan moe_few_gate_up(const MoeProblem& P) {
+    if (!P.lut_in || P.lut_blocks != 0 || (reinterpret_cast<uintptr_t>(P.lut_in) & 15) != 0 || !moe_few_wanted(P, P.G, P.gu_codes)) return MoeFewPlan{};
+    return moe_few_plan(expected_pairs(P), kCtasPerSm * num_sms(), P.I, 2, P.G, P.H, false);
+}
+static MoeFewPlan moe_few_down(const MoeProblem& P) {
+    if (!moe_few_wanted(P, P.Gi, P.dn_codes)) return MoeFewPlan{};
+    return moe_few_plan(expected_pairs(P), kCtasPerSm * num_sms(), P.H, 1, P.Gi, P.I, true);
+}
+
 template <int D>
 static int launch_moe_experts_t(const MoeProblem& P, cudaStream_t s, const PeerLink& link) {
     int rc;
@@ -951,7 +972,13 @@ static int launch_moe_experts_t(const MoeProblem& P, cudaStream_t s, const PeerL
             OJX_CUDA_TRY(cudaGetLastError());
             ++extra;
         }
-        OJX_CUDA_TRY(launch_chained(moe_gate_up_kernel<D>, gu_items < sms ? gu_items : sms, kThreads, sizeof(CoreSmem), s, P));
+        const MoeFewPlan f = moe_few_gate_up(P);
+        if (f.bytes > 0) {
+            if ((rc = set_smem(moe_gate_up_few_kernel)) != OJX_OK) return rc;
+            OJX_CUDA_TRY(launch_chained(moe_gate_up_few_kernel, pairs * f.tiles, kFewThreads + 32, f.bytes, s, P, f, P.lut_ready));
+        } else {
+            OJX_CUDA_TRY(launch_chained(moe_gate_up_kernel<D>, gu_items < sms ? gu_items : sms, kThreads, sizeof(CoreSmem), s, P));
+        }
     }
     bool chain_down = false;
     if constexpr (D <= 16) {
@@ -961,7 +988,13 @@ static int launch_moe_experts_t(const MoeProblem& P, cudaStream_t s, const PeerL
             chain_down = true;
         }
     }
-    if (!chain_down) OJX_CUDA_TRY(launch_chained(moe_down_kernel<D>, dn_items < sms ? dn_items : sms, kThreads, sizeof(CoreSmem), s, P, link));
+    const MoeFewPlan f = chain_down ? MoeFewPlan{} : moe_few_down(P);
+    if (f.bytes > 0) {
+        if ((rc = set_smem(moe_down_few_kernel<D>)) != OJX_OK) return rc;
+        OJX_CUDA_TRY(launch_chained(moe_down_few_kernel<D>, pairs * f.tiles, kFewThreads, f.bytes, s, P, f, link));
+    } else if (!chain_down) {
+        OJX_CUDA_TRY(launch_chained(moe_down_kernel<D>, dn_items < sms ? dn_items : sms, kThreads, sizeof(CoreSmem), s, P, link));
+    }
     if ((rc = launch_combine(P, link, s)) != OJX_OK) return rc;
     count_launch(3 + extra);
     return OJX_OK;
