@@ -13,7 +13,7 @@
 // tcgen05.commit.  After the last K tile the producer warps become the epilogue: tcgen05.ld the
 // accumulator rows, scale, bias, store bf16.
 //
-// A layer has few 128-row tiles (54 for 6912 rows), so the K axis is split over up to eight CTAs per
+// A layer has few 128-row tiles (54 for 6912 rows), so the K axis is split over up to four CTAs per
 // tile until the GPU is full.  The CTAs of a tile form a thread-block cluster: each leaves its raw fp32
 // partial sums in its own shared memory (the stage buffers are idle by then), and after a cluster barrier
 // every CTA adds the partials of its share of the batch columns in split order, reading the other CTAs'
@@ -98,6 +98,16 @@ __device__ __forceinline__ float4 dq_ld_cluster4(unsigned remote) {
     return v;
 }
 
+// Sixteen accumulator columns of the warp's 32 lanes (all threads of the warp).
+__device__ __forceinline__ void dq_ld16(unsigned taddr, unsigned (&v)[16]) {
+    asm volatile(
+        "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
+        : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]), "=r"(v[8]), "=r"(v[9]),
+          "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15])
+        : "r"(taddr));
+    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+}
+
 // Shared-memory matrix descriptor of a K-major tile stored with the 128-byte swizzle: rows of 128
 // bytes, groups of 8 rows 1024 bytes apart.
 __device__ __forceinline__ unsigned long long make_desc_sw128(unsigned smem_addr) {
@@ -144,6 +154,7 @@ struct DequantGemmProblem {
     int csr_cap;                // outlier entries of the CTA's rows that fit in shared memory
     int ksplit;                 // CTAs per tile along K (gridDim.z = the cluster's size)
     int tiles_per_split;        // K tiles per split (even, so that a split's code bytes start 16-byte aligned)
+    int tiles_per_sum;          // K tiles per accumulator: those of a CTA, or half of them where one CTA does the work of two splits
     // Outliers listed per (128-row tile, 64-column tile) once per layer (dq_list_* kernels), or null: the lists are
     // then made in shared memory by every CTA.  tile_off[rt * (KT_all + 1) + kt] .. [+ 1] = the tile's entries.
     const int* tile_off;
@@ -154,7 +165,7 @@ struct DequantGemmProblem {
 
 // The CTA's share of a tile's columns, summed over the Z splits in split order, scaled and stored (the eight producer warps).  A
 // thread takes four rows of every eighth column, with up to sixteen 16-byte loads in flight, and stores 8 bytes: with single numbers
-// two splits' sums of 256 columns took 15 k clocks of the kernel's 50 k (2560 to 6912 at batch 256 25.5 us, now 21.3).
+// two splits' sums of 256 columns took 15 k clocks of the kernel's 50 k (2560 to 6912 at batch 256 28.9 us, now 23.0).
 template <int Z>
 __device__ __forceinline__ void dq_reduce(const DequantGemmProblem& P, const unsigned char* tiles, unsigned rank, int N, int nb, int m0, int b0) {
     constexpr int C = Z == 1 ? 8 : 16 / Z;   // columns at a time
@@ -444,14 +455,14 @@ __global__ void __launch_bounds__(kDqThreads, 1) vq_dequant_gemm_kernel(const __
             const int cbeg = half * (N >> 1), cstop = cbeg + (N >> 1);
             float* part = reinterpret_cast<float*>(tiles);   // raw sums [column][row] fp32, read by the whole cluster
             for (int c0 = cbeg; c0 < cstop; c0 += 16) {
-                unsigned v[16];
+                unsigned v[16], w[16];
                 const unsigned taddr = tmem_base + ((unsigned)((warp & 3) * 32) << 16) + (unsigned)c0;
-                asm volatile(
-                    "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
-                    : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]), "=r"(v[8]),
-                      "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15])
-                    : "r"(taddr));
-                asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+                dq_ld16(taddr, v);
+                if (KT > P.tiles_per_sum) {   // two sums in one CTA: added as the reduction adds those of two CTAs
+                    dq_ld16(taddr + (unsigned)N, w);
+#pragma unroll
+                    for (int j = 0; j < 16; ++j) v[j] = __float_as_uint(__uint_as_float(v[j]) + __uint_as_float(w[j]));
+                }
 #pragma unroll
                 for (int j = 0; j < 16; ++j)
                     if (c0 + j < cstop) part[(c0 + j) * kDqBlockM + trow] = __uint_as_float(v[j]);
@@ -466,14 +477,15 @@ __global__ void __launch_bounds__(kDqThreads, 1) vq_dequant_gemm_kernel(const __
             if (!ok) break;
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
             const unsigned a_addr = smem_u32(tiles + s * stage_bytes), b_addr = a_addr + a_bytes;
+            const unsigned dst = tmem_base + (unsigned)(kt / P.tiles_per_sum * N);
 #pragma unroll
             for (int j = 0; j < kDqBlockK / 16; ++j) {
                 const unsigned long long da = make_desc_sw128(a_addr + j * 32), db = make_desc_sw128(b_addr + j * 32);
-                const unsigned acc = (kt > 0 || j > 0) ? 1u : 0u;
+                const unsigned acc = (kt % P.tiles_per_sum > 0 || j > 0) ? 1u : 0u;
                 asm volatile(
                     "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
                     "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}"
-                    ::"r"(tmem_base), "l"(da), "l"(db), "r"(idesc), "r"(acc)
+                    ::"r"(dst), "l"(da), "l"(db), "r"(idesc), "r"(acc)
                     : "memory");
             }
             // frees the stage when the MMAs that read it have completed
@@ -500,11 +512,7 @@ __global__ void __launch_bounds__(kDqThreads, 1) vq_dequant_gemm_kernel(const __
                 case 1: dq_reduce<1>(P, tiles, rank, N, nb, m0, b0); break;
                 case 2: dq_reduce<2>(P, tiles, rank, N, nb, m0, b0); break;
                 case 3: dq_reduce<3>(P, tiles, rank, N, nb, m0, b0); break;
-                case 4: dq_reduce<4>(P, tiles, rank, N, nb, m0, b0); break;
-                case 5: dq_reduce<5>(P, tiles, rank, N, nb, m0, b0); break;
-                case 6: dq_reduce<6>(P, tiles, rank, N, nb, m0, b0); break;
-                case 7: dq_reduce<7>(P, tiles, rank, N, nb, m0, b0); break;
-                default: dq_reduce<8>(P, tiles, rank, N, nb, m0, b0); break;
+                default: dq_reduce<4>(P, tiles, rank, N, nb, m0, b0); break;
             }
         }
         dq_cluster_sync();   // nobody leaves while its partial sums may still be read
@@ -807,41 +815,14 @@ bool dequant_gemm_supported(const LinearProblem& P, bool csr_sorted) {
            (reinterpret_cast<uintptr_t>(P.x) & 15) == 0;
 }
 
-// Clusters of z CTAs of one SM each that are resident at once (a cluster lies inside a GPC); cached per device.
-static int dq_resident_clusters(int z) {
-    static std::atomic<int> cache[64][9];
-    int dev = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return 0;
-    int n = cache[dev][z].load(std::memory_order_relaxed);
-    if (n != 0) return n > 0 ? n : 0;
-    cudaLaunchConfig_t cfg{};
-    cfg.gridDim = dim3(64, 1, z);
-    cfg.blockDim = dim3(kDqThreads);
-    cfg.dynamicSmemBytes = kDqSmemBudget;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeClusterDimension;
-    attr[0].val.clusterDim.x = 1;
-    attr[0].val.clusterDim.y = 1;
-    attr[0].val.clusterDim.z = z;
-    cfg.attrs = attr;
-    cfg.numAttrs = 1;
-    n = 0;
-    if (cudaFuncSetAttribute(vq_dequant_gemm_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kDqSmemBudget) != cudaSuccess ||
-        cudaOccupancyMaxActiveClusters(&n, vq_dequant_gemm_kernel, &cfg) != cudaSuccess) {
-        cudaGetLastError();
-        n = 0;
-    }
-    cache[dev][z].store(n > 0 ? n : -1, std::memory_order_relaxed);
-    return n;
-}
-
 // Splits along K for `ctas` (row tile, batch tile) pairs and KT tiles of 64 columns: fill the SMs, at most
-// zmax splits (one thread-block cluster), at least eight tiles per split, an even number of tiles per split, all clusters resident at
-// once.  us, 6912 to 2560 (20 tiles) at batch 32 and 256 by splits: 4 18.1 / 24.3, 5 15.7 / 21.8, 6 14.1 / 20.4, 7 (two rounds) 25.3 / 36.7.
+// zmax splits (one thread-block cluster), at least eight tiles per split, an even number of tiles per split.  The splits are the
+// boundaries between a result's fp32 sums: they follow from the layer and the batch alone, so that a layer gives the same bits on
+// its own and inside a block.
 static void plan_ksplit(int ctas, int KT, int sms, int zmax, int* ksplit, int* per) {
     int z = sms / (ctas > 0 ? ctas : 1);
     z = z < 1 ? 1 : z > zmax ? zmax : z;
-    while (z > 1 && (KT / z < 8 || dq_resident_clusters(z) < ctas)) --z;
+    while (z > 1 && KT / z < 8) --z;
     int p = (KT + z - 1) / z;
     p += p & 1;
     *per = z > 1 ? p : KT;
@@ -999,7 +980,15 @@ static int dq_problem(DequantGemmProblem* out, const LinearProblem& L, cudaStrea
     return OJX_OK;
 }
 
-// One launch of the 128-row kernel for a layer, or for two of one width and batch on the same activations.
+// Splits of a layer in the 128-row kernel.
+static void plan_dq128(const LinearProblem& L, int* z, int* per) {
+    const int tiles = (L.row_stop - L.row_start + kDqBlockM - 1) / kDqBlockM, KT = L.K / kDqBlockK;
+    *z = 1;
+    *per = KT;
+    if (!getenv("OJASX_B200_TENSOR_NO_KSPLIT")) plan_ksplit(tiles * ((L.batch + 255) / 256), KT, num_sms(), 4, z, per);
+}
+
+// One launch of the 128-row kernel for a layer, or for two of one shape and batch on the same activations.
 static int launch_dq128(DequantGemmProblem* P, const LinearProblem* L, int count, cudaStream_t stream) {
     bool glists = true;   // outliers of both, where there are any, are listed already
     for (int i = 0; i < count; ++i) glists = glists && (P[i].tile_off != nullptr || L[i].csr.nnz == 0);
@@ -1033,7 +1022,12 @@ static int launch_dq128(DequantGemmProblem* P, const LinearProblem* L, int count
     dim3 grid(tiles[0] + tiles[1], (L[0].batch + 255) / 256, 1);
     const int KT = L[0].K / kDqBlockK;
     int z = 1, per = KT;
-    if (!getenv("OJASX_B200_TENSOR_NO_KSPLIT")) plan_ksplit((int)(grid.x * grid.y), KT, num_sms(), 8, &z, &per);
+    plan_dq128(L[0], &z, &per);
+    if (z == 2 && (int)(grid.x * grid.y) * z > num_sms()) {   // a pair: both sums of a tile in one CTA's tensor memory
+        z = 1;
+        for (int i = 0; i < count; ++i)
+            while (P[i].tmem_cols < 2 * n_pad) P[i].tmem_cols <<= 1;
+    }
     grid.z = z;
     // X tiles by the copy engine when the tensor map can be made (OJASX_B200_TENSOR_TMA=0 keeps the 16-byte copies)
     CUtensorMap xmap{};
@@ -1046,6 +1040,7 @@ static int launch_dq128(DequantGemmProblem* P, const LinearProblem* L, int count
         P[i].csr_cap = csr_cap;
         P[i].ksplit = z;
         P[i].tiles_per_split = z > 1 ? per : KT;
+        P[i].tiles_per_sum = per;
         P[i].use_tma = tma ? 1 : 0;
         pair.P[i] = P[i];
     }
@@ -1069,12 +1064,17 @@ static int launch_dq128(DequantGemmProblem* P, const LinearProblem* L, int count
     return OJX_OK;
 }
 
-// Gate and up of a SwiGLU block in one launch, if their tiles do not need more than a round of the SMs: then nothing, or less, is
-// split along K.  us for both, 2560 to 6912, two launches and one: batch 32 30 / 21, 64 31 / 23, 128 34 / 25, 256 43 / 33.  The block:
-// 62 / 40, 72 / 44, 76 / 50, 94 / 64, with a call into the library for each layer before.
+// Gate and up of a SwiGLU block in one launch, with the splits that each has on its own (the sums of two splits in one CTA where the
+// tiles of both layers leave no SMs for them), if that is at most a round of the SMs.  With three or four splits a CTA would do
+// three or four times the work of one of the separate launches.  us per block of 2560 and 6912, three calls of a layer and one call
+// of the block: batch 32 61.8 / 48.9, 64 65.5 / 52.2, 128 76.1 / 58.5, 256 94.3 / 69.8; 3840 wide (four splits) 44.8 / 41.4, 70.0 / 57.4
+// at 32 and 256.
 bool dequant_gemm_pair_pays(const LinearProblem& A, const LinearProblem& B) {
-    const int tiles = (A.row_stop - A.row_start + kDqBlockM - 1) / kDqBlockM + (B.row_stop - B.row_start + kDqBlockM - 1) / kDqBlockM;
-    return A.K == B.K && A.batch == B.batch && A.x == B.x && tiles * ((A.batch + 255) / 256) <= num_sms();
+    const int rows = A.row_stop - A.row_start, tiles = 2 * ((rows + kDqBlockM - 1) / kDqBlockM) * ((A.batch + 255) / 256);
+    if (A.K != B.K || A.batch != B.batch || A.x != B.x || rows != B.row_stop - B.row_start || A.K / kDqBlockK > kDqMaxTiles) return false;
+    int z = 1, per = 0;
+    plan_dq128(A, &z, &per);
+    return tiles * (z > 2 ? z : 1) <= num_sms();
 }
 int launch_dequant_gemm_pair(const LinearProblem* L, cudaStream_t stream, DqLists* const* lists, const unsigned* generation) {
     DequantGemmProblem P[2]{};
