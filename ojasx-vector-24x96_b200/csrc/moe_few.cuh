@@ -91,8 +91,18 @@ struct FewBars {
 };
 static_assert((2 * kFewMaxBlocks + 2 * kFewSlots) * 8 <= kFewBars, "room for the barriers");
 
+// Warps that gather for nrb warps that add.  A wait for a phase of a barrier cannot tell "two phases behind" from "done", so a warp may
+// wait for a slot's phase only when it knows the phase before it to be over.  What a gathering warp knows is its own last wait: all
+// blocks up to kFewSlots before its last piece's are added (they are added in order).  Its next piece must therefore lie at most
+// kFewSlots blocks further, and a block has 2 * nrb pieces.
+__host__ __device__ constexpr int few_gatherers(int nrb) {
+    return kFewThreads / 32 - nrb < kFewSlots * 2 * nrb ? kFewThreads / 32 - nrb : kFewSlots * 2 * nrb;
+}
+
 // Sum of row threadIdx.x of the item, in the threads of the first ceil(rows / 32) warps; the other warps gather.  RING: the table comes
 // through the ring of `blocks` blocks, otherwise it lies there whole.  A piece of work is 8 groups of 32 rows.
+// Order of a gathering warp's waits: the slot first.  Block b - kFewSlots is then known to be added and its table to have landed, so
+// that a ring of at least kFewSlots blocks is at most one phase behind at the second wait.
 template <bool RING>
 __device__ __forceinline__ float few_sums(const FewBars& B, const unsigned char* tab, int blocks, const unsigned char* codes, int stride, float* val,
                                           int rows, int G) {
@@ -121,11 +131,11 @@ __device__ __forceinline__ float few_sums(const FewBars& B, const unsigned char*
         }
         return acc;
     }
-    const int ng = kFewThreads / 32 - nrb;
-    for (int u = warp - nrb; u < nblk * upb; u += ng) {
+    const int ng = few_gatherers(nrb);
+    for (int u = warp - nrb; u < nblk * upb && warp < nrb + ng; u += ng) {
         const int b = u / upb, r = u - b * upb, lr = (r >> 1) * 32 + lane, g = b * kFewBlock + (r & 1) * 8, at = RING ? b % blocks : b;
-        if (RING) bulk_copy_wait(B.full + at, (unsigned)(b / blocks) & 1u);
         if (b >= kFewSlots) bulk_copy_wait(B.vempty + b % kFewSlots, (unsigned)(b / kFewSlots - 1) & 1u);
+        if (RING) bulk_copy_wait(B.full + at, (unsigned)(b / blocks) & 1u);
         if (lr < rows && g < G)
             few_gather8(reinterpret_cast<const float*>(tab) + (size_t)(at * kFewBlock + (r & 1) * 8) * 256, codes + (size_t)lr * stride + g,
                         val + (size_t)(b % kFewSlots) * slot + lr * kFewValRow + (r & 1) * 8);
@@ -348,7 +358,7 @@ static MoeFewPlan moe_few_plan(int pairs, int sms, int outputs, int mats, int G,
         const long long val = kFewSlots * rows * kFewValRow * 4, codes = up16(rows * f.stride), x = up16(4LL * K), prod = 4 * kFewProd, res = up16(4 * rows);
         const long long rest = kFewBars + val + codes + x + prod + res, cap = (long long)sizeof(CoreSmem);
         const long long fit = rest < cap ? (cap - rest) / (kFewBlock * 1024) : 0;
-        const int most = whole_table ? nblk : (nblk < kFewMaxBlocks ? nblk : kFewMaxBlocks), least = whole_table ? nblk : (nblk < 4 ? nblk : 4);
+        const int most = whole_table ? nblk : (nblk < kFewMaxBlocks ? nblk : kFewMaxBlocks), least = whole_table ? nblk : (nblk < kFewSlots ? nblk : kFewSlots);   // (fewer than kFewSlots: see few_sums)
         if (fit < least) continue;
         f.blocks = fit < most ? (int)fit : most;
         f.tab = kFewBars;

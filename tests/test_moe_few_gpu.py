@@ -16,7 +16,12 @@ pytestmark = pytest.mark.gpu
     (1088, 320, 5, 4, 3, 0.01, 8),    # eight and a half blocks, 40 down groups
     (2560, 640, 12, 10, 1, 0.0038, 8),
     (2560, 640, 12, 10, 2, 0.01, 8),  # two waves of items
-    (2560, 640, 6, 2, 1, 0.3, 8),     # several passes of outlier products
+    (2560, 640, 3, 2, 1, 0.1, 8),     # one block of rows (18 rows), twenty table blocks; two passes of outlier products
+    (2560, 256, 6, 4, 1, 0.01, 8),    # one block of rows (14), twenty table blocks
+    (2560, 1280, 3, 1, 1, 0.01, 8),   # one block of rows in both passes (18), ten down blocks
+    (2560, 576, 6, 4, 1, 0.0, 8),     # one block of rows, full (32)
+    (1152, 256, 4, 3, 1, 0.01, 8),    # one block of rows, nine table blocks
+    (4096, 128, 4, 2, 2, 0.01, 8),    # one block of rows (8), 32 table blocks, a ring of twelve
     (2560, 640, 12, 8, 8, 0.01, 8),   # the values do not fit: row-per-lane
     (1024, 256, 6, 5, 1, 0.01, 4),
     (1024, 512, 6, 5, 2, 0.01, 16),
