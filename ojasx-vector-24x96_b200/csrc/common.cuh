@@ -141,4 +141,36 @@ void set_last_error(const char* what, cudaError_t e);
 void set_last_error_msg(const char* what);
 int num_sms();
 
+#ifdef __CUDACC__
+// Waits for a phase of an mbarrier (shared-space address) for at most about an eighth of a second: between the warps of a CTA a
+// phase takes microseconds, and a wait that has not ended by then never will.  False: it ran out.  gone: shared-space address
+// of a word that such a wait sets and that makes the others on it give up at once (0: none).
+constexpr long long kBarClocks = 1LL << 28;
+__device__ __forceinline__ bool bar_wait(unsigned bar, unsigned parity, unsigned gone = 0) {
+    long long begin = 0;
+    for (bool first = true;; first = false) {
+        unsigned done;
+        asm volatile(
+            "{\n\t.reg .pred p;\n\t"
+            "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+            "selp.u32 %0, 1, 0, p;\n\t}"
+            : "=r"(done)
+            : "r"(bar), "r"(parity)
+            : "memory");
+        if (done) return true;
+        if (gone != 0) {
+            int set;
+            asm volatile("ld.volatile.shared.s32 %0, [%1];" : "=r"(set) : "r"(gone) : "memory");
+            if (set) return false;
+        }
+        const long long now = clock64();
+        if (first) begin = now;
+        else if (now - begin > kBarClocks) {
+            if (gone != 0) asm volatile("st.volatile.shared.s32 [%0], %1;" ::"r"(gone), "r"(1) : "memory");
+            return false;
+        }
+    }
+}
+#endif
+
 }  // namespace ojx

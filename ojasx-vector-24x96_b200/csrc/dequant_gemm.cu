@@ -43,7 +43,6 @@ constexpr int kDqThreads = kDqProducers + 32;   // + 1 MMA warp
 constexpr int kDqBlockM = 128;
 constexpr int kDqBlockK = 64;        // bf16 elements per K tile = one 128-byte swizzle row
 constexpr int kDqStages = 8;        // most stage buffers; as many as fit next to the batch tile are used (3 at N = 256)
-constexpr int kDqSpin = 1 << 22;     // bounded mbarrier polling
 
 
 
@@ -60,21 +59,8 @@ __device__ __forceinline__ void mbar_init(unsigned bar, unsigned count) {
 __device__ __forceinline__ void mbar_arrive(unsigned bar) {
     asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
 }
-// Returns false if the phase did not complete within the polling budget.
-__device__ __forceinline__ bool mbar_wait(unsigned bar, unsigned parity) {
-    for (int i = 0; i < kDqSpin; ++i) {
-        unsigned done;
-        asm volatile(
-            "{\n\t.reg .pred p;\n\t"
-            "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-            "selp.u32 %0, 1, 0, p;\n\t}"
-            : "=r"(done)
-            : "r"(bar), "r"(parity)
-            : "memory");
-        if (done) return true;
-    }
-    return false;
-}
+// Returns false if the phase did not complete in time.
+__device__ __forceinline__ bool mbar_wait(unsigned bar, unsigned parity) { return bar_wait(bar, parity); }
 
 __device__ __forceinline__ void dq_cluster_sync() {
     asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");

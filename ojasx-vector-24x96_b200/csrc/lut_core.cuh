@@ -77,9 +77,8 @@ constexpr int slice_groups() { return (kXsFloats / D) < kSliceGroups ? (kXsFloat
 // ---- bulk copy of a contiguous run of global memory into shared memory by the copy engine (TMA), tracked by an
 // mbarrier.  Used where a whole table slice is brought in at once: per-thread 16-byte copies keep too few bytes
 // in flight per SM for that (about 18 bytes per clock measured), the copy engine does not have that limit.
-// Every wait is bounded; a wait that runs out raises g_bulk_copy_timeout and carries on.
+// Every wait is bounded; a wait that runs out raises g_bulk_copy_timeout, and what the launch then stores is not valid.
 static __device__ int g_bulk_copy_timeout;   // one per translation unit; moe.cu is the one that copies tables this way
-constexpr int kBulkSpin = 1 << 22;
 __device__ __forceinline__ void bulk_bar_init(void* bar) {
     const unsigned a = static_cast<unsigned>(__cvta_generic_to_shared(bar));
     asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(a) : "memory");
@@ -115,18 +114,7 @@ __device__ __forceinline__ void bulk_copy_add(void* bar, void* dst, const void* 
                  : "memory");
 }
 __device__ __forceinline__ bool bulk_copy_wait(void* bar, unsigned parity) {
-    const unsigned b = static_cast<unsigned>(__cvta_generic_to_shared(bar));
-    for (int i = 0; i < kBulkSpin; ++i) {
-        unsigned done;
-        asm volatile(
-            "{\n\t.reg .pred p;\n\t"
-            "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-            "selp.u32 %0, 1, 0, p;\n\t}"
-            : "=r"(done)
-            : "r"(b), "r"(parity)
-            : "memory");
-        if (done) return true;
-    }
+    if (bar_wait(static_cast<unsigned>(__cvta_generic_to_shared(bar)), parity)) return true;
     atomicExch(&g_bulk_copy_timeout, 1);
     return false;
 }

@@ -20,7 +20,7 @@
 // multiplication, and ptxas cannot merge it with the addition that follows, as it does with a packed multiplication.
 //
 // Shared memory, by absolute shared-space address (the dynamic area must start at 1024; checked at run time):
-//     1024  mbarriers and control words; 1120 a sum of zero; 1152 a place for the sums of rows that do not exist
+//     1024  mbarriers and control words; 1104 set when a wait ran out; 1120 a sum of zero; 1152 a place for the sums of rows that do not exist
 //     1664  activations of a slice, [2][8 units x 272 bytes]: element e of a unit at e*16, its four vectors side by side
 //     6144  codebook f32[256][8], every number twice
 //    22528  parked sums float4[2688]
@@ -35,7 +35,7 @@ namespace ojx {
 
 constexpr int kQuWalkers = 8, kQuBuilders = 4, kQuSets = 1, kQuChunks = 8, kQuThreads = 32 * (kQuWalkers + kQuBuilders), kQuVecs = 4;
 constexpr int kQuSlice = 16;                                   // groups
-constexpr uint32_t kQuCtl = 1024, kQuZero = 1120, kQuDump = 1152, kQuXs = 1664, kQuBook = 6144, kQuAcc = 22528, kQuTab = 65536, kQuRing = 196608;
+constexpr uint32_t kQuCtl = 1024, kQuGone = 1104, kQuZero = 1120, kQuDump = 1152, kQuXs = 1664, kQuBook = 6144, kQuAcc = 22528, kQuTab = 65536, kQuRing = 196608;
 constexpr uint32_t kQuXsBytes = 2176, kQuTabBytes = 65536, kQuRingBytes = kQuChunks * 512;
 constexpr int kQuRows = (int)(kQuTab - kQuAcc) / 16;           // rows of a work item
 constexpr size_t kQuSmemBytes = kQuRing + kQuWalkers * kQuRingBytes - kQuCtl;
@@ -43,7 +43,6 @@ constexpr int kQuMaxK = (int)(2 * kQuTabBytes / 16);           // activations st
 static_assert(kQuSmemBytes <= 227 * 1024 && kQuRows == 2688, "shared memory of one SM");
 
 static __device__ int g_quad_error;   // 1: shared memory does not start at 1024, 2: a bounded wait ran out
-constexpr int kQuSpin = 1 << 22;
 
 // A work item: rows [0, n0) at base0, [n0, n) at base1, four vectors (an unused one repeats the first).
 struct QuadItem {
@@ -97,18 +96,7 @@ __device__ __forceinline__ uint32_t qu_full(int slice) { return kQuCtl + (slice 
 __device__ __forceinline__ uint32_t qu_empty(int slice) { return kQuCtl + 16 + (slice & 1) * 8; }
 __device__ __forceinline__ void qu_arrive(uint32_t bar) { asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory"); }
 __device__ __forceinline__ void qu_wait(uint32_t bar, unsigned parity) {
-    for (int i = 0; i < kQuSpin; ++i) {
-        unsigned done;
-        asm volatile(
-            "{\n\t.reg .pred p;\n\t"
-            "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-            "selp.u32 %0, 1, 0, p;\n\t}"
-            : "=r"(done)
-            : "r"(bar), "r"(parity)
-            : "memory");
-        if (done) return;
-    }
-    atomicExch(&g_quad_error, 2);
+    if (!bar_wait(bar, parity, kQuGone)) atomicExch(&g_quad_error, 2);
 }
 
 template <class T>
@@ -124,6 +112,7 @@ __device__ __forceinline__ bool quad_begin(unsigned char* raw, const float* __re
         asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(kQuCtl + threadIdx.x * 8), "r"(threadIdx.x < 2 ? kQuBuilders : kQuWalkers) : "memory");
     }
     if (threadIdx.x < 4) *qu_at<float>(raw, kQuZero + threadIdx.x * 4) = 0.0f;
+    if (threadIdx.x == 0) *qu_at<int>(raw, kQuGone) = 0;
     float2* book = qu_at<float2>(raw, kQuBook);
     for (int i = threadIdx.x; i < 256 * 8; i += kQuThreads) {
         const float c = i < Kcb * 8 ? codebook[i] : 0.0f;
@@ -336,6 +325,10 @@ __device__ __forceinline__ void quad_run(unsigned char* raw, const QuadItem& it,
     else quad_walk<false>(it, first);
     first += (it.G + kQuSlice - 1) / kQuSlice;
     __syncthreads();
+    if (*qu_at<volatile int>(raw, kQuGone)) {   // a wait ran out: no sum of this item is what it should be
+        for (int i = threadIdx.x; i < it.n; i += kQuThreads) qu_at<float4>(raw, kQuAcc)[i] = make_float4(NAN, NAN, NAN, NAN);
+        __syncthreads();
+    }
 }
 
 // The four vectors side by side in the (idle) table area: xs[k] for the outliers of the rows.  Ends with a barrier.

@@ -21,7 +21,7 @@ constexpr int kFewBlock = 16;                       // groups in a block of tabl
 constexpr int kFewValRow = kFewBlock + 4;           // floats a row of values takes: 128-bit accesses of eight rows do not share banks
 constexpr int kFewMaxBlocks = 12;
 constexpr int kFewSlots = 4;                        // slots of values
-constexpr int kFewBars = 256;                       // bytes of barriers
+constexpr int kFewBars = 272;                       // bytes of barriers and of the word that a wait sets when it runs out
 
 // Map of the dynamic shared memory (byte offsets).
 struct MoeFewPlan {
@@ -74,8 +74,10 @@ __device__ __forceinline__ void few_gather8(const float* tab, const unsigned cha
 // values is written; vempty[i]: it has been added.
 struct FewBars {
     unsigned long long *full, *empty, *vfull, *vempty;
+    int* gone;
     __device__ __forceinline__ explicit FewBars(unsigned char* smem)
-        : full(reinterpret_cast<unsigned long long*>(smem)), empty(full + kFewMaxBlocks), vfull(empty + kFewMaxBlocks), vempty(vfull + kFewSlots) {}
+        : full(reinterpret_cast<unsigned long long*>(smem)), empty(full + kFewMaxBlocks), vfull(empty + kFewMaxBlocks), vempty(vfull + kFewSlots),
+          gone(reinterpret_cast<int*>(vempty + kFewSlots)) {}
     __device__ __forceinline__ void init(int blocks, int rows) const {   // one thread; a barrier follows
         const int nrb = (rows + 31) >> 5;
         for (int i = 0; i < blocks; ++i) {
@@ -86,10 +88,17 @@ struct FewBars {
             few_bar_init(vfull + i, 2 * nrb);
             few_bar_init(vempty + i, nrb);
         }
+        *gone = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
+    // A wait inside the hand-over.  One that runs out makes all later ones of the CTA give up at once, and the item's sums NaN.
+    __device__ __forceinline__ void wait(unsigned long long* bar, unsigned parity) const {
+        if (!bar_wait(static_cast<unsigned>(__cvta_generic_to_shared(bar)), parity, static_cast<unsigned>(__cvta_generic_to_shared(gone))))
+            atomicExch(&g_bulk_copy_timeout, 1);
+    }
+    __device__ __forceinline__ bool failed() const { return *const_cast<volatile int*>(gone) != 0; }
 };
-static_assert((2 * kFewMaxBlocks + 2 * kFewSlots) * 8 <= kFewBars, "room for the barriers");
+static_assert((2 * kFewMaxBlocks + 2 * kFewSlots) * 8 + 4 <= kFewBars && kFewBars % 16 == 0, "room for the barriers");
 
 // Warps that gather for nrb warps that add.  A wait for a phase of a barrier cannot tell "two phases behind" from "done", so a warp may
 // wait for a slot's phase only when it knows the phase before it to be over.  What a gathering warp knows is its own last wait: all
@@ -112,7 +121,7 @@ __device__ __forceinline__ float few_sums(const FewBars& B, const unsigned char*
     if (warp < nrb) {
         const int lr = threadIdx.x;
         for (int b = 0; b < nblk; ++b) {
-            bulk_copy_wait(B.vfull + b % kFewSlots, (unsigned)(b / kFewSlots) & 1u);
+            B.wait(B.vfull + b % kFewSlots, (unsigned)(b / kFewSlots) & 1u);
             if (lr < rows) {
                 const float4* v = reinterpret_cast<const float4*>(val + (size_t)(b % kFewSlots) * slot + lr * kFewValRow);
                 const float4 v0 = v[0], v1 = v[1];
@@ -134,8 +143,8 @@ __device__ __forceinline__ float few_sums(const FewBars& B, const unsigned char*
     const int ng = few_gatherers(nrb);
     for (int u = warp - nrb; u < nblk * upb && warp < nrb + ng; u += ng) {
         const int b = u / upb, r = u - b * upb, lr = (r >> 1) * 32 + lane, g = b * kFewBlock + (r & 1) * 8, at = RING ? b % blocks : b;
-        if (b >= kFewSlots) bulk_copy_wait(B.vempty + b % kFewSlots, (unsigned)(b / kFewSlots - 1) & 1u);
-        if (RING) bulk_copy_wait(B.full + at, (unsigned)(b / blocks) & 1u);
+        if (b >= kFewSlots) B.wait(B.vempty + b % kFewSlots, (unsigned)(b / kFewSlots - 1) & 1u);
+        if (RING) B.wait(B.full + at, (unsigned)(b / blocks) & 1u);
         if (lr < rows && g < G)
             few_gather8(reinterpret_cast<const float*>(tab) + (size_t)(at * kFewBlock + (r & 1) * 8) * 256, codes + (size_t)lr * stride + g,
                         val + (size_t)(b % kFewSlots) * slot + lr * kFewValRow + (r & 1) * 8);
@@ -221,12 +230,13 @@ __global__ void __launch_bounds__(kFewThreads + 32, 1) moe_gate_up_few_kernel(co
         if (early) chain_begin();
         const bool mine = decode_pair(P, pair).expert >= 0;
         if (lane == 0) {
-            if (!mine)
-                for (int b = 0; b < first; ++b) bulk_copy_wait(B.full + b, 0);   // nothing may land after the CTA has left
-            for (int b = first; mine && b < nblk; ++b) {
-                bulk_copy_wait(B.empty + b % F.blocks, (unsigned)(b / F.blocks - 1) & 1u);
+            int b = first;
+            for (; mine && b < nblk; ++b) {
+                B.wait(B.empty + b % F.blocks, (unsigned)(b / F.blocks - 1) & 1u);
+                if (B.failed()) break;
                 bring(b);
             }
+            for (int c = b - first; c < b; ++c) bulk_copy_wait(B.full + c % F.blocks, (unsigned)(c / F.blocks) & 1u);   // nothing may land after the CTA has left
         }
         return;
     }
@@ -264,7 +274,7 @@ __global__ void __launch_bounds__(kFewThreads + 32, 1) moe_gate_up_few_kernel(co
             gate = fminf(gate, P.gate_limit);
             up = fminf(fmaxf(up, -P.gate_limit), P.gate_limit);
         }
-        P.inter[(size_t)pair * P.I + i0 + threadIdx.x] = __fmul_rn(silu_ref(gate), up);
+        P.inter[(size_t)pair * P.I + i0 + threadIdx.x] = B.failed() ? NAN : __fmul_rn(silu_ref(gate), up);
     }
 }
 
@@ -333,7 +343,8 @@ __global__ void __launch_bounds__(kFewThreads, 1) moe_down_few_kernel(const __gr
         if (P.dn_scales) sum = __fmul_rn(sum, scale);
         if (has)
             sum = __fadd_rn(sum, c.sum(P.dn_csr, xs, reinterpret_cast<float*>(smem_raw + F.prod), mine, c.number(p0, 0, R), c.number(p1, 0, R)));
-        if (mine) peer_store(link, P.expert_out + (size_t)pair * P.H + h0 + threadIdx.x, sum);
+        else few_sync();
+        if (mine) peer_store(link, P.expert_out + (size_t)pair * P.H + h0 + threadIdx.x, B.failed() ? NAN : sum);
     } else {
         chain_begin();
     }
