@@ -24,7 +24,6 @@
 // bf16), so it is used only for bf16 I/O, inside the rel 2e-2 tolerance of the bf16 activation path.
 // Every wait on an mbarrier is bounded; on a timeout the kernel raises a flag that the host reads.
 #include <algorithm>
-#include <atomic>
 #include <cstdlib>
 
 #include <cuda.h>   // CUtensorMap and the types of cuTensorMapEncodeTiled (the entry point is looked up at run time)
@@ -995,14 +994,8 @@ static int launch_dq128(DequantGemmProblem* P, const LinearProblem* L, int count
         csr_cap = (int)(left / 8 < 8192 ? left / 8 : 8192);
     }
     const size_t smem = dequant_gemm_smem(n_pad, stages, csr_cap, copies);
-    // the opt-in is a per-device attribute of the kernel: remember what each device was given
-    static thread_local size_t configured[64] = {};
-    int cur_dev = 0;
-    OJX_CUDA_TRY(cudaGetDevice(&cur_dev));
-    if (cur_dev < 0 || cur_dev >= 64 || smem > configured[cur_dev]) {
-        OJX_CUDA_TRY(cudaFuncSetAttribute(vq_dequant_gemm_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-        if (cur_dev >= 0 && cur_dev < 64) configured[cur_dev] = smem;
-    }
+    static std::atomic<bool> opted[64];
+    OJX_CUDA_TRY(opt_in_smem(reinterpret_cast<const void*>(vq_dequant_gemm_kernel), kDqSmemBudget, opted));
     int tiles[2] = {0, 0};
     for (int i = 0; i < count; ++i) tiles[i] = (L[i].row_stop - L[i].row_start + kDqBlockM - 1) / kDqBlockM;
     dim3 grid(tiles[0] + tiles[1], (L[0].batch + 255) / 256, 1);
@@ -1101,13 +1094,8 @@ int launch_dequant_gemm(const LinearProblem& L, cudaStream_t stream, DqLists* li
                 P.use_tma = 1;
                 P.book_copies = dequant_gemm256_smem(P.n_pad, 8) <= kDqSmemBudget ? 8 : 4;
                 const size_t smem = dequant_gemm256_smem(P.n_pad, P.book_copies);
-                static thread_local size_t configured2[64] = {};
-                int dev = 0;
-                OJX_CUDA_TRY(cudaGetDevice(&dev));
-                if (dev < 0 || dev >= 64 || smem > configured2[dev]) {
-                    OJX_CUDA_TRY(cudaFuncSetAttribute(vq_dequant_gemm256_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-                    if (dev >= 0 && dev < 64) configured2[dev] = smem;
-                }
+                static std::atomic<bool> opted[64];
+                OJX_CUDA_TRY(opt_in_smem(reinterpret_cast<const void*>(vq_dequant_gemm256_kernel), kDqSmemBudget, opted));
                 grid.z = z;
                 cudaLaunchConfig_t cfg{};
                 cfg.gridDim = grid;

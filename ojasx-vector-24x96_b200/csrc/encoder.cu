@@ -73,7 +73,8 @@ static int launch_assign_t(const float* vectors, size_t n, const float* centroid
                            unsigned long long* counts, cudaStream_t s) {
     const size_t smem = sizeof(float) * ((size_t)(Kcb * D + 1) & ~(size_t)1) + (sums ? sizeof(double) * Kcb * D + sizeof(unsigned) * Kcb : 0);
     if (smem > 200 * 1024) return OJX_ERR_TOO_LARGE;
-    if (smem > 48 * 1024) OJX_CUDA_TRY(cudaFuncSetAttribute(vq_assign_kernel<D>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    static std::atomic<bool> opted[64];
+    OJX_CUDA_TRY(opt_in_smem(reinterpret_cast<const void*>(vq_assign_kernel<D>), 200 * 1024, opted));
     const size_t want = (n + kEncThreads - 1) / kEncThreads;
     const size_t cap = (size_t)num_sms() * 8;
     const int grid = (int)(want < cap ? want : cap);

@@ -852,18 +852,13 @@ int launch_kvq_append(const KvqProblem& P, cudaStream_t s) {
 
 template <int R, int D>
 static int launch_decode_t(const KvqProblem& P, cudaStream_t s, const PeerLink& link) {
-    const size_t smem = kvq_decode_smem(P, R);
-    if (smem + 64 > 227 * 1024) return OJX_ERR_TOO_LARGE;   // 64: the kernel's few static bytes
+    const size_t smem = kvq_decode_smem(P, R), most = 227 * 1024 - 64;   // 64: the kernel's few static bytes
+    if (smem > most) return OJX_ERR_TOO_LARGE;
     KvqProblem Q = P;
     Q.v_copies = kvq_decode_v_copies(P, R);
     Q.direct = kvq_direct_smem<R, D>(P.G, P.head_dim) <= smem && P.head_dim <= kvq_decode_threads(R, D) ? (R == 8 ? kDirectTokens / 2 : kDirectTokens) : 0;
-    static thread_local size_t configured[64] = {};  // largest opt-in made for this instantiation, per device
-    int cur_dev = 0;
-    OJX_CUDA_TRY(cudaGetDevice(&cur_dev));
-    if (cur_dev < 0 || cur_dev >= 64 || smem > configured[cur_dev]) {
-        OJX_CUDA_TRY(cudaFuncSetAttribute(kvq_decode_kernel<R, D>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-        if (cur_dev >= 0 && cur_dev < 64) configured[cur_dev] = smem;
-    }
+    static std::atomic<bool> opted[64];
+    OJX_CUDA_TRY(opt_in_smem(reinterpret_cast<const void*>(kvq_decode_kernel<R, D>), most, opted));
     OJX_CUDA_TRY(launch_chained(kvq_decode_kernel<R, D>, dim3(P.n_chunks, P.Hkv, P.n_pos > 0 ? P.n_pos * P.B : P.B), kvq_decode_threads(R, D), smem, s, Q, link));
     count_launch(1);
     return OJX_OK;
@@ -1003,8 +998,8 @@ int launch_legacy_attention(const float* q, int head_dim, int block_dim, int T, 
     const int G = head_dim / block_dim;
     if (G > 128) return OJX_ERR_UNSUPPORTED;
     const size_t smem = sizeof(float) * (size_t)G * 256;
-    if (smem > 48 * 1024)
-        OJX_CUDA_TRY(cudaFuncSetAttribute(legacy_attention_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    static std::atomic<bool> opted[64];
+    OJX_CUDA_TRY(opt_in_smem(reinterpret_cast<const void*>(legacy_attention_kernel), 128 * 1024, opted));
     legacy_attention_kernel<<<1, 256, smem, s>>>(q, head_dim, block_dim, T, k_codes, v_codes, k_scales, v_scales,
                                                  scale_factor, logits, out);
     OJX_CUDA_TRY(cudaGetLastError());

@@ -1,5 +1,7 @@
 // Host-side launch entry points shared by the C ABI translation unit.
 #pragma once
+#include <atomic>
+
 #include "common.cuh"
 
 namespace ojx {
@@ -30,6 +32,19 @@ __device__ __forceinline__ void chain_begin() {
     cudaTriggerProgrammaticLaunchCompletion();
 }
 #endif
+
+// A kernel's opt-in to `bytes` of dynamic shared memory, the most that any of its launches takes, once per device.  The attribute belongs
+// to the kernel, not to a thread or a launch: one that follows the size of a launch is lowered by another thread's.
+inline cudaError_t opt_in_smem(const void* kernel, size_t bytes, std::atomic<bool> (&done)[64]) {
+    int dev = 0;
+    const cudaError_t e = cudaGetDevice(&dev);
+    if (e != cudaSuccess) return e;
+    const bool known = dev >= 0 && dev < 64;
+    if (known && done[dev].load(std::memory_order_acquire)) return cudaSuccess;
+    const cudaError_t set = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+    if (set == cudaSuccess && known) done[dev].store(true, std::memory_order_release);
+    return set;
+}
 
 struct PeerLink;   // peer.cuh: exchange over peer memory fused into a kernel's epilogue (null / n == 0: none)
 const PeerLink* peer_link_of(void* peer_link_handle);

@@ -943,7 +943,8 @@ static int launch_moe_experts_t(const MoeProblem& P, cudaStream_t s, const PeerL
     int extra = 0;
     if (P.pair_list) {
         const size_t hs = sizeof(int) * 2 * (size_t)P.E;
-        if (hs > 48 * 1024) OJX_CUDA_TRY(cudaFuncSetAttribute(moe_plan_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)hs));
+        static std::atomic<bool> opted[64];
+        OJX_CUDA_TRY(opt_in_smem(reinterpret_cast<const void*>(moe_plan_kernel), 226 * 1024, opted));
         OJX_CUDA_TRY(launch_chained(moe_plan_kernel, 1, 1024, hs, s, P, const_cast<int*>(P.pair_list)));
         ++extra;
     }
@@ -1124,7 +1125,8 @@ int launch_moe_router(const float* Wr, const void* x, int io_dtype, int n_tokens
     }
     const size_t tsm = sizeof(float) * kTopkWarps * (size_t)E;
     if (tsm > 200 * 1024) return OJX_ERR_TOO_LARGE;
-    if (tsm > 48 * 1024) OJX_CUDA_TRY(cudaFuncSetAttribute(moe_router_topk_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tsm));
+    static std::atomic<bool> opted[64];
+    OJX_CUDA_TRY(opt_in_smem(reinterpret_cast<const void*>(moe_router_topk_kernel), 200 * 1024, opted));
     const int tgrid = (n_tokens + kTopkWarps - 1) / kTopkWarps;
     if (E <= 512) OJX_CUDA_TRY(launch_chained(moe_router_topk_reg_kernel<16>, n_tokens, kTopkWarps * 32, 0, s, logits, n_tokens, E, k, idx_out, w_out, probs, link));
     else OJX_CUDA_TRY(launch_chained(moe_router_topk_kernel, tgrid, kTopkWarps * 32, tsm, s, logits, n_tokens, E, k, idx_out, w_out, probs, link));

@@ -153,14 +153,8 @@ static int launch_rvq_lut(const uint8_t* packed, const float* codebooks, const f
     const int grid = tiles < cap ? tiles : cap;
     if (D % 4 != 0 || (reinterpret_cast<uintptr_t>(codebooks) & 15)) return OJX_ERR_UNSUPPORTED;
     auto go = [&](auto kern) -> int {
-        static thread_local size_t opted[16][3] = {};   // largest opt-in so far, per device and width
-        int dev = 0;
-        if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 16) dev = 0;
-        size_t& have = opted[dev][bits == 1 ? 0 : bits == 2 ? 1 : 2];
-        if (smem > 48 * 1024 && smem > have) {
-            OJX_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-            have = smem;
-        }
+        static std::atomic<bool> opted[3][64];   // per width
+        OJX_CUDA_TRY(opt_in_smem(reinterpret_cast<const void*>(kern), 200 * 1024, opted[bits == 1 ? 0 : bits == 2 ? 1 : 2]));
         kern<<<grid, kRvqLutThreads, smem, s>>>(packed, codebooks, row_scales, bias, x, batch, stages, D, rows, columns,
                                                 row_start, row_stop, out);
         OJX_CUDA_TRY(cudaGetLastError());
