@@ -208,7 +208,7 @@ int launch_linear(LinearProblem P, cudaStream_t stream, const PeerLink* link) {
         rc = try_launch_linear_cluster(P, stream, link);
         if (rc != OJX_ERR_UNSUPPORTED) return rc;
     }
-    if (P.tile_rows <= 0 && !force_persistent() && quad_linear_pays(P)) return launch_quad_linear(P, stream, L);
+    if (P.tile_rows <= 0 && !force_persistent() && chain_walk_enabled() && quad_linear_pays(P)) return launch_quad_linear(P, stream, L);
     if (P.tile_rows <= 0) P.tile_rows = plan_tile_rows(rows, P.batch);
     P.tiles = (rows + P.tile_rows - 1) / P.tile_rows;
     P.item_begin = 0;

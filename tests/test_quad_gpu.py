@@ -21,6 +21,8 @@ pytestmark = pytest.mark.gpu
     (2624, 3201, 4, "f32"),     # two row tiles
     (4096, 2560, 40, "f32"),
     (8256, 300, 4, "f32"),      # more activations than are staged: the kernels of one vector
+    (2112, 200, 604, "f32"),    # more groups of vectors than SMs: second work items behind 17 slices
+    (2048, 33, 1201, "f32"),    # third ones, 16 slices
     (1280, 700, 9, "bf16"),
 ])
 def test_linear_batches(cuda, oracle, monkeypatch, K, M, batch, dtype):
@@ -42,6 +44,17 @@ def test_linear_batches(cuda, oracle, monkeypatch, K, M, batch, dtype):
     if M > 64:   # a run of rows in the middle
         assert np.array_equal(layer(xt, 31, M - 7).float().cpu().numpy(), want[:, 31:M - 7])
     assert ojasx_b200.lib().ojasx_b200_take_device_error() == 0
+
+
+def test_row_walk_switch_keeps_its_walk(cuda, kernels_of, monkeypatch):
+    """OJASX_B200_LINEAR_WALK=rows names a walk of one vector, also for batches that four vectors at a time would be faster for."""
+    layer = ops.VQLinear.from_weights(synth.make_vq_linear(3, 1024, 2048, block_dim=8, outlier_frac=0.01))
+    x = torch.randn(200, 1024, generator=torch.Generator("cuda").manual_seed(3), device=cuda)
+    four, quad = layer(x), kernels_of(lambda: layer(x))
+    monkeypatch.setenv("OJASX_B200_LINEAR_WALK", "rows")
+    rows, walk = layer(x), kernels_of(lambda: layer(x))
+    assert "lut_linear_quad_kernel" in quad and "lut_linear_quad_kernel" not in walk and "lut_linear_kernel" in walk
+    assert torch.equal(four, rows)
 
 
 def test_linear_special_values(cuda, oracle, monkeypatch):
@@ -70,6 +83,8 @@ def test_linear_special_values(cuda, oracle, monkeypatch):
     (2560, 640, 16, 10, 24, 0.0),
     (2560, 640, 16, 10, 25, 0.0038),
     (3584, 512, 6, 2, 31, 0.01),    # more hidden rows than a tile holds
+    (2816, 64, 160, 2, 200, 0.01),  # more groups of pairs than SMs: whole rounds, of two tiles of hidden rows; 22 slices and one
+    (1152, 320, 320, 4, 200, 0.003),   # two whole rounds and a rest; nine slices and three
 ])
 @pytest.mark.parametrize("dtype", ["f32", "bf16"])
 def test_moe_batches(cuda, oracle, monkeypatch, H, I, E, k, B, frac, dtype):
