@@ -383,12 +383,13 @@ __global__ void __launch_bounds__(kPfThreads) kvq_prefill_kernel(const __grid_co
 // up to 1.5 times as much as position by position), so the products are packed fp32 FMAs here.  128 threads, thread = 8 rows x 4 tokens
 // of the scores and 8 rows x HD/16 dimensions of the outputs; keys and values of a tile are expanded one after the other into the same
 // place, so that two CTAs (105 KB each) share an SM.  Sums are formed in short runs: a score in runs of 32 dimensions, even and odd ones apart,
-// outputs in runs of 16 tokens, and of 512 tokens, which are added up in `out`.  Relative error against 64 bits (2-norm), position by
-// position through the query tables and here: 512 positions 1.02e-7 / 9.3e-8, 1000 behind 4000 tokens 1.08e-7 / 8.8e-8, 32 7.5e-8 /
-// 7.1e-8.
+// outputs in runs of 16 tokens, of a tile, and of 512 tokens, which are added up in `out`.  Relative error against 64 bits (2-norm), position
+// by position through the query tables and here: 64 positions 8.7e-8 / 7.6e-8, 512 1.04e-7 / 8.9e-8, 112 behind 400 1.13e-7 / 9.9e-8 (1.22e-7
+// with runs of 16 added to the running outputs; block_dim 4 1.15e-7 / 1.09e-7, eight query heads 1.03e-7 / 9.9e-8), 100 behind 4000
+// 1.04e-7 / 7.9e-8.
 // Bound: fp32 FMAs (8.2 k clocks per tile of 64 x 64 x 128 with packed pairs) and the latency of shared memory; two CTAs take 21 k for
-// two tiles.  us per chunk of 512 positions with its codes, 8 KV heads of 4 query heads, head_dim 128: 750 / 173; 1000 behind 4000
-// 16740 / 2340.  With the rounding errors of the running outputs kept beside them the score loop had no registers left for its loads
+// two tiles.  us per chunk of 512 positions with its codes, 8 KV heads of 4 query heads, head_dim 128: 768 / 191; behind 2000
+// 5375 / 707.  With the rounding errors of the running outputs kept beside them the score loop had no registers left for its loads
 // (14 k clocks a tile instead of 8); 256 threads of half the rows read shared memory twice as often (no faster).
 constexpr int kPf32Pad = 4, kPf32Dims = 32, kPf32Run = 16, kPf32Tiles = 8;
 __device__ __forceinline__ uint64_t pf_pack(float a, float b) {
@@ -612,7 +613,10 @@ __global__ void __launch_bounds__(kPfThreads, D == 16 && HD == 128 ? 1 : 2) kvq_
         if (t0 + kPfTok < t_all) keep(buf ^ 1);
         __syncthreads();
 #pragma unroll
-        for (int c = 0; c < NC; ++c)
+        for (int c = 0; c < NC; ++c) {
+            uint64_t tsum[8][2];                                 // the tile's sums: one addition a tile to the running outputs
+#pragma unroll
+            for (int i = 0; i < 8; ++i) tsum[i][0] = tsum[i][1] = 0ull;
 #pragma unroll 1
             for (int r0 = 0; r0 < kPfTok && t0 + r0 < t_all; r0 += kPf32Run) {
                 uint64_t a[8][2];
@@ -635,10 +639,18 @@ __global__ void __launch_bounds__(kPfThreads, D == 16 && HD == 128 ? 1 : 2) kvq_
                 for (int i = 0; i < 8; ++i)
 #pragma unroll
                     for (int e = 0; e < 2; ++e) {
-                        const float2 sum = pf_unpack(o[i][c][e]), f = pf_unpack(a[i][e]);
-                        o[i][c][e] = pf_pack(sum.x + f.x, sum.y + f.y);
+                        const float2 sum = pf_unpack(tsum[i][e]), f = pf_unpack(a[i][e]);
+                        tsum[i][e] = pf_pack(sum.x + f.x, sum.y + f.y);
                     }
             }
+#pragma unroll
+            for (int i = 0; i < 8; ++i)
+#pragma unroll
+                for (int e = 0; e < 2; ++e) {
+                    const float2 sum = pf_unpack(o[i][c][e]), f = pf_unpack(tsum[i][e]);
+                    o[i][c][e] = pf_pack(sum.x + f.x, sum.y + f.y);
+                }
+        }
         if (++tiles % kPf32Tiles == 0 && t0 + kPfTok < t_all) flush(false);
     }
     flush(true);

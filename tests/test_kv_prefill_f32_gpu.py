@@ -1,5 +1,5 @@
 """fp32 prompt chunks through the prefill kernel: against 64 bits at the edges of its tiles (64 query rows, 64 tokens, runs of 512),
-with special values, and the same routes for calls that it does not take."""
+no further off than position by position, with special values, and the same routes for calls that it does not take."""
 import numpy as np
 import pytest
 import torch
@@ -48,7 +48,11 @@ def test_against_64_bits(cuda, B, Hkv, R, hd, D, T0, S):
     books, cache, k, v, q = _cache(T0 + S, B, Hkv, R, hd, D, T0, S)
     got = cache.prefill(k, v, q)
     want = _exact(q, books, cache.read(0, T0 + S), T0)
-    assert (got.double() - want).norm() <= 2.5 * 2.0 ** -24 * want.norm()   # an output's rounding and those of its sums in short runs
+    many = float((got.double() - want).norm() / want.norm())
+    cache.crop(T0)
+    one = torch.stack([(cache.append(k[s], v[s]), cache.decode(q[s]))[1] for s in range(S)])
+    single = float((one.double() - want).norm() / want.norm())
+    assert many < max(1.15 * single, 1.2e-7), (many, single)       # 1.2e-7: two roundings of an output
 
 
 def test_special_values(cuda):
