@@ -121,7 +121,7 @@ LinearProblem LinearHandle::problem(const void* x, void* y, int batch, int io_dt
     P.codes = codes; P.codebook = codebook; P.scales = scales; P.bias = bias;
     P.csr = CsrView{row_ptrs, cols, vals, nnz};
     P.x = x; P.y = y; P.K = in; P.G = G; P.D = D; P.Kcb = Kcb;
-    P.row_start = row_start; P.row_stop = row_stop; P.batch = batch; P.io_dtype = io_dtype;
+    P.rows_all = out; P.row_start = row_start; P.row_stop = row_stop; P.batch = batch; P.io_dtype = io_dtype;
     return P;
 }
 
@@ -342,7 +342,7 @@ int ojasx_b200_linear_forward_raw(const uint8_t* d_codes, const float* d_codeboo
     P.x = d_x; P.y = d_y; P.K = columns;
     P.G = (columns + block_dim - 1) / block_dim;  // blocks_per_row of the packed layout (codec.py:108)
     P.D = block_dim; P.Kcb = codebook_size;
-    P.row_start = row_start; P.row_stop = row_stop; P.batch = batch_size; P.io_dtype = io_dtype;
+    P.rows_all = rows; P.row_start = row_start; P.row_stop = row_stop; P.batch = batch_size; P.io_dtype = io_dtype;
     return launch_linear(P, static_cast<cudaStream_t>(stream));
 }
 

@@ -43,6 +43,7 @@ struct LinearProblem {
     int G;                    // groups per row (code bytes per row)
     int D;                    // block_dim
     int Kcb;                  // codebook entries (<= 256)
+    int rows_all;             // rows of the whole matrix, whose outliers csr.nnz counts
     int row_start, row_stop;
     int batch;
     int io_dtype;             // OJX_F32 / OJX_BF16

@@ -178,10 +178,12 @@ static int quad_configure() {   // the kernels' opt-in to large shared memory, o
 }
 
 // Clocks of an item of n rows with `entries` outliers each.  A slice takes 5050 where its table is the bound, 6600 with 1280 rows and
-// 9200 with 2560; the rest are the first table, the staging of the activations, the outliers and the results.
+// 9200 with 2560; the rest are the first table, the staging of the activations, and the outliers and results, a thread for every
+// kQuThreads-th row.
 static double quad_item_clocks(int n, int G, double entries) {
     const double slices = (G + kQuSlice - 1) / kQuSlice;
-    return slices * std::max(5050.0, 3900.0 + 2.1 * ((n + 255) / 256 * 256)) + 10000.0 + n * (2.5 + 1.1 * entries);
+    return slices * std::max(5050.0, 3900.0 + 2.1 * ((n + 255) / 256 * 256)) + 10000.0 +
+           0.5 * (n + (n + kQuThreads - 1) / kQuThreads * kQuThreads) * (2.5 + 1.5 * entries);
 }
 
 static bool quad_codes_fit(const uint8_t* codes, int G) { return G > 0 && G % 8 == 0 && (reinterpret_cast<uintptr_t>(codes) & 7) == 0; }
@@ -190,10 +192,13 @@ static bool quad_linear_fits(const LinearProblem& P) {
     return P.D == 8 && P.Kcb <= 256 && quad_codes_fit(P.codes, P.G) && (P.csr.nnz <= 0 || P.K <= kQuMaxK);
 }
 
+// Outlier entries of a row, on average.
+static double linear_entries(const LinearProblem& P) { return P.csr.nnz > 0 ? (double)P.csr.nnz / P.rows_all : 0.0; }
+
 // Tile of a linear's rows that makes the last CTA finish first, and that CTA's clocks.
 static int quad_linear_tile(const LinearProblem& P, double* clocks) {
     const int rows = P.row_stop - P.row_start, quads = (P.batch + kQuVecs - 1) / kQuVecs, sms = num_sms();
-    const double entries = P.csr.nnz > 0 ? 0.0038 * P.K : 0.0;   // (the rows of the whole matrix are not known here)
+    const double entries = linear_entries(P);
     int best = 0;
     for (int cut = 1; cut <= 64; ++cut) {
         const int tile = quad_tile(rows, kQuRows, 32, cut), items = quads * ((rows + tile - 1) / tile);
@@ -204,11 +209,13 @@ static int quad_linear_tile(const LinearProblem& P, double* clocks) {
     return best;
 }
 
-// Whether a linear is faster with four vectors at a time.  The persistent kernel's items take the groups times (135 + 0.096 per row)
-// clocks, 2 per row where code rows are no multiples of 16 bytes (its walk then loads them byte by byte).  us, that kernel / this:
-//   2560 -> 4096, batch 64 55.6 / 65.8, 96 82 / 71, 512 318 / 203; 2560 -> 1024, 128 41 / 62, 512 152 / 80; 4096 -> 2560, 512 368 / 184
-//   1024 -> 16384, batch 8 21.7 / 28.9, 32 39.2 / 37.1, 64 109 / 47; 2560 -> 32768, 8 54 / 66, 32 237 / 101; 3136 -> 13106, 54 2794 / 135
-// Of 40 linears drawn over 512 to 6912 columns, 256 to 32768 rows and 3 to 512 vectors none was sent to the slower one by more than 3 %.
+// Whether a linear is faster with four vectors at a time.  The persistent kernel's items take the groups times (140 + 0.066 per row)
+// clocks, 2 per row where code rows are no multiples of 16 bytes (its walk then loads them byte by byte), and 1 + 0.66 per entry for
+// a row with outliers.  us, that kernel / this, at no, 0.38 % and 5 % outliers:
+//   2560 -> 4096, batch 64 47 / 58, 54 / 64, 162 / 122; 96 70 / 63, 83 / 69, 296 / 145; 256 138 / 90, 161 / 104, 587 / 314
+//   4096 -> 2560, 64 58 / 87, 66 / 93, 207 / 140; 96 81 / 89, 95 / 98, 372 / 189; 128 80 / 93, 94 / 102, 371 / 213
+//   1024 -> 16384, 16 20 / 27, 24 / 30, 53 / 56; 32 29 / 32, 38 / 35, 99 / 80; 64 82 / 40, 108 / 45, 307 / 125
+//   2560 -> 1024, 128 36 / 56, 40 / 60, 97 / 85; 256 69 / 59, 77 / 65, 190 / 123; 3136 -> 3106, 4 52 / 75, 54 / 80, 57 / 110; 8 98 / 75, 101 / 80, 108 / 110
 bool quad_linear_pays(const LinearProblem& P) {
     if (!quad_linear_fits(P)) return false;
     const char* e = std::getenv("OJASX_B200_QUAD_MIN_BATCH");   // vectors from which a linear comes here, instead of the estimate
@@ -217,7 +224,8 @@ bool quad_linear_pays(const LinearProblem& P) {
     const int rows = P.row_stop - P.row_start, sms = num_sms(), tile = plan_tile_rows(rows, P.batch), items = P.batch * ((rows + tile - 1) / tile);
     double four = 0.0;
     quad_linear_tile(P, &four);
-    return four < (double)((items + sms - 1) / sms) * P.G * (135.0 + (P.G % 16 ? 2.0 : 0.096) * tile);
+    const double row = P.csr.nnz > 0 ? 1.0 + 0.66 * linear_entries(P) : 0.0;
+    return four < (double)((items + sms - 1) / sms) * (P.G * (140.0 + (P.G % 16 ? 2.0 : 0.066) * tile) + row * tile);
 }
 
 int launch_quad_linear(LinearProblem P, cudaStream_t s, const PeerLink& link) {
@@ -239,10 +247,12 @@ static void quad_passes(const MoeProblem& P, QuadMoe (&pass)[2]) {
 }
 
 // Routed pairs are taken four of an expert at a time where that is estimated to be faster than the chain walk pair by pair, whose
-// gate/up and down rows take the groups times (135 + 0.096 per row) clocks each (0.5 where code rows are no multiples of 16 bytes and
-// every lane walks its own row) and whose tables 0.8 per group and token.  us per routed layer at hidden 2560 / inter 640, that / this:
-//   512 experts, top 10: 64 tokens 340 / 476, 128 618 / 626, 192 899 / 732, 256 1179 / 861, 512 2278 / 1523
-//   128 experts, top 8: 32 tokens 169 / 221, 48 227 / 211, 64 267 / 301, 128 478 / 438, 256 913 / 561; 64, top 4: 128 273 / 289, 256 496 / 299
+// gate/up and down rows take the groups times (113 + 0.08 per row) clocks each (0.5 where code rows are no multiples of 16 bytes and
+// every lane walks its own row), and 1 + 0.6 per entry for a row with outliers, whose last round is half a gate/up item longer, and
+// whose tables take 0.8 per group and token.  us per routed layer at hidden 2560 / inter 640, that / this, at no and at 0.38 % outliers:
+//   512 experts, top 10: 64 tokens 293 / 359, 342 / 398; 96 402 / 465, 469 / 510; 128 531 / 505, 622 / 559; 256 997 / 761, 1174 / 838
+//   128 experts, top 8: 32 tokens 143 / 144, 165 / 167; 48 196 / 162, 227 / 172; 64 235 / 225, 270 / 250; 256 773 / 492, 907 / 544
+//   64 experts, top 8, 2048 / 768: 32 117 / 127, 133 / 142; 48 160 / 128, 183 / 141; top 4, 1024 / 512: 64 68 / 72, 77 / 78; 96 94 / 73, 107 / 79
 bool moe_quad_wanted(const MoeProblem& P) {
     if (!P.plan || P.D != 8 || P.Kcb > 256 || P.E > 4096 || !quad_codes_fit(P.gu_codes, P.G) || !quad_codes_fit(P.dn_codes, P.Gi)) return false;
     if ((P.gu_csr.nnz > 0 && P.H > kQuMaxK) || (P.dn_csr.nnz > 0 && P.I > kQuMaxK)) return false;
@@ -271,8 +281,9 @@ bool moe_quad_wanted(const MoeProblem& P) {
         four += whole * ((A.rows + tile0 - 1) / tile0) * quad_item_clocks(unit[i] * tile0, Gs[i], entries[i]);
         if (rest) four += std::max(1.0, (double)rest * ((A.rows + tile1 - 1) / tile1) / sms) * quad_item_clocks(unit[i] * tile1, Gs[i], entries[i]);
     }
-    const double pair = P.G * (135.0 + (P.G % 16 ? 0.5 : 0.096) * 2 * P.I) + P.Gi * (135.0 + (P.Gi % 16 ? 0.5 : 0.096) * P.H);
-    return four < ((double)expect / sms + 0.5) * pair + 0.8 * P.n_tokens * P.G;
+    auto rows = [](double n, int G, double e) { return G * (113.0 + (G % 16 ? 0.5 : 0.08) * n) + (e > 0.0 ? n * (1.0 + 0.6 * e) : 0.0); };
+    const double up = rows(2.0 * P.I, P.G, entries[0]), pair = up + rows(P.H, P.Gi, entries[1]);
+    return four < 0.97 * ((double)expect / sms * pair + 0.5 * up + 0.8 * P.n_tokens * P.G);   // (the estimates are 3 % off)
 }
 
 int launch_moe_quad(const MoeProblem& P, cudaStream_t s, const PeerLink& link) {

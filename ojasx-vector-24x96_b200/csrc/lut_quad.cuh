@@ -13,7 +13,8 @@
 // A slice is 16 groups: 256 codes x 16 groups x 4 vectors = 64 KB, kept twice.  Warps 0..7 walk one slice (shared-memory
 // pipe) while warps 8..11 build the next (fp32 pipe), handing the buffers over through mbarriers with bounded waits.
 //
-// Bound: the shared-memory pipe (72 to 85 % busy).  A step of a warp (32 rows x 2 groups x 4 vectors) is two gathers of 4 wavefronts each, a
+// Bound: the shared-memory pipe (over whole launches 60 % busy in a linear of 2560 to 4096 at batch 512, 53 % in both passes of a MoE
+// layer; issue slots 50 to 57 %), the rest are the ends of the work items: first tables, outliers, results.  A step of a warp (32 rows x 2 groups x 4 vectors) is two gathers of 4 wavefronts each, a
 // 2-byte code read and shares of parking and code copies, about 10 wavefronts for 256 entries; the walk with one vector needs
 // 8.5 for 128, and fills and drains 31 steps per slice.  The build of a slice takes 16384 x 15 fp32 operations (1920 clocks),
 // as packed pairs half as many issue slots: a product is fma(a, b, -0) with the -0 from a kernel argument -- the same bits as a
