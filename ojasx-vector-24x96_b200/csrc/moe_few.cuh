@@ -8,7 +8,8 @@
 // in shared memory, and the row's thread in another warp adds them in order (g ascending, one accumulator: the same bits).  The
 // tables of gate/up arrive in blocks through a ring of their own.  Whatever does not depend on the launch before is asked for
 // before the wait: the first table blocks of gate/up (built two launches earlier); codes, scales and row pointers of down.
-// Hidden 2560, 640 wide, 512 experts, ten pairs, us from the end of the launch before: gate/up 16.2 -> @GU@, down 10.9 -> @DN@.
+// us per routed layer of 64 experts, row-per-lane kernels / these: 2560 / 640, one pair 35.7 / 31.1, 4 36.2 / 26.6, 10 40.8 / 32.7, 20
+// 68 / 49; 2560 / 256, 10 37.1 / 28.0; 1024 / 256, 4 26.7 / 21.2; 4096 / 1024, 4 45.8 / 35.2, 10 64 / 59; 512 experts, 10 41.4 / 33.5.
 #pragma once
 
 namespace ojx {
@@ -351,19 +352,24 @@ __global__ void __launch_bounds__(kFewThreads, 1) moe_down_few_kernel(const __gr
     peer_signal_when_last(link, gridDim.x);
 }
 
-// Items of `pairs` pairs with `outputs` rows of K inputs each (G blocks of codes; `mats` matrices side by side): one to four waves of
-// the SMs, or nothing (bytes = 0) when they do not fit.  @RULE@
+// Items of `pairs` pairs with `outputs` rows of K inputs each (G blocks of codes; `mats` matrices side by side): few rounds of
+// the SMs, or nothing (bytes = 0) when they do not fit or the row-per-lane kernels are faster.  Those walk any number of rows per CTA at
+// little more than the price of few, while every round here waits for table, codes and outliers anew; down, and gate/up of a short table,
+// pay up to the third round, a second round of gate/up over 128 groups only with fewer than 160 rows an item.  us, row-per-lane / the
+// rounds that this leaves out: 2560 / 640, 48 pairs 77.8 / 95.1, 64 83.9 / 113.5; 1024 / 640, 64 57.3 / 63.9; 4096 / 1024, 24 99 / 115;
+// 2048 / 384, 60 66.3 / 72.6.  Kept: 2560 / 640, 32 71.4 / 70.2; 2560 / 256, 64 65.4 / 59.7; 4096 / 512, 24 81 / 67.
 static MoeFewPlan moe_few_plan(int pairs, int sms, int outputs, int mats, int G, int K, bool whole_table) {
     MoeFewPlan f{};
     if (G < 8 || (G & 7) != 0) return f;
     const int nblk = (G + kFewBlock - 1) / kFewBlock;
-    for (int waves = 1; waves <= 4 && waves * G <= 4000; ++waves) {
+    const int most_waves = whole_table || G <= 64 ? 3 : 2;
+    for (int waves = 1; waves <= most_waves; ++waves) {
         const int want = sms * waves / pairs;
         if (want < 1) continue;
         f.tile = (outputs + want - 1) / want;
         f.tiles = (outputs + f.tile - 1) / f.tile;
         const long long rows = (long long)f.tile * mats;
-        if (rows > kFewMaxRows) continue;
+        if (rows > kFewMaxRows || (!whole_table && G > 128 && waves > 1 && rows > 160)) continue;
         f.stride = (G >> 3) & 1 ? G : G + 8;
         auto up16 = [](long long b) { return (b + 15) & ~15LL; };
         const long long val = kFewSlots * rows * kFewValRow * 4, codes = up16(rows * f.stride), x = up16(4LL * K), prod = 4 * kFewProd, res = up16(4 * rows);
