@@ -466,7 +466,7 @@ static int kvq_decode_impl(OjasxKvqHandle handle, const void* d_q, void* d_out, 
 
 // The prefill kernels walk a CTA's whole context for 64 query rows; few positions on a long context split the context instead: the
 // decode kernel with a position axis.  bf16: the former once its CTAs fill half the GPU or the context is short.  fp32: by estimates of
-// both in us, 12 and 9.7 per 64 tokens of context (11.2 with two CTAs on an SM) against 13 per wave of decode CTAs and thousand tokens, a
+// both in us, 12 and another 9.7 per 64 tokens of context (11.2 with two CTAs on an SM) against 13 per wave of decode CTAs and thousand tokens, a
 // CTA's tables counting as a thousand.  us per chunk, decode kernel / prefill kernel, 8 KV heads of 4 query heads, head_dim 128:
 //   16 positions behind 0, 500, 1000 tokens 42 / 43, 74 / 126, 88 / 195; 32: 54 / 43, 118 / 127, 171 / 209; 64: 87 / 46, 206 / 130,
 //   327 / 212; 256: 251 / 86, 742 / 169, 1234 / 250.  Under a static plan the context is not known: up to 1024 tokens of capacity it is taken to be short.

@@ -354,7 +354,8 @@ template <int R, int D>
 __global__ void __launch_bounds__(kvq_decode_threads(R, D), 1) kvq_decode_kernel(const __grid_constant__ KvqProblem P,
                                                                                  const __grid_constant__ PeerLink link) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    {   // the head's codebooks, which nothing in the stream writes, for a range of few tokens (see kvq_decode_direct)
+    // The head's codebooks for a range of few tokens (see kvq_decode_direct): nothing in the stream writes them.
+    auto bring_books = [&]() {
         float4* cb = reinterpret_cast<float4*>(smem_raw);
         const size_t at = (size_t)blockIdx.y * P.Kcb * D / 4;
         for (int i = threadIdx.x; i < 64 * D; i += kvq_decode_threads(R, D)) {
@@ -364,7 +365,11 @@ __global__ void __launch_bounds__(kvq_decode_threads(R, D), 1) kvq_decode_kernel
             cb[i] = k;
             cb[64 * D + i] = v;
         }
-    }
+    };
+    // Before the wait where the launch's ranges may all go that way; books of 16 KB each cost a CTA that then builds tables 2.5 us
+    // (4 sequences of 32768 tokens, head_dim 128: 74.0 without, 76.5 with them), smaller ones nothing that shows.
+    const bool early = P.direct && (D <= 8 || P.chunk <= P.direct);
+    if (early) bring_books();
     chain_begin();
     constexpr int kThreads = kvq_decode_threads(R, D), kHalf = kThreads / 2;   // score threads = value threads
     constexpr int kTpt = 2, kSub = kTpt * kHalf;                               // tokens per pass
@@ -404,6 +409,7 @@ __global__ void __launch_bounds__(kvq_decode_threads(R, D), 1) kvq_decode_kernel
     const uint8_t* kc = P.k_codes + (((size_t)b * P.Hkv + h) * P.max_seq) * G;
     const uint8_t* vc = P.v_codes + (((size_t)b * P.Hkv + h) * P.max_seq) * G;
     if (P.direct && t_end - t_begin <= P.direct) {
+        if (!early) bring_books();   // (a barrier follows before they are read)
         kvq_decode_direct<R, D>(P, smem_raw, z, h, kc + (size_t)t_begin * G, vc + (size_t)t_begin * G, t_end - t_begin, part);
         kvq_merge_if_last<R>(P, z, h, link);
         peer_signal_when_last(link, gridDim.x * gridDim.y * gridDim.z);
