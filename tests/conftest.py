@@ -34,18 +34,3 @@ def cuda():
         pytest.skip("no CUDA device")
     torch.cuda.set_device(0)
     return torch.device("cuda", 0)
-
-
-@pytest.fixture
-def kernels_of(cuda):
-    """kernels_of(call): names of the kernels that a call launches."""
-    import torch
-
-    def names(call):
-        torch.cuda.synchronize()
-        with torch.profiler.profile(activities=[torch.profiler.ProfilerActivity.CUDA]) as p:
-            call()
-            torch.cuda.synchronize()
-        return " ".join(e.name for e in p.events())
-
-    return names

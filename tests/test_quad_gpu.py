@@ -46,17 +46,6 @@ def test_linear_batches(cuda, oracle, monkeypatch, K, M, batch, dtype):
     assert ojasx_b200.lib().ojasx_b200_take_device_error() == 0
 
 
-def test_row_walk_switch_keeps_its_walk(cuda, kernels_of, monkeypatch):
-    """OJASX_B200_LINEAR_WALK=rows names a walk of one vector, also for batches that four vectors at a time would be faster for."""
-    layer = ops.VQLinear.from_weights(synth.make_vq_linear(3, 1024, 2048, block_dim=8, outlier_frac=0.01))
-    x = torch.randn(200, 1024, generator=torch.Generator("cuda").manual_seed(3), device=cuda)
-    four, quad = layer(x), kernels_of(lambda: layer(x))
-    monkeypatch.setenv("OJASX_B200_LINEAR_WALK", "rows")
-    rows, walk = layer(x), kernels_of(lambda: layer(x))
-    assert "lut_linear_quad_kernel" in quad and "lut_linear_quad_kernel" not in walk and "lut_linear_kernel" in walk
-    assert torch.equal(four, rows)
-
-
 def test_linear_special_values(cuda, oracle, monkeypatch):
     """Infinities, NaN and sums of exactly -0 travel as they do in the kernels of one vector; a short codebook; no outliers."""
     w = synth.make_vq_linear(5, 320, 300, block_dim=8, outlier_frac=0.0)
